@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "rmn_b200.h"
 
 namespace rmn {
@@ -167,6 +169,24 @@ inline bool coords_aligned(const void* p, int W) {
 }
 
 void count_launch();
+
+// Opts a kernel in to more than 48 KB of dynamic shared memory, once per device (one object per kernel
+// instantiation; safe when several host threads make the first call together).
+class SmemOptIn {
+public:
+  cudaError_t apply(const void* kernel, size_t bytes) {
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    auto set = [&] { err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+    if (dev >= 0 && dev < 64) std::call_once(once_[dev], set);
+    else set();
+    return err;
+  }
+
+private:
+  std::once_flag once_[64];
+};
 
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? RMN_OK : RMN_ERR_CUDA; }
 

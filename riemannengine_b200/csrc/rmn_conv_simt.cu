@@ -1,6 +1,8 @@
 // SIMT (CUDA-core) sparse convolution over a neighbour table, fp32
 // accumulation. This is the exact-arithmetic path: fp32 features (the 1e-4
-// parity bar) and any channel count the tensor-core kernels do not take.
+// parity bar) and any channel count the tensor-core kernels do not take. fp32
+// features whose channel counts are multiples of four run in rmn_conv_f32.cu;
+// the generic kernels here take the rest.
 //
 // All three passes are output-stationary, so there are no atomics and results
 // are bit-reproducible:
@@ -12,6 +14,14 @@
 #include <cuda_bf16.h>
 
 namespace rmn {
+
+// rmn_conv_f32.cu
+bool f32_fast_shape(int c_in, int c_out);
+int f32_conv(const float* src, const float* w, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, float* out,
+             const float* ep_scale, const float* ep_shift, int ep_relu, cudaStream_t stream);
+size_t f32_wgrad_workspace_bytes(uint32_t n_dst, int K, int c_in, int c_out);
+int f32_conv_backward_weight(const float* feats, const float* grad_out, uint32_t n_dst, const int32_t* nbr, int K, int c_in,
+                             int c_out, float* dw, float* workspace, cudaStream_t stream);
 
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
@@ -213,9 +223,13 @@ int simt_conv_forward(const void* feats, int c_in, const void* w, int K, int c_o
                       const int32_t* nbr, uint32_t n_dst, void* out, int dtype, const float* ep_scale,
                       const float* ep_shift, int ep_relu, cudaStream_t stream) {
   const long long ws_k = (long long)c_in * c_out;
-  if (dtype == RMN_F32)
+  if (dtype == RMN_F32) {
+    const int st = f32_conv((const float*)feats, (const float*)w, nbr, n_dst, K, c_in, c_out, (float*)out, ep_scale,
+                            ep_shift, ep_relu, stream);
+    if (st != RMN_ERR_UNSUPPORTED) return st;
     return launch_gather_gemm<float>(feats, w, nbr, n_dst, K, c_in, c_out, ws_k, c_out, 1, out, ep_scale, ep_shift,
                                      ep_relu, stream);
+  }
   return launch_gather_gemm<__nv_bfloat16>(feats, w, nbr, n_dst, K, c_in, c_out, ws_k, c_out, 1, out, ep_scale,
                                            ep_shift, ep_relu, stream);
 }
@@ -224,6 +238,7 @@ int simt_conv_backward_input(const void* grad_out, int c_out, const void* w, int
                              const int32_t* nbr_t, uint32_t n_src, void* grad_feats, int dtype,
                              cudaStream_t stream) {
   const long long ws_k = (long long)c_in * c_out;
+  // (fp32 hosts transpose the weights first and call the forward pass: rmn_conv_transpose_weights)
   if (dtype == RMN_F32)
     return launch_gather_gemm<float>(grad_out, w, nbr_t, n_src, K, c_out, c_in, ws_k, 1, c_out, grad_feats, nullptr,
                                      nullptr, 0, stream);
@@ -232,7 +247,9 @@ int simt_conv_backward_input(const void* grad_out, int c_out, const void* w, int
 }
 
 size_t simt_wgrad_workspace_bytes(uint32_t n_dst, int K, int c_in, int c_out) {
-  return (size_t)wgrad_chunks(n_dst) * K * c_in * c_out * sizeof(float);
+  const size_t generic = (size_t)wgrad_chunks(n_dst) * K * c_in * c_out * sizeof(float);
+  const size_t fast = f32_fast_shape(c_in, c_out) ? f32_wgrad_workspace_bytes(n_dst, K, c_in, c_out) : 0;
+  return fast > generic ? fast : generic;
 }
 
 template <typename T>
@@ -253,8 +270,12 @@ int launch_wgrad(const void* feats, const void* grad_out, const int32_t* nbr, ui
 int simt_conv_backward_weight(const void* feats, int c_in, const void* grad_out, uint32_t n_dst,
                               int c_out, const int32_t* nbr, int K, float* dw, int dtype,
                               void* workspace, cudaStream_t stream) {
-  if (dtype == RMN_F32)
+  if (dtype == RMN_F32) {
+    const int st = f32_conv_backward_weight((const float*)feats, (const float*)grad_out, n_dst, nbr, K, c_in, c_out, dw,
+                                            (float*)workspace, stream);
+    if (st != RMN_ERR_UNSUPPORTED) return st;
     return launch_wgrad<float>(feats, grad_out, nbr, n_dst, K, c_in, c_out, dw, (float*)workspace, stream);
+  }
   return launch_wgrad<__nv_bfloat16>(feats, grad_out, nbr, n_dst, K, c_in, c_out, dw, (float*)workspace, stream);
 }
 

@@ -292,6 +292,15 @@ def conv_backward_input(grad_out: torch.Tensor, weights: torch.Tensor, nbr_t: to
     n_src = int(nbr_t.size(1))
     out = torch.empty((n_src, c_in), dtype=grad_out.dtype, device=grad_out.device)
     with torch.cuda.device(grad_out.device):
+        if grad_out.dtype == torch.float32 and n_src and grad_out.size(0):
+            # fp32: the forward pass on transposed weights (rmn_conv_transpose_weights)
+            wt = torch.empty((K, c_out, c_in), dtype=weights.dtype, device=weights.device)
+            capi.check(capi.lib().rmn_conv_transpose_weights(_ptr(weights), K, c_in, c_out, capi.F32, 0, _ptr(wt),
+                                                             _stream()), "rmn_conv_transpose_weights")
+            capi.check(capi.lib().rmn_conv_forward_planned(_ptr(grad_out), int(grad_out.size(0)), c_out, _ptr(wt), K,
+                                                           c_in, _ptr(nbr_t), None, n_src, _ptr(out), capi.F32, None,
+                                                           None, 0, _stream()), "rmn_conv_forward_planned")
+            return out
         capi.check(capi.lib().rmn_conv_backward_input_planned(_ptr(grad_out), int(grad_out.size(0)), c_out,
                                                               _ptr(weights), K, c_in, _ptr(nbr_t), _ptr(plan), n_src,
                                                               _ptr(out), _dtype_code(grad_out), _stream()),

@@ -1014,10 +1014,21 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
   return out;
 }
 
+// reverse: nbr_t is the forward table of a point-symmetric self map, i.e. its offsets run backwards
 at::Tensor conv_backward_input(const at::Tensor& grad_in, const at::Tensor& kernel_in, const at::Tensor& nbr_t,
-                               const at::Tensor& plan_t = at::Tensor()) {
-  auto grad = grad_in.contiguous(), kernel = kernel_in.contiguous();
+                               bool reverse, const at::Tensor& plan_t = at::Tensor()) {
+  auto grad = grad_in.contiguous();
   c10::cuda::CUDAGuard guard(grad.device());
+  if (grad.scalar_type() == at::kFloat && grad.size(0) > 0 && nbr_t.size(1) > 0) {
+    // fp32: the forward pass on transposed weights
+    auto w = kernel_in.contiguous();
+    auto wt = at::empty({w.size(0), w.size(2), w.size(1)}, w.options());
+    check(rmn_conv_transpose_weights(ptr(w), static_cast<int>(w.size(0)), static_cast<int>(w.size(1)),
+                                     static_cast<int>(w.size(2)), RMN_F32, reverse ? 1 : 0, ptr(wt), current_stream()),
+          "rmn_conv_transpose_weights");
+    return conv_forward(grad, wt, nbr_t);
+  }
+  auto kernel = reverse ? kernel_in.flip(0) : kernel_in.contiguous();
   const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(kernel.size(1)),
             c_out = static_cast<int>(kernel.size(2));
   auto out = at::empty({nbr_t.size(1), c_in}, grad.options());
@@ -1115,7 +1126,7 @@ public:
       for (auto const& t : reduce) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), side_stream);
       if (ctx->needs_input_grad(0)) {
         auto plan_in = ctx->saved_data["plan_in"].toTensor();
-        g_feat = conv_backward_input(grad, ctx->saved_data["flip_kernel"].toBool() ? saved[1].flip(0) : saved[1], nbr_in,
+        g_feat = conv_backward_input(grad, saved[1], nbr_in, ctx->saved_data["flip_kernel"].toBool(),
                                      plan_in.numel() > 0 ? plan_in : at::Tensor());
       }
       c10::Event reduced(c10::DeviceType::CUDA);
@@ -1127,7 +1138,7 @@ public:
     }
     if (ctx->needs_input_grad(0)) {
       auto plan_in = ctx->saved_data["plan_in"].toTensor();
-      g_feat = conv_backward_input(grad, ctx->saved_data["flip_kernel"].toBool() ? saved[1].flip(0) : saved[1], nbr_in,
+      g_feat = conv_backward_input(grad, saved[1], nbr_in, ctx->saved_data["flip_kernel"].toBool(),
                                    plan_in.numel() > 0 ? plan_in : at::Tensor());
     }
     if (ctx->needs_input_grad(1)) g_kernel = conv_backward_weight(saved[0], grad, nbr_out).to(saved[1].scalar_type());
