@@ -379,6 +379,27 @@ int rmn_conv_backward_input(const void *d_grad_out, uint32_t n_dst, int c_out,
 int rmn_conv_transpose_weights(const void *d_weights, int K, int c_in, int c_out, int dtype, int reverse,
                                void *d_out, void *stream);
 
+/*
+ * Prepared weights for the fastest bf16 kernels. rmn_conv_weight_image_bytes: size of the image of [K, c_in, c_out]
+ * weights, 0 when no such kernel covers the dtype and channel counts (use the plain entry points then).
+ * rmn_conv_weight_image builds it (one small kernel); transpose != 0 makes the image of the transposed weights, for
+ * rmn_conv_forward_image to compute the input gradient from grad_out (c_in and c_out exchanged there); reverse != 0
+ * exchanges offsets k and K - 1 - k, for the input gradient of a point-symmetric self map over its own forward table.
+ * rmn_conv_forward_image: rmn_conv_forward_planned with an image in place of the weights (bf16; d_feats 32-byte
+ * aligned, d_image and d_out 16-byte aligned). rmn_conv_forward_image_stats: also the channel statistics of
+ * rmn_conv_forward_stats.
+ */
+size_t rmn_conv_weight_image_bytes(int K, int c_in, int c_out, int dtype);
+int rmn_conv_weight_image(const void *d_weights, int K, int c_in, int c_out, int dtype, int transpose, int reverse,
+                          void *d_image, void *stream);
+int rmn_conv_forward_image(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
+                           const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out, const float *d_scale,
+                           const float *d_shift, int relu, void *stream);
+int rmn_conv_forward_image_stats(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
+                                 const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out,
+                                 const float *d_scale, const float *d_shift, int relu, double *d_stats, void *d_workspace,
+                                 size_t workspace_bytes, void *stream);
+
 /* Scratch bytes of rmn_conv_backward_weight. */
 size_t rmn_conv_backward_weight_workspace_bytes(uint32_t n_dst, int K, int c_in, int c_out,
                                                 int dtype);

@@ -536,6 +536,7 @@ int launch(const void* src, const void* w, const int32_t* nbr, uint32_t n_dst, i
 
 #include "rmn_conv_tc_tma.cuh"
 #include "rmn_conv_tc_wgrad.cuh"
+#include "rmn_conv_ta.cuh"
 
 #include <cstdlib>
 

@@ -16,6 +16,10 @@ int tc_conv_stats(const void* src, uint32_t n_src, const void* w, const int32_t*
                   int c_col, void* out, const float* ep_scale, const float* ep_shift, int ep_relu,
                   float* stats_partial, uint32_t* n_partials, cudaStream_t stream, const void* plan);
 
+int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
+            const float* ep_scale, const float* ep_shift, int ep_relu, float* stats_partial, uint32_t* n_partials,
+            cudaStream_t stream, const void* plan);
+
 constexpr uint32_t kMaxStatPartials = 1024;
 
 __device__ __forceinline__ float ld_f32(const float* p) { return __ldg(p); }
@@ -176,6 +180,28 @@ extern "C" int rmn_conv_forward_stats_planned(const void* d_feats, uint32_t n_sr
                                         d_shift, relu, stream_);
   if (st != RMN_OK) return st;
   return channel_stats(d_out, n_dst, c_out, dtype, d_stats, (float*)d_workspace, stream);
+}
+
+extern "C" int rmn_conv_forward_image_stats(const void* d_feats, uint32_t n_src, int c_in, const void* d_image, int K,
+                                            int c_out, const int32_t* d_nbr, const void* d_plan, uint32_t n_dst,
+                                            void* d_out, const float* d_scale, const float* d_shift, int relu,
+                                            double* d_stats, void* d_workspace, size_t workspace_bytes, void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  if (!d_stats || c_out < 1) return RMN_ERR_BAD_ARG;
+  if (n_dst == 0) {
+    RMN_CUDA_TRY(cudaMemsetAsync(d_stats, 0, 2 * (size_t)c_out * sizeof(double), stream));
+    return RMN_OK;
+  }
+  if (!d_image || !d_nbr || !d_out || !d_workspace || (n_src > 0 && !d_feats) || K < 1 || K > 65535) return RMN_ERR_BAD_ARG;
+  if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_image & 15) || ((uintptr_t)d_out & 15)) return RMN_ERR_BAD_ARG;
+  if (workspace_bytes < rmn_channel_stats_workspace_bytes(c_out)) return RMN_ERR_ALLOC;
+  uint32_t n_partials = 0;
+  const int st = ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, relu, (float*)d_workspace,
+                         &n_partials, stream, d_plan);
+  if (st != RMN_OK) return st;
+  k_stats_reduce<<<(2 * c_out + 127) / 128, 128, 0, stream>>>((const float*)d_workspace, n_partials, c_out, d_stats);
+  RMN_LAUNCH_CHECK();
+  return RMN_OK;
 }
 
 extern "C" int rmn_affine_act(const void* d_x, uint32_t n_rows, int channels, const float* d_scale,

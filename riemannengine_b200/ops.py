@@ -251,6 +251,20 @@ def conv_plan_build(nbr: torch.Tensor, offsets: np.ndarray) -> Optional[torch.Te
     return plan
 
 
+def _weight_image(weights: torch.Tensor, transpose: bool, feats: torch.Tensor,
+                  reverse: bool = False) -> Optional[torch.Tensor]:
+    """Prepared weights (rmn_conv_weight_image) for the tensor-memory kernels, or None when they do not cover the shape
+    or the features are not aligned for them. The current device is the tensors'."""
+    K, c_in, c_out = (int(s) for s in weights.shape)
+    nbytes = capi.lib().rmn_conv_weight_image_bytes(K, c_in, c_out, _dtype_code(weights))
+    if nbytes == 0 or feats.data_ptr() % 32:
+        return None
+    image = torch.empty(nbytes, dtype=torch.uint8, device=weights.device)
+    capi.check(capi.lib().rmn_conv_weight_image(_ptr(weights), K, c_in, c_out, _dtype_code(weights), int(transpose),
+                                                int(reverse), _ptr(image), _stream()), "rmn_conv_weight_image")
+    return image
+
+
 def conv_forward(feats: torch.Tensor, weights: torch.Tensor, nbr: torch.Tensor,
                  scale: Optional[torch.Tensor] = None, shift: Optional[torch.Tensor] = None,
                  relu: bool = False, plan: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -275,6 +289,12 @@ def conv_forward(feats: torch.Tensor, weights: torch.Tensor, nbr: torch.Tensor,
 
     sc, sh = vec(scale), vec(shift)
     with torch.cuda.device(feats.device):
+        image = _weight_image(weights, False, feats) if n_dst and feats.size(0) else None
+        if image is not None:
+            capi.check(capi.lib().rmn_conv_forward_image(_ptr(feats), int(feats.size(0)), c_in, _ptr(image), K, c_out,
+                                                         _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _ptr(sc), _ptr(sh),
+                                                         int(bool(relu)), _stream()), "rmn_conv_forward_image")
+            return out
         capi.check(capi.lib().rmn_conv_forward_planned(_ptr(feats), int(feats.size(0)), c_in, _ptr(weights), K, c_out,
                                                        _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _dtype_code(feats),
                                                        _ptr(sc), _ptr(sh), int(bool(relu)), _stream()),
@@ -300,6 +320,12 @@ def conv_backward_input(grad_out: torch.Tensor, weights: torch.Tensor, nbr_t: to
             capi.check(capi.lib().rmn_conv_forward_planned(_ptr(grad_out), int(grad_out.size(0)), c_out, _ptr(wt), K,
                                                            c_in, _ptr(nbr_t), None, n_src, _ptr(out), capi.F32, None,
                                                            None, 0, _stream()), "rmn_conv_forward_planned")
+            return out
+        image = _weight_image(weights, True, grad_out) if n_src and grad_out.size(0) else None
+        if image is not None:
+            capi.check(capi.lib().rmn_conv_forward_image(_ptr(grad_out), int(grad_out.size(0)), c_out, _ptr(image), K,
+                                                         c_in, _ptr(nbr_t), _ptr(plan), n_src, _ptr(out), None, None, 0,
+                                                         _stream()), "rmn_conv_forward_image")
             return out
         capi.check(capi.lib().rmn_conv_backward_input_planned(_ptr(grad_out), int(grad_out.size(0)), c_out,
                                                               _ptr(weights), K, c_in, _ptr(nbr_t), _ptr(plan), n_src,
@@ -409,6 +435,13 @@ def conv_forward_stats(feats: torch.Tensor, weights: torch.Tensor, nbr: torch.Te
     wbytes = lib.rmn_channel_stats_workspace_bytes(c_out)
     ws = torch.empty(wbytes, dtype=torch.uint8, device=feats.device)
     with torch.cuda.device(feats.device):
+        image = _weight_image(weights, False, feats) if n_dst and feats.size(0) else None
+        if image is not None:
+            capi.check(lib.rmn_conv_forward_image_stats(_ptr(feats), int(feats.size(0)), c_in, _ptr(image), K, c_out,
+                                                        _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _ptr(sc), _ptr(sh),
+                                                        int(bool(relu)), _ptr(stats), _ptr(ws), wbytes, _stream()),
+                       "rmn_conv_forward_image_stats")
+            return out, stats
         capi.check(lib.rmn_conv_forward_stats_planned(_ptr(feats), int(feats.size(0)), c_in, _ptr(weights), K, c_out,
                                                       _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _dtype_code(feats),
                                                       _ptr(sc), _ptr(sh), int(bool(relu)), _ptr(stats), _ptr(ws),

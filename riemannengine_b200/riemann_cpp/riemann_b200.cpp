@@ -984,6 +984,22 @@ void allreduce_gradients(const std::vector<at::Tensor>& gradients) {
 // ---------------------------------------------------------------------------------------------
 namespace {
 
+// The prepared weights of rmn_conv_forward_image, of [K, c_in, c_out] weights or (transpose) of their transposes;
+// undefined where no such kernel covers the shape and type, or the operand is not aligned for it.
+at::Tensor weight_image(const at::Tensor& kernel, bool transpose, bool reverse, const at::Tensor& operand) {
+  if (kernel.scalar_type() != at::kBFloat16 || reinterpret_cast<uintptr_t>(operand.data_ptr()) % 32 != 0) return at::Tensor();
+  const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(kernel.size(1)),
+            c_out = static_cast<int>(kernel.size(2));
+  const size_t bytes = transpose ? rmn_conv_weight_image_bytes(K, c_out, c_in, RMN_BF16)
+                                 : rmn_conv_weight_image_bytes(K, c_in, c_out, RMN_BF16);
+  if (bytes == 0) return at::Tensor();
+  auto image = at::empty({static_cast<int64_t>(bytes)}, kernel.options().dtype(at::kByte));
+  check(rmn_conv_weight_image(ptr(kernel), K, c_in, c_out, RMN_BF16, transpose ? 1 : 0, reverse ? 1 : 0, ptr(image),
+                              current_stream()),
+        "rmn_conv_weight_image");
+  return image;
+}
+
 // bias (if defined) is folded into the kernel's epilogue as a per-channel shift
 at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in, const at::Tensor& nbr,
                         const at::Tensor& bias = at::Tensor(), const at::Tensor& scale_in = at::Tensor(),
@@ -1004,6 +1020,16 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
   if (scale_in.defined() && scale_in.numel() > 0) {
     scale = scale_in.detach().reshape({-1}).to(at::kFloat).contiguous();
     TORCH_CHECK(scale.numel() == c_out, "scale must have one entry per output channel");
+  }
+  if (feats.size(0) > 0 && nbr.size(1) > 0) {
+    if (auto image = weight_image(kernel, false, false, feats); image.defined()) {
+      check(rmn_conv_forward_image(ptr(feats), static_cast<uint32_t>(feats.size(0)), c_in, ptr(image), K, c_out,
+                                   static_cast<const int32_t*>(ptr(nbr)), ptr(plan), static_cast<uint32_t>(nbr.size(1)),
+                                   ptr(out), static_cast<const float*>(ptr(scale)), static_cast<const float*>(ptr(shift)),
+                                   relu ? 1 : 0, current_stream()),
+            "rmn_conv_forward_image");
+      return out;
+    }
   }
   check(rmn_conv_forward_planned(ptr(feats), static_cast<uint32_t>(feats.size(0)), c_in, ptr(kernel), K, c_out,
                                  static_cast<const int32_t*>(ptr(nbr)), ptr(plan), static_cast<uint32_t>(nbr.size(1)),
@@ -1028,10 +1054,19 @@ at::Tensor conv_backward_input(const at::Tensor& grad_in, const at::Tensor& kern
           "rmn_conv_transpose_weights");
     return conv_forward(grad, wt, nbr_t);
   }
-  auto kernel = reverse ? kernel_in.flip(0) : kernel_in.contiguous();
-  const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(kernel.size(1)),
-            c_out = static_cast<int>(kernel.size(2));
+  const int K = static_cast<int>(kernel_in.size(0)), c_in = static_cast<int>(kernel_in.size(1)),
+            c_out = static_cast<int>(kernel_in.size(2));
   auto out = at::empty({nbr_t.size(1), c_in}, grad.options());
+  if (grad.size(0) > 0 && nbr_t.size(1) > 0) {
+    if (auto image = weight_image(kernel_in.contiguous(), true, reverse, grad); image.defined()) {
+      check(rmn_conv_forward_image(ptr(grad), static_cast<uint32_t>(grad.size(0)), c_out, ptr(image), K, c_in,
+                                   static_cast<const int32_t*>(ptr(nbr_t)), ptr(plan_t),
+                                   static_cast<uint32_t>(nbr_t.size(1)), ptr(out), nullptr, nullptr, 0, current_stream()),
+            "rmn_conv_forward_image");
+      return out;
+    }
+  }
+  auto kernel = reverse ? kernel_in.flip(0) : kernel_in.contiguous();
   check(rmn_conv_backward_input_planned(ptr(grad), static_cast<uint32_t>(grad.size(0)), c_out, ptr(kernel), K, c_in,
                                         static_cast<const int32_t*>(ptr(nbr_t)), ptr(plan_t),
                                         static_cast<uint32_t>(nbr_t.size(1)), ptr(out), dtype_code(grad),
