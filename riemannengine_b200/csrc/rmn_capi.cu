@@ -16,7 +16,7 @@ int simt_conv_backward_weight(const void* feats, int c_in, const void* grad_out,
 int tc_conv(const void* src, uint32_t n_src, const void* w, const int32_t* nbr, uint32_t n_dst, int K, int c_red,
             int c_col, bool transposed_weights, void* out, const float* ep_scale, const float* ep_shift, int ep_relu,
             cudaStream_t stream, const void* plan);
-bool ta_shape(int c_red, int c_col);
+size_t ta_image_bytes(int K, int c_red, int c_col);
 int ta_weight_image(const void* w, int K, int c_red, int c_col, int transpose, int reverse, void* image, cudaStream_t stream);
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, int ep_relu, float* stats_partial, uint32_t* n_partials,
@@ -106,8 +106,9 @@ extern "C" int rmn_conv_forward(const void* d_feats, uint32_t n_src, int c_in,
 }
 
 extern "C" size_t rmn_conv_weight_image_bytes(int K, int c_in, int c_out, int dtype) {
-  if (K < 1 || K > 65535 || dtype != RMN_BF16 || !ta_shape(c_in, c_out)) return 0;
-  return (size_t)K * c_in * c_out * 2;
+  if (K < 1 || K > 65535 || dtype != RMN_BF16) return 0;
+  const size_t plain = ta_image_bytes(K, c_in, c_out), transposed = ta_image_bytes(K, c_out, c_in);
+  return plain > transposed ? plain : transposed;  // (both orders of every pair have a kernel)
 }
 
 extern "C" int rmn_conv_weight_image(const void* d_weights, int K, int c_in, int c_out, int dtype, int transpose, int reverse,

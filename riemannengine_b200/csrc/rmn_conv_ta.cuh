@@ -23,8 +23,9 @@ namespace tc {
 
 template <int CR, int CC>
 struct TaCfg {
-  static constexpr int KB = CR < 64 ? CR : 64;  // reduction channels per stage
-  static constexpr int NKB = CR / KB;
+  static constexpr int KB = 64;                 // reduction channels per stage ...
+  static constexpr int OPS = CR < KB ? 2 : 1;   // ... those of two offsets where a row has only 32 ...
+  static constexpr int NKB = CR < KB ? 1 : CR / KB;  // ... or one of the NKB blocks of an offset
   static constexpr int T = CC <= 64 ? 4 : (CC <= 128 ? 2 : 1);  // row tiles that share one stage of W[k]
   static constexpr int GROUPS = 4, PHASES = GROUPS / T;         // the PHASES groups of a tile take its stages in turn
   static constexpr int A_COLS = KB / 2;                         // tensor-memory columns of one A slot
@@ -39,6 +40,7 @@ struct TaCfg {
   static constexpr uint32_t EP_OFFSET = BAR_OFFSET + 1024;                // 2 * CC floats of epilogue scale / shift
   static constexpr uint32_t STATS_OFFSET = EP_OFFSET + 2 * CC * 4;        // per-warp channel statistics, 4 * 2 * CC floats
   static constexpr uint32_t SMEM = STATS_OFFSET + 4 * 2 * CC * 4;
+  static_assert(CR * OPS == KB * NKB && (OPS == 1 || (PHASES == 1 && CC <= 64)), "stages");
   static_assert(FIT >= 2 && BARRIERS * 8 + 4 <= 1024, "tensor / shared memory");
 };
 
@@ -59,7 +61,8 @@ __device__ __forceinline__ constexpr uint32_t n_channel(uint32_t p) {
 }
 
 // The weight image: per offset and KB-channel block, the MN-major swizzled operand image of the stage (one line of 128 or
-// 64 bytes per reduction position and 64-column atom, 16-byte chunk c of line p at swz(p, c)). One thread per chunk.
+// 64 bytes per reduction position and 64-column atom, 16-byte chunk c of line p at swz(p, c)). Where a stage has two
+// offsets their lines follow one another; the second half of an odd last stage is zero. One thread per chunk.
 // transpose: w is [K][CC][CR] (input gradient); reverse: offset k of the image is W[K - 1 - k].
 template <int CR, int CC>
 __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, int transpose, int reverse,
@@ -67,11 +70,11 @@ __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __res
   using C = TaCfg<CR, CC>;
   constexpr int KB = C::KB, NBLK = CC < 64 ? CC : 64, CPL = NBLK / 8, CHUNKS = KB * CC / 8;
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
-  if (i >= (uint32_t)K * C::NKB * CHUNKS) return;
+  if (i >= (uint32_t)((K + C::OPS - 1) / C::OPS) * C::NKB * CHUNKS) return;
   const uint32_t stage = i / CHUNKS, r = i % CHUNKS;
-  const uint32_t k = stage / C::NKB, kb = stage % C::NKB;
   const uint32_t atom = r / (KB * CPL), p = (r / CPL) % KB, c = r % CPL;
-  const uint32_t ci = kb * KB + k_channel(p);
+  const uint32_t ci = k_channel(C::OPS > 1 ? p % CR : stage % C::NKB * KB + p);
+  const int k = (int)(C::OPS > 1 ? stage * C::OPS + p / CR : stage / C::NKB);
   const __nv_bfloat16* wk = w + (size_t)(reverse ? K - 1 - k : k) * CR * CC;
   uint32_t v[4];
 #pragma unroll
@@ -80,31 +83,35 @@ __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __res
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const uint32_t co = atom * NBLK + n_channel<NBLK>(c * 8 + q * 2 + h);
-      e[h] = *reinterpret_cast<const uint16_t*>(transpose ? wk + (size_t)co * CR + ci : wk + (size_t)ci * CC + co);
+      e[h] = k >= K ? (uint16_t)0 : *reinterpret_cast<const uint16_t*>(transpose ? wk + (size_t)co * CR + ci : wk + (size_t)ci * CC + co);
     }
     v[q] = e[0] | ((uint32_t)e[1] << 16);
   }
   image[stage * CHUNKS + atom * (KB * CPL) + p * CPL + swz<NBLK * 2>(p, c)] = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-// The 32 rows of a gather warp, one KB-channel block of each, on their way from global to tensor memory. Two lanes share
-// a row of each half of 16 (lane t: row t / 4 + 8 (t & 1), 32-byte piece t / 2 & 1 of every 64 bytes). The registers are
-// loaded in the order tcgen05.st.16x64b takes them in, so nothing is moved in between: a move, like a spill, of a
-// register whose load is in flight waits for the load (four lanes per row and 16x256b stores would halve the pieces
-// per row, but need the moves and three times the registers).
-template <int KB>
+// The 32 rows of a gather warp on their way from global to tensor memory: 64 channels of one row each, or the 32 channels
+// of two (OPS = 2, idx2: the rows of the second offset). Two lanes share a row of each half of 16 (lane t: row
+// t / 4 + 8 (t & 1), 32-byte piece t / 2 & 1 of every 64 bytes). The registers are loaded in the order tcgen05.st.16x64b
+// takes them in, so nothing is moved in between: a move, like a spill, of a register whose load is in flight waits for
+// the load (four lanes per row and 16x256b stores would halve the pieces per row, but need the moves and three times the
+// registers).
 struct RowBlock {
-  static constexpr int W = KB / 4;  // words per lane and row
-  uint32_t v[2][W];
-  template <int CR>
-  __device__ __forceinline__ void load(const __nv_bfloat16* __restrict__ src_lane, int32_t idx, int lane) {
+  uint32_t v[2][16];
+  template <int CR, int OPS>
+  __device__ __forceinline__ void load(const __nv_bfloat16* __restrict__ src_lane, int32_t idx, int32_t idx2, int lane) {
     const int mine = (lane >> 2) + 8 * (lane & 1);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int32_t row = __shfl_sync(0xFFFFFFFFu, idx, h * 16 + mine);
       const __nv_bfloat16* p = src_lane + (size_t)(uint32_t)row * CR;
       ldg32_or_zero<0>(p, row >= 0, v[h]);
-      if constexpr (W == 16) ldg32_or_zero<8>(p + 32, row >= 0, v[h]);
+      if constexpr (OPS == 1) {
+        ldg32_or_zero<8>(p + 32, row >= 0, v[h]);
+      } else {
+        const int32_t row2 = __shfl_sync(0xFFFFFFFFu, idx2, h * 16 + mine);
+        ldg32_or_zero<8>(src_lane + (size_t)(uint32_t)row2 * CR, row2 >= 0, v[h]);
+      }
     }
   }
   __device__ __forceinline__ void store(uint32_t taddr) const {
@@ -126,7 +133,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
               const float* __restrict__ ep_shift, int ep_relu, float* __restrict__ stats_partial,
               const int32_t* __restrict__ perm, const uint32_t* __restrict__ tile_mask) {
   using C = TaCfg<CR, CC>;
-  constexpr int KB = C::KB, NKB = C::NKB, T = C::T, G = C::GROUPS, PH = C::PHASES, SLOTS = C::SLOTS, BST = C::B_STAGES;
+  constexpr int KB = C::KB, NKB = C::NKB, OPS = C::OPS, T = C::T, G = C::GROUPS, PH = C::PHASES, SLOTS = C::SLOTS, BST = C::B_STAGES;
   constexpr int KSTEP = PH > NKB ? PH / NKB : 1;  // every KSTEP-th offset belongs to one group of a tile ...
   constexpr int NB = NKB > PH ? NKB / PH : 1;     // ... with NB of its channel blocks, PH apart
   constexpr int NBLK = CC < 64 ? CC : 64;         // columns of one atom
@@ -141,6 +148,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   uint64_t* acc_empty = acc_full + C::ACC_BUFS * T;  // [buffer][tile]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + C::ACC_BUFS * T);
   float* s_ep = reinterpret_cast<float*>(smem + C::EP_OFFSET);  // per-channel scale | shift
+  const int n_off = (K + OPS - 1) / OPS;  // offsets, or pairs of them
   const bool has_ep = ep_scale != nullptr || ep_shift != nullptr || ep_relu != 0;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -186,13 +194,14 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     const uint32_t a_base = tmem_base + C::ACC_COLS + g * SLOTS * C::A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t bars = smem_u32(a_full + g * SLOTS);  // full barriers; the empty ones lie G * SLOTS further
 
-    // Cursor over the table entries of this lane's rows; kEnd behind the last one
+    // Cursor over the table entries of this lane's rows (OPS = 2: `second` goes with the entry returned); kEnd behind the
+    // last one
     constexpr int32_t kEnd = INT32_MIN;
     uint32_t st = blockIdx.x, todo = 0;
     int k = K, kb = NB - 1;
     const int32_t* entry = nbr;
     bool row_ok = false, fresh = true;
-    int32_t last = -1;
+    int32_t last = -1, second = -1;
     auto next = [&]() -> int32_t {
       if constexpr (NB > 1) {
         if (++kb < NB) return last;
@@ -210,8 +219,9 @@ __global__ void __launch_bounds__(kTaThreads, 1)
         } else {
           if (k < K) {
             last = row_ok ? __ldg(entry) : -1;
-            entry += (size_t)KSTEP * n_dst;
-            k += KSTEP;
+            if constexpr (OPS == 2) second = row_ok && k + 1 < K ? __ldg(entry + n_dst) : -1;
+            entry += (size_t)(KSTEP * OPS) * n_dst;
+            k += KSTEP * OPS;
             return last;
           }
         }
@@ -241,9 +251,9 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     // whose loads are in flight, and a copy waits for its source. A spilled register of a block does the same: 80
     // registers were 3 times slower.)
     uint32_t cnt = 0;
-    RowBlock<KB> b0, b1;
-    auto load = [&](RowBlock<KB>& b, int32_t idx, int block) {
-      b.template load<CR>(src_lane + (NB > 1 ? block * PH * KB : 0), idx, lane);
+    RowBlock b0, b1;
+    auto load = [&](RowBlock& b, int32_t idx, int32_t idx2, int block) {
+      b.template load<CR, OPS>(src_lane + (NB > 1 ? block * PH * KB : 0), idx, idx2, lane);
     };
     auto arrive = [&]() {  // the block stored last has reached tensor memory
       tc_wait_st();
@@ -251,7 +261,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(bars + ((cnt - 1u) % SLOTS) * 8);
     };
-    auto put = [&](const RowBlock<KB>& b) {
+    auto put = [&](const RowBlock& b) {
       if (cnt) arrive();
       const uint32_t s = cnt % SLOTS, ph = (cnt / SLOTS) & 1u;
       ++cnt;
@@ -262,34 +272,36 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     };
     constexpr int ODD = NB > 1 ? 1 : 0;
     static_assert(NB <= 2, "the blocks of an offset alternate");
-    int32_t w0 = next(), w1 = next(), w2, w3;
-    load(b0, w0, 0);
-    load(b1, w1, ODD);
-    w2 = next();
-    w3 = next();
+    int32_t w0, w1, w2, w3, x0 = -1, x1 = -1, x2 = -1, x3 = -1;
+    w0 = next(), x0 = second;
+    w1 = next(), x1 = second;
+    load(b0, w0, x0, 0);
+    load(b1, w1, x1, ODD);
     bool live0 = w0 != kEnd, live1 = w1 != kEnd;
-    w0 = next();
-    w1 = next();
+    w2 = next(), x2 = second;
+    w3 = next(), x3 = second;
+    w0 = next(), x0 = second;
+    w1 = next(), x1 = second;
     while (live0) {
       put(b0);
-      load(b0, w2, 0);
+      load(b0, w2, x2, 0);
       live0 = w2 != kEnd;
-      w2 = next();
+      w2 = next(), x2 = second;
       if (!live1) break;
       put(b1);
-      load(b1, w3, ODD);
+      load(b1, w3, x3, ODD);
       live1 = w3 != kEnd;
-      w3 = next();
+      w3 = next(), x3 = second;
       if (!live0) break;
       put(b0);
-      load(b0, w0, 0);
+      load(b0, w0, x0, 0);
       live0 = w0 != kEnd;
-      w0 = next();
+      w0 = next(), x0 = second;
       if (!live1) break;
       put(b1);
-      load(b1, w1, ODD);
+      load(b1, w1, x1, ODD);
       live1 = w1 != kEnd;
-      w1 = next();
+      w1 = next(), x1 = second;
       if (__any_sync(0xFFFFFFFFu, timed_out)) break;
     }
     if (cnt) arrive();
@@ -315,7 +327,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
         }
       }
       uint32_t started = 0, odd = 0;  // per tile: an MMA has been issued; parity of its offset count
-      for (int k = 0; kPlan ? todo != 0 : k < K; ++k) {
+      for (int k = 0; kPlan ? todo != 0 : k < n_off; ++k) {
         if constexpr (kPlan) {
           k = __ffs(todo) - 1;
           todo &= todo - 1u;
@@ -370,7 +382,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
 #pragma unroll
           for (int t = 0; t < T; ++t) todo |= __ldg(tile_mask + (size_t)st * T + t);
         }
-        for (int k = 0; (kPlan ? todo != 0 : k < K) && !timed_out; ++k) {
+        for (int k = 0; (kPlan ? todo != 0 : k < n_off) && !timed_out; ++k) {
           if constexpr (kPlan) {
             k = __ffs(todo) - 1;
             todo &= todo - 1u;
@@ -542,9 +554,16 @@ int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n
   return RMN_OK;
 }
 
+// K rounded up to whole stages, times the bytes of one offset's weights
+template <int CR, int CC>
+size_t image_bytes(int K) {
+  using C = TaCfg<CR, CC>;
+  return (size_t)((K + C::OPS - 1) / C::OPS) * C::NKB * C::B_BYTES;
+}
+
 template <int CR, int CC>
 int launch_image(const void* w, int K, int transpose, int reverse, void* image, cudaStream_t stream) {
-  const uint32_t chunks = (uint32_t)K * CR * CC / 8;
+  const uint32_t chunks = (uint32_t)(image_bytes<CR, CC>(K) / 16);
   k_weight_image<CR, CC><<<(chunks + 255) / 256, 256, 0, stream>>>((const __nv_bfloat16*)w, K, transpose, reverse,
                                                                   (uint4*)image);
   RMN_LAUNCH_CHECK();
@@ -556,11 +575,14 @@ int launch_image(const void* w, int K, int transpose, int reverse, void* image, 
 #define RMN_TA_SHAPES(CASE) \
   CASE(32, 32) CASE(32, 64) CASE(64, 32) CASE(64, 64) CASE(64, 128) CASE(128, 64) CASE(128, 128) CASE(128, 256) CASE(256, 128) CASE(256, 256)
 
-bool ta_shape(int c_red, int c_col) {
-#define RMN_TA_CASE(R, Cc) if (c_red == R && c_col == Cc) return true;
+constexpr int kPlanMinWeight = 128 * 128;
+
+// 0: no kernel for these channel counts
+size_t ta_image_bytes(int K, int c_red, int c_col) {
+#define RMN_TA_CASE(R, Cc) if (c_red == R && c_col == Cc) return tc::image_bytes<R, Cc>(K);
   RMN_TA_SHAPES(RMN_TA_CASE)
 #undef RMN_TA_CASE
-  return false;
+  return 0;
 }
 
 // image of [K][c_red][c_col] weights (transpose: given as [K][c_col][c_red])
@@ -576,13 +598,18 @@ int ta_weight_image(const void* w, int K, int c_red, int c_col, int transpose, i
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, int ep_relu, float* stats_partial, uint32_t* n_partials,
             cudaStream_t stream, const void* plan) {
-  if (K > kPlanMaxK) plan = nullptr;
+  // A plan pays where a skipped tile saves more MMA time than the gather of its rows takes anyway: from 128 x 128 channels
+  // on (1.2 M rows: 128->128 716 -> 645 us, but 64->64 281 -> 288, 32->64 221 -> 249). The rows come out the same.
 #define RMN_TA_ARGS src, image, nbr, n_dst, K, out, ep_scale, ep_shift, ep_relu, stream, stats_partial, n_partials, plan
 #define RMN_TA_CASE(R, Cc)                                                                                            \
   if (c_red == R && c_col == Cc) {                                                                                    \
-    if (stats_partial)                                                                                                \
-      return plan ? tc::launch_ta<R, Cc, true, true>(RMN_TA_ARGS) : tc::launch_ta<R, Cc, true, false>(RMN_TA_ARGS);    \
-    return plan ? tc::launch_ta<R, Cc, false, true>(RMN_TA_ARGS) : tc::launch_ta<R, Cc, false, false>(RMN_TA_ARGS);    \
+    if constexpr (R * Cc >= kPlanMinWeight) {                                                                         \
+      if (plan && K <= kPlanMaxK)                                                                                     \
+        return stats_partial ? tc::launch_ta<R, Cc, true, true>(RMN_TA_ARGS)                                          \
+                             : tc::launch_ta<R, Cc, false, true>(RMN_TA_ARGS);                                        \
+    }                                                                                                                 \
+    return stats_partial ? tc::launch_ta<R, Cc, true, false>(RMN_TA_ARGS)                                             \
+                         : tc::launch_ta<R, Cc, false, false>(RMN_TA_ARGS);                                           \
   }
   RMN_TA_SHAPES(RMN_TA_CASE)
 #undef RMN_TA_CASE

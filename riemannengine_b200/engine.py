@@ -140,19 +140,22 @@ class KernelMap:
         self._uses_out = self._uses_in = 0
 
     # Convolution plans (ops.conv_plan_build), built lazily under the same rule as the C++ host layer
-    # (KernelMap::plan_out in riemann_cpp): by the pass that brings the work done on the table (sum of
-    # c_in * c_out over the passes) to four 64 x 64 layers' worth, where the plan repays its build.
+    # (KernelMap::plan_out in riemann_cpp): passes of 128 x 128 channels or more count, by c_in * c_out, and
+    # the one that brings the sum to two 128 x 128 layers' worth builds the plan; narrower ones gain nothing.
     plan_policy = 0  # 0 automatic, 1 always, 2 never
+    _WIDE_PASS = 128 * 128
 
     @staticmethod
     def _want_plan(weight_sum: int, rows: int) -> bool:
         if KernelMap.plan_policy == 2 or rows < 8192:
             return False
-        return KernelMap.plan_policy == 1 or weight_sum >= 4 * 64 * 64
+        return KernelMap.plan_policy == 1 or weight_sum >= 2 * KernelMap._WIDE_PASS
 
     def plan_out(self, weight: int):
         if self._parent is not None:
             return self._parent.plan_in(weight)
+        if weight < self._WIDE_PASS and KernelMap.plan_policy == 0:
+            return None
         self._uses_out += weight
         if (self._plan_out is None and self.region_offsets is not None
                 and self._want_plan(self._uses_out, self.n_out)):
@@ -164,6 +167,8 @@ class KernelMap:
             return self._parent.plan_out(weight)
         if self.self_symmetric:
             return self.plan_out(weight)
+        if weight < self._WIDE_PASS and KernelMap.plan_policy == 0:
+            return None
         self._uses_in += weight
         if (self._plan_in is None and self.region_offsets is not None
                 and self._want_plan(self._uses_in, self.n_in)):
