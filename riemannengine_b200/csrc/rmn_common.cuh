@@ -58,7 +58,15 @@ struct __align__(16) TableHeader {
   // number of trailing zeros. The position inside a bucket is taken from the bits above them.
   uint32_t x_or;
   uint32_t pos_shift;
-  uint32_t pad[4];
+  uint32_t yz_or[2];  // x_or of the second and third spatial columns
+  uint32_t pad[2];
+
+  // low bits that all rows share in spatial column `axis` (of the first three)
+  __device__ __forceinline__ uint32_t low_shift(int axis) const {
+    if (axis == 0) return pos_shift;
+    const uint32_t o = yz_or[axis - 1];
+    return o ? (uint32_t)__ffs((int)o) - 1u : 0u;
+  }
 };
 static_assert(sizeof(TableHeader) == 256, "header must be 256 bytes");
 

@@ -350,7 +350,20 @@ __global__ void __launch_bounds__(256) k_kmap_transpose(const int32_t* __restric
 
 inline uint32_t kmap_blocks(uint32_t n_query) { return (n_query + kKmapBlock - 1) / kKmapBlock; }
 
+// Self maps whose hash table does not fit the 126 MB L2 go over the occupancy index (rmn_kmap_blocks.cuh); below that a
+// probe of the table is an L2 hit and the index saves nothing (1.2 M rows x 27 offsets: 137 us by probing, 240 us with it).
+inline bool use_block_index(uint32_t n, int K) {
+  return (size_t)n * 64 > ((size_t)120 << 20) && (K & 1) && K >= 9 && K <= 2048;
+}
+
+// counts per (offset, 256 query rows), totals, flags
+inline size_t kmap_counts_bytes(uint32_t n_query, int K) {
+  return (((size_t)K * kmap_blocks(n_query) + (size_t)K + 64) * sizeof(uint32_t) + 255) & ~(size_t)255;
+}
+
 }  // namespace rmn
+
+#include "rmn_kmap_blocks.cuh"
 
 using namespace rmn;
 
@@ -409,7 +422,7 @@ extern "C" int rmn_region_offsets(int region_type, int D, const int32_t* kernel_
 
 extern "C" size_t rmn_kmap_workspace_bytes(uint32_t n_query, int K) {
   if (K < 1) K = 1;
-  return ((size_t)K * kmap_blocks(n_query) + (size_t)K + 64) * sizeof(uint32_t);
+  return kmap_counts_bytes(n_query, K) + (use_block_index(n_query, K) ? block_index_bytes(n_query) : 0);
 }
 
 extern "C" int rmn_kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_query, int W,
@@ -463,6 +476,25 @@ extern "C" int rmn_kmap_build_self(const void* d_table, const int32_t* d_coords,
   auto* slots =
       reinterpret_cast<const Slot*>(reinterpret_cast<const char*>(d_table) + sizeof(TableHeader));
   const int half = K / 2;
+  if (use_block_index(n_rows, K) && ((uintptr_t)d_workspace & 15) == 0) {
+    const BlockIndex ix = block_index(static_cast<char*>(d_workspace) + kmap_counts_bytes(n_rows, K), n_rows);
+    RMN_CUDA_TRY(cudaMemsetAsync(ix.slots, 0xFF, (size_t)ix.capacity * sizeof(BlockSlot) + 32, stream));
+    RMN_DISPATCH_W(W, k_block_insert<kW><<<nb, 256, 0, stream>>>(h, d_coords, n_rows, ix));
+    RMN_LAUNCH_CHECK();
+    k_block_bases<<<(ix.capacity + 255) / 256, 256, 0, stream>>>(ix);
+    RMN_LAUNCH_CHECK();
+    RMN_DISPATCH_W(W, k_block_scatter<kW><<<nb, 256, 0, stream>>>(h, d_coords, n_rows, ix));
+    RMN_LAUNCH_CHECK();
+    const size_t smem = (size_t)8 * kKmapBlock * 12 + (size_t)K * 4 + (size_t)half * 4;
+    RMN_DISPATCH_W(W, k_kmap_blocks_self<kW><<<nb, kKmapBlock, smem, stream>>>(h, slots, d_coords, n_rows, d_offsets, K,
+                                                                              d_nbr, block_counts, nb, ix));
+    RMN_LAUNCH_CHECK();
+    k_kmap_scan_blocks<<<half + 1, 1024, 0, stream>>>(block_counts, nb, totals);
+    RMN_LAUNCH_CHECK();
+    k_kmap_offset_ptr<<<1, 32, 0, stream>>>(totals, K, d_offset_ptr, half, totals + K + 1);
+    RMN_LAUNCH_CHECK();
+    return RMN_OK;
+  }
   if (half > 0)  // the mirrored half starts as "no neighbour"
     RMN_CUDA_TRY(cudaMemsetAsync(d_nbr + (size_t)(half + 1) * n_rows, 0xFF, (size_t)half * n_rows * sizeof(int32_t),
                                  stream));

@@ -1,0 +1,316 @@
+// Self map over an occupancy index: the rows of a map grouped into 4 x 4 x 4 blocks of voxels, one 64-bit mask per block.
+//
+// What bounds k_kmap_probe_self on a large map is random access: a hash-table line per (row, x-triple of offsets), and
+// for every hit a scattered 4-byte store of the mirror entry into a table that no cache holds; once the hash table
+// exceeds the L2 the probes go to DRAM as well (4.8 M rows x 81 offsets: 3740 us). Here a row looks up the blocks that its
+// neighbourhood can touch (at most 8 per position on the axes behind the third; the slots of all blocks stay in L2), and
+// every offset is a bit test; a hit ranks its bit in the mask and reads the row number from `perm`, where the rows of a
+// block lie next to one another. All K offsets are computed, nothing is mirrored, and the table is written once,
+// coalesced: 2180 us for that map, still bound by the row numbers' random reads (26 per row; more registers or wider
+// shared entries leave less L1 and are slower: 2030 and 2350 us against 1980 us for the kernel alone).
+//
+// Included by rmn_kmap.cu.
+#pragma once
+
+namespace rmn {
+
+struct __align__(32) BlockSlot {  // one 32-byte sector: a lookup is one access
+  unsigned long long key;   // packed block coordinates, kEmptyKey when free
+  unsigned long long free;  // bit per voxel of the block: 0 where a row exists (so that a fill with ones is "empty")
+  uint32_t base;            // position in perm of the first row of the block
+  uint32_t pad[3];
+};
+
+// Index in a workspace of block_index_bytes(n). One slot per eight rows, so that the slots fit the L2 where the hash table
+// does not: a surface fills a block with about twenty rows. Rows that lie too thinly for that (a lidar sweep) overflow
+// the index; its user then falls back to the hash table.
+struct BlockIndex {
+  BlockSlot* slots;
+  uint32_t* counter;      // rows numbered so far, minus one
+  uint32_t* overflow;     // all ones; 0: the blocks did not fit
+  int32_t* perm;          // row numbers, block by block
+  uint32_t* slot_of_row;  // build scratch
+  uint32_t capacity;
+};
+constexpr uint32_t kBlockMaxProbes = 32;
+inline uint32_t block_index_capacity(uint32_t n) { return n / 8 + 64; }
+inline size_t block_index_bytes(uint32_t n) {
+  return (size_t)block_index_capacity(n) * sizeof(BlockSlot) + 32 + (size_t)n * 8;
+}
+inline BlockIndex block_index(void* workspace, uint32_t n) {
+  BlockIndex b;
+  b.capacity = block_index_capacity(n);
+  b.slots = static_cast<BlockSlot*>(workspace);
+  b.counter = reinterpret_cast<uint32_t*>(b.slots + b.capacity);  // (filled together with the slots)
+  b.overflow = b.counter + 1;
+  b.perm = reinterpret_cast<int32_t*>(b.counter + 8);
+  b.slot_of_row = reinterpret_cast<uint32_t*>(b.perm + n);
+  return b;
+}
+
+__device__ __forceinline__ uint32_t block_hash(unsigned long long key, uint32_t capacity) {
+  uint32_t h = (uint32_t)key ^ ((uint32_t)(key >> 32) * 0x9E3779B1u);
+  h *= 0x85ebca6bu;
+  h ^= h >> 13;
+  h *= 0xc2b2ae35u;
+  h ^= h >> 16;
+  return __umulhi(h, capacity);
+}
+
+// Coordinates of a row relative to the box, split into block and position. The first three spatial columns (fewer in
+// two or one dimensions) are the block's axes; the low bits that all rows share (tensor stride) are left out of them.
+template <int W>
+struct BlockCoords {
+  static constexpr int NA = W - 1 < 3 ? W - 1 : 3;
+  uint32_t local;           // 2 bits per block axis, in nibbles
+  uint32_t block[NA];       // block coordinate per block axis
+  unsigned long long key;   // packed block coordinates with the remaining columns
+  uint32_t dist[W];         // distance from the box minimum per column
+
+  __device__ __forceinline__ void load(const TableHeader* h, const int32_t (&c)[W]) {
+    local = 0;
+    key = 0;
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      dist[i] = (uint32_t)c[i] - (uint32_t)h->mn[i];
+      unsigned long long field = dist[i];
+      if (i >= 1 && i <= NA) {
+        const uint32_t s = h->low_shift(i - 1);
+        local |= ((dist[i] >> s) & 3u) << (4 * (i - 1));
+        block[i - 1] = (dist[i] >> s) >> 2;
+        field = block[i - 1];
+      }
+      key |= field << h->shift[i];
+    }
+  }
+  static __device__ __forceinline__ uint32_t bit(uint32_t nibbles) {  // position of a voxel in its block's mask
+    return (nibbles & 3u) | ((nibbles >> 2) & 0xCu) | ((nibbles >> 4) & 0x30u);
+  }
+};
+
+template <int W>
+__global__ void __launch_bounds__(256) k_block_insert(const TableHeader* __restrict__ h, const int32_t* __restrict__ coords,
+                                                      uint32_t n, BlockIndex ix) {
+  const uint32_t row = blockIdx.x * 256 + threadIdx.x;
+  if (row >= n) return;
+  int32_t c[W];
+  load_row<W>(coords, row, c);
+  BlockCoords<W> b;
+  b.load(h, c);
+  if (*(volatile uint32_t*)ix.overflow == 0) return;
+  uint32_t s = block_hash(b.key, ix.capacity);
+  bool placed = false;
+  for (uint32_t probe = 0; probe < kBlockMaxProbes; ++probe) {
+    unsigned long long cur = *(volatile unsigned long long*)&ix.slots[s].key;
+    if (cur == kEmptyKey) cur = atomicCAS(&ix.slots[s].key, kEmptyKey, b.key);
+    if (cur == kEmptyKey || cur == b.key) {
+      placed = true;
+      break;
+    }
+    if (++s == ix.capacity) s = 0;
+  }
+  if (!placed) {
+    *(volatile uint32_t*)ix.overflow = 0;
+    return;
+  }
+  atomicAnd(&ix.slots[s].free, ~(1ull << b.bit(b.local)));
+  ix.slot_of_row[row] = s;
+}
+
+// Gives every block its range of perm. Which range a block gets depends on the order of the atomics; what the index
+// returns does not.
+__global__ void __launch_bounds__(256) k_block_bases(BlockIndex ix) {
+  __shared__ uint32_t s_warp[8], s_base;
+  if (__ldg(ix.overflow) == 0) return;
+  const uint32_t s = blockIdx.x * 256 + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t count = s < ix.capacity ? (uint32_t)__popcll(~__ldg(&ix.slots[s].free)) : 0u;
+  uint32_t incl = count;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t run = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const uint32_t v = s_warp[w];
+      s_warp[w] = run;
+      run += v;
+    }
+    s_base = run ? atomicAdd(ix.counter, run) + 1u : 0u;  // (the counter starts at all ones)
+  }
+  __syncthreads();
+  if (count) ix.slots[s].base = s_base + s_warp[warp] + incl - count;
+}
+
+template <int W>
+__global__ void __launch_bounds__(256) k_block_scatter(const TableHeader* __restrict__ h, const int32_t* __restrict__ coords,
+                                                       uint32_t n, BlockIndex ix) {
+  const uint32_t row = blockIdx.x * 256 + threadIdx.x;
+  if (row >= n) return;
+  if (__ldg(ix.overflow) == 0) return;
+  const uint32_t s = ix.slot_of_row[row];
+  int32_t c[W];
+  load_row<W>(coords, row, c);
+  BlockCoords<W> b;
+  b.load(h, c);
+  const unsigned long long below = (1ull << b.bit(b.local)) - 1ull;
+  ix.perm[__ldg(&ix.slots[s].base) + (uint32_t)__popcll(~__ldg(&ix.slots[s].free) & below)] = (int32_t)row;
+}
+
+// One thread per row, as in k_kmap_probe. Offsets that reach further than two voxels (in units of the map's grid) along
+// a block axis look their row up in the hash table instead.
+template <int W>
+__global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
+    const TableHeader* __restrict__ h, const Slot* __restrict__ slots, const int32_t* __restrict__ coords, uint32_t n,
+    const int32_t* __restrict__ offsets, int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts,
+    uint32_t n_blocks, BlockIndex ix) {
+  using B = BlockCoords<W>;
+  constexpr int D = W - 1, NA = B::NA, CELLS = 1 << NA;
+  constexpr uint32_t kNever = 1u << 28, kFar = 1u << 29, kNewOuter = 1u << 30;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned long long* s_occ = reinterpret_cast<unsigned long long*>(smem_raw);  // [CELLS][256] masks around every row
+  uint32_t* s_base = reinterpret_cast<uint32_t*>(s_occ + CELLS * kKmapBlock);   // [CELLS][256]
+  uint32_t* s_off = s_base + CELLS * kKmapBlock;                                // [K] offset in nibbles modulo 8, flags
+  uint32_t* s_cnt = s_off + K;                                                  // [half]
+  __shared__ uint32_t s_reach[2 * NA];  // largest step down / up per block axis
+  const int half = K / 2;
+  const bool overflow = __ldg(ix.overflow) == 0;
+  if (threadIdx.x < 2 * NA) s_reach[threadIdx.x] = 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k < K; k += kKmapBlock) {
+    uint32_t e = 0;
+    int32_t step[NA];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+      const int32_t o = __ldg(offsets + k * D + a);
+      const uint32_t s = h->low_shift(a);
+      if (o & ((1 << s) - 1)) e |= kNever;  // off the map's grid
+      step[a] = o >> s;
+      if (step[a] < -2 || step[a] > 2) e |= kFar;
+      e |= ((uint32_t)step[a] & 7u) << (4 * a);
+    }
+    bool new_outer = k == 0;
+#pragma unroll
+    for (int a = NA; a < D; ++a) new_outer |= k > 0 && __ldg(offsets + k * D + a) != __ldg(offsets + (k - 1) * D + a);
+    if (new_outer) e |= kNewOuter;
+    if (!(e & (kNever | kFar))) {
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        if (step[a] < 0) atomicMax(&s_reach[2 * a], (uint32_t)-step[a]);
+        if (step[a] > 0) atomicMax(&s_reach[2 * a + 1], (uint32_t)step[a]);
+      }
+    }
+    if (overflow) e |= kFar;
+    s_off[k] = e;
+    if (k < half) s_cnt[k] = 0;
+  }
+  __syncthreads();
+
+  const uint32_t q = blockIdx.x * kKmapBlock + threadIdx.x;
+  const bool active = q < n;
+  const int lane = threadIdx.x & 31;
+  int32_t c[W];
+#pragma unroll
+  for (int i = 0; i < W; ++i) c[i] = h->mn[i];
+  if (active) load_row<W>(coords, q, c);
+  B b;
+  b.load(h, c);
+  // per block axis: the neighbouring block on the side of the row's half of its block, if any offset reaches it
+  long long side[NA];
+  uint32_t reach = 0;
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+    const uint32_t l = (b.local >> (4 * a)) & 3u;
+    const uint32_t last = (((uint32_t)(h->mx[a + 1] - h->mn[a + 1])) >> h->low_shift(a)) >> 2;
+    const bool up = l >= 2;
+    if (up ? (l + s_reach[2 * a + 1] > 3 && b.block[a] < last) : (s_reach[2 * a] > l && b.block[a] > 0)) reach |= 1u << a;
+    side[a] = (up ? 1ll : -1ll) * (1ll << h->shift[a + 1]);
+  }
+  unsigned long long* occ = s_occ + threadIdx.x;
+  uint32_t* base = s_base + threadIdx.x;
+  int32_t* dst = nbr + q;
+  for (int k = 0; k < K; ++k, dst += n) {
+    const uint32_t e = s_off[k];
+    if (!overflow && (e & kNewOuter)) {  // (same for the whole block) look up the blocks around the row
+      unsigned long long key0 = b.key;
+      bool in_box = active;
+#pragma unroll
+      for (int a = NA; a < D; ++a) {
+        const int32_t o = __ldg(offsets + k * D + a);
+        in_box = in_box && b.dist[a + 1] + (uint32_t)o <= (uint32_t)(h->mx[a + 1] - h->mn[a + 1]);
+        key0 += (unsigned long long)((long long)o << h->shift[a + 1]);
+      }
+      constexpr int BATCH = CELLS < 4 ? CELLS : 4;  // independent lookups in flight
+#pragma unroll
+      for (int i0 = 0; i0 < CELLS; i0 += BATCH) {
+        ulonglong2 v[BATCH];
+        uint32_t at[BATCH];
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) {
+          const int i = i0 + j;
+          v[j] = make_ulonglong2(kEmptyKey, ~0ull);
+          at[j] = 0;
+          if (in_box && (i & ~reach) == 0) {
+            unsigned long long key = key0;
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+              if ((i >> a) & 1) key += (unsigned long long)side[a];
+            at[j] = block_hash(key, ix.capacity);
+            v[j] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[j]));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) {
+          const int i = i0 + j;
+          unsigned long long key = key0;
+#pragma unroll
+          for (int a = 0; a < NA; ++a)
+            if ((i >> a) & 1) key += (unsigned long long)side[a];
+          for (uint32_t probe = 1; v[j].x != key && v[j].x != kEmptyKey && probe < kBlockMaxProbes; ++probe) {
+            if (++at[j] == ix.capacity) at[j] = 0;
+            v[j] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[j]));
+          }
+          const bool found = v[j].x == key;
+          occ[i * kKmapBlock] = found ? ~v[j].y : 0ull;
+          if (found) base[i * kKmapBlock] = __ldg(&ix.slots[at[j]].base);
+        }
+      }
+    }
+    uint32_t uid = 0xFFFFFFFFu;
+    bool hit = false;
+    if (!(e & (kNever | kFar))) {
+      const uint32_t p = b.local + (e & 0xFFFu), bit = B::bit(p);
+      // bits 2, 6 and 10: is the voxel in the row's own block or in the next one along the axis
+      const uint32_t cell = ((((p & 0x444u) * 0x124u) >> 10) & 7u) * kKmapBlock;
+      const unsigned long long m = occ[cell];
+      hit = (m >> bit) & 1ull;
+      if (hit) uid = (uint32_t)__ldg(ix.perm + base[cell] + __popcll(m & ((1ull << bit) - 1ull)));
+    } else if (e & kFar && !(e & kNever)) {
+      bool in_box = active;
+      unsigned long long key = 0;
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        const uint32_t d = b.dist[i] + (i > 0 ? (uint32_t)__ldg(offsets + k * D + i - 1) : 0u);
+        in_box = in_box && d <= (uint32_t)(h->mx[i] - h->mn[i]);
+        key |= (unsigned long long)d << h->shift[i];
+      }
+      if (in_box) uid = table_find(slots, h->capacity, h->pos_shift, key);
+      hit = uid != 0xFFFFFFFFu;
+    }
+    if (active) __stcs(dst, (int32_t)uid);
+    if (k < half) {  // (the other half has the same counts, see k_kmap_offset_ptr)
+      const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+      if (lane == 0) atomicAdd(&s_cnt[k], (uint32_t)__popc(hits));
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < half; k += kKmapBlock) block_counts[(size_t)k * n_blocks + blockIdx.x] = s_cnt[k];
+  if (threadIdx.x == 0) block_counts[(size_t)half * n_blocks + blockIdx.x] = min((uint32_t)kKmapBlock, n - blockIdx.x * kKmapBlock);
+}
+
+}  // namespace rmn

@@ -39,23 +39,28 @@ template <int W>
 __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ coords, uint32_t n,
                                                     TableHeader* h, uint4* __restrict__ slots, uint32_t capacity) {
   __shared__ int32_t s_mn[8][W], s_mx[8][W];
-  __shared__ uint32_t s_or[8];
+  constexpr int NA = W - 1 < 3 ? W - 1 : 3;
+  __shared__ uint32_t s_or[8][NA];
   const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < capacity; i += gridDim.x * blockDim.x)
     slots[i] = ones;
   int32_t mn[W], mx[W];
 #pragma unroll
   for (int c = 0; c < W; ++c) { mn[c] = INT_MAX; mx[c] = INT_MIN; }
-  // OR of (x - x of row 0) over the rows: its trailing zeros are the bits of the first spatial
-  // column that all rows share
-  const uint32_t x0 = n > 0 ? (uint32_t)__ldg(coords + 1) : 0u;
-  uint32_t x_or = 0;
+  // OR of (x - x of row 0) over the rows: its trailing zeros are the bits of a spatial column that all rows share
+  uint32_t first[NA], col_or[NA];
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+    first[a] = n > 0 ? (uint32_t)__ldg(coords + 1 + a) : 0u;
+    col_or[a] = 0;
+  }
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     int32_t v[W];
     load_row<W>(coords, r, v);
 #pragma unroll
     for (int c = 0; c < W; ++c) { mn[c] = min(mn[c], v[c]); mx[c] = max(mx[c], v[c]); }
-    x_or |= (uint32_t)v[1] - x0;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) col_or[a] |= (uint32_t)v[1 + a] - first[a];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -64,8 +69,11 @@ __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ 
     const int32_t b = __reduce_max_sync(0xFFFFFFFFu, mx[c]);
     if (lane == 0) { s_mn[warp][c] = a; s_mx[warp][c] = b; }
   }
-  x_or = __reduce_or_sync(0xFFFFFFFFu, x_or);
-  if (lane == 0) s_or[warp] = x_or;
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+    const uint32_t o = __reduce_or_sync(0xFFFFFFFFu, col_or[a]);
+    if (lane == 0) s_or[warp][a] = o;
+  }
   __syncthreads();
   // one atomic per block and column (per-warp atomics on eight addresses serialise badly); blocks that
   // saw no row leave the zero ("no row yet") in place
@@ -76,11 +84,12 @@ __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ 
     atomicMax(&h->mn_enc[threadIdx.x], ~((uint32_t)a ^ 0x80000000u));
     atomicMax(&h->mx_enc[threadIdx.x], (uint32_t)b ^ 0x80000000u);
   }
-  if (threadIdx.x == 32 && blockIdx.x * blockDim.x < n) {
+  if (threadIdx.x >= 32 && threadIdx.x < 32 + NA && blockIdx.x * blockDim.x < n) {
+    const int a = (int)threadIdx.x - 32;
     uint32_t o = 0;
 #pragma unroll
-    for (int w2 = 0; w2 < 8; ++w2) o |= s_or[w2];
-    if (o) atomicOr(&h->x_or, o);
+    for (int w2 = 0; w2 < 8; ++w2) o |= s_or[w2][a];
+    if (o) atomicOr(a == 0 ? &h->x_or : &h->yz_or[a - 1], o);
   }
   __threadfence();
   __syncthreads();
