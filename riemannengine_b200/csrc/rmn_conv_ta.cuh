@@ -21,12 +21,13 @@
 namespace rmn {
 namespace tc {
 
-template <int CR, int CC>
+// CC: columns of a CTA (of the whole product, or one of its 64-column blocks), T: row tiles that share one stage of W[k]
+template <int CR, int CC, int T_>
 struct TaCfg {
   static constexpr int KB = 64;                 // reduction channels per stage ...
   static constexpr int OPS = CR < KB ? 2 : 1;   // ... those of two offsets where a row has only 32 ...
   static constexpr int NKB = CR < KB ? 1 : CR / KB;  // ... or one of the NKB blocks of an offset
-  static constexpr int T = CC <= 64 ? 4 : (CC <= 128 ? 2 : 1);  // row tiles that share one stage of W[k]
+  static constexpr int T = T_;
   static constexpr int GROUPS = 4, PHASES = GROUPS / T;         // the PHASES groups of a tile take its stages in turn
   static constexpr int A_COLS = KB / 2;                         // tensor-memory columns of one A slot
   static constexpr int ACC_BUFS = T * CC * 2 + GROUPS * 2 * A_COLS <= 512 ? 2 : 1;
@@ -40,7 +41,7 @@ struct TaCfg {
   static constexpr uint32_t EP_OFFSET = BAR_OFFSET + 1024;                // 2 * CC floats of epilogue scale / shift
   static constexpr uint32_t STATS_OFFSET = EP_OFFSET + 2 * CC * 4;        // per-warp channel statistics, 4 * 2 * CC floats
   static constexpr uint32_t SMEM = STATS_OFFSET + 4 * 2 * CC * 4;
-  static_assert(CR * OPS == KB * NKB && (OPS == 1 || (PHASES == 1 && CC <= 64)), "stages");
+  static_assert(CR * OPS == KB * NKB && (OPS == 1 || CC <= 64), "stages");
   static_assert(FIT >= 2 && BARRIERS * 8 + 4 <= 1024, "tensor / shared memory");
 };
 
@@ -64,10 +65,13 @@ __device__ __forceinline__ constexpr uint32_t n_channel(uint32_t p) {
 // 64 bytes per reduction position and 64-column atom, 16-byte chunk c of line p at swz(p, c)). Where a stage has two
 // offsets their lines follow one another; the second half of an odd last stage is zero. One thread per chunk.
 // transpose: w is [K][CC][CR] (input gradient); reverse: offset k of the image is W[K - 1 - k].
+template <int CC>
+constexpr int ta_tiles() { return CC <= 64 ? 4 : (CC <= 128 ? 2 : 1); }
+
 template <int CR, int CC>
 __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, int transpose, int reverse,
                                                       uint4* __restrict__ image) {
-  using C = TaCfg<CR, CC>;
+  using C = TaCfg<CR, CC, ta_tiles<CC>()>;
   constexpr int KB = C::KB, NBLK = CC < 64 ? CC : 64, CPL = NBLK / 8, CHUNKS = KB * CC / 8;
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (i >= (uint32_t)((K + C::OPS - 1) / C::OPS) * C::NKB * CHUNKS) return;
@@ -126,13 +130,14 @@ struct RowBlock {
 // (tile, offset) pairs take no gather, no slot and no MMA, offsets that no tile of the super-tile has no copy of W[k].
 // kStats: the epilogue also accumulates, per output channel, the sum and the sum of squares of the values it stores
 // and writes them to stats_partial[blockIdx.x][2][CC].
-template <int CR, int CC, bool kStats, bool kPlan>
+// The columns [CC * blockIdx.y, CC * (blockIdx.y + 1)) of n_cols are computed.
+template <int CR, int CC, int T_, bool kStats, bool kPlan>
 __global__ void __launch_bounds__(kTaThreads, 1)
     k_conv_ta(const __nv_bfloat16* __restrict__ src, const uint8_t* __restrict__ image, const int32_t* __restrict__ nbr,
               uint32_t n_dst, int K, __nv_bfloat16* __restrict__ out, uint32_t n_super, const float* __restrict__ ep_scale,
-              const float* __restrict__ ep_shift, int ep_relu, float* __restrict__ stats_partial,
+              const float* __restrict__ ep_shift, int ep_relu, uint32_t n_cols, float* __restrict__ stats_partial,
               const int32_t* __restrict__ perm, const uint32_t* __restrict__ tile_mask) {
-  using C = TaCfg<CR, CC>;
+  using C = TaCfg<CR, CC, T_>;
   constexpr int KB = C::KB, NKB = C::NKB, OPS = C::OPS, T = C::T, G = C::GROUPS, PH = C::PHASES, SLOTS = C::SLOTS, BST = C::B_STAGES;
   constexpr int KSTEP = PH > NKB ? PH / NKB : 1;  // every KSTEP-th offset belongs to one group of a tile ...
   constexpr int NB = NKB > PH ? NKB / PH : 1;     // ... with NB of its channel blocks, PH apart
@@ -148,13 +153,15 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   uint64_t* acc_empty = acc_full + C::ACC_BUFS * T;  // [buffer][tile]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + C::ACC_BUFS * T);
   float* s_ep = reinterpret_cast<float*>(smem + C::EP_OFFSET);  // per-channel scale | shift
+  static_assert(KSTEP <= 2 || !kPlan, "planned tiles count their offsets modulo 2");
+  const uint32_t col0 = blockIdx.y * CC;
   const int n_off = (K + OPS - 1) / OPS;  // offsets, or pairs of them
   const bool has_ep = ep_scale != nullptr || ep_shift != nullptr || ep_relu != 0;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (has_ep && tid < CC) {
-    s_ep[tid] = ep_scale ? __ldg(ep_scale + tid) : 1.f;
-    s_ep[CC + tid] = ep_shift ? __ldg(ep_shift + tid) : 0.f;
+    s_ep[tid] = ep_scale ? __ldg(ep_scale + col0 + tid) : 1.f;
+    s_ep[CC + tid] = ep_shift ? __ldg(ep_shift + col0 + tid) : 0.f;
   }
   if (tid == 0) {
     for (int s = 0; s < BST; ++s) {
@@ -189,7 +196,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     // Stages of a tile are its (offset, channel block) pairs in order; group g takes every PH-th one from g / T on. A warp
     // fills the 32 lanes of tensor memory it may access with its 32 rows of the tile.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTaGatherRegs));
-    const int g = warp >> 2, t = g % T, k_first = (g / T) / NKB;
+    const int g = warp >> 2, t = g % T, k_first = (g / T) / NKB * OPS;
     const __nv_bfloat16* src_lane = src + ((g / T) % NKB) * KB + ((lane >> 1) & 1) * 16;
     const uint32_t a_base = tmem_base + C::ACC_COLS + g * SLOTS * C::A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t bars = smem_u32(a_full + g * SLOTS);  // full barriers; the empty ones lie G * SLOTS further
@@ -342,7 +349,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
             if constexpr (kPlan) {
               if (!((m[t] >> k) & 1u)) continue;
             }
-            const uint32_t g = t + T * (KSTEP > 1 ? ((odd >> t) & 1u) * NKB + kb : kb % PH);
+            const uint32_t g = t + T * (KSTEP > 1 ? (kPlan ? (odd >> t) & 1u : (uint32_t)k % KSTEP) * NKB + kb : kb % PH);
             const uint32_t c = (cnts >> (8 * g)) & 7u, s = c % SLOTS;
             const uint32_t begun = (started >> t) & 1u;
             if (!mbar_wait(&a_full[g * SLOTS + s], (c / SLOTS) & 1u)) { timed_out = true; goto mma_done; }
@@ -359,7 +366,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
             tc_commit_elect(&a_empty[g * SLOTS + s]);
             cnts = (cnts + (1u << (8 * g))) & 0x07070707u;
             started |= 1u << t;
-            if (KSTEP > 1 && kb == NKB - 1) odd ^= 1u << t;
+            if (kPlan && KSTEP > 1 && kb == NKB - 1) odd ^= 1u << t;
           }
           tc_commit_elect(&b_empty[bs]);
         }
@@ -390,7 +397,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
           for (int kb = 0; kb < NKB; ++kb, ++b_it) {
             const uint32_t s = b_it % BST;
             if (!mbar_wait(&b_empty[s], ((b_it / BST) & 1u) ^ 1u)) { timed_out = true; break; }
-            bulk_load(smem_base + s * C::B_BYTES, image + (size_t)(k * NKB + kb) * C::B_BYTES, C::B_BYTES,
+            bulk_load(smem_base + s * C::B_BYTES, image + ((size_t)(k * NKB + kb) * n_cols + col0) * (KB * 2), C::B_BYTES,
                       smem_u32(&b_full[s]));
           }
         }
@@ -468,12 +475,12 @@ __global__ void __launch_bounds__(kTaThreads, 1)
               }
             }
             if (rows[2 * h] != 0xFFFFFFFFu) {
-              uint4* d = reinterpret_cast<uint4*>(out + (size_t)rows[2 * h] * CC + ch);
+              uint4* d = reinterpret_cast<uint4*>(out + (size_t)rows[2 * h] * n_cols + col0 + ch);
 #pragma unroll
               for (int v = 0; v < NW / 4; ++v) d[v] = make_uint4(w0[4 * v], w0[4 * v + 1], w0[4 * v + 2], w0[4 * v + 3]);
             }
             if (rows[2 * h + 1] != 0xFFFFFFFFu) {
-              uint4* d = reinterpret_cast<uint4*>(out + (size_t)rows[2 * h + 1] * CC + ch);
+              uint4* d = reinterpret_cast<uint4*>(out + (size_t)rows[2 * h + 1] * n_cols + col0 + ch);
 #pragma unroll
               for (int v = 0; v < NW / 4; ++v) d[v] = make_uint4(w1[4 * v], w1[4 * v + 1], w1[4 * v + 2], w1[4 * v + 3]);
             }
@@ -508,7 +515,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps, added in warp order
       const float* all = reinterpret_cast<const float*>(smem + C::STATS_OFFSET);
       for (int c = (int)(quad * 32) + lane; c < 2 * CC; c += 128)
-        stats_partial[(size_t)blockIdx.x * 2 * CC + c] = all[c] + all[2 * CC + c] + all[4 * CC + c] + all[6 * CC + c];
+        stats_partial[((size_t)blockIdx.x * 2 + c / CC) * n_cols + col0 + c % CC] = all[c] + all[2 * CC + c] + all[4 * CC + c] + all[6 * CC + c];
     }
   }
 
@@ -522,12 +529,12 @@ __global__ void __launch_bounds__(kTaThreads, 1)
 }
 
 // grid_out receives the number of CTAs, i.e. of [2][CC] partials written to stats_partial.
-template <int CR, int CC, bool kStats, bool kPlan>
+template <int CR, int CC, int T, bool kStats, bool kPlan>
 int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, void* out, const float* ep_scale,
-              const float* ep_shift, int ep_relu, cudaStream_t stream, float* stats_partial, uint32_t* grid_out,
-              const void* plan) {
-  using C = TaCfg<CR, CC>;
-  auto kern = k_conv_ta<CR, CC, kStats, kPlan>;
+              const float* ep_shift, int ep_relu, uint32_t n_cols, int sms, cudaStream_t stream, float* stats_partial,
+              uint32_t* grid_out, const void* plan) {
+  using C = TaCfg<CR, CC, T>;
+  auto kern = k_conv_ta<CR, CC, T, kStats, kPlan>;
   const int32_t* perm = nullptr;
   const uint32_t* tile_mask = nullptr;
   if constexpr (kPlan) {
@@ -540,14 +547,12 @@ int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n
   }
   static SmemOptIn opt_in;
   RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(kern), C::SMEM));
-  int dev = 0, sms = 148;
-  RMN_CUDA_TRY(cudaGetDevice(&dev));
-  RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const uint32_t n_super = (n_dst + kTileM * C::T - 1) / (kTileM * C::T);
-  const uint32_t grid = (uint32_t)sms < n_super ? (uint32_t)sms : n_super;  // one CTA per SM owns its tensor memory
-  kern<<<grid, kTaThreads, C::SMEM, stream>>>((const __nv_bfloat16*)src, (const uint8_t*)image, nbr, n_dst, K,
-                                             (__nv_bfloat16*)out, n_super, ep_scale, ep_shift, ep_relu, stats_partial, perm,
-                                             tile_mask);
+  const uint32_t n_blocks = n_cols / CC, fit = (uint32_t)sms > n_blocks ? (uint32_t)sms / n_blocks : 1u;
+  const uint32_t grid = fit < n_super ? fit : n_super;  // one CTA per SM owns its tensor memory
+  kern<<<dim3(grid, n_blocks), kTaThreads, C::SMEM, stream>>>((const __nv_bfloat16*)src, (const uint8_t*)image, nbr, n_dst, K,
+                                             (__nv_bfloat16*)out, n_super, ep_scale, ep_shift, ep_relu, n_cols, stats_partial,
+                                             perm, tile_mask);
   RMN_LAUNCH_CHECK();
   count_tc_launch();
   if (grid_out) *grid_out = grid;
@@ -557,7 +562,7 @@ int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n
 // K rounded up to whole stages, times the bytes of one offset's weights
 template <int CR, int CC>
 size_t image_bytes(int K) {
-  using C = TaCfg<CR, CC>;
+  using C = TaCfg<CR, CC, ta_tiles<CC>()>;
   return (size_t)((K + C::OPS - 1) / C::OPS) * C::NKB * C::B_BYTES;
 }
 
@@ -594,22 +599,47 @@ int ta_weight_image(const void* w, int K, int c_red, int c_col, int transpose, i
   return RMN_ERR_UNSUPPORTED;
 }
 
+// Whether to run single row tiles and 64-column blocks, not super-tiles of all columns. Super-tiles share a copy of W[k] and
+// a gathered row among all columns, but few of them leave SMs idle: the time goes with the tiles of the busiest SM, a
+// tile on its own costing about 30 % more, and one of more than 128 columns 60 % more than one of 64.
+bool ta_small(uint32_t n_dst, int c_col, int sms) {
+  const uint32_t tiles = (n_dst + tc::kTileM - 1) / tc::kTileM, t = c_col <= 64 ? 4u : c_col <= 128 ? 2u : 1u;
+  const uint32_t blocks = c_col <= 64 ? 1u : (uint32_t)c_col / 64, fit = (uint32_t)sms > blocks ? (uint32_t)sms / blocks : 1u;
+  const uint32_t supers = (tiles + t - 1) / t;
+  const uint32_t whole = (supers + sms - 1) / sms * t * (c_col > 128 ? 16u : 10u), single = (tiles + fit - 1) / fit * 13u;
+  return single < whole;
+}
+
 // stats_partial != nullptr: also leave per-CTA channel statistics ([*n_partials][2][c_col] floats)
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, int ep_relu, float* stats_partial, uint32_t* n_partials,
             cudaStream_t stream, const void* plan) {
+  int dev = 0, sms = 148;
+  RMN_CUDA_TRY(cudaGetDevice(&dev));
+  RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+#define RMN_TA_ARGS \
+  src, image, nbr, n_dst, K, out, ep_scale, ep_shift, ep_relu, (uint32_t)c_col, sms, stream, stats_partial, n_partials, plan
+  if (ta_small(n_dst, c_col, sms)) {
+    plan = nullptr;
+#define RMN_TA_CASE(R, Cc)                                                                   \
+  if (c_red == R && (Cc == 32 ? c_col == 32 : c_col != 32))                                  \
+    return stats_partial ? tc::launch_ta<R, Cc, 1, true, false>(RMN_TA_ARGS)                 \
+                         : tc::launch_ta<R, Cc, 1, false, false>(RMN_TA_ARGS);
+    RMN_TA_CASE(32, 32) RMN_TA_CASE(32, 64) RMN_TA_CASE(64, 32) RMN_TA_CASE(64, 64) RMN_TA_CASE(128, 64) RMN_TA_CASE(256, 64)
+#undef RMN_TA_CASE
+  }
   // A plan pays where a skipped tile saves more MMA time than the gather of its rows takes anyway: from 128 x 128 channels
   // on (1.2 M rows: 128->128 716 -> 645 us, but 64->64 281 -> 288, 32->64 221 -> 249). The rows come out the same.
-#define RMN_TA_ARGS src, image, nbr, n_dst, K, out, ep_scale, ep_shift, ep_relu, stream, stats_partial, n_partials, plan
-#define RMN_TA_CASE(R, Cc)                                                                                            \
-  if (c_red == R && c_col == Cc) {                                                                                    \
-    if constexpr (R * Cc >= kPlanMinWeight) {                                                                         \
-      if (plan && K <= kPlanMaxK)                                                                                     \
-        return stats_partial ? tc::launch_ta<R, Cc, true, true>(RMN_TA_ARGS)                                          \
-                             : tc::launch_ta<R, Cc, false, true>(RMN_TA_ARGS);                                        \
-    }                                                                                                                 \
-    return stats_partial ? tc::launch_ta<R, Cc, true, false>(RMN_TA_ARGS)                                             \
-                         : tc::launch_ta<R, Cc, false, false>(RMN_TA_ARGS);                                           \
+#define RMN_TA_CASE(R, Cc)                                                                       \
+  if (c_red == R && c_col == Cc) {                                                               \
+    constexpr int T = tc::ta_tiles<Cc>();                                                        \
+    if constexpr (R * Cc >= kPlanMinWeight) {                                                    \
+      if (plan && K <= kPlanMaxK)                                                                \
+        return stats_partial ? tc::launch_ta<R, Cc, T, true, true>(RMN_TA_ARGS)                  \
+                             : tc::launch_ta<R, Cc, T, false, true>(RMN_TA_ARGS);                \
+    }                                                                                            \
+    return stats_partial ? tc::launch_ta<R, Cc, T, true, false>(RMN_TA_ARGS)                     \
+                         : tc::launch_ta<R, Cc, T, false, false>(RMN_TA_ARGS);                   \
   }
   RMN_TA_SHAPES(RMN_TA_CASE)
 #undef RMN_TA_CASE

@@ -1,5 +1,5 @@
 """bf16 convolution on prepared weights (gathered operand in tensor memory) against a float64 reference: every channel
-pair, row counts around one 128-row tile and around a super-tile, even and odd numbers of offsets, transposed and
+pair, row counts around one 128-row tile and around those that fill the SMs, even and odd numbers of offsets, transposed and
 reversed weights, epilogue and channel statistics."""
 import pytest
 import torch
@@ -24,7 +24,7 @@ def _close(got, want):
 
 @pytest.mark.parametrize("c_in,c_out", SHAPES)
 @pytest.mark.parametrize("n,K,fill", [(1, 1, 1.0), (127, 2, 0.5), (129, 27, 0.4), (513, 8, 1.0), (1030, 5, 0.01),
-                                      (100_003, 3, 0.5)])
+                                      (75_775, 2, 0.5), (100_003, 3, 0.5), (150_001, 3, 0.5)])
 def test_image_passes_match_float64(c_in, c_out, n, K, fill):
     from riemannengine_b200 import capi, ops
     assert capi.lib().rmn_conv_weight_image_bytes(K, c_in, c_out, capi.BF16) > 0
