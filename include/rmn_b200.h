@@ -382,19 +382,32 @@ int rmn_conv_transpose_weights(const void *d_weights, int K, int c_in, int c_out
 /*
  * Prepared weights for the fastest bf16 kernels. rmn_conv_weight_image_bytes: size of the image of [K, c_in, c_out]
  * weights, 0 when no such kernel covers the dtype and channel counts (use the plain entry points then).
- * rmn_conv_weight_image builds it (one small kernel); transpose != 0 makes the image of the transposed weights, for
+ * rmn_conv_weight_image builds it (one small kernel) from [K, w_in, w_out] weights, w_in <= c_in and w_out <= c_out: the
+ * other channels are zero, so that narrower layers run on padded features (rmn_pad_channels). transpose != 0 makes the image of the transposed weights, for
  * rmn_conv_forward_image to compute the input gradient from grad_out (c_in and c_out exchanged there); reverse != 0
  * exchanges offsets k and K - 1 - k, for the input gradient of a point-symmetric self map over its own forward table.
+ * fold (may be NULL; not with transpose): also turn a batch norm in evaluation mode into the scale and shift vectors
+ * [c_out] of the epilogue (an absent conv_bias, gamma or beta is NULL).
  * rmn_conv_forward_image: rmn_conv_forward_planned with an image in place of the weights (bf16; d_feats 32-byte
- * aligned, d_image and d_out 16-byte aligned). rmn_conv_forward_image_stats: also the channel statistics of
+ * aligned, d_image, d_add and d_out 16-byte aligned); d_add (may be NULL): [n_dst, c_out], added behind scale and
+ * shift, before the ReLU (a residual connection). rmn_conv_forward_image_stats: also the channel statistics of
  * rmn_conv_forward_stats.
  */
 size_t rmn_conv_weight_image_bytes(int K, int c_in, int c_out, int dtype);
-int rmn_conv_weight_image(const void *d_weights, int K, int c_in, int c_out, int dtype, int transpose, int reverse,
-                          void *d_image, void *stream);
+typedef struct {
+  const void *mean, *var, *gamma, *beta, *conv_bias;  /* device, [w_out], param_dtype */
+  int param_dtype;
+  float eps;
+  float *scale, *shift;                               /* device, [c_out], written */
+} rmn_bn_fold;
+int rmn_conv_weight_image(const void *d_weights, int K, int w_in, int w_out, int c_in, int c_out, int dtype, int transpose,
+                          int reverse, const rmn_bn_fold *fold, void *d_image, void *stream);
 int rmn_conv_forward_image(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
                            const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out, const float *d_scale,
-                           const float *d_shift, int relu, void *stream);
+                           const float *d_shift, const void *d_add, int relu, void *stream);
+/* d_dst [n_rows, c_dst] = d_src [n_rows, c_src] with c_dst - c_src zero channels behind (bf16; c_dst a multiple of 8,
+ * d_dst 16-byte aligned). */
+int rmn_pad_channels(const void *d_src, uint32_t n_rows, int c_src, void *d_dst, int c_dst, void *stream);
 int rmn_conv_forward_image_stats(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
                                  const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out,
                                  const float *d_scale, const float *d_shift, int relu, double *d_stats, void *d_workspace,

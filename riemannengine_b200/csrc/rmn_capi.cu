@@ -17,10 +17,11 @@ int tc_conv(const void* src, uint32_t n_src, const void* w, const int32_t* nbr, 
             int c_col, bool transposed_weights, void* out, const float* ep_scale, const float* ep_shift, int ep_relu,
             cudaStream_t stream, const void* plan);
 size_t ta_image_bytes(int K, int c_red, int c_col);
-int ta_weight_image(const void* w, int K, int c_red, int c_col, int transpose, int reverse, void* image, cudaStream_t stream);
+int ta_weight_image(const void* w, int K, int w_red, int w_col, int c_red, int c_col, int transpose, int reverse,
+                    const rmn_bn_fold& fold, void* image, cudaStream_t stream);
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
-            const float* ep_scale, const float* ep_shift, int ep_relu, float* stats_partial, uint32_t* n_partials,
-            cudaStream_t stream, const void* plan);
+            const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial,
+            uint32_t* n_partials, cudaStream_t stream, const void* plan);
 int tc_read_status(cudaStream_t stream, uint32_t* status);
 unsigned long long tc_launch_count();
 int tc_conv_wgrad(const void* feats, const void* grad_out, const int32_t* nbr, uint32_t n_dst, int K, int c_in,
@@ -111,22 +112,30 @@ extern "C" size_t rmn_conv_weight_image_bytes(int K, int c_in, int c_out, int dt
   return plain > transposed ? plain : transposed;  // (both orders of every pair have a kernel)
 }
 
-extern "C" int rmn_conv_weight_image(const void* d_weights, int K, int c_in, int c_out, int dtype, int transpose, int reverse,
-                                     void* d_image, void* stream_) {
+extern "C" int rmn_conv_weight_image(const void* d_weights, int K, int w_in, int w_out, int c_in, int c_out, int dtype,
+                                     int transpose, int reverse, const rmn_bn_fold* fold, void* d_image, void* stream_) {
   if (!d_weights || !d_image || K < 1 || K > 65535 || ((uintptr_t)d_image & 15)) return RMN_ERR_BAD_ARG;
+  if (w_in < 1 || w_in > c_in || w_out < 1 || w_out > c_out) return RMN_ERR_BAD_ARG;
+  rmn_bn_fold f = {};
+  if (fold) {
+    f = *fold;
+    if (transpose || !f.scale || !f.shift || (f.param_dtype != RMN_F32 && f.param_dtype != RMN_BF16)) return RMN_ERR_BAD_ARG;
+  }
   if (rmn_conv_weight_image_bytes(K, c_in, c_out, dtype) == 0) return RMN_ERR_UNSUPPORTED;
-  return transpose ? ta_weight_image(d_weights, K, c_out, c_in, 1, reverse, d_image, (cudaStream_t)stream_)
-                   : ta_weight_image(d_weights, K, c_in, c_out, 0, reverse, d_image, (cudaStream_t)stream_);
+  return transpose ? ta_weight_image(d_weights, K, w_out, w_in, c_out, c_in, 1, reverse, f, d_image, (cudaStream_t)stream_)
+                   : ta_weight_image(d_weights, K, w_in, w_out, c_in, c_out, 0, reverse, f, d_image, (cudaStream_t)stream_);
 }
 
 extern "C" int rmn_conv_forward_image(const void* d_feats, uint32_t n_src, int c_in, const void* d_image, int K, int c_out,
                                       const int32_t* d_nbr, const void* d_plan, uint32_t n_dst, void* d_out,
-                                      const float* d_scale, const float* d_shift, int relu, void* stream_) {
+                                      const float* d_scale, const float* d_shift, const void* d_add, int relu,
+                                      void* stream_) {
   if (n_dst == 0) return RMN_OK;
   // (with no source rows every table entry is -1 and nothing is read through d_feats)
   if (!d_image || !d_nbr || !d_out || (n_src > 0 && !d_feats) || K < 1 || K > 65535) return RMN_ERR_BAD_ARG;
-  if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_image & 15) || ((uintptr_t)d_out & 15)) return RMN_ERR_BAD_ARG;
-  return ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, relu, nullptr, nullptr,
+  if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_image & 15) || ((uintptr_t)d_out & 15) || ((uintptr_t)d_add & 15))
+    return RMN_ERR_BAD_ARG;
+  return ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, d_add, relu, nullptr, nullptr,
                  (cudaStream_t)stream_, d_plan);
 }
 

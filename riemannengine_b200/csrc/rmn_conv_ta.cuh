@@ -64,13 +64,27 @@ __device__ __forceinline__ constexpr uint32_t n_channel(uint32_t p) {
 // The weight image: per offset and KB-channel block, the MN-major swizzled operand image of the stage (one line of 128 or
 // 64 bytes per reduction position and 64-column atom, 16-byte chunk c of line p at swz(p, c)). Where a stage has two
 // offsets their lines follow one another; the second half of an odd last stage is zero. One thread per chunk.
-// transpose: w is [K][CC][CR] (input gradient); reverse: offset k of the image is W[K - 1 - k].
+// w has w_red <= CR and w_col <= CC channels, the rest is zero. transpose: w is [K][w_col][w_red] (input gradient);
+// reverse: offset k of the image is W[K - 1 - k]. Block 0 also turns the batch norm of `fold` into epilogue scale and shift.
 template <int CC>
 constexpr int ta_tiles() { return CC <= 64 ? 4 : (CC <= 128 ? 2 : 1); }
 
 template <int CR, int CC>
-__global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, int transpose, int reverse,
+__global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, uint32_t w_red,
+                                                      uint32_t w_col, int transpose, int reverse, rmn_bn_fold fold,
                                                       uint4* __restrict__ image) {
+  if (fold.scale && blockIdx.x == 0) {
+    for (uint32_t c = threadIdx.x; c < CC; c += 256) {
+      auto param = [&](const void* p, float absent) {
+        if (!p || c >= w_col) return absent;
+        return fold.param_dtype == RMN_F32 ? static_cast<const float*>(p)[c]
+                                           : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[c]);
+      };
+      const float s = param(fold.gamma, 1.f) / sqrtf(param(fold.var, 1.f) + fold.eps);
+      fold.scale[c] = s;
+      fold.shift[c] = param(fold.beta, 0.f) + (param(fold.conv_bias, 0.f) - param(fold.mean, 0.f)) * s;
+    }
+  }
   using C = TaCfg<CR, CC, ta_tiles<CC>()>;
   constexpr int KB = C::KB, NBLK = CC < 64 ? CC : 64, CPL = NBLK / 8, CHUNKS = KB * CC / 8;
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
@@ -79,7 +93,7 @@ __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __res
   const uint32_t atom = r / (KB * CPL), p = (r / CPL) % KB, c = r % CPL;
   const uint32_t ci = k_channel(C::OPS > 1 ? p % CR : stage % C::NKB * KB + p);
   const int k = (int)(C::OPS > 1 ? stage * C::OPS + p / CR : stage / C::NKB);
-  const __nv_bfloat16* wk = w + (size_t)(reverse ? K - 1 - k : k) * CR * CC;
+  const __nv_bfloat16* wk = w + (size_t)(reverse ? K - 1 - k : k) * w_red * w_col;
   uint32_t v[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -87,7 +101,9 @@ __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __res
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const uint32_t co = atom * NBLK + n_channel<NBLK>(c * 8 + q * 2 + h);
-      e[h] = k >= K ? (uint16_t)0 : *reinterpret_cast<const uint16_t*>(transpose ? wk + (size_t)co * CR + ci : wk + (size_t)ci * CC + co);
+      e[h] = k >= K || ci >= w_red || co >= w_col
+                 ? (uint16_t)0
+                 : *reinterpret_cast<const uint16_t*>(wk + (transpose ? (size_t)co * w_red + ci : (size_t)ci * w_col + co));
     }
     v[q] = e[0] | ((uint32_t)e[1] << 16);
   }
@@ -135,7 +151,7 @@ template <int CR, int CC, int T_, bool kStats, bool kPlan>
 __global__ void __launch_bounds__(kTaThreads, 1)
     k_conv_ta(const __nv_bfloat16* __restrict__ src, const uint8_t* __restrict__ image, const int32_t* __restrict__ nbr,
               uint32_t n_dst, int K, __nv_bfloat16* __restrict__ out, uint32_t n_super, const float* __restrict__ ep_scale,
-              const float* __restrict__ ep_shift, int ep_relu, uint32_t n_cols, float* __restrict__ stats_partial,
+              const float* __restrict__ ep_shift, const __nv_bfloat16* __restrict__ ep_add, int ep_relu, uint32_t n_cols, float* __restrict__ stats_partial,
               const int32_t* __restrict__ perm, const uint32_t* __restrict__ tile_mask) {
   using C = TaCfg<CR, CC, T_>;
   constexpr int KB = C::KB, NKB = C::NKB, OPS = C::OPS, T = C::T, G = C::GROUPS, PH = C::PHASES, SLOTS = C::SLOTS, BST = C::B_STAGES;
@@ -156,7 +172,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   static_assert(KSTEP <= 2 || !kPlan, "planned tiles count their offsets modulo 2");
   const uint32_t col0 = blockIdx.y * CC;
   const int n_off = (K + OPS - 1) / OPS;  // offsets, or pairs of them
-  const bool has_ep = ep_scale != nullptr || ep_shift != nullptr || ep_relu != 0;
+  const bool has_ep = ep_scale != nullptr || ep_shift != nullptr || ep_add != nullptr || ep_relu != 0;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (has_ep && tid < CC) {
@@ -441,7 +457,19 @@ __global__ void __launch_bounds__(kTaThreads, 1)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const uint32_t taddr = tmem_base + ((quad * 32u + h * 16u) << 16) + (buf * T + t) * CC + nb * NBLK;
-            uint32_t w0[NW], w1[NW];  // rows 2 h and 2 h + 1
+            uint32_t w0[NW], w1[NW];  // rows 2 h and 2 h + 1: first what is added to them, then the result
+            if (ep_add) {
+              auto fetch = [&](uint32_t row, uint32_t (&w)[NW]) {
+                const uint4* a = reinterpret_cast<const uint4*>(ep_add + (size_t)row * n_cols + col0 + ch);
+#pragma unroll
+                for (int v = 0; v < NW / 4; ++v) {
+                  const uint4 x = row != 0xFFFFFFFFu ? __ldg(a + v) : make_uint4(0u, 0u, 0u, 0u);
+                  w[4 * v] = x.x, w[4 * v + 1] = x.y, w[4 * v + 2] = x.z, w[4 * v + 3] = x.w;
+                }
+              };
+              fetch(rows[2 * h], w0);
+              fetch(rows[2 * h + 1], w1);
+            }
 #pragma unroll
             for (int q = 0; q < NBLK / 32; ++q) {
               uint32_t r[16];
@@ -464,6 +492,11 @@ __global__ void __launch_bounds__(kTaThreads, 1)
                   f[1] = fmaf(f[1], sc.y, sh.y);
                   f[2] = fmaf(f[2], sc.x, sh.x);
                   f[3] = fmaf(f[3], sc.y, sh.y);
+                  if (ep_add) {
+                    const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w0[q * 4 + gg]));
+                    const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w1[q * 4 + gg]));
+                    f[0] += a0.x, f[1] += a0.y, f[2] += a1.x, f[3] += a1.y;
+                  }
                   if (ep_relu) {
 #pragma unroll
                     for (int v = 0; v < 4; ++v) f[v] = fmaxf(f[v], 0.f);
@@ -531,7 +564,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
 // grid_out receives the number of CTAs, i.e. of [2][CC] partials written to stats_partial.
 template <int CR, int CC, int T, bool kStats, bool kPlan>
 int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, void* out, const float* ep_scale,
-              const float* ep_shift, int ep_relu, uint32_t n_cols, int sms, cudaStream_t stream, float* stats_partial,
+              const float* ep_shift, const void* ep_add, int ep_relu, uint32_t n_cols, int sms, cudaStream_t stream, float* stats_partial,
               uint32_t* grid_out, const void* plan) {
   using C = TaCfg<CR, CC, T>;
   auto kern = k_conv_ta<CR, CC, T, kStats, kPlan>;
@@ -551,7 +584,8 @@ int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n
   const uint32_t n_blocks = n_cols / CC, fit = (uint32_t)sms > n_blocks ? (uint32_t)sms / n_blocks : 1u;
   const uint32_t grid = fit < n_super ? fit : n_super;  // one CTA per SM owns its tensor memory
   kern<<<dim3(grid, n_blocks), kTaThreads, C::SMEM, stream>>>((const __nv_bfloat16*)src, (const uint8_t*)image, nbr, n_dst, K,
-                                             (__nv_bfloat16*)out, n_super, ep_scale, ep_shift, ep_relu, n_cols, stats_partial,
+                                             (__nv_bfloat16*)out, n_super, ep_scale, ep_shift,
+                                             (const __nv_bfloat16*)ep_add, ep_relu, n_cols, stats_partial,
                                              perm, tile_mask);
   RMN_LAUNCH_CHECK();
   count_tc_launch();
@@ -567,10 +601,11 @@ size_t image_bytes(int K) {
 }
 
 template <int CR, int CC>
-int launch_image(const void* w, int K, int transpose, int reverse, void* image, cudaStream_t stream) {
+int launch_image(const void* w, int K, int w_red, int w_col, int transpose, int reverse, const rmn_bn_fold& fold, void* image,
+                 cudaStream_t stream) {
   const uint32_t chunks = (uint32_t)(image_bytes<CR, CC>(K) / 16);
-  k_weight_image<CR, CC><<<(chunks + 255) / 256, 256, 0, stream>>>((const __nv_bfloat16*)w, K, transpose, reverse,
-                                                                  (uint4*)image);
+  k_weight_image<CR, CC><<<(chunks + 255) / 256, 256, 0, stream>>>((const __nv_bfloat16*)w, K, w_red, w_col, transpose,
+                                                                  reverse, fold, (uint4*)image);
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -590,10 +625,11 @@ size_t ta_image_bytes(int K, int c_red, int c_col) {
   return 0;
 }
 
-// image of [K][c_red][c_col] weights (transpose: given as [K][c_col][c_red])
-int ta_weight_image(const void* w, int K, int c_red, int c_col, int transpose, int reverse, void* image, cudaStream_t stream) {
+// image of c_red x c_col products of [K][w_red][w_col] weights (transpose: given as [K][w_col][w_red])
+int ta_weight_image(const void* w, int K, int w_red, int w_col, int c_red, int c_col, int transpose, int reverse,
+                    const rmn_bn_fold& fold, void* image, cudaStream_t stream) {
 #define RMN_TA_CASE(R, Cc) \
-  if (c_red == R && c_col == Cc) return tc::launch_image<R, Cc>(w, K, transpose, reverse, image, stream);
+  if (c_red == R && c_col == Cc) return tc::launch_image<R, Cc>(w, K, w_red, w_col, transpose, reverse, fold, image, stream);
   RMN_TA_SHAPES(RMN_TA_CASE)
 #undef RMN_TA_CASE
   return RMN_ERR_UNSUPPORTED;
@@ -612,13 +648,13 @@ bool ta_small(uint32_t n_dst, int c_col, int sms) {
 
 // stats_partial != nullptr: also leave per-CTA channel statistics ([*n_partials][2][c_col] floats)
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
-            const float* ep_scale, const float* ep_shift, int ep_relu, float* stats_partial, uint32_t* n_partials,
+            const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial, uint32_t* n_partials,
             cudaStream_t stream, const void* plan) {
   int dev = 0, sms = 148;
   RMN_CUDA_TRY(cudaGetDevice(&dev));
   RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 #define RMN_TA_ARGS \
-  src, image, nbr, n_dst, K, out, ep_scale, ep_shift, ep_relu, (uint32_t)c_col, sms, stream, stats_partial, n_partials, plan
+  src, image, nbr, n_dst, K, out, ep_scale, ep_shift, ep_add, ep_relu, (uint32_t)c_col, sms, stream, stats_partial, n_partials, plan
   if (ta_small(n_dst, c_col, sms)) {
     plan = nullptr;
 #define RMN_TA_CASE(R, Cc)                                                                   \

@@ -17,8 +17,8 @@ int tc_conv_stats(const void* src, uint32_t n_src, const void* w, const int32_t*
                   float* stats_partial, uint32_t* n_partials, cudaStream_t stream, const void* plan);
 
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
-            const float* ep_scale, const float* ep_shift, int ep_relu, float* stats_partial, uint32_t* n_partials,
-            cudaStream_t stream, const void* plan);
+            const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial,
+            uint32_t* n_partials, cudaStream_t stream, const void* plan);
 
 constexpr uint32_t kMaxStatPartials = 1024;
 
@@ -196,8 +196,8 @@ extern "C" int rmn_conv_forward_image_stats(const void* d_feats, uint32_t n_src,
   if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_image & 15) || ((uintptr_t)d_out & 15)) return RMN_ERR_BAD_ARG;
   if (workspace_bytes < rmn_channel_stats_workspace_bytes(c_out)) return RMN_ERR_ALLOC;
   uint32_t n_partials = 0;
-  const int st = ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, relu, (float*)d_workspace,
-                         &n_partials, stream, d_plan);
+  const int st = ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, nullptr, relu,
+                         (float*)d_workspace, &n_partials, stream, d_plan);
   if (st != RMN_OK) return st;
   k_stats_reduce<<<(2 * c_out + 127) / 128, 128, 0, stream>>>((const float*)d_workspace, n_partials, c_out, d_stats);
   RMN_LAUNCH_CHECK();

@@ -260,8 +260,8 @@ def _weight_image(weights: torch.Tensor, transpose: bool, feats: torch.Tensor,
     if nbytes == 0 or feats.data_ptr() % 32:
         return None
     image = torch.empty(nbytes, dtype=torch.uint8, device=weights.device)
-    capi.check(capi.lib().rmn_conv_weight_image(_ptr(weights), K, c_in, c_out, _dtype_code(weights), int(transpose),
-                                                int(reverse), _ptr(image), _stream()), "rmn_conv_weight_image")
+    capi.check(capi.lib().rmn_conv_weight_image(_ptr(weights), K, c_in, c_out, c_in, c_out, _dtype_code(weights),
+                                                int(transpose), int(reverse), None, _ptr(image), _stream()), "rmn_conv_weight_image")
     return image
 
 
@@ -293,7 +293,7 @@ def conv_forward(feats: torch.Tensor, weights: torch.Tensor, nbr: torch.Tensor,
         if image is not None:
             capi.check(capi.lib().rmn_conv_forward_image(_ptr(feats), int(feats.size(0)), c_in, _ptr(image), K, c_out,
                                                          _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _ptr(sc), _ptr(sh),
-                                                         int(bool(relu)), _stream()), "rmn_conv_forward_image")
+                                                         None, int(bool(relu)), _stream()), "rmn_conv_forward_image")
             return out
         capi.check(capi.lib().rmn_conv_forward_planned(_ptr(feats), int(feats.size(0)), c_in, _ptr(weights), K, c_out,
                                                        _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _dtype_code(feats),
@@ -324,8 +324,8 @@ def conv_backward_input(grad_out: torch.Tensor, weights: torch.Tensor, nbr_t: to
         image = _weight_image(weights, True, grad_out) if n_src and grad_out.size(0) else None
         if image is not None:
             capi.check(capi.lib().rmn_conv_forward_image(_ptr(grad_out), int(grad_out.size(0)), c_out, _ptr(image), K,
-                                                         c_in, _ptr(nbr_t), _ptr(plan), n_src, _ptr(out), None, None, 0,
-                                                         _stream()), "rmn_conv_forward_image")
+                                                         c_in, _ptr(nbr_t), _ptr(plan), n_src, _ptr(out), None, None,
+                                                         None, 0, _stream()), "rmn_conv_forward_image")
             return out
         capi.check(capi.lib().rmn_conv_backward_input_planned(_ptr(grad_out), int(grad_out.size(0)), c_out,
                                                               _ptr(weights), K, c_in, _ptr(nbr_t), _ptr(plan), n_src,

@@ -986,97 +986,6 @@ void allreduce_gradients(const std::vector<at::Tensor>& gradients) {
 // ---------------------------------------------------------------------------------------------
 namespace {
 
-// The prepared weights of rmn_conv_forward_image, of [K, c_in, c_out] weights or (transpose) of their transposes;
-// undefined where no such kernel covers the shape and type, or the operand is not aligned for it.
-at::Tensor weight_image(const at::Tensor& kernel, bool transpose, bool reverse, const at::Tensor& operand) {
-  if (kernel.scalar_type() != at::kBFloat16 || reinterpret_cast<uintptr_t>(operand.data_ptr()) % 32 != 0) return at::Tensor();
-  const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(kernel.size(1)),
-            c_out = static_cast<int>(kernel.size(2));
-  const size_t bytes = transpose ? rmn_conv_weight_image_bytes(K, c_out, c_in, RMN_BF16)
-                                 : rmn_conv_weight_image_bytes(K, c_in, c_out, RMN_BF16);
-  if (bytes == 0) return at::Tensor();
-  auto image = at::empty({static_cast<int64_t>(bytes)}, kernel.options().dtype(at::kByte));
-  check(rmn_conv_weight_image(ptr(kernel), K, c_in, c_out, RMN_BF16, transpose ? 1 : 0, reverse ? 1 : 0, ptr(image),
-                              current_stream()),
-        "rmn_conv_weight_image");
-  return image;
-}
-
-// bias (if defined) is folded into the kernel's epilogue as a per-channel shift
-at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in, const at::Tensor& nbr,
-                        const at::Tensor& bias = at::Tensor(), const at::Tensor& scale_in = at::Tensor(),
-                        bool relu = false, const at::Tensor& plan = at::Tensor()) {
-  TORCH_CHECK(feats_in.is_cuda() && kernel_in.is_cuda(), "features and kernel must be CUDA tensors");
-  TORCH_CHECK(feats_in.scalar_type() == kernel_in.scalar_type(), "expected features and kernel to have the same dtype");
-  auto feats = feats_in.contiguous(), kernel = kernel_in.contiguous();
-  c10::cuda::CUDAGuard guard(feats.device());
-  const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(kernel.size(1)),
-            c_out = static_cast<int>(kernel.size(2));
-  auto out = at::empty({nbr.size(1), c_out}, feats.options());
-  at::Tensor shift;
-  if (bias.defined() && bias.numel() > 0) {
-    shift = bias.detach().reshape({-1}).to(at::kFloat).contiguous();
-    TORCH_CHECK(shift.numel() == c_out, "bias must have one entry per output channel");
-  }
-  at::Tensor scale;
-  if (scale_in.defined() && scale_in.numel() > 0) {
-    scale = scale_in.detach().reshape({-1}).to(at::kFloat).contiguous();
-    TORCH_CHECK(scale.numel() == c_out, "scale must have one entry per output channel");
-  }
-  if (feats.size(0) > 0 && nbr.size(1) > 0) {
-    if (auto image = weight_image(kernel, false, false, feats); image.defined()) {
-      check(rmn_conv_forward_image(ptr(feats), static_cast<uint32_t>(feats.size(0)), c_in, ptr(image), K, c_out,
-                                   static_cast<const int32_t*>(ptr(nbr)), ptr(plan), static_cast<uint32_t>(nbr.size(1)),
-                                   ptr(out), static_cast<const float*>(ptr(scale)), static_cast<const float*>(ptr(shift)),
-                                   relu ? 1 : 0, current_stream()),
-            "rmn_conv_forward_image");
-      return out;
-    }
-  }
-  check(rmn_conv_forward_planned(ptr(feats), static_cast<uint32_t>(feats.size(0)), c_in, ptr(kernel), K, c_out,
-                                 static_cast<const int32_t*>(ptr(nbr)), ptr(plan), static_cast<uint32_t>(nbr.size(1)),
-                                 ptr(out), dtype_code(feats),
-                                 scale.defined() ? static_cast<const float*>(ptr(scale)) : nullptr,
-                                 static_cast<const float*>(ptr(shift)), relu ? 1 : 0, current_stream()),
-        "rmn_conv_forward_planned");
-  return out;
-}
-
-// reverse: nbr_t is the forward table of a point-symmetric self map, i.e. its offsets run backwards
-at::Tensor conv_backward_input(const at::Tensor& grad_in, const at::Tensor& kernel_in, const at::Tensor& nbr_t,
-                               bool reverse, const at::Tensor& plan_t = at::Tensor()) {
-  auto grad = grad_in.contiguous();
-  c10::cuda::CUDAGuard guard(grad.device());
-  if (grad.scalar_type() == at::kFloat && grad.size(0) > 0 && nbr_t.size(1) > 0) {
-    // fp32: the forward pass on transposed weights
-    auto w = kernel_in.contiguous();
-    auto wt = at::empty({w.size(0), w.size(2), w.size(1)}, w.options());
-    check(rmn_conv_transpose_weights(ptr(w), static_cast<int>(w.size(0)), static_cast<int>(w.size(1)),
-                                     static_cast<int>(w.size(2)), RMN_F32, reverse ? 1 : 0, ptr(wt), current_stream()),
-          "rmn_conv_transpose_weights");
-    return conv_forward(grad, wt, nbr_t);
-  }
-  const int K = static_cast<int>(kernel_in.size(0)), c_in = static_cast<int>(kernel_in.size(1)),
-            c_out = static_cast<int>(kernel_in.size(2));
-  auto out = at::empty({nbr_t.size(1), c_in}, grad.options());
-  if (grad.size(0) > 0 && nbr_t.size(1) > 0) {
-    if (auto image = weight_image(kernel_in.contiguous(), true, reverse, grad); image.defined()) {
-      check(rmn_conv_forward_image(ptr(grad), static_cast<uint32_t>(grad.size(0)), c_out, ptr(image), K, c_in,
-                                   static_cast<const int32_t*>(ptr(nbr_t)), ptr(plan_t),
-                                   static_cast<uint32_t>(nbr_t.size(1)), ptr(out), nullptr, nullptr, 0, current_stream()),
-            "rmn_conv_forward_image");
-      return out;
-    }
-  }
-  auto kernel = reverse ? kernel_in.flip(0) : kernel_in.contiguous();
-  check(rmn_conv_backward_input_planned(ptr(grad), static_cast<uint32_t>(grad.size(0)), c_out, ptr(kernel), K, c_in,
-                                        static_cast<const int32_t*>(ptr(nbr_t)), ptr(plan_t),
-                                        static_cast<uint32_t>(nbr_t.size(1)), ptr(out), dtype_code(grad),
-                                        current_stream()),
-        "rmn_conv_backward_input_planned");
-  return out;
-}
-
 // (reduction channels, output channels) with a tensor-core forward / input-gradient kernel (csrc/rmn_conv_tc.cu);
 // the weight-gradient kernels cover the same pairs
 bool tc_forward_shape(int64_t c_red, int64_t c_col) {
@@ -1102,6 +1011,141 @@ std::pair<int64_t, int64_t> tc_legal_shape(int64_t c_in, int64_t c_out) {
   return best;
 }
 
+// bf16 features [n, c] with zero channels behind, up to `channels`
+at::Tensor pad_channels(const at::Tensor& x_in, int64_t channels) {
+  if (x_in.size(1) == channels) return x_in;
+  auto x = x_in.contiguous();
+  auto out = at::empty({x.size(0), channels}, x.options());
+  check(rmn_pad_channels(ptr(x), static_cast<uint32_t>(x.size(0)), static_cast<int>(x.size(1)), ptr(out),
+                         static_cast<int>(channels), current_stream()),
+        "rmn_pad_channels");
+  return out;
+}
+
+// bf16 channel counts without a tensor-core kernel (a 4-channel stem, 48 or 96 channels ...) run as the next pair that
+// has one: padded input channels multiply zero weights, padded output channels are cut off again.
+std::pair<int64_t, int64_t> run_shape(const at::Tensor& kernel) {
+  return kernel.scalar_type() == at::kBFloat16 ? tc_legal_shape(kernel.size(1), kernel.size(2))
+                                               : std::pair<int64_t, int64_t>{kernel.size(1), kernel.size(2)};
+}
+
+// The prepared weights of rmn_conv_forward_image, of [K, c_in, c_out] weights as the pair `shape` or (transpose) of their
+// transposes; undefined where no such kernel covers the shape and type, or the operand is not aligned for it.
+at::Tensor weight_image(const at::Tensor& kernel, std::pair<int64_t, int64_t> shape, bool transpose, bool reverse,
+                        const at::Tensor& operand, const rmn_bn_fold* fold = nullptr) {
+  if (kernel.scalar_type() != at::kBFloat16 || reinterpret_cast<uintptr_t>(operand.data_ptr()) % 32 != 0) return at::Tensor();
+  const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(shape.first),
+            c_out = static_cast<int>(shape.second);
+  const size_t bytes = rmn_conv_weight_image_bytes(K, c_in, c_out, RMN_BF16);
+  if (bytes == 0) return at::Tensor();
+  auto image = at::empty({static_cast<int64_t>(bytes)}, kernel.options().dtype(at::kByte));
+  check(rmn_conv_weight_image(ptr(kernel), K, static_cast<int>(kernel.size(1)), static_cast<int>(kernel.size(2)), c_in, c_out,
+                              RMN_BF16, transpose ? 1 : 0, reverse ? 1 : 0, fold, ptr(image), current_stream()),
+        "rmn_conv_weight_image");
+  return image;
+}
+
+// Epilogue of a convolution: out = act(conv * scale + shift + add). The vectors are per output channel; with a batch norm
+// (evaluation mode) they are made by the kernel that prepares the weights.
+struct ConvEpilogue {
+  at::Tensor scale, shift, add;
+  bool relu = false;
+};
+
+at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in, const at::Tensor& nbr,
+                        const ConvEpilogue& ep = {}, const at::Tensor& plan = at::Tensor(), torch::nn::BatchNorm1dImpl* bn = nullptr) {
+  TORCH_CHECK(feats_in.is_cuda() && kernel_in.is_cuda(), "features and kernel must be CUDA tensors");
+  TORCH_CHECK(feats_in.scalar_type() == kernel_in.scalar_type(), "expected features and kernel to have the same dtype");
+  auto feats = feats_in.contiguous(), kernel = kernel_in.contiguous();
+  c10::cuda::CUDAGuard guard(feats.device());
+  const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(kernel.size(1)),
+            c_out = static_cast<int>(kernel.size(2));
+  const auto shape = run_shape(kernel);
+  auto vector = [&](const at::Tensor& v, const char* what) {
+    if (!v.defined() || v.numel() == 0) return at::Tensor();
+    auto r = v.detach().reshape({-1}).to(at::kFloat).contiguous();
+    TORCH_CHECK(r.numel() == c_out, what, " must have one entry per output channel");
+    return r;
+  };
+  if (feats.size(0) > 0 && nbr.size(1) > 0) {
+    feats = pad_channels(feats, shape.first);
+    const bool padded = shape.second != c_out;
+    at::Tensor shift, scale;
+    rmn_bn_fold fold{};
+    if (bn) {
+      auto data = [](const at::Tensor& t) { return t.defined() ? ptr(t) : nullptr; };
+      scale = at::empty({2, shape.second}, feats.options().dtype(at::kFloat));
+      shift = scale[1];
+      fold = rmn_bn_fold{data(bn->running_mean), data(bn->running_var), data(bn->weight), data(bn->bias), data(ep.shift),
+                         dtype_code(bn->running_mean), static_cast<float>(bn->options.eps()),
+                         static_cast<float*>(ptr(scale)), static_cast<float*>(ptr(scale)) + shape.second};
+    } else {
+      shift = vector(ep.shift, "bias");
+      scale = vector(ep.scale, "scale");
+      if (padded && shift.defined()) shift = at::constant_pad_nd(shift, {0, shape.second - c_out});
+      if (padded && scale.defined()) scale = at::constant_pad_nd(scale, {0, shape.second - c_out});
+    }
+    if (auto image = weight_image(kernel, shape, false, false, feats, bn ? &fold : nullptr); image.defined()) {
+      TORCH_CHECK(!padded || !ep.add.defined(), "a padded convolution adds nothing");
+      auto out = at::empty({nbr.size(1), shape.second}, feats.options());
+      check(rmn_conv_forward_image(ptr(feats), static_cast<uint32_t>(feats.size(0)), static_cast<int>(shape.first), ptr(image),
+                                   K, static_cast<int>(shape.second), static_cast<const int32_t*>(ptr(nbr)), ptr(plan),
+                                   static_cast<uint32_t>(nbr.size(1)), ptr(out), static_cast<const float*>(ptr(scale)),
+                                   static_cast<const float*>(ptr(shift)), ptr(ep.add), ep.relu ? 1 : 0, current_stream()),
+            "rmn_conv_forward_image");
+      return padded ? out.narrow(1, 0, c_out) : out;
+    }
+    TORCH_CHECK(!bn && !ep.add.defined(), "no kernel folds this layer's batch norm");
+  }
+  auto shift = vector(ep.shift, "bias"), scale = vector(ep.scale, "scale");
+  auto out = at::empty({nbr.size(1), c_out}, feats.options());
+  check(rmn_conv_forward_planned(ptr(feats), static_cast<uint32_t>(feats.size(0)), c_in, ptr(kernel), K, c_out,
+                                 static_cast<const int32_t*>(ptr(nbr)), ptr(plan), static_cast<uint32_t>(nbr.size(1)),
+                                 ptr(out), dtype_code(feats), static_cast<const float*>(ptr(scale)),
+                                 static_cast<const float*>(ptr(shift)), ep.relu ? 1 : 0, current_stream()),
+        "rmn_conv_forward_planned");
+  return out;
+}
+
+// reverse: nbr_t is the forward table of a point-symmetric self map, i.e. its offsets run backwards
+at::Tensor conv_backward_input(const at::Tensor& grad_in, const at::Tensor& kernel_in, const at::Tensor& nbr_t,
+                               bool reverse, const at::Tensor& plan_t = at::Tensor()) {
+  auto grad = grad_in.contiguous();
+  c10::cuda::CUDAGuard guard(grad.device());
+  if (grad.scalar_type() == at::kFloat && grad.size(0) > 0 && nbr_t.size(1) > 0) {
+    // fp32: the forward pass on transposed weights
+    auto w = kernel_in.contiguous();
+    auto wt = at::empty({w.size(0), w.size(2), w.size(1)}, w.options());
+    check(rmn_conv_transpose_weights(ptr(w), static_cast<int>(w.size(0)), static_cast<int>(w.size(1)),
+                                     static_cast<int>(w.size(2)), RMN_F32, reverse ? 1 : 0, ptr(wt), current_stream()),
+          "rmn_conv_transpose_weights");
+    return conv_forward(grad, wt, nbr_t);
+  }
+  const int K = static_cast<int>(kernel_in.size(0)), c_in = static_cast<int>(kernel_in.size(1)),
+            c_out = static_cast<int>(kernel_in.size(2));
+  if (grad.size(0) > 0 && nbr_t.size(1) > 0) {
+    const auto shape = run_shape(kernel_in);
+    grad = pad_channels(grad, shape.second);
+    if (auto image = weight_image(kernel_in.contiguous(), shape, true, reverse, grad); image.defined()) {
+      auto out = at::empty({nbr_t.size(1), shape.first}, grad.options());
+      check(rmn_conv_forward_image(ptr(grad), static_cast<uint32_t>(grad.size(0)), static_cast<int>(shape.second), ptr(image),
+                                   K, static_cast<int>(shape.first), static_cast<const int32_t*>(ptr(nbr_t)), ptr(plan_t),
+                                   static_cast<uint32_t>(nbr_t.size(1)), ptr(out), nullptr, nullptr, nullptr, 0,
+                                   current_stream()),
+            "rmn_conv_forward_image");
+      return shape.first == c_in ? out : out.narrow(1, 0, c_in).contiguous();
+    }
+  }
+  auto out = at::empty({nbr_t.size(1), c_in}, grad.options());
+  auto kernel = reverse ? kernel_in.flip(0) : kernel_in.contiguous();
+  check(rmn_conv_backward_input_planned(ptr(grad), static_cast<uint32_t>(grad.size(0)), c_out, ptr(kernel), K, c_in,
+                                        static_cast<const int32_t*>(ptr(nbr_t)), ptr(plan_t),
+                                        static_cast<uint32_t>(nbr_t.size(1)), ptr(out), dtype_code(grad),
+                                        current_stream()),
+        "rmn_conv_backward_input_planned");
+  return out;
+}
+
 at::Tensor conv_backward_weight(const at::Tensor& feats_in, const at::Tensor& grad_in, const at::Tensor& nbr) {
   auto feats = feats_in.contiguous(), grad = grad_in.contiguous();
   c10::cuda::CUDAGuard guard(feats.device());
@@ -1119,6 +1163,30 @@ at::Tensor conv_backward_weight(const at::Tensor& feats_in, const at::Tensor& gr
   return dw;
 }
 
+// shapes rmn_channel_dot_stats / rmn_affine2 take: 16-byte lanes, a power-of-two number of them (<= 32) per row
+bool bn_fast_shape(const at::Tensor& x) {
+  if (!x.is_cuda() || x.dim() != 2 || x.size(0) == 0) return false;
+  if (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16) return false;
+  const int64_t lanes16 = x.size(1) * x.element_size() / 16;
+  return x.size(1) * x.element_size() % 16 == 0 && lanes16 >= 1 && lanes16 <= 32 && (32 % lanes16) == 0;
+}
+
+// Sums of the first `columns` columns, [1, columns] in x's type (a bias gradient): one streaming pass (1.2 M x 64 bf16:
+// 34 us, torch's reduction of the narrow matrix 131 us).
+at::Tensor column_sums(const at::Tensor& x, int64_t columns) {
+  if (!bn_fast_shape(x) || !x.is_contiguous() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0)
+    return x.narrow(1, 0, columns).sum(0, /*keepdim=*/true);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int C = static_cast<int>(x.size(1));
+  auto sums = at::empty({2, C}, x.options().dtype(at::kDouble));
+  const size_t ws_bytes = rmn_channel_dot_stats_workspace_bytes(C);
+  auto ws = at::empty({static_cast<int64_t>(ws_bytes)}, x.options().dtype(at::kByte));
+  check(rmn_channel_dot_stats(ptr(x), ptr(x), static_cast<uint32_t>(x.size(0)), C, dtype_code(x),
+                              static_cast<double*>(ptr(sums)), ptr(ws), ws_bytes, current_stream()),
+        "rmn_channel_dot_stats");
+  return sums.narrow(0, 0, 1).narrow(1, 0, columns).to(x.scalar_type());
+}
+
 // The neighbour tables travel through autograd as plain (non-differentiable) int32 tensors:
 // nbr_out for the forward pass and the weight gradient, nbr_in for the input gradient.
 class SparseConvolutionAutograd : public torch::autograd::Function<SparseConvolutionAutograd> {
@@ -1127,13 +1195,19 @@ public:
   static at::Tensor forward(torch::autograd::AutogradContext* ctx, at::Tensor features, at::Tensor kernel,
                             at::Tensor nbr_out, at::Tensor nbr_in, bool flip_kernel, at::Tensor bias,
                             at::Tensor plan_out, at::Tensor plan_in) {
+    // (padded once: the weight gradient reads them again)
+    if (features.size(0) > 0 && nbr_out.size(1) > 0 && kernel.scalar_type() == at::kBFloat16 &&
+        features.scalar_type() == at::kBFloat16) {
+      c10::cuda::CUDAGuard guard(features.device());
+      features = pad_channels(features, run_shape(kernel).first);
+    }
     ctx->save_for_backward({features, kernel});
     ctx->saved_data["has_bias"] = bias.numel() > 0;
     ctx->saved_data["nbr_out"] = nbr_out;
     ctx->saved_data["nbr_in"] = nbr_in;
     ctx->saved_data["plan_in"] = plan_in;
     ctx->saved_data["flip_kernel"] = flip_kernel;
-    return conv_forward(features, kernel, nbr_out, bias, at::Tensor(), false,
+    return conv_forward(features, kernel, nbr_out, ConvEpilogue{at::Tensor(), bias, at::Tensor(), false},
                         plan_out.numel() > 0 ? plan_out : at::Tensor());
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
@@ -1142,6 +1216,16 @@ public:
     auto nbr_out = ctx->saved_data["nbr_out"].toTensor();
     auto nbr_in = ctx->saved_data["nbr_in"].toTensor();
     auto grad = grad_outputs[0].contiguous();
+    const auto& kernel = saved[1];
+    if (grad.size(0) > 0 && nbr_out.size(1) > 0 && saved[0].size(0) > 0) {
+      c10::cuda::CUDAGuard guard(grad.device());
+      grad = pad_channels(grad, run_shape(kernel).second);
+    }
+    auto weight_gradient = [&] {
+      auto g = conv_backward_weight(saved[0], grad, nbr_out);
+      return g.sizes() == kernel.sizes() ? g : g.narrow(1, 0, kernel.size(1)).narrow(2, 0, kernel.size(2)).contiguous();
+    };
+    auto bias_gradient = [&] { return column_sums(grad, kernel.size(2)); };
     at::Tensor g_feat, g_kernel, g_bias;
     // (needs_input_grad counts the tensor arguments only: features 0, kernel 1, nbr_out 2, nbr_in 3, bias 4)
     const bool want_bias = ctx->saved_data["has_bias"].toBool() && ctx->needs_input_grad(4);
@@ -1149,8 +1233,8 @@ public:
       // Data-parallel: the weight gradient comes first, its all-reduce runs on the second stream and the
       // input gradient on this one; this stream waits for the reduced gradients before handing them on.
       std::vector<at::Tensor> reduce;
-      if (ctx->needs_input_grad(1)) reduce.push_back(g_kernel = conv_backward_weight(saved[0], grad, nbr_out));
-      if (want_bias) reduce.push_back(g_bias = grad.sum(0, /*keepdim=*/true).to(at::kFloat).contiguous());
+      if (ctx->needs_input_grad(1)) reduce.push_back(g_kernel = weight_gradient());
+      if (want_bias) reduce.push_back(g_bias = bias_gradient().to(at::kFloat).contiguous());
       auto main_stream = c10::cuda::getCurrentCUDAStream();
       auto side_stream = pair_list_stream(main_stream.device_index());
       c10::Event ready(c10::DeviceType::CUDA);
@@ -1178,42 +1262,25 @@ public:
       g_feat = conv_backward_input(grad, saved[1], nbr_in, ctx->saved_data["flip_kernel"].toBool(),
                                    plan_in.numel() > 0 ? plan_in : at::Tensor());
     }
-    if (ctx->needs_input_grad(1)) g_kernel = conv_backward_weight(saved[0], grad, nbr_out).to(saved[1].scalar_type());
-    if (want_bias) g_bias = grad.sum(0, /*keepdim=*/true);
+    if (ctx->needs_input_grad(1)) g_kernel = weight_gradient().to(saved[1].scalar_type());
+    if (want_bias) g_bias = bias_gradient();
     return {g_feat, g_kernel, at::Tensor(), at::Tensor(), at::Tensor(), g_bias, at::Tensor(), at::Tensor()};
   }
 };
 
 }  // namespace
 
-at::Tensor sparse_convolution(const at::Tensor& features_in, const at::Tensor& kernel_in,
-                              const std::shared_ptr<KernelMap>& kmap, const at::Tensor& bias_in) {
-  // bf16 channel counts without a tensor-core kernel (a 4-channel stem, 48 or 96 channels ...) are zero-padded
-  // to the next pair that has one, with differentiable torch ops around the convolution: padded input channels
-  // multiply zero weights, padded output channels are cut off again, and autograd slices the gradients back.
-  at::Tensor features = features_in, kernel = kernel_in, bias = bias_in;
-  const int64_t c_in = kernel.size(1), c_out = kernel.size(2);
-  int64_t pad_out = 0;
-  if (features.scalar_type() == at::kBFloat16 && kernel.scalar_type() == at::kBFloat16) {
-    auto legal = tc_legal_shape(c_in, c_out);
-    if (legal.first != c_in || legal.second != c_out) {
-      pad_out = legal.second - c_out;
-      features = at::constant_pad_nd(features, {0, legal.first - c_in});
-      kernel = at::constant_pad_nd(kernel, {0, pad_out, 0, legal.first - c_in});
-      if (bias.defined() && bias.numel() > 0 && pad_out) bias = at::constant_pad_nd(bias, {0, pad_out});
-    }
-  }
-  if (pad_out) {
-    auto padded = sparse_convolution(features, kernel, kmap, bias);
-    return padded.narrow(1, 0, c_out);
-  }
+at::Tensor sparse_convolution(const at::Tensor& features, const at::Tensor& kernel,
+                              const std::shared_ptr<KernelMap>& kmap, const at::Tensor& bias) {
+  TORCH_CHECK(features.size(1) == kernel.size(1), "Convolution kernel input channels do not match features");
   // the inverse table is cached in the kernel map; it is only needed when the features want a gradient
   at::Tensor nbr_in = kmap->self_symmetric
                           ? kmap->nbr_out
                           : (features.requires_grad() ? kmap->nbr_in() : at::empty({0}, kmap->nbr_out.options()));
   // (autograd functions take defined tensors only: an empty tensor stands for "no bias")
   at::Tensor bias_arg = bias.defined() ? bias : at::empty({0}, kernel.options());
-  const int64_t weight = kernel.size(1) * kernel.size(2);
+  const auto shape = run_shape(kernel);
+  const int64_t weight = shape.first * shape.second;
   auto none = at::empty({0}, kmap->nbr_out.options().dtype(at::kByte));
   at::Tensor plan_out, plan_in;
   if (features.scalar_type() == at::kBFloat16) {  // plans serve the tensor-core kernels only
@@ -1288,7 +1355,8 @@ SparseTensor RiemannConvolutionBaseImpl::forward(const SparseTensor& input) {
     torch::NoGradGuard guard;
     at::Tensor plan;
     if (input.F().scalar_type() == at::kBFloat16) plan = kmap->plan_out(int64_t(in_channels_) * out_channels_);
-    auto result = conv_forward(input.F(), kernel_, kmap->nbr_out, fold_shift_, fold_scale_, fold_relu_, plan);
+    auto result = conv_forward(input.F(), kernel_, kmap->nbr_out,
+                               ConvEpilogue{fold_scale_, fold_shift_, at::Tensor(), fold_relu_}, plan);
     return SparseTensor(std::move(result), output_key, std::move(manager));
   }
   auto result = sparse_convolution(input.F(), kernel_, kmap, bias_);  // the bias add is fused into the epilogue
@@ -1405,14 +1473,6 @@ public:
     return {dx, dgamma, dbeta, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };
-
-// shapes rmn_channel_dot_stats / rmn_affine2 take: 16-byte lanes, a power-of-two number of them (<= 32) per row
-bool bn_fast_shape(const at::Tensor& x) {
-  if (!x.is_cuda() || x.dim() != 2 || x.size(0) == 0) return false;
-  if (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16) return false;
-  const int64_t lanes16 = x.size(1) * x.element_size() / 16;
-  return x.size(1) * x.element_size() % 16 == 0 && lanes16 >= 1 && lanes16 <= 32 && (32 % lanes16) == 0;
-}
 }  // namespace
 
 SparseTensor RiemannBatchNormImpl::forward(const SparseTensor& input) {

@@ -44,10 +44,35 @@ def test_image_passes_match_float64(c_in, c_out, n, K, fill):
     image = ops._weight_image(w.flip(0).contiguous(), False, feats, reverse=True)
     out = torch.empty((n, c_out), dtype=torch.bfloat16, device="cuda")
     capi.check(capi.lib().rmn_conv_forward_image(ops._ptr(feats), n_src, c_in, ops._ptr(image), K, c_out, ops._ptr(nbr),
-                                                 None, n, ops._ptr(out), None, None, 0, ops._stream()), "image")
+                                                 None, n, ops._ptr(out), None, None, None, 0, ops._stream()), "image")
     assert torch.equal(out, ops.conv_forward(feats, w, nbr))
     got, stats = ops.conv_forward_stats(feats, w, nbr, shift=shift)
     _close(got, want + shift.double())
     stored = got.double()
     want_stats = torch.stack([stored.sum(0), (stored * stored).sum(0)])
     assert float((stats - want_stats).abs().max()) <= 1e-4 * max(1.0, float((stored * stored).sum(0).max()))
+
+
+@pytest.mark.parametrize("n,c_in,c_out", [(1, 4, 20), (1000, 20, 96), (4099, 33, 64)])
+def test_padded_layer_with_bias_matches_float64(n, c_in, c_out):
+    """Channel counts without a kernel of their own: padded features, weights and gradients, the bias gradient."""
+    from riemannengine_b200 import cpp, ops
+    C = cpp.load()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    c = torch.unique(torch.randint(0, 40, (2 * n, 3), generator=g, device="cuda"), dim=0)[:n]
+    coords = torch.cat([torch.zeros_like(c[:, :1]), c], 1).int().contiguous()
+    layer = C.RiemannConvolution(c_in, c_out, kernel_size=3, stride=1, bias=True, dimension=3)
+    layer.to("cuda:0")
+    layer.to(torch.bfloat16)
+    feats = torch.randn((coords.size(0), c_in), generator=g, device="cuda").bfloat16().requires_grad_(True)
+    grad = torch.randn((coords.size(0), c_out), generator=g, device="cuda").bfloat16()
+    y = layer(C.SparseTensor(feats, coords))
+    y.F.backward(grad)
+    table = ops.table_build(coords)
+    nbr = ops.kmap_build(table, table.coords, ops.region_offsets(0, [3] * 3, [1] * 3, [1] * 3), self_map=True).nbr
+    w, b = layer.kernel.detach(), layer.bias.detach()
+    _close(y.F.detach(), _reference(feats.detach(), w, nbr) + b.double())
+    _close(feats.grad, _reference(grad, w.flip(0).transpose(1, 2), nbr))
+    _close(layer.bias.grad, grad.double().sum(0, keepdim=True))
+    want = torch.stack([feats.detach()[nbr[k][nbr[k] >= 0].long()].double().t() @ grad[nbr[k] >= 0].double() for k in range(27)])
+    _close(layer.kernel.grad, want)
