@@ -65,7 +65,7 @@ __device__ __forceinline__ constexpr uint32_t n_channel(uint32_t p) {
 // 64 bytes per reduction position and 64-column atom, 16-byte chunk c of line p at swz(p, c)). Where a stage has two
 // offsets their lines follow one another; the second half of an odd last stage is zero. One thread per chunk.
 // w has w_red <= CR and w_col <= CC channels, the rest is zero. transpose: w is [K][w_col][w_red] (input gradient);
-// reverse: offset k of the image is W[K - 1 - k]. Block 0 also turns the batch norm of `fold` into epilogue scale and shift.
+// reverse: offset k of the image is W[K - 1 - k]. One more block turns the batch norm of `fold` into epilogue scale and shift.
 template <int CC>
 constexpr int ta_tiles() { return CC <= 64 ? 4 : (CC <= 128 ? 2 : 1); }
 
@@ -73,7 +73,7 @@ template <int CR, int CC>
 __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, uint32_t w_red,
                                                       uint32_t w_col, int transpose, int reverse, rmn_bn_fold fold,
                                                       uint4* __restrict__ image) {
-  if (fold.scale && blockIdx.x == 0) {
+  if (fold.scale && blockIdx.x == gridDim.x - 1) {
     for (uint32_t c = threadIdx.x; c < CC; c += 256) {
       auto param = [&](const void* p, float absent) {
         if (!p || c >= w_col) return absent;
@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __res
       fold.scale[c] = s;
       fold.shift[c] = param(fold.beta, 0.f) + (param(fold.conv_bias, 0.f) - param(fold.mean, 0.f)) * s;
     }
+    return;
   }
   using C = TaCfg<CR, CC, ta_tiles<CC>()>;
   constexpr int KB = C::KB, NBLK = CC < 64 ? CC : 64, CPL = NBLK / 8, CHUNKS = KB * CC / 8;
@@ -604,7 +605,7 @@ template <int CR, int CC>
 int launch_image(const void* w, int K, int w_red, int w_col, int transpose, int reverse, const rmn_bn_fold& fold, void* image,
                  cudaStream_t stream) {
   const uint32_t chunks = (uint32_t)(image_bytes<CR, CC>(K) / 16);
-  k_weight_image<CR, CC><<<(chunks + 255) / 256, 256, 0, stream>>>((const __nv_bfloat16*)w, K, w_red, w_col, transpose,
+  k_weight_image<CR, CC><<<(chunks + 255) / 256 + (fold.scale ? 1 : 0), 256, 0, stream>>>((const __nv_bfloat16*)w, K, w_red, w_col, transpose,
                                                                   reverse, fold, (uint4*)image);
   RMN_LAUNCH_CHECK();
   return RMN_OK;

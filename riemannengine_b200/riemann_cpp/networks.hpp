@@ -22,7 +22,7 @@ struct ConvNormActImpl : torch::nn::Module {
     norm = register_module("norm", RiemannBatchNorm(c_out));
     act = register_module("act", RiemannReLU());
   }
-  SparseTensor forward(SparseTensor x) { return act->forward(norm->forward(conv->forward(x))); }
+  SparseTensor forward(SparseTensor x) { return conv_norm_relu(x, *conv->base(), *norm); }
 };
 TORCH_MODULE(ConvNormAct);
 
@@ -38,7 +38,7 @@ struct UpNormActImpl : torch::nn::Module {
     norm = register_module("norm", RiemannBatchNorm(c_out));
     act = register_module("act", RiemannReLU());
   }
-  SparseTensor forward(SparseTensor x) { return act->forward(norm->forward(conv->forward(x))); }
+  SparseTensor forward(SparseTensor x) { return conv_norm_relu(x, *conv->base(), *norm); }
 };
 TORCH_MODULE(UpNormAct);
 
@@ -58,8 +58,7 @@ struct BasicBlockImpl : torch::nn::Module {
     act = register_module("act", RiemannReLU());
   }
   SparseTensor forward(SparseTensor x) {
-    auto y = norm->forward(conv->forward(first->forward(x)));
-    return act->forward(y + x);
+    return conv_norm_relu(first->forward(x), *conv->base(), *norm, &x);
   }
 };
 TORCH_MODULE(BasicBlock);

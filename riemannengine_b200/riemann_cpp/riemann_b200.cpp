@@ -1319,7 +1319,28 @@ void RiemannConvolutionBaseImpl::reset_parameters(bool is_transpose) {
   if (bias_.defined()) bias_.uniform_(-bound, bound);
 }
 
-SparseTensor RiemannConvolutionBaseImpl::forward(const SparseTensor& input) {
+namespace {
+// whether the kernel that prepares a layer's weights also folds this batch norm (bf16 on tensor cores, parameters of one type)
+bool folds_batch_norm(const RiemannConvolutionBaseImpl& conv, const SparseTensor& input, const torch::nn::BatchNorm1dImpl& bn) {
+  auto const& kernel = conv.kernel_;
+  auto const& mean = bn.running_mean;
+  if (!mean.defined() || !bn.running_var.defined() || input.F().scalar_type() != at::kBFloat16 ||
+      kernel.scalar_type() != at::kBFloat16 || !input.F().is_cuda() || input.F().size(0) == 0)
+    return false;
+  if (mean.scalar_type() != at::kBFloat16 && mean.scalar_type() != at::kFloat) return false;
+  for (auto const& p : {bn.running_var, bn.weight, bn.bias, conv.bias_, mean})
+    if (p.defined() && (p.scalar_type() != mean.scalar_type() || !p.is_contiguous() || p.numel() != conv.out_channels_ ||
+                        p.device() != input.F().device()))
+      return false;
+  const auto shape = run_shape(kernel);
+  auto x = input.F();
+  return rmn_conv_weight_image_bytes(static_cast<int>(kernel.size(0)), static_cast<int>(shape.first),
+                                     static_cast<int>(shape.second), RMN_BF16) > 0 &&
+         (shape.first != x.size(1) || !x.is_contiguous() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 == 0);
+}
+}  // namespace
+
+std::pair<std::shared_ptr<KernelMap>, CoordinateMapKey> RiemannConvolutionBaseImpl::kernel_map(const SparseTensor& input) {
   TORCH_CHECK(input.dimension() == dimension_, "Input dimension mismatch");
   TORCH_CHECK(input.F().size(1) == in_channels_, "Input channel count does not match convolution");
   const auto params = kernel_generator_.get_kernel(input.tensor_stride(), is_transpose_);
@@ -1351,51 +1372,70 @@ SparseTensor RiemannConvolutionBaseImpl::forward(const SparseTensor& input) {
   auto kmap = manager->kernel_map(input.coordinate_map_key(), output_key, params.kernel_size, params.kernel_stride,
                                   params.kernel_dilation, params.region_type, params.region_offsets, is_transpose_,
                                   false);
-  if (fold_scale_.defined() || fold_shift_.defined() || fold_relu_) {  // set by fused_conv_bn_relu for one call
-    torch::NoGradGuard guard;
-    at::Tensor plan;
-    if (input.F().scalar_type() == at::kBFloat16) plan = kmap->plan_out(int64_t(in_channels_) * out_channels_);
-    auto result = conv_forward(input.F(), kernel_, kmap->nbr_out,
-                               ConvEpilogue{fold_scale_, fold_shift_, at::Tensor(), fold_relu_}, plan);
-    return SparseTensor(std::move(result), output_key, std::move(manager));
-  }
+  return {std::move(kmap), output_key};
+}
+
+SparseTensor RiemannConvolutionBaseImpl::forward(const SparseTensor& input) {
+  auto [kmap, output_key] = kernel_map(input);
   auto result = sparse_convolution(input.F(), kernel_, kmap, bias_);  // the bias add is fused into the epilogue
-  return SparseTensor(std::move(result), output_key, std::move(manager));
+  return SparseTensor(std::move(result), output_key, input.coordinate_manager());
+}
+
+SparseTensor RiemannConvolutionBaseImpl::forward_fused(const SparseTensor& input, torch::nn::BatchNorm1d bn, bool relu,
+                                                       const at::Tensor& add) {
+  torch::NoGradGuard guard;
+  auto [kmap, output_key] = kernel_map(input);
+  const auto shape = run_shape(kernel_);
+  at::Tensor plan;
+  if (input.F().scalar_type() == at::kBFloat16) plan = kmap->plan_out(shape.first * shape.second);
+  ConvEpilogue ep;
+  ep.shift = bias_;
+  ep.add = add;
+  ep.relu = relu;
+  torch::nn::BatchNorm1dImpl* folded = nullptr;
+  if (!bn.is_empty()) {
+    if (folds_batch_norm(*this, input, *bn) && kmap->nbr_out.size(1) > 0) {
+      folded = bn.get();
+    } else {  // the affine by torch ops
+      auto inv = torch::rsqrt(bn->running_var.to(at::kFloat) + bn->options.eps());
+      ep.scale = bn->weight.defined() ? inv * bn->weight.to(at::kFloat) : inv;
+      ep.shift = -bn->running_mean.to(at::kFloat) * ep.scale;
+      if (bn->bias.defined()) ep.shift = ep.shift + bn->bias.to(at::kFloat);
+      if (bias_.defined()) ep.shift = ep.shift + bias_.reshape({-1}).to(at::kFloat) * ep.scale;
+    }
+  }
+  auto result = conv_forward(input.F(), kernel_, kmap->nbr_out, ep, plan, folded);
+  return SparseTensor(std::move(result), output_key, input.coordinate_manager());
 }
 
 // conv -> batch norm (running statistics) -> ReLU as ONE kernel (inference): the norm's affine and the
 // layer's bias are folded into the convolution epilogue (engine/nn/residual.cpp:44-52 runs three modules).
 SparseTensor fused_conv_bn_relu(const SparseTensor& input, RiemannConvolutionBaseImpl& conv,
                                 torch::nn::BatchNorm1d bn, bool relu) {
-  torch::NoGradGuard guard;
-  at::Tensor scale, shift;
-  at::Tensor bias = conv.bias_.defined() ? conv.bias_.reshape({-1}).to(at::kFloat) : at::Tensor();
   if (!bn.is_empty()) {
     TORCH_CHECK(!bn->is_training(), "fused_conv_bn_relu folds running statistics: call bn->eval() first");
     TORCH_CHECK(bn->running_var.defined(), "fused_conv_bn_relu needs running statistics");
-    auto inv = torch::rsqrt(bn->running_var.to(at::kFloat) + bn->options.eps());
-    scale = bn->weight.defined() ? inv * bn->weight.to(at::kFloat) : inv;
-    shift = -bn->running_mean.to(at::kFloat) * scale;
-    if (bn->bias.defined()) shift = shift + bn->bias.to(at::kFloat);
-    if (bias.defined()) shift = shift + bias * scale;
-  } else {
-    shift = bias;
   }
-  conv.fold_scale_ = scale;
-  conv.fold_shift_ = shift;
-  conv.fold_relu_ = relu;
-  try {
-    auto out = conv.forward(input);
-    conv.fold_scale_ = at::Tensor();
-    conv.fold_shift_ = at::Tensor();
-    conv.fold_relu_ = false;
-    return out;
-  } catch (...) {
-    conv.fold_scale_ = at::Tensor();
-    conv.fold_shift_ = at::Tensor();
-    conv.fold_relu_ = false;
-    throw;
+  return conv.forward_fused(input, bn, relu);
+}
+
+SparseTensor conv_norm_relu(const SparseTensor& input, RiemannConvolutionBaseImpl& conv, RiemannBatchNormImpl& norm,
+                            const SparseTensor* residual) {
+  auto bn = norm.normalization();
+  bool fuse = !at::GradMode::is_enabled() && !bn->is_training() && folds_batch_norm(conv, input, *bn);
+  if (fuse && residual) {  // (a stride-1 layer: the output lies on the input's map)
+    auto const& r = residual->F();
+    fuse = conv.kernel_generator_.kernel_stride() == stride_type(conv.dimension_, 1) && !conv.is_transpose_ &&
+           residual->coordinate_manager() == input.coordinate_manager() &&
+           residual->coordinate_map_key() == input.coordinate_map_key() && r.size(0) == input.F().size(0) &&
+           r.size(1) == conv.out_channels_ && r.scalar_type() == at::kBFloat16 && r.is_contiguous() &&
+           r.device() == input.F().device() && reinterpret_cast<uintptr_t>(r.data_ptr()) % 16 == 0 &&
+           run_shape(conv.kernel_).second == conv.out_channels_;
   }
+  if (fuse) return conv.forward_fused(input, bn, true, residual ? residual->F() : at::Tensor());
+  auto y = norm.forward(conv.forward(input));
+  if (residual) y = y + *residual;
+  return SparseTensor(at::relu(y.F()), y.coordinate_map_key(), y.coordinate_manager());
 }
 
 RiemannBatchNormImpl::RiemannBatchNormImpl(int64_t num_features, double eps, double momentum, bool affine,

@@ -390,9 +390,13 @@ public:
   KernelGenerator kernel_generator_;
   torch::Tensor kernel_{nullptr};
   torch::Tensor bias_{nullptr};
-  // per-call epilogue fold (scale, shift, ReLU) installed by fused_conv_bn_relu; empty otherwise
-  at::Tensor fold_scale_, fold_shift_;
-  bool fold_relu_ = false;
+  // out = act(conv(input) (+ bias) * scale + shift + add) with the batch norm's running statistics as scale and shift
+  // (a missing holder: bias only); inference only
+  SparseTensor forward_fused(const SparseTensor& input, torch::nn::BatchNorm1d bn, bool relu, const at::Tensor& add = {});
+
+private:
+  // input map -> (kernel map, output key), building or reusing the output map
+  std::pair<std::shared_ptr<KernelMap>, CoordinateMapKey> kernel_map(const SparseTensor& input);
 };
 
 // RiemannBatchNormImpl (engine/nn/normalization.hpp:11-34): torch's BatchNorm1d over the feature matrix.
@@ -413,6 +417,11 @@ using RiemannSyncBatchNorm = RiemannBatchNorm;
 // Inference-only conv -> batch norm -> ReLU as one kernel; `bn` may be an empty holder (bias + ReLU only).
 SparseTensor fused_conv_bn_relu(const SparseTensor& input, RiemannConvolutionBaseImpl& conv,
                                 torch::nn::BatchNorm1d bn = nullptr, bool relu = true);
+
+// relu(norm(conv(input)) [+ residual]): one kernel in evaluation mode without gradients, where bf16 kernels cover the layer;
+// otherwise (training, fp32, a residual on other coordinates) the layers one after the other.
+SparseTensor conv_norm_relu(const SparseTensor& input, RiemannConvolutionBaseImpl& conv, RiemannBatchNormImpl& norm,
+                            const SparseTensor* residual = nullptr);
 
 #define RIEMANN_B200_CONV_WRAPPER(Name)                                                                   \
   class Name##Impl : public torch::nn::Cloneable<Name##Impl> {                                            \

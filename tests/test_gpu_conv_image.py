@@ -76,3 +76,24 @@ def test_padded_layer_with_bias_matches_float64(n, c_in, c_out):
     _close(layer.bias.grad, grad.double().sum(0, keepdim=True))
     want = torch.stack([feats.detach()[nbr[k][nbr[k] >= 0].long()].double().t() @ grad[nbr[k] >= 0].double() for k in range(27)])
     _close(layer.kernel.grad, want)
+
+
+def test_network_in_evaluation_mode_matches_its_layers():
+    """Without gradients conv, batch norm, residual and ReLU run as one kernel; with them, layer by layer."""
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    torch.manual_seed(5)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    c = torch.unique(torch.randint(0, 24, (3000, 3), generator=g, device="cuda"), dim=0)
+    coords = torch.cat([torch.zeros_like(c[:, :1]), c], 1).int().contiguous()
+    net = C.MinkUNet(4, 20, width=32, dimension=3)
+    net.to("cuda:0")
+    net.to(torch.bfloat16)
+    feats = torch.randn((coords.size(0), 4), generator=g, device="cuda").bfloat16()
+    for _ in range(3):   # running statistics that are not the identity
+        net(C.SparseTensor(feats, coords))
+    net.train(False)
+    want = net(C.SparseTensor(feats, coords)).F.detach().double()
+    with torch.no_grad():
+        got = net(C.SparseTensor(feats, coords)).F.double()
+    assert float((got - want).norm()) <= 2e-2 * float(want.norm())
