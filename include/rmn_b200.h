@@ -122,6 +122,16 @@ int rmn_table_build_finish(const int32_t *d_coords, uint32_t n_rows, int W, void
                            int64_t *d_inverse, int32_t *d_unique_coords, void *d_workspace, void *stream);
 
 /*
+ * rmn_table_build followed by rmn_table_info, for a host that needs the number of unique rows before it can go on: the
+ * build itself stores the words into page-locked memory and the call returns as soon as they are there, while the second
+ * half of the build may still be running on the stream. d_mapping and d_inverse may be NULL. expect_duplicates != 0: most
+ * rows are expected to repeat (strided or quantised coordinates); a hint, the result is the same.
+ */
+int rmn_table_build_counted(const int32_t *d_coords, uint32_t n_rows, int W, void *d_table, size_t table_bytes,
+                            int64_t *d_mapping, int64_t *d_inverse, int32_t *d_unique_coords, void *d_workspace,
+                            size_t workspace_bytes, int expect_duplicates, uint32_t info[4], void *stream);
+
+/*
  * rmn_table_build for callers that cannot allocate device memory. It has no
  * counterpart in the reference. Same inputs, outputs and results as
  * rmn_table_build, but there is no workspace argument: the build's scratch is
@@ -291,6 +301,14 @@ int rmn_kmap_build(const void *d_table, const int32_t *d_query, uint32_t n_query
  */
 int rmn_kmap_build_self(const void *d_table, const int32_t *d_coords, uint32_t n_rows, int W,
                         const int32_t *d_offsets, int K, int32_t *d_nbr, int64_t *d_offset_ptr,
+                        void *d_workspace, size_t workspace_bytes, void *stream);
+
+/*
+ * rmn_kmap_build (self = 0) or rmn_kmap_build_self that also stores the K + 1 offset pointers into page-locked mapped host
+ * memory: final once the work queued here has run.
+ */
+int rmn_kmap_build_host(const void *d_table, const int32_t *d_query, uint32_t n_query, int W, const int32_t *d_offsets,
+                        int K, int self, int32_t *d_nbr, int64_t *d_offset_ptr, int64_t *h_offset_ptr_pinned,
                         void *d_workspace, size_t workspace_bytes, void *stream);
 
 /*

@@ -156,6 +156,17 @@ __device__ __forceinline__ void load_row(const int32_t* __restrict__ coords, uin
   }
 }
 
+template <int W, bool kVec>
+__device__ __forceinline__ void store_row(int32_t* __restrict__ coords, uint32_t row, const int32_t (&c)[W]) {
+  if constexpr (kVec) {
+    static_assert(W == 4, "one 16-byte access per row");
+    reinterpret_cast<int4*>(coords)[row] = make_int4(c[0], c[1], c[2], c[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; ++i) coords[(size_t)row * W + i] = c[i];
+  }
+}
+
 // Slot count for n_rows inserted rows: load factor <= 1/4 (<= 1/3 for large tables, below), a multiple of 32,
 // at least 64. (Measured on
 // 1.2 M voxels, insert + self-map probe / general 27-offset probe: 2 n slots 0.312 / 0.435 ms, 3 n

@@ -8,13 +8,16 @@
 // (one vectorised 16-byte load for W = 4), loops over the K offsets held in
 // shared memory, probes, writes nbr[k][q] (coalesced: consecutive lanes are
 // consecutive rows) and counts hits per offset with warp ballots.
-// Pass 2 (k_kmap_scan): exclusive scan of the per-(offset, block) hit counts
-// and of the per-offset totals -> offset_ptr[K+1].
+// On small maps the offsets are split over gridDim.y, so that more blocks share the chain of probes.
+// Pass 2 (k_kmap_scan): exclusive scan of the per-(offset, block) hit counts; the last block turns
+// the per-offset totals into offset_ptr[K+1].
 // Pass 3 (k_kmap_pairs, optional): ballot compaction of nbr into (a, q) pair
 // lists at deterministic positions (pairs of one offset sorted by query row),
 // with no sort and no atomics. The reference instead sorts all triplets by
 // offset (engine/grid/lattice_gpu.cuh:440-488).
 #include "rmn_common.cuh"
+
+#include <string.h>
 
 #include <mutex>
 
@@ -29,14 +32,17 @@ template <int W>
 __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots,
     const int32_t* __restrict__ query, uint32_t n_query, const int32_t* __restrict__ offsets,
-    int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks) {
+    int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks,
+    uint32_t* __restrict__ scan_ticket) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int D = W - 1;
+  const int k_begin = (int)((uint32_t)K * blockIdx.y / gridDim.y), k_end = (int)((uint32_t)K * (blockIdx.y + 1) / gridDim.y);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scan_ticket = 0;
   long long* s_delta = reinterpret_cast<long long*>(smem_raw);           // [K]
   int32_t* s_off = reinterpret_cast<int32_t*>(s_delta + K);              // [K][D]
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_off + K * D);          // [K]
-  for (int i = threadIdx.x; i < K * D; i += kKmapBlock) s_off[i] = offsets[i];
-  for (int k = threadIdx.x; k < K; k += kKmapBlock) {
+  for (int i = k_begin * D + threadIdx.x; i < k_end * D; i += kKmapBlock) s_off[i] = offsets[i];
+  for (int k = k_begin + threadIdx.x; k < k_end; k += kKmapBlock) {
     long long d = 0;
 #pragma unroll
     for (int a = 0; a < D; ++a) d += (long long)offsets[k * D + a] << h->shift[a + 1];
@@ -75,8 +81,8 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe(
   // every warp pay a second and third dependent table read per offset; those lookups are noted in
   // a bit mask instead (64 offsets per chunk) and finished, thread by thread, after the chunk.
   constexpr int kUnroll = 3;
-  for (int chunk0 = 0; chunk0 < K; chunk0 += 64) {
-    const int chunk_end = min(K, chunk0 + 64);
+  for (int chunk0 = k_begin; chunk0 < k_end; chunk0 += 64) {
+    const int chunk_end = min(k_end, chunk0 + 64);
     unsigned long long pending = 0ull;
     for (int k0 = chunk0; k0 < chunk_end; k0 += kUnroll) {
       unsigned long long key[kUnroll];
@@ -128,7 +134,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe(
     }
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < K; k += kKmapBlock)
+  for (int k = k_begin + threadIdx.x; k < k_end; k += kKmapBlock)
     block_counts[(size_t)k * n_blocks + blockIdx.x] = s_cnt[k];
 }
 
@@ -141,15 +147,19 @@ template <int W>
 __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots,
     const int32_t* __restrict__ coords, uint32_t n, const int32_t* __restrict__ offsets, int K,
-    int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks) {
+    int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks,
+    uint32_t* __restrict__ scan_ticket) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int D = W - 1;
   const int half = K / 2;
+  const int k_begin = (int)((uint32_t)half * blockIdx.y / gridDim.y);
+  const int k_end = (int)((uint32_t)half * (blockIdx.y + 1) / gridDim.y);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scan_ticket = 0;
   long long* s_delta = reinterpret_cast<long long*>(smem_raw);   // [half]
   int32_t* s_off = reinterpret_cast<int32_t*>(s_delta + (half > 0 ? half : 1));  // [half][D]
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_off + (half > 0 ? half : 1) * D);  // [half]
-  for (int i = threadIdx.x; i < half * D; i += kKmapBlock) s_off[i] = offsets[i];
-  for (int k = threadIdx.x; k < half; k += kKmapBlock) {
+  for (int i = k_begin * D + threadIdx.x; i < k_end * D; i += kKmapBlock) s_off[i] = offsets[i];
+  for (int k = k_begin + threadIdx.x; k < k_end; k += kKmapBlock) {
     long long d = 0;
 #pragma unroll
     for (int a = 0; a < D; ++a) d += (long long)offsets[k * D + a] << h->shift[a + 1];
@@ -178,10 +188,10 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
     ckey += (long long)((long long)c[i] - (long long)mn) << h->shift[i];
   }
   const int lane = threadIdx.x & 31;
-  if (active) __stcs(nbr + (size_t)half * n + q, (int32_t)q);  // centre offset: identity
+  if (active && blockIdx.y == 0) __stcs(nbr + (size_t)half * n + q, (int32_t)q);  // centre offset: identity
   // (Deferring the few lookups that walk past their home slot to a second loop, as the general builder does,
   // made this kernel slower: 0.153 against 0.144 ms.)
-  for (int k = 0; k < half; ++k) {
+  for (int k = k_begin; k < k_end; ++k) {
     bool in_box = active;
 #pragma unroll
     for (int a = 0; a < D; ++a) in_box = in_box && (dist[a + 1] + (uint32_t)s_off[k * D + a] <= span[a + 1]);
@@ -195,20 +205,27 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
     if (lane == 0) atomicAdd(&s_cnt[k], (uint32_t)__popc(hits));
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < half; k += kKmapBlock)
+  for (int k = k_begin + threadIdx.x; k < k_end; k += kKmapBlock)
     block_counts[(size_t)k * n_blocks + blockIdx.x] = s_cnt[k];
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && blockIdx.y == 0) {
     const uint32_t row0 = blockIdx.x * kKmapBlock;
     block_counts[(size_t)half * n_blocks + blockIdx.x] = row0 < n ? min((uint32_t)kKmapBlock, n - row0) : 0u;
   }
 }
 
-// grid = K blocks of 1024 threads: exclusive scan of block_counts[k][0..n_blocks) in place,
-// totals[k] = number of pairs of offset k.
-__global__ void __launch_bounds__(1024) k_kmap_scan_blocks(uint32_t* __restrict__ block_counts,
-                                                           uint32_t n_blocks,
-                                                           uint32_t* __restrict__ totals) {
+// One block of 1024 threads per counted offset: exclusive scan of block_counts[k][0..n_blocks) in place, totals[k] = number
+// of pairs of offset k. The last block to finish writes offset_ptr[0..K] = exclusive scan of the totals, to host_ptr too
+// (mapped page-locked memory) where a host wants them.
+// mirror_half > 0 (self map): offsets K-1-k and k hold the same number of pairs, so only the first mirror_half + 1 offsets
+// have counts and blocks; the flag word records the half: the pair lists of the mirrored offsets are then the exchanged
+// lists of their mirror offsets (written by k_kmap_pairs together with the originals).
+__global__ void __launch_bounds__(1024) k_kmap_scan(uint32_t* __restrict__ block_counts, uint32_t n_blocks, int K,
+                                                    int mirror_half, uint32_t* __restrict__ totals,
+                                                    int64_t* __restrict__ offset_ptr, volatile int64_t* host_ptr) {
   __shared__ uint32_t warp_sums[32];
+  __shared__ int64_t warp_sums64[32];
+  __shared__ uint32_t s_last;
+  uint32_t* flags = totals + K;  // [0] "pair lists did not fit" (see rmn_kmap_pairs_status), [1] half, [2] ticket
   uint32_t* counts = block_counts + (size_t)blockIdx.x * n_blocks;
   const uint32_t per = (n_blocks + 1023u) / 1024u;
   const uint32_t begin = min(n_blocks, threadIdx.x * per), end = min(n_blocks, begin + per);
@@ -231,7 +248,11 @@ __global__ void __launch_bounds__(1024) k_kmap_scan_blocks(uint32_t* __restrict_
       if (lane >= d) wi += t;
     }
     warp_sums[lane] = wi - w;
-    if (lane == 31) totals[blockIdx.x] = wi;
+    if (lane == 31) {
+      totals[blockIdx.x] = wi;
+      __threadfence();
+      s_last = atomicAdd(flags + 2, 1u) == gridDim.x - 1 ? 1u : 0u;
+    }
   }
   __syncthreads();
   uint32_t run = warp_sums[warp] + incl - sum;
@@ -240,25 +261,37 @@ __global__ void __launch_bounds__(1024) k_kmap_scan_blocks(uint32_t* __restrict_
     counts[i] = run;
     run += v;
   }
-}
-
-// one thread: offset_ptr[0..K] = exclusive scan of totals (K is small)
-// mirror_half > 0 (self map): offsets K-1-k and k hold the same number of pairs, so the totals of
-// the mirrored half are copied from the probed half, and *mirror_flag records the half: the pair
-// lists of the mirrored offsets are then the exchanged lists of their mirror offsets (written by
-// k_kmap_pairs together with the originals) and need no per-block counts.
-__global__ void k_kmap_offset_ptr(uint32_t* __restrict__ totals, int K, int64_t* __restrict__ offset_ptr,
-                                  int mirror_half, uint32_t* mirror_flag) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int k = K - mirror_half; k < K; ++k) totals[k] = totals[K - 1 - k];
-  *mirror_flag = (uint32_t)mirror_half;
-  totals[K] = 0;  // "pair lists did not fit" flag of rmn_kmap_pairs (read by rmn_kmap_pairs_status)
-  int64_t run = 0;
-  for (int k = 0; k < K; ++k) {
-    offset_ptr[k] = run;
-    run += totals[k];
+  if (!s_last) return;
+  __threadfence();
+  if (threadIdx.x == 0) {
+    flags[0] = 0;
+    flags[1] = (uint32_t)mirror_half;
   }
-  offset_ptr[K] = run;
+  const int per_k = (K + 1023) / 1024, k0 = min(K, (int)threadIdx.x * per_k), k1 = min(K, k0 + per_k);
+  auto total = [&](int k) { return __ldcg(totals + (k >= K - mirror_half ? K - 1 - k : k)); };
+  int64_t sum64 = 0;
+  for (int k = k0; k < k1; ++k) sum64 += total(k);
+  int64_t incl64 = sum64;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int64_t t = __shfl_up_sync(0xFFFFFFFFu, incl64, d);
+    if (lane >= d) incl64 += t;
+  }
+  if (lane == 31) warp_sums64[warp] = incl64;
+  __syncthreads();
+  int64_t pos = incl64 - sum64;
+  for (int w = 0; w < warp; ++w) pos += warp_sums64[w];
+  for (int k = k0; k < k1; ++k) {
+    const uint32_t t = total(k);
+    offset_ptr[k] = pos;
+    if (host_ptr) host_ptr[k] = pos;
+    if (k >= K - mirror_half) totals[k] = t;
+    pos += t;
+    if (k == K - 1) {
+      offset_ptr[K] = pos;
+      if (host_ptr) host_ptr[K] = pos;
+    }
+  }
 }
 
 // Block b covers query rows [b*256, b*256+256). Warp w handles offsets
@@ -425,90 +458,92 @@ extern "C" size_t rmn_kmap_workspace_bytes(uint32_t n_query, int K) {
   return kmap_counts_bytes(n_query, K) + (use_block_index(n_query, K) ? block_index_bytes(n_query) : 0);
 }
 
+// Blocks that share the offsets of a row block (gridDim.y): about four blocks per SM in all, three offsets each at least.
+static unsigned offset_split(uint32_t n_blocks, int K) {
+  const uint32_t want = 148u * 4u / n_blocks, most = ((uint32_t)K + 2u) / 3u;
+  const uint32_t split = want < most ? want : most;
+  return split > 1 ? split : 1u;
+}
+
+static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_query, int W, const int32_t* d_offsets, int K,
+                      bool self, int32_t* d_nbr, int64_t* d_offset_ptr, void* d_workspace, size_t workspace_bytes,
+                      int64_t* host_ptr, cudaStream_t stream) {
+  if (!d_table || W < 2 || W > RMN_MAX_W || K < 1 || K > 4096 || (self && (K & 1) == 0) || !d_offsets || !d_offset_ptr ||
+      !d_workspace)
+    return RMN_ERR_BAD_ARG;
+  if (workspace_bytes < rmn_kmap_workspace_bytes(n_query, K)) return RMN_ERR_ALLOC;
+  if (n_query == 0) {
+    RMN_CUDA_TRY(cudaMemsetAsync(d_offset_ptr, 0, sizeof(int64_t) * (K + 1), stream));
+    if (host_ptr) memset(host_ptr, 0, sizeof(int64_t) * (K + 1));
+    return RMN_OK;
+  }
+  if (!d_query || !d_nbr || !coords_aligned(d_query, W)) return RMN_ERR_BAD_ARG;
+  int64_t* host_alias = nullptr;
+  if (host_ptr) {
+    void* p = nullptr;
+    RMN_CUDA_TRY(cudaHostGetDevicePointer(&p, host_ptr, 0));
+    host_alias = static_cast<int64_t*>(p);
+  }
+  const uint32_t nb = kmap_blocks(n_query);
+  uint32_t* block_counts = reinterpret_cast<uint32_t*>(d_workspace);
+  uint32_t* totals = block_counts + (size_t)K * nb;
+  uint32_t* ticket = totals + K + 2;
+  auto* h = reinterpret_cast<const TableHeader*>(d_table);
+  auto* slots =
+      reinterpret_cast<const Slot*>(reinterpret_cast<const char*>(d_table) + sizeof(TableHeader));
+  const int half = self ? K / 2 : 0;
+  if (self && use_block_index(n_query, K) && ((uintptr_t)d_workspace & 15) == 0) {
+    const BlockIndex ix = block_index(static_cast<char*>(d_workspace) + kmap_counts_bytes(n_query, K), n_query);
+    RMN_CUDA_TRY(cudaMemsetAsync(ix.slots, 0xFF, (size_t)ix.capacity * sizeof(BlockSlot) + 32, stream));
+    RMN_DISPATCH_W(W, k_block_insert<kW><<<nb, 256, 0, stream>>>(h, d_query, n_query, ix));
+    RMN_LAUNCH_CHECK();
+    k_block_bases<<<(ix.capacity + 255) / 256, 256, 0, stream>>>(ix);
+    RMN_LAUNCH_CHECK();
+    RMN_DISPATCH_W(W, k_block_scatter<kW><<<nb, 256, 0, stream>>>(h, d_query, n_query, ix));
+    RMN_LAUNCH_CHECK();
+    const size_t smem = (size_t)8 * kKmapBlock * 12 + (size_t)K * 4 + (size_t)half * 4;
+    RMN_DISPATCH_W(W, k_kmap_blocks_self<kW><<<nb, kKmapBlock, smem, stream>>>(h, slots, d_query, n_query, d_offsets, K,
+                                                                              d_nbr, block_counts, nb, ticket, ix));
+  } else if (self) {
+    if (half > 0)  // the mirrored half starts as "no neighbour"
+      RMN_CUDA_TRY(cudaMemsetAsync(d_nbr + (size_t)(half + 1) * n_query, 0xFF, (size_t)half * n_query * sizeof(int32_t),
+                                   stream));
+    const int hs = half > 0 ? half : 1;
+    const size_t smem = (size_t)hs * 8 + (size_t)hs * (W - 1) * 4 + (size_t)hs * 4;
+    RMN_DISPATCH_W(W, k_kmap_probe_self<kW><<<dim3(nb, offset_split(nb, half)), kKmapBlock, smem, stream>>>(
+                          h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket));
+  } else {
+    const size_t smem = (size_t)K * 8 + (size_t)K * (W - 1) * 4 + (size_t)K * 4;
+    RMN_DISPATCH_W(W, k_kmap_probe<kW><<<dim3(nb, offset_split(nb, K)), kKmapBlock, smem, stream>>>(
+                          h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket));
+  }
+  RMN_LAUNCH_CHECK();
+  k_kmap_scan<<<self ? half + 1 : K, 1024, 0, stream>>>(block_counts, nb, K, half, totals, d_offset_ptr, host_alias);
+  RMN_LAUNCH_CHECK();
+  return RMN_OK;
+}
+
 extern "C" int rmn_kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_query, int W,
                               const int32_t* d_offsets, int K, int32_t* d_nbr,
                               int64_t* d_offset_ptr, void* d_workspace, size_t workspace_bytes,
                               void* stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
-  if (!d_table || W < 2 || W > RMN_MAX_W || K < 1 || K > 4096 || !d_offsets || !d_offset_ptr ||
-      !d_workspace)
-    return RMN_ERR_BAD_ARG;
-  if (workspace_bytes < rmn_kmap_workspace_bytes(n_query, K)) return RMN_ERR_ALLOC;
-  const uint32_t nb = kmap_blocks(n_query);
-  uint32_t* block_counts = reinterpret_cast<uint32_t*>(d_workspace);
-  uint32_t* totals = block_counts + (size_t)K * nb;
-  if (n_query == 0) {
-    RMN_CUDA_TRY(cudaMemsetAsync(d_offset_ptr, 0, sizeof(int64_t) * (K + 1), stream));
-    return RMN_OK;
-  }
-  if (!d_query || !d_nbr || !coords_aligned(d_query, W)) return RMN_ERR_BAD_ARG;
-  auto* h = reinterpret_cast<const TableHeader*>(d_table);
-  auto* slots =
-      reinterpret_cast<const Slot*>(reinterpret_cast<const char*>(d_table) + sizeof(TableHeader));
-  const size_t smem = (size_t)K * 8 + (size_t)K * (W - 1) * 4 + (size_t)K * 4;
-  RMN_DISPATCH_W(W, k_kmap_probe<kW><<<nb, kKmapBlock, smem, stream>>>(
-                        h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb));
-  RMN_LAUNCH_CHECK();
-  k_kmap_scan_blocks<<<K, 1024, 0, stream>>>(block_counts, nb, totals);
-  RMN_LAUNCH_CHECK();
-  k_kmap_offset_ptr<<<1, 32, 0, stream>>>(totals, K, d_offset_ptr, 0, totals + K + 1);
-  RMN_LAUNCH_CHECK();
-  return RMN_OK;
+  return kmap_build(d_table, d_query, n_query, W, d_offsets, K, false, d_nbr, d_offset_ptr, d_workspace, workspace_bytes,
+                    nullptr, (cudaStream_t)stream_);
 }
 
 extern "C" int rmn_kmap_build_self(const void* d_table, const int32_t* d_coords, uint32_t n_rows, int W,
                                    const int32_t* d_offsets, int K, int32_t* d_nbr, int64_t* d_offset_ptr,
                                    void* d_workspace, size_t workspace_bytes, void* stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
-  if (!d_table || W < 2 || W > RMN_MAX_W || K < 1 || K > 4096 || (K & 1) == 0 || !d_offsets || !d_offset_ptr ||
-      !d_workspace)
-    return RMN_ERR_BAD_ARG;
-  if (workspace_bytes < rmn_kmap_workspace_bytes(n_rows, K)) return RMN_ERR_ALLOC;
-  const uint32_t nb = kmap_blocks(n_rows);
-  uint32_t* block_counts = reinterpret_cast<uint32_t*>(d_workspace);
-  uint32_t* totals = block_counts + (size_t)K * nb;
-  if (n_rows == 0) {
-    RMN_CUDA_TRY(cudaMemsetAsync(d_offset_ptr, 0, sizeof(int64_t) * (K + 1), stream));
-    return RMN_OK;
-  }
-  if (!d_coords || !d_nbr || !coords_aligned(d_coords, W)) return RMN_ERR_BAD_ARG;
-  auto* h = reinterpret_cast<const TableHeader*>(d_table);
-  auto* slots =
-      reinterpret_cast<const Slot*>(reinterpret_cast<const char*>(d_table) + sizeof(TableHeader));
-  const int half = K / 2;
-  if (use_block_index(n_rows, K) && ((uintptr_t)d_workspace & 15) == 0) {
-    const BlockIndex ix = block_index(static_cast<char*>(d_workspace) + kmap_counts_bytes(n_rows, K), n_rows);
-    RMN_CUDA_TRY(cudaMemsetAsync(ix.slots, 0xFF, (size_t)ix.capacity * sizeof(BlockSlot) + 32, stream));
-    RMN_DISPATCH_W(W, k_block_insert<kW><<<nb, 256, 0, stream>>>(h, d_coords, n_rows, ix));
-    RMN_LAUNCH_CHECK();
-    k_block_bases<<<(ix.capacity + 255) / 256, 256, 0, stream>>>(ix);
-    RMN_LAUNCH_CHECK();
-    RMN_DISPATCH_W(W, k_block_scatter<kW><<<nb, 256, 0, stream>>>(h, d_coords, n_rows, ix));
-    RMN_LAUNCH_CHECK();
-    const size_t smem = (size_t)8 * kKmapBlock * 12 + (size_t)K * 4 + (size_t)half * 4;
-    RMN_DISPATCH_W(W, k_kmap_blocks_self<kW><<<nb, kKmapBlock, smem, stream>>>(h, slots, d_coords, n_rows, d_offsets, K,
-                                                                              d_nbr, block_counts, nb, ix));
-    RMN_LAUNCH_CHECK();
-    k_kmap_scan_blocks<<<half + 1, 1024, 0, stream>>>(block_counts, nb, totals);
-    RMN_LAUNCH_CHECK();
-    k_kmap_offset_ptr<<<1, 32, 0, stream>>>(totals, K, d_offset_ptr, half, totals + K + 1);
-    RMN_LAUNCH_CHECK();
-    return RMN_OK;
-  }
-  if (half > 0)  // the mirrored half starts as "no neighbour"
-    RMN_CUDA_TRY(cudaMemsetAsync(d_nbr + (size_t)(half + 1) * n_rows, 0xFF, (size_t)half * n_rows * sizeof(int32_t),
-                                 stream));
-  const int hs = half > 0 ? half : 1;
-  const size_t smem = (size_t)hs * 8 + (size_t)hs * (W - 1) * 4 + (size_t)hs * 4;
-  RMN_DISPATCH_W(W, k_kmap_probe_self<kW><<<nb, kKmapBlock, smem, stream>>>(
-                        h, slots, d_coords, n_rows, d_offsets, K, d_nbr, block_counts, nb));
-  RMN_LAUNCH_CHECK();
-  // only the probed half (and the centre) is scanned here; see k_kmap_offset_ptr
-  k_kmap_scan_blocks<<<half + 1, 1024, 0, stream>>>(block_counts, nb, totals);
-  RMN_LAUNCH_CHECK();
-  k_kmap_offset_ptr<<<1, 32, 0, stream>>>(totals, K, d_offset_ptr, half, totals + K + 1);
-  RMN_LAUNCH_CHECK();
-  return RMN_OK;
+  return kmap_build(d_table, d_coords, n_rows, W, d_offsets, K, true, d_nbr, d_offset_ptr, d_workspace, workspace_bytes,
+                    nullptr, (cudaStream_t)stream_);
+}
+
+extern "C" int rmn_kmap_build_host(const void* d_table, const int32_t* d_query, uint32_t n_query, int W,
+                                   const int32_t* d_offsets, int K, int self, int32_t* d_nbr, int64_t* d_offset_ptr,
+                                   int64_t* h_offset_ptr_pinned, void* d_workspace, size_t workspace_bytes, void* stream_) {
+  if (!h_offset_ptr_pinned) return RMN_ERR_BAD_ARG;
+  return kmap_build(d_table, d_query, n_query, W, d_offsets, K, self != 0, d_nbr, d_offset_ptr, d_workspace,
+                    workspace_bytes, h_offset_ptr_pinned, (cudaStream_t)stream_);
 }
 
 static int kmap_pairs_launch(const int32_t* d_nbr, uint32_t n_query, int K, const int64_t* d_offset_ptr,

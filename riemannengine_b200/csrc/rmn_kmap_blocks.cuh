@@ -168,7 +168,8 @@ template <int W>
 __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots, const int32_t* __restrict__ coords, uint32_t n,
     const int32_t* __restrict__ offsets, int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts,
-    uint32_t n_blocks, BlockIndex ix) {
+    uint32_t n_blocks, uint32_t* __restrict__ scan_ticket, BlockIndex ix) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scan_ticket = 0;
   using B = BlockCoords<W>;
   constexpr int D = W - 1, NA = B::NA, CELLS = 1 << NA;
   constexpr uint32_t kNever = 1u << 28, kFar = 1u << 29, kNewOuter = 1u << 30;

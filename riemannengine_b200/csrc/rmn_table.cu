@@ -5,9 +5,11 @@
 //   256-byte memset of the header
 //   -> fill + range (slots to the empty pattern, column min/max; the last block plans the bit packing)
 //   -> insert (one 16-byte CAS on the packed key, atomicMin on the first row)
-//   -> count (rows that are the first occurrence, per 256-row block; the last block scans the counts)
+//   -> count (rows that are the first occurrence, per 256-row block; the last block scans the counts and, where the
+//      caller waits for them, stores the header's words into the host's memory)
 //   -> finalize (unique ids, mapping, unique coordinates; identity inverse when nothing was a duplicate)
 //   -> inverse (only does work when there were duplicates)
+// Up to kSmallRows rows one block does all of it in one launch.
 // Numbering unique rows by first occurrence reproduces the reference CPU map
 // (engine/grid/lattice_cpu.hpp:419-444) deterministically; the reference GPU
 // map lets a CAS race pick the surviving duplicate
@@ -17,8 +19,10 @@
 #include <cuda_bf16.h>
 
 #include <limits.h>
+#include <string.h>
 #include <stddef.h>
 
+#include <atomic>
 #include <mutex>
 
 namespace rmn {
@@ -28,8 +32,68 @@ int tc_clear_status();
 const uint32_t* tc_status_device_address();
 
 constexpr int kRowsPerBlock = 256;
+constexpr uint32_t kGrid = 148 * 8;  // blocks of the passes that may have nothing to do
+
+// Scratch of a build of n rows: slot of every row, rows that are the first of their key per 256-row block (then the
+// blocks' offsets), and one bit per row for them
+struct Scratch {
+  uint32_t* slot_of_row;
+  uint32_t* block_counts;
+  uint32_t* first_bits;
+};
+constexpr size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
+constexpr size_t scratch_bytes(size_t n) {
+  const size_t nb = (n + kRowsPerBlock - 1) / kRowsPerBlock;
+  return align16(n * 4) + align16((nb + 1) * 4) + nb * (kRowsPerBlock / 8) + 256;
+}
+inline Scratch scratch(void* workspace, uint32_t n) {
+  const size_t nb = (n + kRowsPerBlock - 1) / kRowsPerBlock;
+  char* p = reinterpret_cast<char*>(((uintptr_t)workspace + 15) & ~(uintptr_t)15);
+  Scratch s;
+  s.slot_of_row = reinterpret_cast<uint32_t*>(p);
+  s.block_counts = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4));
+  s.first_bits = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4) + align16((nb + 1) * 4));
+  return s;
+}
+
+// Words that a build stores into page-locked host memory for a host that polls: rmn_table_info's four, the convolution
+// kernels' status word and, last, the number of this build.
+struct HostPost {
+  volatile uint32_t* words;  // NULL: nobody waits
+  const uint32_t* conv_status;
+  uint32_t sequence;
+
+  __device__ void store(const TableHeader* h, uint32_t n_unique) const {
+    if (!words) return;
+    words[0] = n_unique;
+    words[1] = *(const volatile uint32_t*)&h->status;
+    words[2] = h->capacity;
+    words[3] = h->n_rows;
+    words[4] = conv_status ? *conv_status : 0u;
+    __threadfence_system();
+    words[5] = sequence;
+  }
+};
 
 __device__ void plan_packing(TableHeader* h);
+
+// One thread: the header's constants, the decoded column bounds and the key packing.
+__device__ void write_header(TableHeader* h, uint32_t W, uint32_t n, uint32_t capacity) {
+  h->magic = kTableMagic;
+  h->W = W;
+  h->n_rows = n;
+  h->capacity = capacity;
+  for (uint32_t c = 0; c < RMN_MAX_W; ++c) {
+    const uint32_t en = *(volatile uint32_t*)&h->mn_enc[c], ex = *(volatile uint32_t*)&h->mx_enc[c];
+    h->mn[c] = (c < W && n > 0) ? (int32_t)(~en ^ 0x80000000u) : 0;
+    h->mx[c] = (c < W && n > 0) ? (int32_t)(ex ^ 0x80000000u) : 0;
+    h->bits[c] = 0;
+    h->shift[c] = 0;
+  }
+  const uint32_t o = *(volatile uint32_t*)&h->x_or;
+  h->pos_shift = o ? (uint32_t)(__ffs((int)o) - 1) : 0u;
+  plan_packing(h);
+}
 
 // First kernel of a build, on a header that a 256-byte memset has zeroed: fills the slots with the empty
 // pattern (all ones) and reduces the column bounds of the rows in the same pass (the fill writes, the
@@ -95,23 +159,7 @@ __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ 
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(&h->range_blocks_done, 1u) == gridDim.x - 1) {
     __threadfence();
-    h->magic = kTableMagic;
-    h->W = W;
-    h->n_rows = n;
-    h->capacity = capacity;
-    for (int c = 0; c < RMN_MAX_W; ++c) {
-      // volatile: the bounds were written by other blocks' atomics
-      const uint32_t en = *(volatile uint32_t*)&h->mn_enc[c], ex = *(volatile uint32_t*)&h->mx_enc[c];
-      h->mn[c] = (c < W && n > 0) ? (int32_t)(~en ^ 0x80000000u) : 0;
-      h->mx[c] = (c < W && n > 0) ? (int32_t)(ex ^ 0x80000000u) : 0;
-      h->bits[c] = 0;
-      h->shift[c] = 0;
-    }
-    {
-      const uint32_t o = *(volatile uint32_t*)&h->x_or;
-      h->pos_shift = o ? (uint32_t)(__ffs((int)o) - 1) : 0u;
-    }
-    plan_packing(h);
+    write_header(h, W, n, capacity);
   }
 }
 
@@ -150,125 +198,164 @@ __device__ __forceinline__ void cas_slot(Slot* slot, unsigned long long key, uns
       : "memory");
 }
 
+// Claims the slot of a row's key: {key, first_row = row, uid = row}. Without duplicates the unique numbering is the row
+// numbering and the slot is final after this single 16-byte compare-and-swap. A row that finds its key taken lowers
+// first_row; *dup tells (k_finalize then renumbers). look_first: read a slot before the compare-and-swap and spare it, and
+// the atomic minimum, where the key is there already with a smaller row - the usual case among many duplicates (1.2 M rows
+// on 0.27 M strided cells: 60 -> 25 us), a second round trip to the slot without them.
+__device__ __forceinline__ bool insert_row(Slot* slots, uint32_t capacity, uint32_t pos_shift, unsigned long long key,
+                                           uint32_t row, bool look_first, uint32_t* slot_of_row, bool* dup) {
+  uint32_t s = hash_key(key, capacity, pos_shift);
+  const unsigned long long mine = (unsigned long long)row | ((unsigned long long)row << 32);
+  for (uint32_t probe = 0; probe < (capacity >> 3); ++probe) {
+    unsigned long long cur_key = kEmptyKey, cur_rows = ~0ull;
+    if (look_first) {
+      const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(slots + s));
+      cur_key = v.x;
+      cur_rows = v.y;
+    }
+    if (cur_key == kEmptyKey) {
+      cas_slot(&slots[s], key, mine, cur_key, cur_rows);
+    }
+    if (cur_key == kEmptyKey || cur_key == key) {
+      if (cur_key == key) {
+        if ((uint32_t)cur_rows > row) atomicMin(&slots[s].first_row, row);
+        *dup = true;
+      }
+      slot_of_row[row] = s;
+      return true;
+    }
+    // another key lives here and this one walks on: leave word for the lookups (kPassedBit)
+    // (all ones: the key has been seen before its rows)
+    if (cur_rows == ~0ull || !((uint32_t)(cur_rows >> 32) & kPassedBit)) atomicOr(&slots[s].uid, kPassedBit);
+    s = next_slot(s, capacity);
+  }
+  return false;
+}
+
 template <int W>
 __global__ void __launch_bounds__(256) k_insert(const int32_t* __restrict__ coords, uint32_t n,
                                                 TableHeader* h, Slot* slots,
-                                                uint32_t* __restrict__ slot_of_row) {
+                                                uint32_t* __restrict__ slot_of_row, int look_first) {
   if (h->status != RMN_OK) return;
   const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= n) return;
-  Packer<W> pk;
-  pk.load(h);
-  const uint32_t capacity = h->capacity;
-  int32_t c[W];
-  load_row<W>(coords, row, c);
-  unsigned long long key;
-  pk.pack(c, key);
-  uint32_t s = hash_key(key, capacity, h->pos_shift);
-  bool placed = false;
-  // One 16-byte compare-and-swap claims a free slot (all ones) with {key, first_row = row,
-  // uid = row}: without duplicates the unique numbering is the row numbering and the slot is
-  // final after this single memory operation. A row that finds its key taken lowers first_row
-  // and counts itself as a duplicate (k_finalize then renumbers).
-  const unsigned long long mine = (unsigned long long)row | ((unsigned long long)row << 32);
-  for (uint32_t probe = 0; probe < (capacity >> 3); ++probe) {
-    unsigned long long cur_key, cur_rows;
-    cas_slot(&slots[s], key, mine, cur_key, cur_rows);
-    if (cur_key == kEmptyKey || cur_key == key) {
-      if (cur_key == key) {
-        atomicMin(&slots[s].first_row, row);
-        atomicAdd(&h->n_dups, 1u);
-      }
-      slot_of_row[row] = s;
-      placed = true;
-      break;
-    }
-    // another key lives here and this one walks on: leave word for the lookups (kPassedBit)
-    if (!((uint32_t)(cur_rows >> 32) & kPassedBit)) atomicOr(&slots[s].uid, kPassedBit);
-    s = next_slot(s, capacity);
+  bool dup = false;
+  if (row < n) {
+    Packer<W> pk;
+    pk.load(h);
+    int32_t c[W];
+    load_row<W>(coords, row, c);
+    unsigned long long key;
+    pk.pack(c, key);
+    if (!insert_row(slots, h->capacity, h->pos_shift, key, row, look_first != 0, slot_of_row, &dup))
+      atomicExch(&h->status, (uint32_t)RMN_ERR_PROBE_LIMIT);
   }
-  if (!placed) atomicExch(&h->status, (uint32_t)RMN_ERR_PROBE_LIMIT);
+  const int dups = __syncthreads_count(dup);  // one atomic per block: the rows' own would serialise on the word
+  if (threadIdx.x == 0 && dups) atomicAdd(&h->n_dups, (uint32_t)dups);
 }
 
-// In-place exclusive scan of counts[n] by ONE block (any multiple of 32 threads up to 1024); the total goes
-// to *total_out. Reads bypass the L1: the counts may have been written by other blocks of the same launch.
-__device__ __forceinline__ void scan_u32_block(uint32_t* __restrict__ counts, uint32_t n, uint32_t* total_out) {
-  __shared__ uint32_t warp_sums[32];
-  const uint32_t nthreads = blockDim.x, nwarps = nthreads >> 5;
-  const uint32_t per = (n + nthreads - 1u) / nthreads;
-  const uint32_t begin = min(n, threadIdx.x * per), end = min(n, begin + per);
-  uint32_t sum = 0;
-  for (uint32_t i = begin; i < end; ++i) sum += __ldcg(counts + i);
-  // block exclusive scan of `sum`
-  uint32_t incl = sum;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// In-place exclusive scan of counts[n] by ONE block (any multiple of 32 threads up to 1024), sixteen counts per thread and
+// step; returns the total. Reads bypass the L1: the counts may have been written by other blocks of the same launch.
+// counts is 16-byte aligned and may be read up to the next multiple of four.
+__device__ __forceinline__ uint32_t scan_u32_block(uint32_t* __restrict__ counts, uint32_t n) {
+  __shared__ uint32_t warp_sums[33];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < n; base += blockDim.x * 16u) {
+    const uint32_t i0 = base + threadIdx.x * 16u;
+    uint32_t v[16];
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-    if (lane >= (uint32_t)d) incl += t;
-  }
-  if (lane == 31) warp_sums[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = lane < nwarps ? warp_sums[lane] : 0u, wi = w;
+    for (int q = 0; q < 4; ++q) {
+      uint4 x = make_uint4(0u, 0u, 0u, 0u);
+      if (i0 + 4 * q < n) x = __ldcg(reinterpret_cast<const uint4*>(counts + i0) + q);
+      v[4 * q] = x.x, v[4 * q + 1] = x.y, v[4 * q + 2] = x.z, v[4 * q + 3] = x.w;
+    }
+    uint32_t sum = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t x = i0 + i < n ? v[i] : 0u;
+      v[i] = sum;
+      sum += x;
+    }
+    uint32_t incl = sum;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wi, d);
-      if (lane >= (uint32_t)d) wi += t;
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= (uint32_t)d) incl += t;
     }
-    warp_sums[lane] = wi - w;  // exclusive
-    if (lane == 31 && total_out) *total_out = wi;
+    __syncthreads();  // (the sums of the step before have been read)
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t w = lane < nwarps ? warp_sums[lane] : 0u;
+      uint32_t wi = w;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wi, d);
+        if (lane >= (uint32_t)d) wi += t;
+      }
+      warp_sums[lane] = wi - w;  // exclusive
+      if (lane == 31) warp_sums[32] = wi;
+    }
+    __syncthreads();
+    const uint32_t before = carry + warp_sums[warp] + incl - sum;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (i0 + i < n) counts[i0 + i] = before + v[i];
+    carry += warp_sums[32];
   }
-  __syncthreads();
-  uint32_t run = warp_sums[warp] + incl - sum;
-  for (uint32_t i = begin; i < end; ++i) {
-    uint32_t v = __ldcg(counts + i);
-    counts[i] = run;
-    run += v;
-  }
+  return carry;
 }
 
-// Rows that are the first occurrence of their key, counted per 256-row block; the last block to finish
-// turns the counts into block offsets (exclusive scan) and writes n_unique. Returns at once when the
-// insert pass met no duplicate: nothing is compacted then (see k_finalize).
-__global__ void __launch_bounds__(kRowsPerBlock) k_count_first(const Slot* __restrict__ slots,
-                                                              const uint32_t* __restrict__ slot_of_row,
-                                                              uint32_t n, TableHeader* h,
-                                                              uint32_t* __restrict__ block_counts) {
-  if (h->status != RMN_OK) return;
-  if (h->n_dups == 0) {  // every row is its own first occurrence: publish the count, nothing to compact
-    if (blockIdx.x == 0 && threadIdx.x == 0) h->n_unique = n;
+// Rows that are the first occurrence of their key: a bit per row, and their number per 256-row block; the last block to
+// finish turns the numbers into block offsets (exclusive scan) and writes n_unique. Nothing to do when the insert pass
+// met no duplicate: nothing is compacted then (see k_finalize).
+__global__ void __launch_bounds__(kRowsPerBlock) k_count_first(const Slot* __restrict__ slots, uint32_t n, TableHeader* h,
+                                                              Scratch sc, HostPost post) {
+  const bool failed = h->status != RMN_OK;
+  if (failed || h->n_dups == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (!failed) h->n_unique = n;
+      post.store(h, failed ? 0u : n);
+    }
     return;
   }
   __shared__ uint32_t s_last;
-  const uint32_t row = blockIdx.x * kRowsPerBlock + threadIdx.x;
-  int flag = 0;
-  if (row < n) flag = slots[slot_of_row[row]].first_row == row;
-  int total = __syncthreads_count(flag);
+  const uint32_t nb = (n + kRowsPerBlock - 1) / kRowsPerBlock;
+  for (uint32_t block = blockIdx.x; block < nb; block += gridDim.x) {
+    const uint32_t row = block * kRowsPerBlock + threadIdx.x;
+    bool first = false;
+    if (row < n) first = slots[sc.slot_of_row[row]].first_row == row;
+    const uint32_t bits = __ballot_sync(0xFFFFFFFFu, first);
+    if ((threadIdx.x & 31) == 0) sc.first_bits[block * (kRowsPerBlock / 32) + (threadIdx.x >> 5)] = bits;
+    const int total = __syncthreads_count(first);
+    if (threadIdx.x == 0) sc.block_counts[block] = (uint32_t)total;
+  }
   if (threadIdx.x == 0) {
-    block_counts[blockIdx.x] = (uint32_t)total;
     __threadfence();
     s_last = atomicAdd(&h->count_blocks_done, 1u) == gridDim.x - 1 ? 1u : 0u;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  scan_u32_block(block_counts, gridDim.x, &h->n_unique);
+  const uint32_t n_unique = scan_u32_block(sc.block_counts, nb);
+  if (threadIdx.x == 0) {
+    h->n_unique = n_unique;
+    post.store(h, n_unique);
+  }
 }
 
 template <int W>
 __global__ void __launch_bounds__(kRowsPerBlock) k_finalize(
     const int32_t* __restrict__ coords, uint32_t n, const TableHeader* h, Slot* slots,
-    const uint32_t* __restrict__ slot_of_row, const uint32_t* __restrict__ block_offsets,
-    int64_t* __restrict__ mapping, int32_t* __restrict__ unique_coords, int64_t* __restrict__ inverse) {
-  __shared__ uint32_t warp_counts[kRowsPerBlock / 32];
+    Scratch sc, int64_t* __restrict__ mapping, int32_t* __restrict__ unique_coords, int64_t* __restrict__ inverse) {
   if (h->status != RMN_OK) return;
   const uint32_t row = blockIdx.x * kRowsPerBlock + threadIdx.x;
   if (h->n_dups == 0) {
     // Fast path (all rows distinct): unique row == input row, already stored in the slots by
     // k_insert; only the identity mapping and the coordinate copy remain (both streaming).
     if (row < n) {
-      mapping[row] = (int64_t)row;
+      if (mapping) mapping[row] = (int64_t)row;
       if (inverse) inverse[row] = (int64_t)row;
       if (unique_coords) {
         int32_t c[W];
@@ -280,28 +367,20 @@ __global__ void __launch_bounds__(kRowsPerBlock) k_finalize(
     if (row == 0) const_cast<TableHeader*>(h)->n_unique = n;
     return;
   }
+  if (row >= n) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t s = 0;
-  int flag = 0;
-  if (row < n) {
-    s = slot_of_row[row];
-    flag = slots[s].first_row == row;
-  }
-  const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, flag);
-  if (lane == 0) warp_counts[warp] = __popc(ballot);
-  __syncthreads();
-  uint32_t base = block_offsets[blockIdx.x];
-  for (int w = 0; w < warp; ++w) base += warp_counts[w];
-  if (flag) {
-    const uint32_t uid = base + __popc(ballot & ((1u << lane) - 1u));
-    slots[s].uid = uid | (slots[s].uid & kPassedBit);
-    mapping[uid] = (int64_t)row;
-    if (unique_coords) {
-      int32_t c[W];
-      load_row<W>(coords, row, c);
+  const uint32_t* bits = sc.first_bits + blockIdx.x * (kRowsPerBlock / 32);
+  if (!((__ldg(bits + warp) >> lane) & 1u)) return;
+  uint32_t uid = sc.block_counts[blockIdx.x] + __popc(__ldg(bits + warp) & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) uid += __popc(__ldg(bits + w));
+  const uint32_t s = sc.slot_of_row[row];
+  slots[s].uid = uid | (slots[s].uid & kPassedBit);
+  if (mapping) mapping[uid] = (int64_t)row;
+  if (unique_coords) {
+    int32_t c[W];
+    load_row<W>(coords, row, c);
 #pragma unroll
-      for (int i = 0; i < W; ++i) unique_coords[(size_t)uid * W + i] = c[i];
-    }
+    for (int i = 0; i < W; ++i) unique_coords[(size_t)uid * W + i] = c[i];
   }
 }
 
@@ -311,9 +390,134 @@ __global__ void __launch_bounds__(256) k_inverse(const Slot* __restrict__ slots,
                                                  int64_t* __restrict__ inverse) {
   // without duplicates k_finalize has already written the identity
   if (h->n_dups == 0 || h->status != RMN_OK) return;
-  const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= n) return;
-  inverse[row] = (int64_t)(slots[slot_of_row[row]].uid & ~kPassedBit);
+  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n; row += gridDim.x * blockDim.x)
+    inverse[row] = (int64_t)(slots[slot_of_row[row]].uid & ~kPassedBit);
+}
+
+// The whole build of a small table by one block: what a chain of six launches costs there is the launches (900 rows:
+// 20 us with their gaps).
+constexpr uint32_t kSmallRows = 2048;
+template <int W>
+__global__ void __launch_bounds__(1024) k_build_small(const int32_t* __restrict__ coords, uint32_t n, TableHeader* h,
+                                                      Slot* slots, uint32_t capacity, Scratch sc,
+                                                      int64_t* __restrict__ mapping, int32_t* __restrict__ unique_coords,
+                                                      int64_t* __restrict__ inverse, int look_first, HostPost post) {
+  constexpr int NA = W - 1 < 3 ? W - 1 : 3;
+  __shared__ TableHeader s_h;
+  __shared__ uint32_t s_ok;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  if (tid < sizeof(TableHeader) / 4) reinterpret_cast<uint32_t*>(&s_h)[tid] = 0u;
+  if (tid == 0) s_ok = 1u;
+  const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (uint32_t i = tid; i < capacity; i += 1024) reinterpret_cast<uint4*>(slots)[i] = ones;
+  int32_t row_c[2][W];
+  int32_t mn[W], mx[W];
+  uint32_t first[NA], col_or[NA];
+#pragma unroll
+  for (int c = 0; c < W; ++c) { mn[c] = INT_MAX; mx[c] = INT_MIN; }
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+    first[a] = (uint32_t)__ldg(coords + 1 + a);
+    col_or[a] = 0;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t row = tid + i * 1024;
+    if (row >= n) continue;
+    load_row<W>(coords, row, row_c[i]);
+#pragma unroll
+    for (int c = 0; c < W; ++c) { mn[c] = min(mn[c], row_c[i][c]); mx[c] = max(mx[c], row_c[i][c]); }
+#pragma unroll
+    for (int a = 0; a < NA; ++a) col_or[a] |= (uint32_t)row_c[i][1 + a] - first[a];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < W; ++c) {
+    const int32_t a = __reduce_min_sync(0xFFFFFFFFu, mn[c]), b = __reduce_max_sync(0xFFFFFFFFu, mx[c]);
+    if (lane == 0 && a <= b) {
+      atomicMax(&s_h.mn_enc[c], ~((uint32_t)a ^ 0x80000000u));
+      atomicMax(&s_h.mx_enc[c], (uint32_t)b ^ 0x80000000u);
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+    const uint32_t o = __reduce_or_sync(0xFFFFFFFFu, col_or[a]);
+    if (lane == 0 && o) atomicOr(a == 0 ? &s_h.x_or : &s_h.yz_or[a - 1], o);
+  }
+  __syncthreads();
+  if (tid == 0) write_header(&s_h, W, n, capacity);
+  __syncthreads();
+  const bool range_ok = s_h.status == RMN_OK;
+  uint32_t dups = 0;
+  if (range_ok) {
+    Packer<W> pk;
+    pk.load(&s_h);
+    bool dup[2] = {false, false};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t row = tid + i * 1024;
+      if (row >= n) continue;
+      unsigned long long key;
+      pk.pack(row_c[i], key);
+      if (!insert_row(slots, capacity, s_h.pos_shift, key, row, look_first != 0, sc.slot_of_row, &dup[i])) s_ok = 0u;
+    }
+    dups = (uint32_t)(__syncthreads_count(dup[0]) + __syncthreads_count(dup[1]));
+    if (tid == 0) {
+      s_h.n_dups = dups;
+      if (!s_ok) s_h.status = RMN_ERR_PROBE_LIMIT;
+    }
+    __syncthreads();
+  }
+  const bool ok = range_ok && s_h.status == RMN_OK;
+  if (ok && dups == 0) {
+    if (tid == 0) s_h.n_unique = n;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t row = tid + i * 1024;
+      if (row >= n) continue;
+      if (mapping) mapping[row] = (int64_t)row;
+      if (inverse) inverse[row] = (int64_t)row;
+      if (unique_coords) {
+#pragma unroll
+        for (int c = 0; c < W; ++c) unique_coords[(size_t)row * W + c] = row_c[i][c];
+      }
+    }
+  } else if (ok) {
+    __shared__ uint32_t s_warp[33];
+    uint32_t carry = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t row = tid + i * 1024;
+      const uint32_t s = row < n ? sc.slot_of_row[row] : 0u;
+      const bool is_first = row < n && __ldcg(&slots[s].first_row) == row;
+      const uint32_t bits = __ballot_sync(0xFFFFFFFFu, is_first);
+      if (lane == 0) s_warp[tid >> 5] = (uint32_t)__popc(bits);
+      __syncthreads();
+      uint32_t before = carry, total = 0;
+      for (uint32_t w = 0; w < 32; ++w) {
+        if (w < (tid >> 5)) before += s_warp[w];
+        total += s_warp[w];
+      }
+      carry += total;
+      if (is_first) {
+        const uint32_t uid = before + __popc(bits & ((1u << lane) - 1u));
+        slots[s].uid = uid | (__ldcg(&slots[s].uid) & kPassedBit);
+        if (mapping) mapping[uid] = (int64_t)row;
+        if (unique_coords) {
+#pragma unroll
+          for (int c = 0; c < W; ++c) unique_coords[(size_t)uid * W + c] = row_c[i][c];
+        }
+      }
+      __syncthreads();
+    }
+    if (tid == 0) s_h.n_unique = carry;
+    if (inverse)
+      for (uint32_t row = tid; row < n; row += 1024)
+        inverse[row] = (int64_t)(__ldcg(&slots[sc.slot_of_row[row]].uid) & ~kPassedBit);
+  }
+  __syncthreads();
+  if (tid < sizeof(TableHeader) / 4) reinterpret_cast<uint32_t*>(h)[tid] = reinterpret_cast<const uint32_t*>(&s_h)[tid];
+  if (tid == 0) post.store(&s_h, s_h.n_unique);
 }
 
 template <int W>
@@ -338,38 +542,57 @@ struct StrideArg {
   int32_t s[RMN_MAX_W];
 };
 
-__global__ void __launch_bounds__(256) k_stride(const int32_t* __restrict__ coords, uint64_t total,
-                                                int W, StrideArg st, int32_t* __restrict__ out) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int col = (int)(i % (uint64_t)W);
-  int32_t c = coords[i];
-  if (col > 0) {
-    const int32_t s = st.s[col - 1];
-    int32_t q = c / s;
-    if ((c % s != 0) && (c < 0)) --q;  // floor for negative coordinates
-    c = q * s;
+// floor(c / s) * s; s == 1 and powers of two without a division
+__device__ __forceinline__ int32_t floor_to(int32_t c, int32_t s) {
+  if ((s & (s - 1)) == 0) return c & -s;
+  int32_t q = c / s;
+  if (c < 0 && q * s != c) --q;  // floor for negative coordinates
+  return q * s;
+}
+
+// One thread per row (1.2 M rows of four columns: 24 -> 8 us against one thread per element with a 64-bit remainder).
+// kVec: rows of four columns as one 16-byte access (aligned pointers).
+template <int W, bool kVec>
+__global__ void __launch_bounds__(256) k_stride(const int32_t* __restrict__ coords, uint32_t n, StrideArg st,
+                                                int32_t* __restrict__ out) {
+  const uint32_t row = blockIdx.x * 256 + threadIdx.x;
+  if (row >= n) return;
+  int32_t c[W];
+  if constexpr (kVec) {
+    load_row<W>(coords, row, c);
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; ++i) c[i] = __ldg(coords + (size_t)row * W + i);
   }
-  out[i] = c;
+#pragma unroll
+  for (int i = 1; i < W; ++i) c[i] = floor_to(c[i], st.s[i - 1]);
+  store_row<W, kVec>(out, row, c);
 }
 
 // Continuous (field) coordinates -> integer voxel coordinates, the reference's rule in float32:
 // batch column lroundf(v), spatial column j: stride_j * (int)floor(v / stride_j)
-// (engine/grid/lattice_cpu.hpp:944-984, engine/grid/lattice_gpu.cu:78-151). One thread per element, streaming.
-__global__ void __launch_bounds__(256) k_field_quantize(const float* __restrict__ field, uint64_t total, int W,
-                                                        StrideArg st, int32_t* __restrict__ out) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int col = (int)(i % (uint64_t)W);
-  const float v = field[i];
-  int32_t c;
-  if (col == 0) {
-    c = (int32_t)lroundf(v);
+// (engine/grid/lattice_cpu.hpp:944-984, engine/grid/lattice_gpu.cu:78-151). One thread per row, streaming.
+template <int W, bool kVec>
+__global__ void __launch_bounds__(256) k_field_quantize(const float* __restrict__ field, uint32_t n, StrideArg st,
+                                                        int32_t* __restrict__ out) {
+  const uint32_t row = blockIdx.x * 256 + threadIdx.x;
+  if (row >= n) return;
+  float v[W];
+  if constexpr (kVec) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(field) + row);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
   } else {
-    const int32_t s = st.s[col - 1];
-    c = s == 1 ? (int32_t)floorf(v) : s * (int32_t)floorf(__fdiv_rn(v, (float)s));
+#pragma unroll
+    for (int i = 0; i < W; ++i) v[i] = __ldg(field + (size_t)row * W + i);
   }
-  out[i] = c;
+  int32_t c[W];
+  c[0] = (int32_t)lroundf(v[0]);
+#pragma unroll
+  for (int i = 1; i < W; ++i) {
+    const int32_t s = st.s[i - 1];
+    c[i] = s == 1 ? (int32_t)floorf(v[i]) : s * (int32_t)floorf(__fdiv_rn(v[i], (float)s));
+  }
+  store_row<W, kVec>(out, row, c);
 }
 
 // out = (int32)floor((double)v / q) on EVERY column (q <= 0: floor only): the discretisation step of
@@ -459,8 +682,11 @@ extern "C" int rmn_field_quantize(const float* d_field, uint32_t n_rows, int W, 
     if (tensor_stride[a] <= 0) return RMN_ERR_BAD_ARG;
     st.s[a] = tensor_stride[a];
   }
-  const uint64_t total = (uint64_t)n_rows * W;
-  k_field_quantize<<<(uint32_t)((total + 255) / 256), 256, 0, stream>>>(d_field, total, W, st, d_out);
+  const uint32_t nb = (n_rows + 255) / 256;
+  if (W == 4 && !((uintptr_t)d_field & 15) && !((uintptr_t)d_out & 15))
+    k_field_quantize<4, true><<<nb, 256, 0, stream>>>(d_field, n_rows, st, d_out);
+  else
+    RMN_DISPATCH_W(W, k_field_quantize<kW, false><<<nb, 256, 0, stream>>>(d_field, n_rows, st, d_out));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -509,8 +735,74 @@ extern "C" size_t rmn_table_bytes(uint32_t n_rows) {
 }
 
 extern "C" size_t rmn_table_build_workspace_bytes(uint32_t n_rows) {
-  const size_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
-  return (size_t)n_rows * 4 + (nb + 1) * 4 + 256;
+  return scratch_bytes(n_rows);
+}
+
+static int table_build_args(const int32_t* d_coords, uint32_t n_rows, int W, const void* d_table, size_t table_bytes,
+                            const void* d_workspace, size_t workspace_bytes) {
+  if (!d_table || W < 2 || W > RMN_MAX_W || n_rows >= 0x7FFFFFFFu) return RMN_ERR_BAD_ARG;
+  if (n_rows > 0 && (!d_coords || !d_workspace)) return RMN_ERR_BAD_ARG;
+  if (((uintptr_t)d_table & 15) || !coords_aligned(d_coords, W)) return RMN_ERR_BAD_ARG;
+  if (table_bytes < rmn_table_bytes(n_rows) ||
+      (n_rows > 0 && workspace_bytes < rmn_table_build_workspace_bytes(n_rows)))
+    return RMN_ERR_ALLOC;
+  return RMN_OK;
+}
+
+static int table_build_begin(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table, void* d_workspace,
+                             int look_first, const HostPost& post, cudaStream_t stream) {
+  auto* h = reinterpret_cast<TableHeader*>(d_table);
+  auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
+  const uint32_t capacity = table_capacity(n_rows);
+  RMN_CUDA_TRY(cudaMemsetAsync(h, 0, sizeof(TableHeader), stream));
+  {
+    const uint32_t fill_blocks = (capacity + 255u) / 256u;
+    const uint32_t blocks = fill_blocks < kGrid ? fill_blocks : kGrid;
+    RMN_DISPATCH_W(W, k_fill_range<kW><<<blocks, 256, 0, stream>>>(d_coords, n_rows, h,
+                                                                    reinterpret_cast<uint4*>(slots), capacity));
+    RMN_LAUNCH_CHECK();
+  }
+  if (n_rows == 0) return RMN_OK;
+  const Scratch sc = scratch(d_workspace, n_rows);
+  const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
+  RMN_DISPATCH_W(W, k_insert<kW><<<nb, 256, 0, stream>>>(d_coords, n_rows, h, slots, sc.slot_of_row, look_first));
+  RMN_LAUNCH_CHECK();
+  k_count_first<<<nb < kGrid ? nb : kGrid, kRowsPerBlock, 0, stream>>>(slots, n_rows, h, sc, post);
+  RMN_LAUNCH_CHECK();
+  return RMN_OK;
+}
+
+static int table_build_finish(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table, int64_t* d_mapping,
+                              int64_t* d_inverse, int32_t* d_unique_coords, void* d_workspace, cudaStream_t stream) {
+  auto* h = reinterpret_cast<TableHeader*>(d_table);
+  auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
+  const Scratch sc = scratch(d_workspace, n_rows);
+  const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
+  RMN_DISPATCH_W(W, k_finalize<kW><<<nb, kRowsPerBlock, 0, stream>>>(d_coords, n_rows, h, slots, sc, d_mapping,
+                                                                     d_unique_coords, d_inverse));
+  RMN_LAUNCH_CHECK();
+  if (d_inverse) {  // optional: only the quantisation modes that average or sample features read it
+    k_inverse<<<nb < kGrid ? nb : kGrid, 256, 0, stream>>>(slots, sc.slot_of_row, n_rows, h, d_inverse);
+    RMN_LAUNCH_CHECK();
+  }
+  return RMN_OK;
+}
+
+static int table_build(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table, int64_t* d_mapping,
+                       int64_t* d_inverse, int32_t* d_unique_coords, void* d_workspace, int look_first,
+                       const HostPost& post, cudaStream_t stream) {
+  if (n_rows > 0 && n_rows <= kSmallRows) {
+    auto* h = reinterpret_cast<TableHeader*>(d_table);
+    auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
+    RMN_DISPATCH_W(W, k_build_small<kW><<<1, 1024, 0, stream>>>(d_coords, n_rows, h, slots, table_capacity(n_rows),
+                                                                scratch(d_workspace, n_rows), d_mapping, d_unique_coords,
+                                                                d_inverse, look_first, post));
+    RMN_LAUNCH_CHECK();
+    return RMN_OK;
+  }
+  const int rc = table_build_begin(d_coords, n_rows, W, d_table, d_workspace, look_first, post, stream);
+  if (rc != RMN_OK || n_rows == 0) return rc;
+  return table_build_finish(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace, stream);
 }
 
 // First half of a build: header, slot fill + bounding box, insert, first-occurrence counts. When it has
@@ -519,33 +811,9 @@ extern "C" size_t rmn_table_build_workspace_bytes(uint32_t n_rows) {
 extern "C" int rmn_table_build_begin(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table,
                                      size_t table_bytes, void* d_workspace, size_t workspace_bytes,
                                      void* stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
-  if (!d_table || W < 2 || W > RMN_MAX_W || n_rows >= 0x7FFFFFFFu) return RMN_ERR_BAD_ARG;
-  if (n_rows > 0 && (!d_coords || !d_workspace)) return RMN_ERR_BAD_ARG;
-  if (((uintptr_t)d_table & 15) || !coords_aligned(d_coords, W)) return RMN_ERR_BAD_ARG;
-  if (table_bytes < rmn_table_bytes(n_rows) ||
-      (n_rows > 0 && workspace_bytes < rmn_table_build_workspace_bytes(n_rows)))
-    return RMN_ERR_ALLOC;
-  auto* h = reinterpret_cast<TableHeader*>(d_table);
-  auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
-  const uint32_t capacity = table_capacity(n_rows);
-  RMN_CUDA_TRY(cudaMemsetAsync(h, 0, sizeof(TableHeader), stream));
-  {
-    const uint32_t fill_blocks = (capacity + 255u) / 256u;
-    const uint32_t blocks = fill_blocks < 148u * 8u ? fill_blocks : 148u * 8u;
-    RMN_DISPATCH_W(W, k_fill_range<kW><<<blocks, 256, 0, stream>>>(d_coords, n_rows, h,
-                                                                    reinterpret_cast<uint4*>(slots), capacity));
-    RMN_LAUNCH_CHECK();
-  }
-  if (n_rows == 0) return RMN_OK;
-  uint32_t* slot_of_row = reinterpret_cast<uint32_t*>(d_workspace);
-  uint32_t* block_counts = slot_of_row + n_rows;
-  const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
-  RMN_DISPATCH_W(W, k_insert<kW><<<nb, 256, 0, stream>>>(d_coords, n_rows, h, slots, slot_of_row));
-  RMN_LAUNCH_CHECK();
-  k_count_first<<<nb, kRowsPerBlock, 0, stream>>>(slots, slot_of_row, n_rows, h, block_counts);
-  RMN_LAUNCH_CHECK();
-  return RMN_OK;
+  const int rc = table_build_args(d_coords, n_rows, W, d_table, table_bytes, d_workspace, workspace_bytes);
+  if (rc != RMN_OK) return rc;
+  return table_build_begin(d_coords, n_rows, W, d_table, d_workspace, 0, HostPost{}, (cudaStream_t)stream_);
 }
 
 // Second half: unique ids, mapping, unique coordinates, inverse. Same table, coordinates and workspace as
@@ -553,24 +821,11 @@ extern "C" int rmn_table_build_begin(const int32_t* d_coords, uint32_t n_rows, i
 extern "C" int rmn_table_build_finish(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table,
                                       int64_t* d_mapping, int64_t* d_inverse, int32_t* d_unique_coords,
                                       void* d_workspace, void* stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
   if (!d_table || W < 2 || W > RMN_MAX_W || n_rows >= 0x7FFFFFFFu) return RMN_ERR_BAD_ARG;
   if (n_rows == 0) return RMN_OK;
   if (!d_coords || !d_mapping || !d_workspace) return RMN_ERR_BAD_ARG;
-  auto* h = reinterpret_cast<TableHeader*>(d_table);
-  auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
-  uint32_t* slot_of_row = reinterpret_cast<uint32_t*>(d_workspace);
-  uint32_t* block_counts = slot_of_row + n_rows;
-  const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
-  RMN_DISPATCH_W(W, k_finalize<kW><<<nb, kRowsPerBlock, 0, stream>>>(
-                        d_coords, n_rows, h, slots, slot_of_row, block_counts, d_mapping,
-                        d_unique_coords, d_inverse));
-  RMN_LAUNCH_CHECK();
-  if (d_inverse) {  // optional: only the quantisation modes that average or sample features read it
-    k_inverse<<<nb, 256, 0, stream>>>(slots, slot_of_row, n_rows, h, d_inverse);
-    RMN_LAUNCH_CHECK();
-  }
-  return RMN_OK;
+  return table_build_finish(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace,
+                            (cudaStream_t)stream_);
 }
 
 extern "C" int rmn_table_build(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table,
@@ -578,11 +833,10 @@ extern "C" int rmn_table_build(const int32_t* d_coords, uint32_t n_rows, int W, 
                                int32_t* d_unique_coords, void* d_workspace,
                                size_t workspace_bytes, void* stream_) {
   if (n_rows > 0 && n_rows < 0x7FFFFFFFu && !d_mapping) return RMN_ERR_BAD_ARG;
-  const int rc = rmn_table_build_begin(d_coords, n_rows, W, d_table, table_bytes, d_workspace, workspace_bytes,
-                                       stream_);
+  const int rc = table_build_args(d_coords, n_rows, W, d_table, table_bytes, d_workspace, workspace_bytes);
   if (rc != RMN_OK) return rc;
-  return rmn_table_build_finish(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace,
-                                stream_);
+  return table_build(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace, 0, HostPost{},
+                     (cudaStream_t)stream_);
 }
 
 // ---------------------------------------------------------------------------
@@ -604,8 +858,7 @@ extern "C" int rmn_table_build(const int32_t* d_coords, uint32_t n_rows, int W, 
 // device (with that device current) on the first call made on it.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kStaticMaxRows = 1u << 20;
-constexpr size_t kStaticScratchBytes =
-    (size_t)kStaticMaxRows * 4 + ((kStaticMaxRows + rmn::kRowsPerBlock - 1) / rmn::kRowsPerBlock + 1) * 4 + 256;
+constexpr size_t kStaticScratchBytes = rmn::scratch_bytes(kStaticMaxRows);
 static __device__ __align__(256) unsigned char g_table_static_scratch[kStaticScratchBytes];
 
 static int static_scratch_address(void** out) {
@@ -739,6 +992,74 @@ extern "C" int rmn_table_info(const void* d_table, uint32_t info[4], void* strea
   return (int)h.status;
 }
 
+// What a waiting host polls: page-locked words of the calling thread, never freed (a build may still store into them).
+struct HostWords {
+  uint32_t* host = nullptr;
+  uint32_t* device = nullptr;
+  uint32_t sequence = 0;
+};
+static HostWords& host_words() {
+  thread_local HostWords w;
+  if (!w.host) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+    } else if (void* alias = device_alias(p)) {
+      memset(p, 0, 64);
+      w.host = static_cast<uint32_t*>(p);
+      w.device = static_cast<uint32_t*>(alias);
+    }
+  }
+  return w;
+}
+
+// The host waits by polling a word that the build stores, not for the stream: no read-back kernel, no event, no second
+// stream, and the host goes on while the second half of the build runs.
+extern "C" int rmn_table_build_counted(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table, size_t table_bytes,
+                                       int64_t* d_mapping, int64_t* d_inverse, int32_t* d_unique_coords, void* d_workspace,
+                                       size_t workspace_bytes, int expect_duplicates, uint32_t info[4], void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  if (!info) return RMN_ERR_BAD_ARG;
+  int rc = table_build_args(d_coords, n_rows, W, d_table, table_bytes, d_workspace, workspace_bytes);
+  if (rc != RMN_OK) return rc;
+  HostWords& hw = host_words();
+  HostPost post{};
+  if (hw.host && n_rows > 0) {
+    post.words = hw.device;
+    post.conv_status = tc_status_device_address();
+    post.sequence = ++hw.sequence ? hw.sequence : ++hw.sequence;
+  }
+  rc = table_build(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace, expect_duplicates, post,
+                   stream);
+  if (rc != RMN_OK) return rc;
+  if (!post.words) return rmn_table_info(d_table, info, stream_);
+  const volatile uint32_t* words = hw.host;
+  for (uint32_t spin = 1; words[5] != post.sequence; ++spin) {
+    if (spin % 4096 != 0) {
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+      continue;
+    }
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) {
+      cudaGetLastError();
+      continue;
+    }
+    if (e != cudaSuccess) return RMN_ERR_CUDA;
+    if (words[5] == post.sequence) break;
+    return rmn_table_info(d_table, info, stream_);  // the build has ended without storing
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  for (int i = 0; i < 4; ++i) info[i] = words[i];
+  if (info[1] == RMN_OK && words[4] != 0) {
+    const int st = (int)words[4];
+    tc_clear_status();
+    return st;
+  }
+  return (int)info[1];
+}
+
 extern "C" int rmn_table_find(const void* d_table, const int32_t* d_query, uint32_t n_query, int W,
                               int32_t* d_rows, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
@@ -766,9 +1087,11 @@ extern "C" int rmn_coords_stride(const int32_t* d_coords, uint32_t n_rows, int W
     if (out_tensor_stride[a] <= 0) return RMN_ERR_BAD_ARG;
     st.s[a] = out_tensor_stride[a];
   }
-  const uint64_t total = (uint64_t)n_rows * W;
-  const uint32_t nb = (uint32_t)((total + 255) / 256);
-  k_stride<<<nb, 256, 0, stream>>>(d_coords, total, W, st, d_out);
+  const uint32_t nb = (n_rows + 255) / 256;
+  if (W == 4 && !((uintptr_t)d_coords & 15) && !((uintptr_t)d_out & 15))
+    k_stride<4, true><<<nb, 256, 0, stream>>>(d_coords, n_rows, st, d_out);
+  else
+    RMN_DISPATCH_W(W, k_stride<kW, false><<<nb, 256, 0, stream>>>(d_coords, n_rows, st, d_out));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

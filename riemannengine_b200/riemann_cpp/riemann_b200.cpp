@@ -287,7 +287,8 @@ CoordinateManager::CoordinateManager(int D, CoordinateMapBackend::Type map_type,
 }
 
 CoordinateManager::Map CoordinateManager::build(const at::Tensor& coords, const stride_type& tensor_stride,
-                                                at::Tensor* mapping_out, at::Tensor* inverse_out) {
+                                                at::Tensor* mapping_out, at::Tensor* inverse_out,
+                                                bool expect_duplicates) {
   c10::cuda::CUDAGuard guard(coords.device());
   const uint32_t n = static_cast<uint32_t>(coords.size(0));
   const int W = static_cast<int>(coords.size(1));
@@ -298,25 +299,18 @@ CoordinateManager::Map CoordinateManager::build(const at::Tensor& coords, const 
   const size_t table_bytes = rmn_table_bytes(n), ws_bytes = rmn_table_build_workspace_bytes(n);
   m.table = at::empty({static_cast<int64_t>(table_bytes)}, bytes);
   auto ws = at::empty({static_cast<int64_t>(ws_bytes)}, bytes);
-  auto mapping = at::empty({n}, longs), inverse = at::empty({n}, longs);
+  at::Tensor mapping, inverse;
+  if (mapping_out) mapping = at::empty({n}, longs);
+  if (inverse_out) inverse = at::empty({n}, longs);
   auto unique = at::empty({n, W}, coords.options());
-  // The header (number of unique rows) is final after the first half of the build: it is read back on the
-  // second stream while the second half still runs on the caller's, so the host is already preparing the
-  // next launches when the build ends.
-  auto main_stream = c10::cuda::getCurrentCUDAStream();
-  check(rmn_table_build_begin(static_cast<const int32_t*>(ptr(coords)), n, W, ptr(m.table), table_bytes, ptr(ws),
-                              ws_bytes, main_stream.stream()),
-        "rmn_table_build");
-  c10::Event counted(c10::DeviceType::CUDA);
-  counted.record(main_stream);
-  check(rmn_table_build_finish(static_cast<const int32_t*>(ptr(coords)), n, W, ptr(m.table),
-                               static_cast<int64_t*>(ptr(mapping)), static_cast<int64_t*>(ptr(inverse)),
-                               static_cast<int32_t*>(ptr(unique)), ptr(ws), main_stream.stream()),
-        "rmn_table_build");
-  auto side_stream = pair_list_stream(main_stream.device_index());
-  counted.block(side_stream);
+  // The number of unique rows is known after the first half of the build: the call returns with it while the second half
+  // still runs, so the host is already preparing the next launches when the build ends.
   uint32_t info[4];
-  check(rmn_table_info(ptr(m.table), info, side_stream.stream()), "rmn_table_build");
+  check(rmn_table_build_counted(static_cast<const int32_t*>(ptr(coords)), n, W, ptr(m.table), table_bytes,
+                                static_cast<int64_t*>(ptr(mapping)), static_cast<int64_t*>(ptr(inverse)),
+                                static_cast<int32_t*>(ptr(unique)), ptr(ws), ws_bytes, expect_duplicates ? 1 : 0, info,
+                                current_stream()),
+        "rmn_table_build");
   m.size = info[0];
   m.coords = unique.narrow(0, 0, m.size);
   if (mapping_out) *mapping_out = mapping.narrow(0, 0, m.size);
@@ -339,6 +333,13 @@ at::Tensor CoordinateManager::get_coordinates(const CoordinateMapKey& key) const
 
 std::pair<CoordinateMapKey, std::pair<at::Tensor, at::Tensor>>
 CoordinateManager::insert_and_map(const at::Tensor& coordinates, stride_type tensor_stride, std::string string_id) {
+  at::Tensor mapping, inverse;
+  auto key = insert(coordinates, std::move(tensor_stride), std::move(string_id), &mapping, &inverse);
+  return {std::move(key), {mapping, inverse}};
+}
+
+CoordinateMapKey CoordinateManager::insert(const at::Tensor& coordinates, stride_type tensor_stride, std::string string_id,
+                                           at::Tensor* mapping, at::Tensor* inverse) {
   check_coordinates(coordinates);
   const auto coordinate_size = static_cast<size_type>(coordinates.size(1));
   if (coordinate_size - 1 != tensor_stride.size())
@@ -351,9 +352,8 @@ CoordinateManager::insert_and_map(const at::Tensor& coordinates, stride_type ten
     for (int i = 0; i < 8; ++i) suffix.push_back(static_cast<char>('a' + std::rand() % 26));
     map_key.second = string_id + suffix;
   }
-  at::Tensor mapping, inverse;
-  maps_[map_key] = build(coordinates, tensor_stride, &mapping, &inverse);
-  return {CoordinateMapKey(coordinate_size, map_key), {mapping, inverse}};
+  maps_[map_key] = build(coordinates, tensor_stride, mapping, inverse, /*expect_duplicates=*/false);
+  return CoordinateMapKey(coordinate_size, map_key);
 }
 
 CoordinateMapKey CoordinateManager::insert_field(const at::Tensor& coordinates, stride_type tensor_stride,
@@ -415,7 +415,7 @@ CoordinateMapKey CoordinateManager::stride(const CoordinateMapKey& in_key, const
                             static_cast<int>(in_map.coords.size(1)), st.data(),
                             static_cast<int32_t*>(ptr(aligned)), current_stream()),
           "rmn_coords_stride");
-    maps_[out_key] = build(aligned, out_stride, nullptr, nullptr);
+    maps_[out_key] = build(aligned, out_stride, nullptr, nullptr, /*expect_duplicates=*/true);
   }
   return CoordinateMapKey(in_key.get_coordinate_size(), out_key);
 }
@@ -433,7 +433,7 @@ std::pair<CoordinateMapKey, bool> CoordinateManager::origin() {
     c10::cuda::CUDAGuard guard(seed->coords.device());
     auto zeroed = at::zeros_like(seed->coords);
     zeroed.select(1, 0).copy_(seed->coords.select(1, 0));
-    maps_[origin_key] = build(zeroed, origin_key.first, nullptr, nullptr);  // dedup on the batch column
+    maps_[origin_key] = build(zeroed, origin_key.first, nullptr, nullptr, true);  // dedup on the batch column
   }
   return {CoordinateMapKey(static_cast<size_type>(D + 1), origin_key), created};
 }
@@ -570,19 +570,17 @@ std::shared_ptr<KernelMap> CoordinateManager::kernel_map(const CoordinateMapKey&
     for (int k = 0; self_symmetric && k < K; ++k)
       for (int a = 0; a < D; ++a)
         if (off[static_cast<size_t>(k) * D + a] != -off[static_cast<size_t>(K - 1 - k) * D + a]) self_symmetric = false;
-    auto build = self_symmetric ? rmn_kmap_build_self : rmn_kmap_build;
-    check(build(ptr(in_map.table), static_cast<const int32_t*>(ptr(out_map.coords)), out_map.size, W,
-                static_cast<const int32_t*>(ptr(d_off)), K, static_cast<int32_t*>(ptr(result->nbr_out)),
-                static_cast<int64_t*>(ptr(result->offset_ptr)), ptr(result->workspace), ws_bytes, current_stream()),
-          self_symmetric ? "rmn_kmap_build_self" : "rmn_kmap_build");
     result->self_symmetric = self_symmetric;
     result->region_offsets = off;
+    // stored by the build's last kernel, not a copy engine: behind a large device-to-host copy of the caller's (the
+    // previous step's result) an engine copy of these few bytes would wait for all of it
     result->host_offset_ptr = at::empty({K + 1}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
-    // stored by a kernel, not a copy engine: behind a large device-to-host copy of the caller's (the previous
-    // step's result) an engine copy of these few bytes would wait for all of it
-    check(rmn_readback_small(ptr(result->offset_ptr), result->host_offset_ptr.data_ptr(),
-                             static_cast<size_t>(K + 1) * sizeof(int64_t), current_stream()),
-          "rmn_readback_small");
+    check(rmn_kmap_build_host(ptr(in_map.table), static_cast<const int32_t*>(ptr(out_map.coords)), out_map.size, W,
+                              static_cast<const int32_t*>(ptr(d_off)), K, self_symmetric ? 1 : 0,
+                              static_cast<int32_t*>(ptr(result->nbr_out)),
+                              static_cast<int64_t*>(ptr(result->offset_ptr)), result->host_offset_ptr.data_ptr<int64_t>(),
+                              ptr(result->workspace), ws_bytes, current_stream()),
+          "rmn_kmap_build");
     result->offset_ptr_ready.emplace(c10::DeviceType::CUDA);
     result->offset_ptr_ready->record(c10::cuda::getCurrentCUDAStream());
   }
@@ -654,10 +652,12 @@ SparseTensor::SparseTensor(at::Tensor features, at::Tensor coordinates, std::sha
   TORCH_CHECK(manager->D() == dimension_, "Coordinate manager dimension does not match coordinates");
   manager_ = std::move(manager);
   stride_type unit_stride(static_cast<size_t>(dimension_), 1);
-  auto inserted = manager_->insert_and_map(coordinates.contiguous(), unit_stride);
-  key_ = std::move(inserted.first);
-  features_ = quantize_features(features_, inserted.second.first, inserted.second.second, manager_->size(key_),
-                                quantization_mode);
+  // (only the modes that combine rows read the inverse mapping)
+  const bool combines = quantization_mode != SparseTensorQuantizationMode::RANDOM_SUBSAMPLE &&
+                        quantization_mode != SparseTensorQuantizationMode::NO_QUANTIZATION;
+  at::Tensor mapping, inverse;
+  key_ = manager_->insert(coordinates.contiguous(), unit_stride, "", &mapping, combines ? &inverse : nullptr);
+  features_ = quantize_features(features_, mapping, inverse, manager_->size(key_), quantization_mode);
 }
 
 SparseTensor::SparseTensor(at::Tensor features, CoordinateMapKey coordinate_map_key,

@@ -157,6 +157,9 @@ public:
                     GPUMemoryAllocatorBackend::Type alloc_type = GPUMemoryAllocatorBackend::PYTORCH,
                     RiemannAlgorithm::Mode algo = RiemannAlgorithm::DEFAULT);
 
+  // insert_and_map with only the mappings that are asked for (each may be null)
+  CoordinateMapKey insert(const at::Tensor& coordinates, stride_type tensor_stride, std::string string_id,
+                          at::Tensor* mapping, at::Tensor* inverse);
   std::pair<CoordinateMapKey, std::pair<at::Tensor, at::Tensor>>
   insert_and_map(const at::Tensor& coordinates, stride_type tensor_stride, std::string string_id = "");
 
@@ -212,7 +215,8 @@ private:
     uint32_t size = 0;
   };
   Map const& find(const CoordinateMapKey& key, const char* what = "") const;
-  Map build(const at::Tensor& coords, const stride_type& tensor_stride, at::Tensor* mapping, at::Tensor* inverse);
+  Map build(const at::Tensor& coords, const stride_type& tensor_stride, at::Tensor* mapping, at::Tensor* inverse,
+            bool expect_duplicates);
 
   int D_;
   CoordinateMapBackend::Type map_type_;

@@ -1,0 +1,85 @@
+"""rmn_table_build_counted (counts stored by the build itself) and rmn_kmap_build_host against the calls without them: row
+counts around the one-block build and around 256-row blocks, with and without duplicates, the hint either way, a packing
+overflow; row counts at which the offsets of a map are split over blocks."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _coords(n, D, extent, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    c = torch.randint(-extent, extent, (n, D), generator=g, device="cuda")
+    return torch.cat([torch.randint(0, 2, (n, 1), generator=g, device="cuda"), c], 1).int().contiguous()
+
+
+def _counted(coords, hint):
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    n, W = coords.shape
+    new = lambda size, dtype: torch.empty(size, dtype=dtype, device="cuda")  # noqa: E731
+    table, ws = new(lib.rmn_table_bytes(n), torch.uint8), new(lib.rmn_table_build_workspace_bytes(n), torch.uint8)
+    mapping, inverse, unique = new(n, torch.int64), new(n, torch.int64), new((n, W), torch.int32)
+    info = torch.zeros(4, dtype=torch.int32)
+    rc = lib.rmn_table_build_counted(ops._ptr(coords), n, W, ops._ptr(table), table.numel(), ops._ptr(mapping),
+                                     ops._ptr(inverse), ops._ptr(unique), ops._ptr(ws), ws.numel(), hint, info.data_ptr(),
+                                     ops._stream())
+    return rc, info, mapping, inverse, unique, table
+
+
+@pytest.mark.parametrize("hint", [0, 1])
+@pytest.mark.parametrize("D", [1, 3, 4])
+@pytest.mark.parametrize("n,extent", [(1, 5), (1023, 4), (1025, 10_000), (2048, 9), (2048, 10_000), (2049, 9), (4097, 10_000),
+                                      (300_001, 30)])
+def test_counted_build_matches_torch(n, D, extent, hint):
+    c = _coords(n, D, extent, n + D)
+    rc, info, mapping, inverse, unique, table = _counted(c, hint)
+    assert rc == 0
+    rows, inv = torch.unique(c, dim=0, return_inverse=True)
+    first = torch.full((rows.size(0),), n, dtype=torch.int64, device="cuda").scatter_reduce(
+        0, inv, torch.arange(n, device="cuda"), "amin")
+    order = first.argsort()
+    m = rows.size(0)
+    assert info.tolist()[0] == m and info.tolist()[3] == n
+    assert torch.equal(mapping[:m], first[order])
+    assert torch.equal(unique[:m], rows[order])
+    assert torch.equal(inverse, order.argsort()[inv])
+    from riemannengine_b200 import capi, ops
+    found = torch.empty(n, dtype=torch.int32, device="cuda")
+    capi.check(capi.lib().rmn_table_find(ops._ptr(table), ops._ptr(c), n, c.size(1), ops._ptr(found), ops._stream()), "find")
+    assert torch.equal(found.long(), inverse)
+
+
+@pytest.mark.parametrize("n", [3, 3000])
+def test_counted_build_reports_a_range_that_does_not_pack(n):
+    from riemannengine_b200 import capi
+    c = _coords(n, 3, 2 ** 30, 1)
+    c[0, 1:], c[1, 1:] = -2 ** 31, 2 ** 31 - 1
+    rc, info, *_ = _counted(c, 0)
+    assert rc != capi.OK and info.tolist()[1] == rc
+
+
+@pytest.mark.parametrize("n", [1, 255, 900, 20_000, 60_000])
+def test_split_offsets_and_host_pointers(n):
+    from riemannengine_b200 import capi, ops
+    c = torch.unique(_coords(n, 3, max(3, int(n ** (1 / 3))), n), dim=0).contiguous()
+    table = ops.table_build(c)
+    off = ops.region_offsets(0, [3] * 3, [1] * 3, [1] * 3)
+    d_off = torch.from_numpy(off).int().cuda()
+    m, K = c.size(0), off.shape[0]
+    want = torch.full((K, m), -1, dtype=torch.int32, device="cuda")
+    for k in range(K):
+        q = c.clone()
+        q[:, 1:] += d_off[k]
+        capi.check(capi.lib().rmn_table_find(ops._ptr(table.buffer), ops._ptr(q), m, 4, ops._ptr(want[k]), ops._stream()), "find")
+    for self_map in (0, 1):
+        nbr = torch.empty((K, m), dtype=torch.int32, device="cuda")
+        ptr, ws = torch.empty(K + 1, dtype=torch.int64, device="cuda"), torch.empty(
+            capi.lib().rmn_kmap_workspace_bytes(m, K), dtype=torch.uint8, device="cuda")
+        host = torch.zeros(K + 1, dtype=torch.int64).pin_memory()
+        capi.check(capi.lib().rmn_kmap_build_host(ops._ptr(table.buffer), ops._ptr(table.coords), m, 4, ops._ptr(d_off), K,
+                                                  self_map, ops._ptr(nbr), ops._ptr(ptr), host.data_ptr(), ops._ptr(ws),
+                                                  ws.numel(), ops._stream()), "kmap")
+        torch.cuda.synchronize()
+        assert torch.equal(nbr, want)
+        assert host.tolist() == ptr.tolist() == [0] + (want >= 0).sum(1).cumsum(0).tolist()
