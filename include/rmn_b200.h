@@ -132,6 +132,13 @@ int rmn_table_build_counted(const int32_t *d_coords, uint32_t n_rows, int W, voi
                             size_t workspace_bytes, int expect_duplicates, uint32_t info[4], void *stream);
 
 /*
+ * d_out [n_unique, channels] = sum (mean != 0: average) of the fp32 rows of every unique row, from a build's mapping and
+ * inverse. d_counts: [n_unique] scratch, rows per unique row. Sums of more than two rows add them in no fixed order.
+ */
+int rmn_segment_reduce(const float *d_feats, uint32_t n_rows, int channels, const int64_t *d_inverse,
+                       const int64_t *d_mapping, uint32_t n_unique, int mean, float *d_out, uint32_t *d_counts, void *stream);
+
+/*
  * rmn_table_build for callers that cannot allocate device memory. It has no
  * counterpart in the reference. Same inputs, outputs and results as
  * rmn_table_build, but there is no workspace argument: the build's scratch is

@@ -33,6 +33,8 @@ SIGNATURES = {
                                        c_void_p]),
     "rmn_table_build_counted": (c_int, [c_void_p, c_uint32, c_int, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_size_t, c_int, c_void_p, c_void_p]),
+    "rmn_segment_reduce": (c_int, [c_void_p, c_uint32, c_int, c_void_p, c_void_p, c_uint32, c_int, c_void_p, c_void_p,
+                                   c_void_p]),
     "rmn_kmap_build_host": (c_int, [c_void_p, c_void_p, c_uint32, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_size_t, c_void_p]),
     "rmn_table_build_static_max_rows": (c_uint32, []),

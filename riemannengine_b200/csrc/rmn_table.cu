@@ -5,7 +5,7 @@
 //   256-byte memset of the header
 //   -> fill + range (slots to the empty pattern, column min/max; the last block plans the bit packing)
 //   -> insert (one 16-byte CAS on the packed key, atomicMin on the first row)
-//   -> count (rows that are the first occurrence, per 256-row block; the last block scans the counts and, where the
+//   -> count (first rows per 256-row block, from the bits of the others; the last block scans the counts and, where the
 //      caller waits for them, stores the header's words into the host's memory)
 //   -> finalize (unique ids, mapping, unique coordinates; identity inverse when nothing was a duplicate)
 //   -> inverse (only does work when there were duplicates)
@@ -35,11 +35,11 @@ constexpr int kRowsPerBlock = 256;
 constexpr uint32_t kGrid = 148 * 8;  // blocks of the passes that may have nothing to do
 
 // Scratch of a build of n rows: slot of every row, rows that are the first of their key per 256-row block (then the
-// blocks' offsets), and one bit per row for them
+// blocks' offsets), and one bit per row that is not the first of its key
 struct Scratch {
   uint32_t* slot_of_row;
   uint32_t* block_counts;
-  uint32_t* first_bits;
+  uint32_t* repeat_bits;
 };
 constexpr size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 constexpr size_t scratch_bytes(size_t n) {
@@ -52,7 +52,7 @@ inline Scratch scratch(void* workspace, uint32_t n) {
   Scratch s;
   s.slot_of_row = reinterpret_cast<uint32_t*>(p);
   s.block_counts = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4));
-  s.first_bits = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4) + align16((nb + 1) * 4));
+  s.repeat_bits = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4) + align16((nb + 1) * 4));
   return s;
 }
 
@@ -101,13 +101,16 @@ __device__ void write_header(TableHeader* h, uint32_t W, uint32_t n, uint32_t ca
 // constants, decodes the bounds and plans the key packing.
 template <int W>
 __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ coords, uint32_t n,
-                                                    TableHeader* h, uint4* __restrict__ slots, uint32_t capacity) {
+                                                    TableHeader* h, uint4* __restrict__ slots, uint32_t capacity,
+                                                    uint32_t* __restrict__ repeat_bits) {
   __shared__ int32_t s_mn[8][W], s_mx[8][W];
   constexpr int NA = W - 1 < 3 ? W - 1 : 3;
   __shared__ uint32_t s_or[8][NA];
   const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < capacity; i += gridDim.x * blockDim.x)
     slots[i] = ones;
+  const uint32_t bit_words = (n + kRowsPerBlock - 1) / kRowsPerBlock * (kRowsPerBlock / 32);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < bit_words; i += gridDim.x * blockDim.x) repeat_bits[i] = 0u;
   int32_t mn[W], mx[W];
 #pragma unroll
   for (int c = 0; c < W; ++c) { mn[c] = INT_MAX; mx[c] = INT_MIN; }
@@ -198,13 +201,16 @@ __device__ __forceinline__ void cas_slot(Slot* slot, unsigned long long key, uns
       : "memory");
 }
 
+constexpr uint32_t kNoRow = 0xFFFFFFFFu;
+
 // Claims the slot of a row's key: {key, first_row = row, uid = row}. Without duplicates the unique numbering is the row
 // numbering and the slot is final after this single 16-byte compare-and-swap. A row that finds its key taken lowers
-// first_row; *dup tells (k_finalize then renumbers). look_first: read a slot before the compare-and-swap and spare it, and
+// first_row; the larger of the two rows is not the first of its key and goes to *repeat (every row but the smallest loses
+// once; kNoRow: none did). look_first: read a slot before the compare-and-swap and spare it, and
 // the atomic minimum, where the key is there already with a smaller row - the usual case among many duplicates (1.2 M rows
 // on 0.27 M strided cells: 60 -> 25 us), a second round trip to the slot without them.
 __device__ __forceinline__ bool insert_row(Slot* slots, uint32_t capacity, uint32_t pos_shift, unsigned long long key,
-                                           uint32_t row, bool look_first, uint32_t* slot_of_row, bool* dup) {
+                                           uint32_t row, bool look_first, uint32_t* slot_of_row, uint32_t* repeat) {
   uint32_t s = hash_key(key, capacity, pos_shift);
   const unsigned long long mine = (unsigned long long)row | ((unsigned long long)row << 32);
   for (uint32_t probe = 0; probe < (capacity >> 3); ++probe) {
@@ -219,8 +225,9 @@ __device__ __forceinline__ bool insert_row(Slot* slots, uint32_t capacity, uint3
     }
     if (cur_key == kEmptyKey || cur_key == key) {
       if (cur_key == key) {
-        if ((uint32_t)cur_rows > row) atomicMin(&slots[s].first_row, row);
-        *dup = true;
+        uint32_t other = (uint32_t)cur_rows;
+        if (other > row) other = atomicMin(&slots[s].first_row, row);
+        *repeat = other > row ? other : row;
       }
       slot_of_row[row] = s;
       return true;
@@ -236,10 +243,10 @@ __device__ __forceinline__ bool insert_row(Slot* slots, uint32_t capacity, uint3
 template <int W>
 __global__ void __launch_bounds__(256) k_insert(const int32_t* __restrict__ coords, uint32_t n,
                                                 TableHeader* h, Slot* slots,
-                                                uint32_t* __restrict__ slot_of_row, int look_first) {
+                                                Scratch sc, int look_first) {
   if (h->status != RMN_OK) return;
   const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-  bool dup = false;
+  uint32_t repeat = kNoRow;
   if (row < n) {
     Packer<W> pk;
     pk.load(h);
@@ -247,10 +254,13 @@ __global__ void __launch_bounds__(256) k_insert(const int32_t* __restrict__ coor
     load_row<W>(coords, row, c);
     unsigned long long key;
     pk.pack(c, key);
-    if (!insert_row(slots, h->capacity, h->pos_shift, key, row, look_first != 0, slot_of_row, &dup))
+    if (!insert_row(slots, h->capacity, h->pos_shift, key, row, look_first != 0, sc.slot_of_row, &repeat))
       atomicExch(&h->status, (uint32_t)RMN_ERR_PROBE_LIMIT);
   }
-  const int dups = __syncthreads_count(dup);  // one atomic per block: the rows' own would serialise on the word
+  const uint32_t own = __ballot_sync(0xFFFFFFFFu, repeat == row);  // (rows of a warp share a word)
+  if ((threadIdx.x & 31) == 0 && own) atomicOr(sc.repeat_bits + (row >> 5), own);
+  if (repeat != kNoRow && repeat != row) atomicOr(sc.repeat_bits + (repeat >> 5), 1u << (repeat & 31));
+  const int dups = __syncthreads_count(repeat != kNoRow);  // one atomic per block: the rows' own would serialise on the word
   if (threadIdx.x == 0 && dups) atomicAdd(&h->n_dups, (uint32_t)dups);
 }
 
@@ -307,11 +317,10 @@ __device__ __forceinline__ uint32_t scan_u32_block(uint32_t* __restrict__ counts
   return carry;
 }
 
-// Rows that are the first occurrence of their key: a bit per row, and their number per 256-row block; the last block to
-// finish turns the numbers into block offsets (exclusive scan) and writes n_unique. Nothing to do when the insert pass
-// met no duplicate: nothing is compacted then (see k_finalize).
-__global__ void __launch_bounds__(kRowsPerBlock) k_count_first(const Slot* __restrict__ slots, uint32_t n, TableHeader* h,
-                                                              Scratch sc, HostPost post) {
+// Rows that are the first of their key, counted per 256-row block from the bits of those that are not (one thread per
+// block); the last CUDA block to finish turns the numbers into block offsets (exclusive scan) and writes n_unique. Nothing
+// to do when the insert pass met no duplicate: nothing is compacted then (see k_finalize).
+__global__ void __launch_bounds__(256) k_count_first(uint32_t n, TableHeader* h, Scratch sc, HostPost post) {
   const bool failed = h->status != RMN_OK;
   if (failed || h->n_dups == 0) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -322,19 +331,16 @@ __global__ void __launch_bounds__(kRowsPerBlock) k_count_first(const Slot* __res
   }
   __shared__ uint32_t s_last;
   const uint32_t nb = (n + kRowsPerBlock - 1) / kRowsPerBlock;
-  for (uint32_t block = blockIdx.x; block < nb; block += gridDim.x) {
-    const uint32_t row = block * kRowsPerBlock + threadIdx.x;
-    bool first = false;
-    if (row < n) first = slots[sc.slot_of_row[row]].first_row == row;
-    const uint32_t bits = __ballot_sync(0xFFFFFFFFu, first);
-    if ((threadIdx.x & 31) == 0) sc.first_bits[block * (kRowsPerBlock / 32) + (threadIdx.x >> 5)] = bits;
-    const int total = __syncthreads_count(first);
-    if (threadIdx.x == 0) sc.block_counts[block] = (uint32_t)total;
-  }
-  if (threadIdx.x == 0) {
+  const uint32_t block = blockIdx.x * 256 + threadIdx.x;
+  if (block < nb) {
+    uint32_t repeats = 0;
+#pragma unroll
+    for (int w = 0; w < kRowsPerBlock / 32; ++w) repeats += __popc(__ldg(sc.repeat_bits + block * (kRowsPerBlock / 32) + w));
+    sc.block_counts[block] = min((uint32_t)kRowsPerBlock, n - block * kRowsPerBlock) - repeats;
     __threadfence();
-    s_last = atomicAdd(&h->count_blocks_done, 1u) == gridDim.x - 1 ? 1u : 0u;
   }
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&h->count_blocks_done, 1u) == gridDim.x - 1 ? 1u : 0u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -369,10 +375,10 @@ __global__ void __launch_bounds__(kRowsPerBlock) k_finalize(
   }
   if (row >= n) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t* bits = sc.first_bits + blockIdx.x * (kRowsPerBlock / 32);
-  if (!((__ldg(bits + warp) >> lane) & 1u)) return;
-  uint32_t uid = sc.block_counts[blockIdx.x] + __popc(__ldg(bits + warp) & ((1u << lane) - 1u));
-  for (int w = 0; w < warp; ++w) uid += __popc(__ldg(bits + w));
+  const uint32_t* bits = sc.repeat_bits + blockIdx.x * (kRowsPerBlock / 32);
+  if ((__ldg(bits + warp) >> lane) & 1u) return;
+  uint32_t uid = sc.block_counts[blockIdx.x] + __popc(~__ldg(bits + warp) & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) uid += __popc(~__ldg(bits + w));
   const uint32_t s = sc.slot_of_row[row];
   slots[s].uid = uid | (slots[s].uid & kPassedBit);
   if (mapping) mapping[uid] = (int64_t)row;
@@ -452,16 +458,16 @@ __global__ void __launch_bounds__(1024) k_build_small(const int32_t* __restrict_
   if (range_ok) {
     Packer<W> pk;
     pk.load(&s_h);
-    bool dup[2] = {false, false};
+    uint32_t repeat[2] = {kNoRow, kNoRow};
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const uint32_t row = tid + i * 1024;
       if (row >= n) continue;
       unsigned long long key;
       pk.pack(row_c[i], key);
-      if (!insert_row(slots, capacity, s_h.pos_shift, key, row, look_first != 0, sc.slot_of_row, &dup[i])) s_ok = 0u;
+      if (!insert_row(slots, capacity, s_h.pos_shift, key, row, look_first != 0, sc.slot_of_row, &repeat[i])) s_ok = 0u;
     }
-    dups = (uint32_t)(__syncthreads_count(dup[0]) + __syncthreads_count(dup[1]));
+    dups = (uint32_t)(__syncthreads_count(repeat[0] != kNoRow) + __syncthreads_count(repeat[1] != kNoRow));
     if (tid == 0) {
       s_h.n_dups = dups;
       if (!s_ok) s_h.status = RMN_ERR_PROBE_LIMIT;
@@ -567,6 +573,43 @@ __global__ void __launch_bounds__(256) k_stride(const int32_t* __restrict__ coor
 #pragma unroll
   for (int i = 1; i < W; ++i) c[i] = floor_to(c[i], st.s[i - 1]);
   store_row<W, kVec>(out, row, c);
+}
+
+// Sum or mean of the rows of every voxel: the first row of a voxel is copied, the others - few, in a lidar sweep - are
+// added to it (atomics), and only voxels of several rows are divided. (960 K points, 4 channels: 57 us by zero fills, two
+// index_add, a ones tensor, a clamp and a division.)
+__global__ void __launch_bounds__(256) k_segment_first(const float* __restrict__ feats, const int64_t* __restrict__ mapping,
+                                                       uint32_t m, int C, float* __restrict__ out, uint32_t* __restrict__ count) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (size_t)m * C) return;
+  const size_t u = i / C, c = i - u * C;
+  out[i] = __ldg(feats + (size_t)__ldg(mapping + u) * C + c);
+  if (c == 0) count[u] = 1u;
+}
+__global__ void __launch_bounds__(256) k_segment_first4(const float4* __restrict__ feats, const int64_t* __restrict__ mapping,
+                                                        uint32_t m, float4* __restrict__ out, uint32_t* __restrict__ count) {
+  const uint32_t u = blockIdx.x * 256 + threadIdx.x;
+  if (u >= m) return;
+  out[u] = __ldg(feats + __ldg(mapping + u));
+  count[u] = 1u;
+}
+__global__ void __launch_bounds__(256) k_segment_add(const float* __restrict__ feats, const int64_t* __restrict__ inverse,
+                                                     const int64_t* __restrict__ mapping, uint32_t n, int C,
+                                                     float* __restrict__ out, uint32_t* __restrict__ count) {
+  const uint32_t row = blockIdx.x * 256 + threadIdx.x;
+  if (row >= n) return;
+  const size_t u = (size_t)__ldg(inverse + row);
+  if ((uint32_t)__ldg(mapping + u) == row) return;
+  for (int c = 0; c < C; ++c) atomicAdd(out + u * C + c, __ldg(feats + (size_t)row * C + c));
+  atomicAdd(count + u, 1u);
+}
+__global__ void __launch_bounds__(256) k_segment_divide(uint32_t m, int C, const uint32_t* __restrict__ count,
+                                                        float* __restrict__ out) {
+  const uint32_t u = blockIdx.x * 256 + threadIdx.x;
+  if (u >= m) return;
+  const uint32_t k = __ldg(count + u);
+  if (k > 1u)
+    for (int c = 0; c < C; ++c) out[(size_t)u * C + c] = __fdiv_rn(out[(size_t)u * C + c], (float)k);
 }
 
 // Continuous (field) coordinates -> integer voxel coordinates, the reference's rule in float32:
@@ -691,6 +734,31 @@ extern "C" int rmn_field_quantize(const float* d_field, uint32_t n_rows, int W, 
   return RMN_OK;
 }
 
+extern "C" int rmn_segment_reduce(const float* d_feats, uint32_t n_rows, int channels, const int64_t* d_inverse,
+                                  const int64_t* d_mapping, uint32_t n_unique, int mean, float* d_out, uint32_t* d_counts,
+                                  void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  if (channels < 1 || n_unique > n_rows) return RMN_ERR_BAD_ARG;
+  if (n_unique == 0) return RMN_OK;
+  if (!d_feats || !d_inverse || !d_mapping || !d_out || !d_counts) return RMN_ERR_BAD_ARG;
+  if (channels == 4 && !((uintptr_t)d_feats & 15) && !((uintptr_t)d_out & 15)) {
+    k_segment_first4<<<(n_unique + 255) / 256, 256, 0, stream>>>((const float4*)d_feats, d_mapping, n_unique, (float4*)d_out,
+                                                                 d_counts);
+  } else {
+    const size_t total = (size_t)n_unique * channels;
+    if (total >= ((size_t)1 << 39)) return RMN_ERR_TOO_LARGE;
+    k_segment_first<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(d_feats, d_mapping, n_unique, channels, d_out, d_counts);
+  }
+  RMN_LAUNCH_CHECK();
+  if (n_unique == n_rows) return RMN_OK;
+  k_segment_add<<<(n_rows + 255) / 256, 256, 0, stream>>>(d_feats, d_inverse, d_mapping, n_rows, channels, d_out, d_counts);
+  RMN_LAUNCH_CHECK();
+  if (!mean) return RMN_OK;
+  k_segment_divide<<<(n_unique + 255) / 256, 256, 0, stream>>>(n_unique, channels, d_counts, d_out);
+  RMN_LAUNCH_CHECK();
+  return RMN_OK;
+}
+
 extern "C" int rmn_coords_discretize(const void* d_in, int in_type, uint64_t n_elems, double quantization_size,
                                      int32_t* d_out, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
@@ -754,20 +822,21 @@ static int table_build_begin(const int32_t* d_coords, uint32_t n_rows, int W, vo
   auto* h = reinterpret_cast<TableHeader*>(d_table);
   auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
   const uint32_t capacity = table_capacity(n_rows);
+  const Scratch sc = scratch(d_workspace, n_rows);
   RMN_CUDA_TRY(cudaMemsetAsync(h, 0, sizeof(TableHeader), stream));
   {
     const uint32_t fill_blocks = (capacity + 255u) / 256u;
     const uint32_t blocks = fill_blocks < kGrid ? fill_blocks : kGrid;
     RMN_DISPATCH_W(W, k_fill_range<kW><<<blocks, 256, 0, stream>>>(d_coords, n_rows, h,
-                                                                    reinterpret_cast<uint4*>(slots), capacity));
+                                                                    reinterpret_cast<uint4*>(slots), capacity,
+                                                                    sc.repeat_bits));
     RMN_LAUNCH_CHECK();
   }
   if (n_rows == 0) return RMN_OK;
-  const Scratch sc = scratch(d_workspace, n_rows);
   const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
-  RMN_DISPATCH_W(W, k_insert<kW><<<nb, 256, 0, stream>>>(d_coords, n_rows, h, slots, sc.slot_of_row, look_first));
+  RMN_DISPATCH_W(W, k_insert<kW><<<nb, 256, 0, stream>>>(d_coords, n_rows, h, slots, sc, look_first));
   RMN_LAUNCH_CHECK();
-  k_count_first<<<nb < kGrid ? nb : kGrid, kRowsPerBlock, 0, stream>>>(slots, n_rows, h, sc, post);
+  k_count_first<<<(nb + 255) / 256, 256, 0, stream>>>(n_rows, h, sc, post);
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

@@ -619,6 +619,21 @@ at::Tensor quantize_features(const at::Tensor& features, const at::Tensor& first
       return features;
     case SparseTensorQuantizationMode::UNWEIGHTED_SUM:
     case SparseTensorQuantizationMode::UNWEIGHTED_AVERAGE: {
+      const bool grad = at::GradMode::is_enabled() && features.requires_grad();
+      if (features.is_cuda() && features.scalar_type() == at::kFloat && !grad && features.size(0) > 0 &&
+          features.size(1) > 0) {
+        c10::cuda::CUDAGuard guard(features.device());
+        auto rows = features.contiguous();
+        auto out = at::empty({unique_count, features.size(1)}, features.options());
+        auto counts = at::empty({unique_count}, features.options().dtype(at::kInt));
+        check(rmn_segment_reduce(static_cast<const float*>(ptr(rows)), static_cast<uint32_t>(rows.size(0)),
+                                 static_cast<int>(rows.size(1)), static_cast<const int64_t*>(ptr(row_to_unique)),
+                                 static_cast<const int64_t*>(ptr(first_rows)), static_cast<uint32_t>(unique_count),
+                                 mode == SparseTensorQuantizationMode::UNWEIGHTED_AVERAGE ? 1 : 0,
+                                 static_cast<float*>(ptr(out)), static_cast<uint32_t*>(ptr(counts)), current_stream()),
+              "rmn_segment_reduce");
+        return out;
+      }
       auto result = torch::zeros({unique_count, features.size(1)}, features.options());
       result.index_add_(0, row_to_unique, features);
       if (mode == SparseTensorQuantizationMode::UNWEIGHTED_SUM) return result;

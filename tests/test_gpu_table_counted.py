@@ -83,3 +83,22 @@ def test_split_offsets_and_host_pointers(n):
         torch.cuda.synchronize()
         assert torch.equal(nbr, want)
         assert host.tolist() == ptr.tolist() == [0] + (want >= 0).sum(1).cumsum(0).tolist()
+
+
+@pytest.mark.parametrize("n,channels,extent,mean", [(1, 1, 3, 1), (5000, 4, 8, 1), (5000, 3, 1000, 1), (70_001, 16, 20, 0),
+                                                    (4096, 4, 2, 0)])
+def test_segment_reduce_matches_float64(n, channels, extent, mean):
+    from riemannengine_b200 import capi, ops
+    c = _coords(n, 3, extent, n)
+    _, info, mapping, inverse, _, _ = _counted(c, 0)
+    m = info.tolist()[0]
+    x = torch.randn((n, channels), device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    out, counts = torch.empty((m, channels), device="cuda"), torch.empty(m, dtype=torch.int32, device="cuda")
+    capi.check(capi.lib().rmn_segment_reduce(ops._ptr(x), n, channels, ops._ptr(inverse), ops._ptr(mapping), m, mean,
+                                             ops._ptr(out), ops._ptr(counts), ops._stream()), "segment")
+    want = torch.zeros((m, channels), dtype=torch.float64, device="cuda").index_add_(0, inverse, x.double())
+    per = torch.bincount(inverse, minlength=m).double().unsqueeze(1)
+    if mean:
+        want /= per
+    assert float((out.double() - want).abs().max()) <= 1e-5 * max(1.0, float(want.abs().max()))
+    assert n == m or torch.equal(counts.double(), per[:, 0])
