@@ -319,9 +319,10 @@ WgradPlan plan(uint32_t n_dst, int K, int sms) {
   p.tmem_cols = pow2_at_least((uint32_t)((p.groups_per_set + C::GP - 1) / C::GP * C::GP) * COUT);
   uint32_t want = (uint32_t)(sms / p.sets);
   if (want < 1) want = 1;
-  // at least 32 row blocks (2048 rows) per slice: fewer, and the fp32 partials cost more than they spread
+  // at least 8 row blocks (512 rows) per slice: fewer, and the fp32 partials cost more than they spread (18 000 rows,
+  // 64 -> 64: 62 us with 32 blocks per slice, i.e. 16 CTAs, 27 with 8, and 5 instead of 2 to add the partials)
   const uint32_t total_blocks = (n_dst + kRowsPerStage - 1) / kRowsPerStage;
-  uint32_t slices = total_blocks / 32;
+  uint32_t slices = total_blocks / 8;
   if (slices < 1) slices = 1;
   p.chunks = slices < want ? slices : want;
   return p;
