@@ -430,9 +430,9 @@ int rmn_conv_weight_image(const void *d_weights, int K, int w_in, int w_out, int
 int rmn_conv_forward_image(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
                            const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out, const float *d_scale,
                            const float *d_shift, const void *d_add, int relu, void *stream);
-/* d_dst [n_rows, c_dst] = d_src [n_rows, c_src] with c_dst - c_src zero channels behind (bf16; c_dst a multiple of 8,
- * d_dst 16-byte aligned). */
-int rmn_pad_channels(const void *d_src, uint32_t n_rows, int c_src, void *d_dst, int c_dst, void *stream);
+/* d_dst [n_rows, c_dst] = the first c_src elements of rows ld_src apart in d_src, with c_dst - c_src zeros behind (2-byte
+ * elements; fp32 as pairs of them). */
+int rmn_pad_channels(const void *d_src, uint32_t n_rows, int c_src, int ld_src, void *d_dst, int c_dst, void *stream);
 int rmn_conv_forward_image_stats(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
                                  const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out,
                                  const float *d_scale, const float *d_shift, int relu, double *d_stats, void *d_workspace,

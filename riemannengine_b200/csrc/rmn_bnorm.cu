@@ -204,19 +204,34 @@ static bool dot_fast_shape(int C) {
   return lpr >= 1 && lpr <= 32 && (32 % lpr) == 0;
 }
 
-// A narrow stem or head as the operand of a tensor-core convolution: one 16-byte store per thread, streaming (600 K rows
-// 4 -> 32 bf16: 9 us; a zero fill and a strided copy took 45).
-__global__ void __launch_bounds__(256) k_pad_channels(const uint16_t* __restrict__ src, size_t total, int c_src, int c_dst,
-                                                      uint4* __restrict__ dst) {
-  const uint32_t per_row = (uint32_t)c_dst / 8;
+// Rows of c_src 2-byte elements, ld_src apart, as rows of c_dst with zeros behind: a narrow stem or head as the operand of a
+// tensor-core convolution, or one half of a concatenation as a matrix of its own. V elements per thread in one store, and
+// in one load too where kVecSrc; streaming (600 K rows 4 -> 32: 9 us, a zero fill and a strided copy took 45; 600 K x 32 of
+// rows of 64: 14 us, a generic strided copy 53).
+template <int V, bool kVecSrc>
+__global__ void __launch_bounds__(256) k_pad_channels(const uint16_t* __restrict__ src, size_t total, int c_src, int ld_src,
+                                                      int c_dst, uint16_t* __restrict__ dst) {
+  struct __align__(2 * V) Chunk {
+    uint16_t v[V];
+  };
+  const uint32_t per_row = (uint32_t)c_dst / V;
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {
     const size_t row = i / per_row;
-    const int c0 = (int)(i - row * per_row) * 8;
-    uint16_t v[8];
+    const int c0 = (int)(i - row * per_row) * V;
+    const uint16_t* p = src + row * ld_src + c0;
+    Chunk x;
+    if constexpr (kVecSrc) {
+      if (c0 < c_src) {
+        x = *reinterpret_cast<const Chunk*>(p);
+      } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = c0 + j < c_src ? __ldg(src + row * c_src + c0 + j) : (uint16_t)0;
-    dst[i] = make_uint4(v[0] | (uint32_t)v[1] << 16, v[2] | (uint32_t)v[3] << 16, v[4] | (uint32_t)v[5] << 16,
-                        v[6] | (uint32_t)v[7] << 16);
+        for (int j = 0; j < V; ++j) x.v[j] = 0;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < V; ++j) x.v[j] = c0 + j < c_src ? __ldg(p + j) : (uint16_t)0;
+    }
+    reinterpret_cast<Chunk*>(dst)[i] = x;
   }
 }
 
@@ -224,16 +239,28 @@ __global__ void __launch_bounds__(256) k_pad_channels(const uint16_t* __restrict
 
 using namespace rmn;
 
-extern "C" int rmn_pad_channels(const void* d_src, uint32_t n_rows, int c_src, void* d_dst, int c_dst, void* stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
-  if (c_src < 1 || c_dst < c_src || c_dst % 8) return RMN_ERR_BAD_ARG;
-  if (n_rows == 0) return RMN_OK;
-  if (!d_src || !d_dst || ((uintptr_t)d_dst & 15) || ((uintptr_t)d_src & 1)) return RMN_ERR_BAD_ARG;
-  const size_t total = (size_t)n_rows * (size_t)(c_dst / 8), blocks = (total + 255) / 256;
-  k_pad_channels<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, stream>>>((const uint16_t*)d_src, total, c_src,
-                                                                                        c_dst, (uint4*)d_dst);
+template <int V>
+static int pad_channels(const void* src, uint32_t n, int c_src, int ld_src, void* dst, int c_dst, cudaStream_t stream) {
+  const size_t total = (size_t)n * (size_t)(c_dst / V), blocks = (total + 255) / 256;
+  const unsigned grid = (unsigned)(blocks < 148 * 32 ? blocks : 148 * 32);
+  const bool vec = c_src % V == 0 && ld_src % V == 0 && (uintptr_t)src % (2 * V) == 0;
+  if (vec)
+    k_pad_channels<V, true><<<grid, 256, 0, stream>>>((const uint16_t*)src, total, c_src, ld_src, c_dst, (uint16_t*)dst);
+  else
+    k_pad_channels<V, false><<<grid, 256, 0, stream>>>((const uint16_t*)src, total, c_src, ld_src, c_dst, (uint16_t*)dst);
   RMN_LAUNCH_CHECK();
   return RMN_OK;
+}
+
+extern "C" int rmn_pad_channels(const void* d_src, uint32_t n_rows, int c_src, int ld_src, void* d_dst, int c_dst,
+                                void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  if (c_src < 1 || c_dst < c_src || ld_src < c_src) return RMN_ERR_BAD_ARG;
+  if (n_rows == 0) return RMN_OK;
+  if (!d_src || !d_dst || ((uintptr_t)d_dst & 1) || ((uintptr_t)d_src & 1)) return RMN_ERR_BAD_ARG;
+  if (c_dst % 8 == 0 && !((uintptr_t)d_dst & 15)) return pad_channels<8>(d_src, n_rows, c_src, ld_src, d_dst, c_dst, stream);
+  if (c_dst % 4 == 0 && !((uintptr_t)d_dst & 7)) return pad_channels<4>(d_src, n_rows, c_src, ld_src, d_dst, c_dst, stream);
+  return pad_channels<1>(d_src, n_rows, c_src, ld_src, d_dst, c_dst, stream);
 }
 
 extern "C" size_t rmn_channel_dot_stats_workspace_bytes(int channels) {

@@ -856,11 +856,58 @@ SparseTensor& SparseTensor::operator+=(const SparseTensor& other) {
 SparseTensor SparseTensor::operator+(at::Scalar scalar) const { return SparseTensor(features_ + scalar, key_, manager_); }
 SparseTensor SparseTensor::operator*(at::Scalar scalar) const { return SparseTensor(features_ * scalar, key_, manager_); }
 
+namespace {
+// Rows of x [n, c] (any distance apart, channels contiguous) with zero channels behind, up to `channels`, as a contiguous
+// matrix; x itself where it is one already.
+at::Tensor pad_channels(const at::Tensor& x, int64_t channels) {
+  if (x.size(1) == channels && x.is_contiguous()) return x;
+  const bool rows = x.is_cuda() && (x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kFloat) && x.size(0) > 0 &&
+                    x.stride(1) == 1 && x.stride(0) >= x.size(1);
+  if (!rows && x.size(1) == channels) return x.contiguous();
+  auto src = rows ? x : x.contiguous();
+  c10::cuda::CUDAGuard guard(src.device());
+  auto out = at::empty({src.size(0), channels}, src.options());
+  const int e = static_cast<int>(src.element_size() / 2);
+  check(rmn_pad_channels(ptr(src), static_cast<uint32_t>(src.size(0)), static_cast<int>(src.size(1)) * e,
+                         static_cast<int>(src.stride(0)) * e, ptr(out), static_cast<int>(channels) * e, current_stream()),
+        "rmn_pad_channels");
+  return out;
+}
+at::Tensor contiguous_rows(const at::Tensor& x) { return x.dim() == 2 ? pad_channels(x, x.size(1)) : x.contiguous(); }
+
+// Concatenation of the channels of two matrices with the same rows (a skip connection). The gradient of a part is made
+// contiguous here: as a view into the whole gradient it would be read with strides by every kernel behind it.
+class ChannelCatAutograd : public torch::autograd::Function<ChannelCatAutograd> {
+public:
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, at::Tensor a, at::Tensor b) {
+    ctx->saved_data["split"] = a.size(1);
+    return at::cat({a, b}, 1);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grad_outputs) {
+    const auto& grad = grad_outputs[0];
+    const int64_t split = ctx->saved_data["split"].toInt();
+    at::Tensor ga, gb;
+    if (ctx->needs_input_grad(0)) ga = contiguous_rows(grad.narrow(1, 0, split));
+    if (ctx->needs_input_grad(1)) gb = contiguous_rows(grad.narrow(1, split, grad.size(1) - split));
+    return {ga, gb};
+  }
+};
+}  // namespace
+
 SparseTensor cat(const std::vector<SparseTensor>& tensors) {
   validate_same_map(tensors, false);
   std::vector<at::Tensor> features;
-  for (auto const& t : tensors) features.push_back(t.F());
-  return SparseTensor(torch::cat(features, 1), tensors.front().coordinate_map_key(),
+  bool grad = false, same = true;
+  for (auto const& t : tensors) {
+    features.push_back(t.F());
+    grad = grad || t.F().requires_grad();
+    same = same && t.F().is_cuda() && t.F().dim() == 2 && t.F().scalar_type() == tensors.front().F().scalar_type();
+  }
+  auto joined = grad && same && features.size() == 2 && at::GradMode::is_enabled()
+                    ? ChannelCatAutograd::apply(features[0], features[1])
+                    : torch::cat(features, 1);
+  return SparseTensor(std::move(joined), tensors.front().coordinate_map_key(),
                       tensors.front().coordinate_manager());
 }
 
@@ -1026,17 +1073,6 @@ std::pair<int64_t, int64_t> tc_legal_shape(int64_t c_in, int64_t c_out) {
   return best;
 }
 
-// bf16 features [n, c] with zero channels behind, up to `channels`
-at::Tensor pad_channels(const at::Tensor& x_in, int64_t channels) {
-  if (x_in.size(1) == channels) return x_in;
-  auto x = x_in.contiguous();
-  auto out = at::empty({x.size(0), channels}, x.options());
-  check(rmn_pad_channels(ptr(x), static_cast<uint32_t>(x.size(0)), static_cast<int>(x.size(1)), ptr(out),
-                         static_cast<int>(channels), current_stream()),
-        "rmn_pad_channels");
-  return out;
-}
-
 // bf16 channel counts without a tensor-core kernel (a 4-channel stem, 48 or 96 channels ...) run as the next pair that
 // has one: padded input channels multiply zero weights, padded output channels are cut off again.
 std::pair<int64_t, int64_t> run_shape(const at::Tensor& kernel) {
@@ -1071,7 +1107,7 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
                         const ConvEpilogue& ep = {}, const at::Tensor& plan = at::Tensor(), torch::nn::BatchNorm1dImpl* bn = nullptr) {
   TORCH_CHECK(feats_in.is_cuda() && kernel_in.is_cuda(), "features and kernel must be CUDA tensors");
   TORCH_CHECK(feats_in.scalar_type() == kernel_in.scalar_type(), "expected features and kernel to have the same dtype");
-  auto feats = feats_in.contiguous(), kernel = kernel_in.contiguous();
+  auto feats = contiguous_rows(feats_in), kernel = kernel_in.contiguous();
   c10::cuda::CUDAGuard guard(feats.device());
   const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(kernel.size(1)),
             c_out = static_cast<int>(kernel.size(2));
@@ -1108,7 +1144,7 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
                                    static_cast<uint32_t>(nbr.size(1)), ptr(out), static_cast<const float*>(ptr(scale)),
                                    static_cast<const float*>(ptr(shift)), ptr(ep.add), ep.relu ? 1 : 0, current_stream()),
             "rmn_conv_forward_image");
-      return padded ? out.narrow(1, 0, c_out) : out;
+      return contiguous_rows(out.narrow(1, 0, c_out));
     }
     TORCH_CHECK(!bn && !ep.add.defined(), "no kernel folds this layer's batch norm");
   }
@@ -1125,7 +1161,7 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
 // reverse: nbr_t is the forward table of a point-symmetric self map, i.e. its offsets run backwards
 at::Tensor conv_backward_input(const at::Tensor& grad_in, const at::Tensor& kernel_in, const at::Tensor& nbr_t,
                                bool reverse, const at::Tensor& plan_t = at::Tensor()) {
-  auto grad = grad_in.contiguous();
+  auto grad = contiguous_rows(grad_in);
   c10::cuda::CUDAGuard guard(grad.device());
   if (grad.scalar_type() == at::kFloat && grad.size(0) > 0 && nbr_t.size(1) > 0) {
     // fp32: the forward pass on transposed weights
@@ -1148,7 +1184,7 @@ at::Tensor conv_backward_input(const at::Tensor& grad_in, const at::Tensor& kern
                                    static_cast<uint32_t>(nbr_t.size(1)), ptr(out), nullptr, nullptr, nullptr, 0,
                                    current_stream()),
             "rmn_conv_forward_image");
-      return shape.first == c_in ? out : out.narrow(1, 0, c_in).contiguous();
+      return contiguous_rows(out.narrow(1, 0, c_in));
     }
   }
   auto out = at::empty({nbr_t.size(1), c_in}, grad.options());
@@ -1230,12 +1266,13 @@ public:
     auto saved = ctx->get_saved_variables();
     auto nbr_out = ctx->saved_data["nbr_out"].toTensor();
     auto nbr_in = ctx->saved_data["nbr_in"].toTensor();
-    auto grad = grad_outputs[0].contiguous();
+    auto grad = grad_outputs[0];
     const auto& kernel = saved[1];
     if (grad.size(0) > 0 && nbr_out.size(1) > 0 && saved[0].size(0) > 0) {
       c10::cuda::CUDAGuard guard(grad.device());
       grad = pad_channels(grad, run_shape(kernel).second);
     }
+    grad = contiguous_rows(grad);
     auto weight_gradient = [&] {
       auto g = conv_backward_weight(saved[0], grad, nbr_out);
       return g.sizes() == kernel.sizes() ? g : g.narrow(1, 0, kernel.size(1)).narrow(2, 0, kernel.size(2)).contiguous();
@@ -1471,7 +1508,7 @@ class BatchNormAutograd : public torch::autograd::Function<BatchNormAutograd> {
 public:
   static at::Tensor forward(torch::autograd::AutogradContext* ctx, at::Tensor x_in, at::Tensor gamma, at::Tensor beta,
                             at::Tensor running_mean, at::Tensor running_var, double momentum, double eps) {
-    auto x = x_in.contiguous();
+    auto x = contiguous_rows(x_in);
     c10::cuda::CUDAGuard guard(x.device());
     const uint32_t n = static_cast<uint32_t>(x.size(0));
     const int C = static_cast<int>(x.size(1));
@@ -1501,7 +1538,7 @@ public:
                                                  torch::autograd::variable_list grad_outputs) {
     auto saved = ctx->get_saved_variables();
     auto x = saved[0], gamma = saved[1], coeffs = saved[2];
-    auto dy = grad_outputs[0].contiguous();
+    auto dy = contiguous_rows(grad_outputs[0]);
     c10::cuda::CUDAGuard guard(x.device());
     const uint32_t n = static_cast<uint32_t>(x.size(0));
     const int C = static_cast<int>(x.size(1));

@@ -97,3 +97,27 @@ def test_network_in_evaluation_mode_matches_its_layers():
     with torch.no_grad():
         got = net(C.SparseTensor(feats, coords)).F.double()
     assert float((got - want).norm()) <= 2e-2 * float(want.norm())
+
+
+@pytest.mark.parametrize("c_src,ld,c_dst,skip", [(4, 4, 32, 0), (20, 32, 20, 0), (32, 64, 32, 32), (33, 70, 33, 3), (7, 9, 40, 1)])
+def test_pad_channels_copies_strided_rows(c_src, ld, c_dst, skip):
+    from riemannengine_b200 import capi, ops
+    n = 1027
+    x = torch.randn((n, ld + skip), device="cuda").bfloat16()
+    out = torch.full((n, c_dst), 7.0, device="cuda", dtype=torch.bfloat16)
+    capi.check(capi.lib().rmn_pad_channels(x.data_ptr() + 2 * skip, n, c_src, ld + skip, ops._ptr(out), c_dst, ops._stream()), "pad")
+    assert torch.equal(out, torch.nn.functional.pad(x[:, skip:skip + c_src], (0, c_dst - c_src)))
+
+
+def test_channel_cat_splits_its_gradient():
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    coords = torch.tensor([[0, i, 0, 0] for i in range(300)], dtype=torch.int32, device="cuda")
+    for dtype in (torch.float32, torch.bfloat16):
+        a, b = (torch.randn((300, c), device="cuda").to(dtype).requires_grad_(True) for c in (32, 20))
+        x = C.SparseTensor(a, coords)
+        y = C.cat([x, C.SparseTensor(b, x.coordinate_map_key, x.coordinate_manager)])
+        g = torch.randn((300, 52), device="cuda").to(dtype)
+        y.F.backward(g)
+        assert torch.equal(y.F, torch.cat([a, b], 1))
+        assert torch.equal(a.grad, g[:, :32]) and torch.equal(b.grad, g[:, 32:])
