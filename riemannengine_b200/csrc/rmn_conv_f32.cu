@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(256)
     k_conv_f32(const float* __restrict__ src, const float* __restrict__ w, const int32_t* __restrict__ nbr, uint32_t n_dst,
                int K, int c_red, int c_col, int splits, float* __restrict__ out, const float* __restrict__ ep_scale,
                const float* __restrict__ ep_shift, int ep_relu) {
+  after_previous_kernel();
   using Cfg = F32FwCfg<NV>;
   constexpr int C = Cfg::C, BATCH = Cfg::BATCH, RGS = Cfg::RGS;
   extern __shared__ __align__(16) float smem_f[];
@@ -243,8 +244,8 @@ static int launch_conv_f32(const float* src, const float* w, const int32_t* nbr,
   const int warps = splits == 8 ? 8 : 4;
   const uint32_t groups = warps / splits;
   dim3 grid((row_groups + groups - 1) / groups, tiles_n);
-  k_conv_f32<NV><<<grid, warps * 32, (size_t)warps * Cfg::WARP_WORDS * 4, stream>>>(src, w, nbr, n_dst, K, c_red, c_col,
-                                                                                   splits, out, ep_scale, ep_shift, ep_relu);
+  RMN_CUDA_TRY(launch_overlapped(k_conv_f32<NV>, dim3(grid), dim3(warps * 32), (size_t)warps * Cfg::WARP_WORDS * 4, stream,
+                                 src, w, nbr, n_dst, K, c_red, c_col, splits, out, ep_scale, ep_shift, ep_relu));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

@@ -73,6 +73,7 @@ template <int CR, int CC>
 __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, uint32_t w_red,
                                                       uint32_t w_col, int transpose, int reverse, rmn_bn_fold fold,
                                                       uint4* __restrict__ image) {
+  after_previous_kernel();
   if (fold.scale && blockIdx.x == gridDim.x - 1) {
     for (uint32_t c = threadIdx.x; c < CC; c += 256) {
       auto param = [&](const void* p, float absent) {
@@ -176,10 +177,6 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   const bool has_ep = ep_scale != nullptr || ep_shift != nullptr || ep_add != nullptr || ep_relu != 0;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (has_ep && tid < CC) {
-    s_ep[tid] = ep_scale ? __ldg(ep_scale + col0 + tid) : 1.f;
-    s_ep[CC + tid] = ep_shift ? __ldg(ep_shift + col0 + tid) : 0.f;
-  }
   if (tid == 0) {
     for (int s = 0; s < BST; ++s) {
       mbar_init(&b_full[s], 1);
@@ -200,6 +197,11 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  after_previous_kernel();
+  if (has_ep && tid < CC) {
+    s_ep[tid] = ep_scale ? __ldg(ep_scale + col0 + tid) : 1.f;
+    s_ep[CC + tid] = ep_shift ? __ldg(ep_shift + col0 + tid) : 0.f;
   }
   tc_fence_before();
   __syncthreads();
@@ -584,10 +586,9 @@ int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n
   const uint32_t n_super = (n_dst + kTileM * C::T - 1) / (kTileM * C::T);
   const uint32_t n_blocks = n_cols / CC, fit = (uint32_t)sms > n_blocks ? (uint32_t)sms / n_blocks : 1u;
   const uint32_t grid = fit < n_super ? fit : n_super;  // one CTA per SM owns its tensor memory
-  kern<<<dim3(grid, n_blocks), kTaThreads, C::SMEM, stream>>>((const __nv_bfloat16*)src, (const uint8_t*)image, nbr, n_dst, K,
-                                             (__nv_bfloat16*)out, n_super, ep_scale, ep_shift,
-                                             (const __nv_bfloat16*)ep_add, ep_relu, n_cols, stats_partial,
-                                             perm, tile_mask);
+  RMN_CUDA_TRY(launch_overlapped(kern, dim3(grid, n_blocks), dim3(kTaThreads), C::SMEM, stream, (const __nv_bfloat16*)src,
+                                 (const uint8_t*)image, nbr, n_dst, K, (__nv_bfloat16*)out, n_super, ep_scale, ep_shift,
+                                 (const __nv_bfloat16*)ep_add, ep_relu, n_cols, stats_partial, perm, tile_mask));
   RMN_LAUNCH_CHECK();
   count_tc_launch();
   if (grid_out) *grid_out = grid;
@@ -605,8 +606,9 @@ template <int CR, int CC>
 int launch_image(const void* w, int K, int w_red, int w_col, int transpose, int reverse, const rmn_bn_fold& fold, void* image,
                  cudaStream_t stream) {
   const uint32_t chunks = (uint32_t)(image_bytes<CR, CC>(K) / 16);
-  k_weight_image<CR, CC><<<(chunks + 255) / 256 + (fold.scale ? 1 : 0), 256, 0, stream>>>((const __nv_bfloat16*)w, K, w_red, w_col, transpose,
-                                                                  reverse, fold, (uint4*)image);
+  RMN_CUDA_TRY(launch_overlapped(k_weight_image<CR, CC>, dim3((chunks + 255) / 256 + (fold.scale ? 1 : 0)), dim3(256), 0,
+                                 stream, (const __nv_bfloat16*)w, K, (uint32_t)w_red, (uint32_t)w_col, transpose, reverse, fold,
+                                 (uint4*)image));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe(
     const int32_t* __restrict__ query, uint32_t n_query, const int32_t* __restrict__ offsets,
     int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks,
     uint32_t* __restrict__ scan_ticket) {
+  after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int D = W - 1;
   const int k_begin = (int)((uint32_t)K * blockIdx.y / gridDim.y), k_end = (int)((uint32_t)K * (blockIdx.y + 1) / gridDim.y);
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
     const int32_t* __restrict__ coords, uint32_t n, const int32_t* __restrict__ offsets, int K,
     int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks,
     uint32_t* __restrict__ scan_ticket) {
+  after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int D = W - 1;
   const int half = K / 2;
@@ -222,6 +224,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
 __global__ void __launch_bounds__(1024) k_kmap_scan(uint32_t* __restrict__ block_counts, uint32_t n_blocks, int K,
                                                     int mirror_half, uint32_t* __restrict__ totals,
                                                     int64_t* __restrict__ offset_ptr, volatile int64_t* host_ptr) {
+  after_previous_kernel();
   __shared__ uint32_t warp_sums[32];
   __shared__ int64_t warp_sums64[32];
   __shared__ uint32_t s_last;
@@ -510,15 +513,16 @@ static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_qu
                                    stream));
     const int hs = half > 0 ? half : 1;
     const size_t smem = (size_t)hs * 8 + (size_t)hs * (W - 1) * 4 + (size_t)hs * 4;
-    RMN_DISPATCH_W(W, k_kmap_probe_self<kW><<<dim3(nb, offset_split(nb, half)), kKmapBlock, smem, stream>>>(
-                          h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket));
+    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(
+                        k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock), smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket)));
   } else {
     const size_t smem = (size_t)K * 8 + (size_t)K * (W - 1) * 4 + (size_t)K * 4;
-    RMN_DISPATCH_W(W, k_kmap_probe<kW><<<dim3(nb, offset_split(nb, K)), kKmapBlock, smem, stream>>>(
-                          h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket));
+    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(
+                        k_kmap_probe<kW>, dim3(nb, offset_split(nb, K)), dim3(kKmapBlock), smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket)));
   }
   RMN_LAUNCH_CHECK();
-  k_kmap_scan<<<self ? half + 1 : K, 1024, 0, stream>>>(block_counts, nb, K, half, totals, d_offset_ptr, host_alias);
+  RMN_CUDA_TRY(launch_overlapped(k_kmap_scan, dim3(self ? half + 1 : K), dim3(1024), 0, stream,
+                        block_counts, nb, K, half, totals, d_offset_ptr, host_alias));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

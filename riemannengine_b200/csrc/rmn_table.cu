@@ -103,6 +103,7 @@ template <int W>
 __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ coords, uint32_t n,
                                                     TableHeader* h, uint4* __restrict__ slots, uint32_t capacity,
                                                     uint32_t* __restrict__ repeat_bits) {
+  after_previous_kernel();
   __shared__ int32_t s_mn[8][W], s_mx[8][W];
   constexpr int NA = W - 1 < 3 ? W - 1 : 3;
   __shared__ uint32_t s_or[8][NA];
@@ -244,6 +245,7 @@ template <int W>
 __global__ void __launch_bounds__(256) k_insert(const int32_t* __restrict__ coords, uint32_t n,
                                                 TableHeader* h, Slot* slots,
                                                 Scratch sc, int look_first) {
+  after_previous_kernel();
   if (h->status != RMN_OK) return;
   const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t repeat = kNoRow;
@@ -321,6 +323,7 @@ __device__ __forceinline__ uint32_t scan_u32_block(uint32_t* __restrict__ counts
 // block); the last CUDA block to finish turns the numbers into block offsets (exclusive scan) and writes n_unique. Nothing
 // to do when the insert pass met no duplicate: nothing is compacted then (see k_finalize).
 __global__ void __launch_bounds__(256) k_count_first(uint32_t n, TableHeader* h, Scratch sc, HostPost post) {
+  after_previous_kernel();
   const bool failed = h->status != RMN_OK;
   if (failed || h->n_dups == 0) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -355,6 +358,7 @@ template <int W>
 __global__ void __launch_bounds__(kRowsPerBlock) k_finalize(
     const int32_t* __restrict__ coords, uint32_t n, const TableHeader* h, Slot* slots,
     Scratch sc, int64_t* __restrict__ mapping, int32_t* __restrict__ unique_coords, int64_t* __restrict__ inverse) {
+  after_previous_kernel();
   if (h->status != RMN_OK) return;
   const uint32_t row = blockIdx.x * kRowsPerBlock + threadIdx.x;
   if (h->n_dups == 0) {
@@ -394,6 +398,7 @@ __global__ void __launch_bounds__(256) k_inverse(const Slot* __restrict__ slots,
                                                  const uint32_t* __restrict__ slot_of_row,
                                                  uint32_t n, const TableHeader* h,
                                                  int64_t* __restrict__ inverse) {
+  after_previous_kernel();
   // without duplicates k_finalize has already written the identity
   if (h->n_dups == 0 || h->status != RMN_OK) return;
   for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n; row += gridDim.x * blockDim.x)
@@ -408,6 +413,7 @@ __global__ void __launch_bounds__(1024) k_build_small(const int32_t* __restrict_
                                                       Slot* slots, uint32_t capacity, Scratch sc,
                                                       int64_t* __restrict__ mapping, int32_t* __restrict__ unique_coords,
                                                       int64_t* __restrict__ inverse, int look_first, HostPost post) {
+  after_previous_kernel();
   constexpr int NA = W - 1 < 3 ? W - 1 : 3;
   __shared__ TableHeader s_h;
   __shared__ uint32_t s_ok;
@@ -580,6 +586,7 @@ __global__ void __launch_bounds__(256) k_stride(const int32_t* __restrict__ coor
 // index_add, a ones tensor, a clamp and a division.)
 __global__ void __launch_bounds__(256) k_segment_first(const float* __restrict__ feats, const int64_t* __restrict__ mapping,
                                                        uint32_t m, int C, float* __restrict__ out, uint32_t* __restrict__ count) {
+  after_previous_kernel();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= (size_t)m * C) return;
   const size_t u = i / C, c = i - u * C;
@@ -588,6 +595,7 @@ __global__ void __launch_bounds__(256) k_segment_first(const float* __restrict__
 }
 __global__ void __launch_bounds__(256) k_segment_first4(const float4* __restrict__ feats, const int64_t* __restrict__ mapping,
                                                         uint32_t m, float4* __restrict__ out, uint32_t* __restrict__ count) {
+  after_previous_kernel();
   const uint32_t u = blockIdx.x * 256 + threadIdx.x;
   if (u >= m) return;
   out[u] = __ldg(feats + __ldg(mapping + u));
@@ -596,6 +604,7 @@ __global__ void __launch_bounds__(256) k_segment_first4(const float4* __restrict
 __global__ void __launch_bounds__(256) k_segment_add(const float* __restrict__ feats, const int64_t* __restrict__ inverse,
                                                      const int64_t* __restrict__ mapping, uint32_t n, int C,
                                                      float* __restrict__ out, uint32_t* __restrict__ count) {
+  after_previous_kernel();
   const uint32_t row = blockIdx.x * 256 + threadIdx.x;
   if (row >= n) return;
   const size_t u = (size_t)__ldg(inverse + row);
@@ -605,6 +614,7 @@ __global__ void __launch_bounds__(256) k_segment_add(const float* __restrict__ f
 }
 __global__ void __launch_bounds__(256) k_segment_divide(uint32_t m, int C, const uint32_t* __restrict__ count,
                                                         float* __restrict__ out) {
+  after_previous_kernel();
   const uint32_t u = blockIdx.x * 256 + threadIdx.x;
   if (u >= m) return;
   const uint32_t k = __ldg(count + u);
@@ -742,19 +752,22 @@ extern "C" int rmn_segment_reduce(const float* d_feats, uint32_t n_rows, int cha
   if (n_unique == 0) return RMN_OK;
   if (!d_feats || !d_inverse || !d_mapping || !d_out || !d_counts) return RMN_ERR_BAD_ARG;
   if (channels == 4 && !((uintptr_t)d_feats & 15) && !((uintptr_t)d_out & 15)) {
-    k_segment_first4<<<(n_unique + 255) / 256, 256, 0, stream>>>((const float4*)d_feats, d_mapping, n_unique, (float4*)d_out,
-                                                                 d_counts);
+    RMN_CUDA_TRY(launch_overlapped(k_segment_first4, dim3((n_unique + 255) / 256), dim3(256), 0, stream,
+                        (const float4*)d_feats, d_mapping, n_unique, (float4*)d_out, d_counts));
   } else {
     const size_t total = (size_t)n_unique * channels;
     if (total >= ((size_t)1 << 39)) return RMN_ERR_TOO_LARGE;
-    k_segment_first<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(d_feats, d_mapping, n_unique, channels, d_out, d_counts);
+    RMN_CUDA_TRY(launch_overlapped(k_segment_first, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream,
+                        d_feats, d_mapping, n_unique, channels, d_out, d_counts));
   }
   RMN_LAUNCH_CHECK();
   if (n_unique == n_rows) return RMN_OK;
-  k_segment_add<<<(n_rows + 255) / 256, 256, 0, stream>>>(d_feats, d_inverse, d_mapping, n_rows, channels, d_out, d_counts);
+  RMN_CUDA_TRY(launch_overlapped(k_segment_add, dim3((n_rows + 255) / 256), dim3(256), 0, stream,
+                        d_feats, d_inverse, d_mapping, n_rows, channels, d_out, d_counts));
   RMN_LAUNCH_CHECK();
   if (!mean) return RMN_OK;
-  k_segment_divide<<<(n_unique + 255) / 256, 256, 0, stream>>>(n_unique, channels, d_counts, d_out);
+  RMN_CUDA_TRY(launch_overlapped(k_segment_divide, dim3((n_unique + 255) / 256), dim3(256), 0, stream,
+                        n_unique, channels, d_counts, d_out));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -827,16 +840,17 @@ static int table_build_begin(const int32_t* d_coords, uint32_t n_rows, int W, vo
   {
     const uint32_t fill_blocks = (capacity + 255u) / 256u;
     const uint32_t blocks = fill_blocks < kGrid ? fill_blocks : kGrid;
-    RMN_DISPATCH_W(W, k_fill_range<kW><<<blocks, 256, 0, stream>>>(d_coords, n_rows, h,
-                                                                    reinterpret_cast<uint4*>(slots), capacity,
-                                                                    sc.repeat_bits));
+    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_fill_range<kW>, dim3(blocks), dim3(256), 0, stream,
+                        d_coords, n_rows, h, reinterpret_cast<uint4*>(slots), capacity, sc.repeat_bits)));
     RMN_LAUNCH_CHECK();
   }
   if (n_rows == 0) return RMN_OK;
   const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
-  RMN_DISPATCH_W(W, k_insert<kW><<<nb, 256, 0, stream>>>(d_coords, n_rows, h, slots, sc, look_first));
+  RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_insert<kW>, dim3(nb), dim3(256), 0, stream,
+                        d_coords, n_rows, h, slots, sc, look_first)));
   RMN_LAUNCH_CHECK();
-  k_count_first<<<(nb + 255) / 256, 256, 0, stream>>>(n_rows, h, sc, post);
+  RMN_CUDA_TRY(launch_overlapped(k_count_first, dim3((nb + 255) / 256), dim3(256), 0, stream,
+                        n_rows, h, sc, post));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -847,11 +861,12 @@ static int table_build_finish(const int32_t* d_coords, uint32_t n_rows, int W, v
   auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
   const Scratch sc = scratch(d_workspace, n_rows);
   const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
-  RMN_DISPATCH_W(W, k_finalize<kW><<<nb, kRowsPerBlock, 0, stream>>>(d_coords, n_rows, h, slots, sc, d_mapping,
-                                                                     d_unique_coords, d_inverse));
+  RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_finalize<kW>, dim3(nb), dim3(kRowsPerBlock), 0, stream,
+                        d_coords, n_rows, h, slots, sc, d_mapping, d_unique_coords, d_inverse)));
   RMN_LAUNCH_CHECK();
   if (d_inverse) {  // optional: only the quantisation modes that average or sample features read it
-    k_inverse<<<nb < kGrid ? nb : kGrid, 256, 0, stream>>>(slots, sc.slot_of_row, n_rows, h, d_inverse);
+    RMN_CUDA_TRY(launch_overlapped(k_inverse, dim3(nb < kGrid ? nb : kGrid), dim3(256), 0, stream,
+                        slots, sc.slot_of_row, n_rows, h, d_inverse));
     RMN_LAUNCH_CHECK();
   }
   return RMN_OK;
@@ -863,9 +878,9 @@ static int table_build(const int32_t* d_coords, uint32_t n_rows, int W, void* d_
   if (n_rows > 0 && n_rows <= kSmallRows) {
     auto* h = reinterpret_cast<TableHeader*>(d_table);
     auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
-    RMN_DISPATCH_W(W, k_build_small<kW><<<1, 1024, 0, stream>>>(d_coords, n_rows, h, slots, table_capacity(n_rows),
-                                                                scratch(d_workspace, n_rows), d_mapping, d_unique_coords,
-                                                                d_inverse, look_first, post));
+    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_build_small<kW>, dim3(1), dim3(1024), 0, stream,
+                        d_coords, n_rows, h, slots, table_capacity(n_rows), scratch(d_workspace, n_rows), d_mapping,
+                        d_unique_coords, d_inverse, look_first, post)));
     RMN_LAUNCH_CHECK();
     return RMN_OK;
   }
