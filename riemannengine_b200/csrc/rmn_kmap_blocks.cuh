@@ -32,7 +32,9 @@ struct BlockIndex {
   uint32_t* slot_of_row;  // build scratch
   uint32_t capacity;
 };
-constexpr uint32_t kBlockMaxProbes = 32;
+// (a surface loads two slots in five: runs of 32 taken slots occur, runs of 128 do not; 4.8 M clip rows overflowed at 32 in
+// some scenes, and took 3.0 ms by the hash table)
+constexpr uint32_t kBlockMaxProbes = 128;
 inline uint32_t block_index_capacity(uint32_t n) { return n / 8 + 64; }
 inline size_t block_index_bytes(uint32_t n) {
   return (size_t)block_index_capacity(n) * sizeof(BlockSlot) + 32 + (size_t)n * 8;
