@@ -57,6 +57,7 @@ struct Vec16<__nv_bfloat16> {
 template <typename T>
 __global__ void __launch_bounds__(256) k_channel_dot_partial(const T* __restrict__ a, const T* __restrict__ b,
                                                              uint32_t n, int C, float* __restrict__ partial) {
+  after_previous_kernel();
   constexpr int VEC = Vec16<T>::N;
   extern __shared__ float s_part[];  // [8 warps][2][C]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(256) k_channel_dot_partial(const T* __restrict
 // channels took 7.3 us with one warp per output, whose lanes read a sector each.
 __global__ void __launch_bounds__(1024) k_dot_reduce(const float* __restrict__ partial, uint32_t n_partials, int C,
                                                      double* __restrict__ stats) {
+  after_previous_kernel();
   __shared__ double s_sum[32][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
   double t = 0.0;
@@ -136,6 +138,7 @@ __global__ void k_bn_forward_coeffs(const double* __restrict__ stats, double cou
                                     void* running_mean, void* running_var, int param_dtype, float momentum, float eps,
                                     int C, float* __restrict__ scale, float* __restrict__ shift,
                                     float* __restrict__ mean_out, float* __restrict__ inv_out) {
+  after_previous_kernel();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const double n = count > 0.0 ? count : 1.0;
@@ -162,6 +165,7 @@ __global__ void k_bn_backward_coeffs(const double* __restrict__ dots, const floa
                                      const float* __restrict__ inv, const void* gamma, int param_dtype, double count,
                                      int C, float* __restrict__ c_dy, float* __restrict__ c_x, float* __restrict__ c_0,
                                      float* __restrict__ dgamma, float* __restrict__ dbeta) {
+  after_previous_kernel();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const double n = count > 0.0 ? count : 1.0;
@@ -183,6 +187,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_affine2(const T* __restrict__ a, const T* __restrict__ b, size_t total_vec, int C,
                                                  const float* __restrict__ c_a, const float* __restrict__ c_b,
                                                  const float* __restrict__ c_0, T* __restrict__ out) {
+  after_previous_kernel();
   constexpr int VEC = Vec16<T>::N;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total_vec; i += (size_t)gridDim.x * blockDim.x) {
     const int c0 = (int)((i * VEC) % (size_t)C);
@@ -211,6 +216,7 @@ static bool dot_fast_shape(int C) {
 template <int V, bool kVecSrc>
 __global__ void __launch_bounds__(256) k_pad_channels(const uint16_t* __restrict__ src, size_t total, int c_src, int ld_src,
                                                       int c_dst, uint16_t* __restrict__ dst) {
+  after_previous_kernel();
   struct __align__(2 * V) Chunk {
     uint16_t v[V];
   };
@@ -245,9 +251,11 @@ static int pad_channels(const void* src, uint32_t n, int c_src, int ld_src, void
   const unsigned grid = (unsigned)(blocks < 148 * 32 ? blocks : 148 * 32);
   const bool vec = c_src % V == 0 && ld_src % V == 0 && (uintptr_t)src % (2 * V) == 0;
   if (vec)
-    k_pad_channels<V, true><<<grid, 256, 0, stream>>>((const uint16_t*)src, total, c_src, ld_src, c_dst, (uint16_t*)dst);
+    RMN_CUDA_TRY(launch_overlapped(k_pad_channels<V, true>, dim3(grid), dim3(256), 0, stream,
+                                   (const uint16_t*)src, total, c_src, ld_src, c_dst, (uint16_t*)dst));
   else
-    k_pad_channels<V, false><<<grid, 256, 0, stream>>>((const uint16_t*)src, total, c_src, ld_src, c_dst, (uint16_t*)dst);
+    RMN_CUDA_TRY(launch_overlapped(k_pad_channels<V, false>, dim3(grid), dim3(256), 0, stream,
+                                   (const uint16_t*)src, total, c_src, ld_src, c_dst, (uint16_t*)dst));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -287,14 +295,14 @@ extern "C" int rmn_channel_dot_stats(const void* d_a, const void* d_b, uint32_t 
   if (blocks > kDotPartials) blocks = kDotPartials;
   const size_t smem = (size_t)8 * 2 * channels * sizeof(float);
   if (dtype == RMN_F32)
-    k_channel_dot_partial<float><<<blocks, 256, smem, stream>>>((const float*)d_a, (const float*)d_b, n_rows, channels,
-                                                                partial);
+    RMN_CUDA_TRY(launch_overlapped(k_channel_dot_partial<float>, dim3(blocks), dim3(256), smem, stream,
+                                   (const float*)d_a, (const float*)d_b, n_rows, channels, partial));
   else
-    k_channel_dot_partial<__nv_bfloat16><<<blocks, 256, smem, stream>>>((const __nv_bfloat16*)d_a,
-                                                                        (const __nv_bfloat16*)d_b, n_rows, channels,
-                                                                        partial);
+    RMN_CUDA_TRY(launch_overlapped(k_channel_dot_partial<__nv_bfloat16>, dim3(blocks), dim3(256), smem, stream,
+                                   (const __nv_bfloat16*)d_a, (const __nv_bfloat16*)d_b, n_rows, channels, partial));
   RMN_LAUNCH_CHECK();
-  k_dot_reduce<<<(2 * channels + 31) / 32, 1024, 0, stream>>>(partial, blocks, channels, d_stats);
+  RMN_CUDA_TRY(launch_overlapped(k_dot_reduce, dim3((2 * channels + 31) / 32), dim3(1024), 0, stream,
+                                 partial, blocks, channels, d_stats));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -307,9 +315,9 @@ extern "C" int rmn_bn_forward_coeffs(const double* d_stats, double count, const 
   if (!d_stats || !d_scale || !d_shift || !d_mean || !d_inv || channels < 1 ||
       (param_dtype != RMN_F32 && param_dtype != RMN_BF16))
     return RMN_ERR_BAD_ARG;
-  k_bn_forward_coeffs<<<(channels + 127) / 128, 128, 0, stream>>>(d_stats, count, d_gamma, d_beta, d_running_mean,
-                                                                  d_running_var, param_dtype, momentum, eps, channels,
-                                                                  d_scale, d_shift, d_mean, d_inv);
+  RMN_CUDA_TRY(launch_overlapped(k_bn_forward_coeffs, dim3((channels + 127) / 128), dim3(128), 0, stream,
+                                 d_stats, count, d_gamma, d_beta, d_running_mean, d_running_var, param_dtype, momentum,
+                                 eps, channels, d_scale, d_shift, d_mean, d_inv));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -321,8 +329,9 @@ extern "C" int rmn_bn_backward_coeffs(const double* d_dots, const float* d_mean,
   if (!d_dots || !d_mean || !d_inv || !d_c_dy || !d_c_x || !d_c_0 || !d_dgamma || !d_dbeta || channels < 1 ||
       (param_dtype != RMN_F32 && param_dtype != RMN_BF16))
     return RMN_ERR_BAD_ARG;
-  k_bn_backward_coeffs<<<(channels + 127) / 128, 128, 0, stream>>>(d_dots, d_mean, d_inv, d_gamma, param_dtype, count,
-                                                                   channels, d_c_dy, d_c_x, d_c_0, d_dgamma, d_dbeta);
+  RMN_CUDA_TRY(launch_overlapped(k_bn_backward_coeffs, dim3((channels + 127) / 128), dim3(128), 0, stream,
+                                 d_dots, d_mean, d_inv, d_gamma, param_dtype, count, channels, d_c_dy, d_c_x, d_c_0,
+                                 d_dgamma, d_dbeta));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -340,11 +349,13 @@ extern "C" int rmn_affine2(const void* d_a, const void* d_b, uint32_t n_rows, in
   const size_t blocks = (total_vec + 255) / 256;
   const unsigned grid = (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);
   if (dtype == RMN_F32)
-    k_affine2<float><<<grid, 256, 0, stream>>>((const float*)d_a, (const float*)d_b, total_vec, channels, d_c_a, d_c_b,
-                                               d_c_0, (float*)d_out);
+    RMN_CUDA_TRY(launch_overlapped(k_affine2<float>, dim3(grid), dim3(256), 0, stream,
+                                   (const float*)d_a, (const float*)d_b, total_vec, channels, d_c_a, d_c_b, d_c_0,
+                                   (float*)d_out));
   else
-    k_affine2<__nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)d_a, (const __nv_bfloat16*)d_b, total_vec,
-                                                       channels, d_c_a, d_c_b, d_c_0, (__nv_bfloat16*)d_out);
+    RMN_CUDA_TRY(launch_overlapped(k_affine2<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream,
+                                   (const __nv_bfloat16*)d_a, (const __nv_bfloat16*)d_b, total_vec, channels, d_c_a,
+                                   d_c_b, d_c_0, (__nv_bfloat16*)d_out));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

@@ -273,6 +273,7 @@ template <int COT>
 __global__ void __launch_bounds__(kWgWarps * 32, 2)
     k_wgrad_f32(const float* __restrict__ feats, const float* __restrict__ grad_out, const int32_t* __restrict__ nbr,
                 uint32_t n_dst, int K, int c_in, int c_out, uint32_t chunk_rows, int tiles_co, float* __restrict__ partial) {
+  after_previous_kernel();
   using Cfg = F32WgCfg<COT>;
   constexpr int NV = COT / 32;  // 4-column groups per lane, 32 columns apart
   extern __shared__ __align__(16) float smem_f[];
@@ -404,6 +405,7 @@ __global__ void __launch_bounds__(kWgWarps * 32, 2)
 template <typename T>
 __global__ void __launch_bounds__(256) k_transpose_weights(const T* __restrict__ w, int K, int c_in, int c_out, int reverse,
                                                            T* __restrict__ out) {
+  after_previous_kernel();
   __shared__ T tile[32][33];
   const int k = blockIdx.z, x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int ci0 = blockIdx.y * 32, co0 = blockIdx.x * 32;
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(256) k_transpose_weights(const T* __restrict__
 // out[e] = sum over the chunks of partial[chunk][e], in chunk order; four elements per thread
 __global__ void __launch_bounds__(128) k_reduce_f32(const float4* __restrict__ partial, uint32_t n_chunks, size_t vecs,
                                                     float4* __restrict__ out) {
+  after_previous_kernel();
   const size_t e = (size_t)blockIdx.x * 128 + threadIdx.x;
   if (e >= vecs) return;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -468,18 +471,19 @@ int f32_conv_backward_weight(const float* feats, const float* grad_out, uint32_t
   if (cot == 32) {
     static SmemOptIn opt_in;
     RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_wgrad_f32<32>), F32WgCfg<32>::SMEM));
-    k_wgrad_f32<32><<<grid, kWgWarps * 32, F32WgCfg<32>::SMEM, stream>>>(feats, grad_out, nbr, n_dst, K, c_in, c_out, rows,
-                                                                         tiles_co, workspace);
+    RMN_CUDA_TRY(launch_overlapped(k_wgrad_f32<32>, dim3(grid), dim3(kWgWarps * 32), F32WgCfg<32>::SMEM, stream,
+                                   feats, grad_out, nbr, n_dst, K, c_in, c_out, rows, tiles_co, workspace));
   } else {
     static SmemOptIn opt_in;
     RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_wgrad_f32<64>), F32WgCfg<64>::SMEM));
-    k_wgrad_f32<64><<<grid, kWgWarps * 32, F32WgCfg<64>::SMEM, stream>>>(feats, grad_out, nbr, n_dst, K, c_in, c_out, rows,
-                                                                         tiles_co, workspace);
+    RMN_CUDA_TRY(launch_overlapped(k_wgrad_f32<64>, dim3(grid), dim3(kWgWarps * 32), F32WgCfg<64>::SMEM, stream,
+                                   feats, grad_out, nbr, n_dst, K, c_in, c_out, rows, tiles_co, workspace));
   }
   RMN_LAUNCH_CHECK();
   const size_t vecs = (size_t)K * c_in * c_out / 4;
-  k_reduce_f32<<<(uint32_t)((vecs + 127) / 128), 128, 0, stream>>>(reinterpret_cast<const float4*>(workspace), chunks, vecs,
-                                                                   reinterpret_cast<float4*>(dw));
+  RMN_CUDA_TRY(launch_overlapped(k_reduce_f32, dim3((uint32_t)((vecs + 127) / 128)), dim3(128), 0, stream,
+                                 reinterpret_cast<const float4*>(workspace), chunks, vecs,
+                                 reinterpret_cast<float4*>(dw)));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -496,9 +500,11 @@ extern "C" int rmn_conv_transpose_weights(const void* d_weights, int K, int c_in
     return RMN_ERR_BAD_ARG;
   const dim3 grid((c_out + 31) / 32, (c_in + 31) / 32, K);
   if (dtype == RMN_F32)
-    k_transpose_weights<<<grid, 256, 0, stream>>>((const uint32_t*)d_weights, K, c_in, c_out, reverse, (uint32_t*)d_out);
+    RMN_CUDA_TRY(launch_overlapped(k_transpose_weights<uint32_t>, dim3(grid), dim3(256), 0, stream,
+                                   (const uint32_t*)d_weights, K, c_in, c_out, reverse, (uint32_t*)d_out));
   else
-    k_transpose_weights<<<grid, 256, 0, stream>>>((const uint16_t*)d_weights, K, c_in, c_out, reverse, (uint16_t*)d_out);
+    RMN_CUDA_TRY(launch_overlapped(k_transpose_weights<uint16_t>, dim3(grid), dim3(256), 0, stream,
+                                   (const uint16_t*)d_weights, K, c_in, c_out, reverse, (uint16_t*)d_out));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

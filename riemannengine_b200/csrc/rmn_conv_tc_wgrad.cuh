@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_conv_tc_wgrad(
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  after_previous_kernel();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -294,6 +295,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_conv_tc_wgrad(
 __global__ void __launch_bounds__(256) k_reduce_chunks(const float* __restrict__ partial, uint32_t n_chunks,
                                                        size_t elems, float* __restrict__ out, uint32_t cin,
                                                        uint32_t cout, uint32_t cin_total, uint32_t col0) {
+  after_previous_kernel();
   const size_t e = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (e >= elems) return;
   float s = 0.f;
@@ -353,14 +355,14 @@ int launch_wgrad(const void* feats, const void* grad_out, const int32_t* nbr, ui
     attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
   RMN_CUDA_TRY(attr_err);
   dim3 grid(p.chunks, p.sets);
-  kern<<<grid, kWgradThreads, C::SMEM, stream>>>((const __nv_bfloat16*)feats + col0, (const __nv_bfloat16*)grad_out,
-                                                 nbr, n_dst, K, p.groups_per_set, p.tmem_cols, (float*)workspace,
-                                                 (uint32_t)cin_total);
+  RMN_CUDA_TRY(launch_overlapped(kern, grid, dim3(kWgradThreads), C::SMEM, stream, (const __nv_bfloat16*)feats + col0,
+                                 (const __nv_bfloat16*)grad_out, nbr, n_dst, K, p.groups_per_set, p.tmem_cols,
+                                 (float*)workspace, (uint32_t)cin_total));
   RMN_LAUNCH_CHECK();
   count_tc_launch();
-  k_reduce_chunks<<<(uint32_t)((elems + 255) / 256), 256, 0, stream>>>((const float*)workspace, p.chunks, elems, dw,
-                                                                        (uint32_t)CIN, (uint32_t)COUT,
-                                                                        (uint32_t)cin_total, (uint32_t)col0);
+  RMN_CUDA_TRY(launch_overlapped(k_reduce_chunks, dim3((uint32_t)((elems + 255) / 256)), dim3(256), 0, stream,
+                                 (const float*)workspace, p.chunks, elems, dw, (uint32_t)CIN, (uint32_t)COUT,
+                                 (uint32_t)cin_total, (uint32_t)col0));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

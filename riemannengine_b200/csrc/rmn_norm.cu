@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(256) k_channel_stats_partial(const T* __restri
 // stats[2][C] (double) = sum over the partials, in partial order (deterministic).
 __global__ void k_stats_reduce(const float* __restrict__ partial, uint32_t n_partials, int C,
                                double* __restrict__ stats) {
+  after_previous_kernel();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * C) return;
   double t = 0.0;
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(256) k_affine_act_bf16x8(const uint4* __restri
                                                            const float* __restrict__ scale,
                                                            const float* __restrict__ shift, int relu,
                                                            uint4* __restrict__ out) {
+  after_previous_kernel();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total_vec; i += (size_t)gridDim.x * blockDim.x) {
     const int c0 = (int)((i * 8) % C);
     const uint4 v = __ldg(x + i);
@@ -116,7 +118,8 @@ static int channel_stats(const void* x, uint32_t n, int C, int dtype, double* st
     k_channel_stats_partial<__nv_bfloat16><<<blocks, 256, 2 * 256 * sizeof(float), stream>>>((const __nv_bfloat16*)x,
                                                                                               n, C, partial);
   RMN_LAUNCH_CHECK();
-  k_stats_reduce<<<(2 * C + 127) / 128, 128, 0, stream>>>(partial, blocks, C, stats);
+  RMN_CUDA_TRY(launch_overlapped(k_stats_reduce, dim3((2 * C + 127) / 128), dim3(128), 0, stream,
+                                 partial, blocks, C, stats));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -168,8 +171,8 @@ extern "C" int rmn_conv_forward_stats_planned(const void* d_feats, uint32_t n_sr
     const int st = tc_conv_stats(d_feats, n_src, d_weights, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift,
                                  relu, (float*)d_workspace, &n_partials, stream, d_plan);
     if (st == RMN_OK) {
-      k_stats_reduce<<<(2 * c_out + 127) / 128, 128, 0, stream>>>((const float*)d_workspace, n_partials, c_out,
-                                                                  d_stats);
+      RMN_CUDA_TRY(launch_overlapped(k_stats_reduce, dim3((2 * c_out + 127) / 128), dim3(128), 0, stream,
+                                     (const float*)d_workspace, n_partials, c_out, d_stats));
       RMN_LAUNCH_CHECK();
       return RMN_OK;
     }
@@ -199,7 +202,8 @@ extern "C" int rmn_conv_forward_image_stats(const void* d_feats, uint32_t n_src,
   const int st = ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, nullptr, relu,
                          (float*)d_workspace, &n_partials, stream, d_plan);
   if (st != RMN_OK) return st;
-  k_stats_reduce<<<(2 * c_out + 127) / 128, 128, 0, stream>>>((const float*)d_workspace, n_partials, c_out, d_stats);
+  RMN_CUDA_TRY(launch_overlapped(k_stats_reduce, dim3((2 * c_out + 127) / 128), dim3(128), 0, stream,
+                                 (const float*)d_workspace, n_partials, c_out, d_stats));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -214,8 +218,8 @@ extern "C" int rmn_affine_act(const void* d_x, uint32_t n_rows, int channels, co
   if (dtype == RMN_BF16 && channels % 8 == 0 && !((uintptr_t)d_x & 15) && !((uintptr_t)d_out & 15)) {
     const size_t vec = total / 8;
     const size_t blocks = (vec + 255) / 256;
-    k_affine_act_bf16x8<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, stream>>>(
-        (const uint4*)d_x, vec, channels, d_scale, d_shift, relu, (uint4*)d_out);
+    RMN_CUDA_TRY(launch_overlapped(k_affine_act_bf16x8, dim3((unsigned)(blocks < 148 * 16 ? blocks : 148 * 16)), dim3(256),
+                                   0, stream, (const uint4*)d_x, vec, channels, d_scale, d_shift, relu, (uint4*)d_out));
   } else {
     const size_t blocks = (total + 255) / 256;
     const unsigned grid = (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);

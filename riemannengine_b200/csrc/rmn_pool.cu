@@ -73,6 +73,7 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(256) k_pool_fwd_vec(const T* __restrict__ feats, const int32_t* __restrict__ nbr,
                                                       uint32_t n_dst, int K, int C, int lanes_per_row,
                                                       T* __restrict__ out, int32_t* __restrict__ aux) {
+  after_previous_kernel();
   constexpr int V = Vec16<T>::N;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane_in_row = gtid % lanes_per_row;
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(256) k_pool_bwd_vec(const T* __restrict__ grad
                                                       const int32_t* __restrict__ nbr_in, uint32_t n_src, int K,
                                                       int C, int lanes_per_row, const int32_t* __restrict__ aux,
                                                       T* __restrict__ grad_in) {
+  after_previous_kernel();
   constexpr int V = Vec16<T>::N;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane_in_row = gtid % lanes_per_row;
@@ -249,8 +251,8 @@ int pool_forward_t(const void* feats, const int32_t* nbr, uint32_t n_dst, int K,
                    cudaStream_t stream) {
   const int lanes = pool_lanes_per_row<T>(C, feats, out);
   if (lanes > 0) {
-    k_pool_fwd_vec<T, MODE><<<pool_grid((uint64_t)n_dst * lanes), 256, 0, stream>>>(
-        (const T*)feats, nbr, n_dst, K, C, lanes, (T*)out, aux);
+    RMN_CUDA_TRY(launch_overlapped(k_pool_fwd_vec<T, MODE>, dim3(pool_grid((uint64_t)n_dst * lanes)), dim3(256), 0, stream,
+                                   (const T*)feats, nbr, n_dst, K, C, lanes, (T*)out, aux));
   } else {
     k_pool_fwd_scalar<T, MODE><<<pool_grid((uint64_t)n_dst * 32), 256, 0, stream>>>((const T*)feats, nbr, n_dst, K, C,
                                                                                     (T*)out, aux);
@@ -264,8 +266,8 @@ int pool_backward_t(const void* grad_out, const int32_t* nbr_in, uint32_t n_src,
                     void* grad_in, cudaStream_t stream) {
   const int lanes = pool_lanes_per_row<T>(C, grad_out, grad_in);
   if (lanes > 0) {
-    k_pool_bwd_vec<T, MODE><<<pool_grid((uint64_t)n_src * lanes), 256, 0, stream>>>(
-        (const T*)grad_out, nbr_in, n_src, K, C, lanes, aux, (T*)grad_in);
+    RMN_CUDA_TRY(launch_overlapped(k_pool_bwd_vec<T, MODE>, dim3(pool_grid((uint64_t)n_src * lanes)), dim3(256), 0, stream,
+                                   (const T*)grad_out, nbr_in, n_src, K, C, lanes, aux, (T*)grad_in));
   } else {
     k_pool_bwd_scalar<T, MODE><<<pool_grid((uint64_t)n_src * 32), 256, 0, stream>>>((const T*)grad_out, nbr_in, n_src,
                                                                                     K, C, aux, (T*)grad_in);
