@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
       hit = uid != 0xFFFFFFFFu;
     }
     if (active) __stcs(dst, (int32_t)uid);
-    if (k < half) {  // (the other half has the same counts, see k_kmap_offset_ptr)
+    if (k < half) {  // (the other half has the same counts, see k_kmap_scan)
       const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
       if (lane == 0) atomicAdd(&s_cnt[k], (uint32_t)__popc(hits));
     }
