@@ -653,6 +653,7 @@ bool ta_small(uint32_t n_dst, int c_col, int sms) {
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial, uint32_t* n_partials,
             cudaStream_t stream, const void* plan) {
+  if (ta_image_bytes(K, c_red, c_col) == 0) return RMN_ERR_UNSUPPORTED;  // (the cases below match blocks of columns)
   int dev = 0, sms = 148;
   RMN_CUDA_TRY(cudaGetDevice(&dev));
   RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -53,6 +53,26 @@ def test_image_passes_match_float64(c_in, c_out, n, K, fill):
     assert float((stats - want_stats).abs().max()) <= 1e-4 * max(1.0, float((stored * stored).sum(0).max()))
 
 
+@pytest.mark.parametrize("n", [100, 150_001])   # single 64-column blocks / super-tiles of all columns
+@pytest.mark.parametrize("c_in,c_out", [(64, 48), (64, 16), (64, 96), (32, 128), (32, 256), (256, 64), (256, 32), (48, 64), (512, 512)])
+def test_image_calls_refuse_pairs_without_a_kernel(n, c_in, c_out):
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    assert lib.rmn_conv_weight_image_bytes(1, c_in, c_out, capi.BF16) == 0
+    feats, out = (torch.full((n, c), 3.0, dtype=torch.bfloat16, device="cuda") for c in (c_in, c_out))
+    image = torch.zeros(4 * 512 * 512, dtype=torch.uint8, device="cuda")
+    nbr = torch.arange(n, dtype=torch.int32, device="cuda")[None].contiguous()
+    args = (ops._ptr(feats), n, c_in, ops._ptr(image), 1, c_out, ops._ptr(nbr), None, n, ops._ptr(out), None, None)
+    assert lib.rmn_conv_forward_image(*args, None, 0, ops._stream()) == capi.ERR_UNSUPPORTED
+    stats = torch.zeros((2, c_out), dtype=torch.float64, device="cuda")
+    size = lib.rmn_channel_stats_workspace_bytes(c_out)
+    work = torch.empty(size, dtype=torch.uint8, device="cuda")
+    assert lib.rmn_conv_forward_image_stats(*args, 0, ops._ptr(stats), ops._ptr(work), size,
+                                            ops._stream()) == capi.ERR_UNSUPPORTED
+    torch.cuda.synchronize()
+    assert bool((out == 3.0).all())
+
+
 @pytest.mark.parametrize("n,c_in,c_out", [(1, 4, 20), (1000, 20, 96), (4099, 33, 64)])
 def test_padded_layer_with_bias_matches_float64(n, c_in, c_out):
     """Channel counts without a kernel of their own: padded features, weights and gradients, the bias gradient."""
