@@ -193,12 +193,13 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
+  // (tensor memory is taken behind the kernels before this one and ahead of the next: see release_next_kernel)
+  wait_previous_kernels();
   if (warp == kTaMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  after_previous_kernel();
   if (has_ep && tid < CC) {
     s_ep[tid] = ep_scale ? __ldg(ep_scale + col0 + tid) : 1.f;
     s_ep[CC + tid] = ep_shift ? __ldg(ep_shift + col0 + tid) : 0.f;
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  release_next_kernel();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
   const uint32_t smem_base = smem_u32(smem);
   bool timed_out = false;
