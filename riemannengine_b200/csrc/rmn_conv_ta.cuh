@@ -176,7 +176,9 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   const int n_off = (K + OPS - 1) / OPS;  // offsets, or pairs of them
   const bool has_ep = ep_scale != nullptr || ep_shift != nullptr || ep_add != nullptr || ep_relu != 0;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // (the shuffle makes the warp number uniform for the compiler, too: with tid >> 5 the MMA warp's loop leaves the uniform
+  // datapath, 919 -> 1005 us in a pass of thirty small layers)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < BST; ++s) {
       mbar_init(&b_full[s], 1);
@@ -333,99 +335,101 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       if (__any_sync(0xFFFFFFFFu, timed_out)) break;
     }
     if (cnt) arrive();
-  } else if (warp == kTaMmaWarp) {
-    // ------------------------------ MMA issuer -----------------------------------------
-    // Warp-uniform code, one elected lane issues. B descriptors differ only in the start address field. Masks of a plan
-    // come through a warp vote (the ballot of "bit `lane` of the mask" is the mask itself), whose result is warp-uniform
-    // by construction, so that branches on it keep the loop on the uniform datapath.
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTaIssueRegs));
-    constexpr uint32_t IDESC = instr_desc(kTileM, CC, true);
-    constexpr uint64_t B_DESC0 = smem_desc_sw_const(KB * SWB, 8 * SWB, SWB == 128 ? 2u : 4u);
-    constexpr uint32_t B_DESC_HI = (uint32_t)(B_DESC0 >> 32);
-    uint32_t cnts = 0;  // stages taken from each group so far, modulo 8 (one byte per group)
-    uint32_t b_it = 0, tile_iter = 0;
-    for (uint32_t st = blockIdx.x; st < n_super && !timed_out; st += gridDim.x, ++tile_iter) {
-      const uint32_t buf = tile_iter % C::ACC_BUFS, acc_ph = (tile_iter / C::ACC_BUFS) & 1u;
-      uint32_t m[T], todo = 0;
-      if constexpr (kPlan) {
-#pragma unroll
-        for (int t = 0; t < T; ++t) {
-          m[t] = __ballot_sync(0xFFFFFFFFu, (__ldg(tile_mask + (size_t)st * T + t) >> lane) & 1u);
-          todo |= m[t];
-        }
-      }
-      uint32_t started = 0, odd = 0;  // per tile: an MMA has been issued; parity of its offset count
-      for (int k = 0; kPlan ? todo != 0 : k < n_off; ++k) {
-        if constexpr (kPlan) {
-          k = __ffs(todo) - 1;
-          todo &= todo - 1u;
-        }
-#pragma unroll
-        for (int kb = 0; kb < NKB; ++kb, ++b_it) {
-          const uint32_t bs = b_it % BST;
-          if (!mbar_wait(&b_full[bs], (b_it / BST) & 1u)) { timed_out = true; goto mma_done; }
-          const uint32_t b_lo = ((smem_base + bs * C::B_BYTES) >> 4) + (uint32_t)(B_DESC0 & 0xFFFFFFFFu);
-#pragma unroll
-          for (int t = 0; t < T; ++t) {
-            if constexpr (kPlan) {
-              if (!((m[t] >> k) & 1u)) continue;
-            }
-            const uint32_t g = t + T * (KSTEP > 1 ? (kPlan ? (odd >> t) & 1u : (uint32_t)k % KSTEP) * NKB + kb : kb % PH);
-            const uint32_t c = (cnts >> (8 * g)) & 7u, s = c % SLOTS;
-            const uint32_t begun = (started >> t) & 1u;
-            if (!mbar_wait(&a_full[g * SLOTS + s], (c / SLOTS) & 1u)) { timed_out = true; goto mma_done; }
-            if (!begun && !mbar_wait(&acc_empty[buf * T + t], acc_ph ^ 1u)) { timed_out = true; goto mma_done; }
-            tc_fence_after();
-            const uint32_t d_tmem = tmem_base + (buf * T + t) * CC;
-            const uint32_t a_tmem = tmem_base + C::ACC_COLS + (g * SLOTS + s) * C::A_COLS;
-#pragma unroll
-            for (int j = 0; j < KB / 16; ++j) {
-              // MN-major B: 8-row K groups 8 * SWB apart (SBO), 64-column atoms KB * SWB apart (LBO), a K step is 16 lines
-              const uint64_t b_desc = ((uint64_t)B_DESC_HI << 32) | (b_lo + (uint32_t)((j * 16 * SWB) >> 4));
-              tc_mma_bf16_ta_elect(d_tmem, a_tmem + j * 8, b_desc, IDESC, j > 0 ? 1u : begun);
-            }
-            tc_commit_elect(&a_empty[g * SLOTS + s]);
-            cnts = (cnts + (1u << (8 * g))) & 0x07070707u;
-            started |= 1u << t;
-            if (kPlan && KSTEP > 1 && kb == NKB - 1) odd ^= 1u << t;
-          }
-          tc_commit_elect(&b_empty[bs]);
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < T; ++t) {
-        if (!((started >> t) & 1u) && !mbar_wait(&acc_empty[buf * T + t], acc_ph ^ 1u)) { timed_out = true; goto mma_done; }
-        tc_commit_elect(&acc_full[buf * T + t]);
-      }
-    }
-  mma_done:;
   } else if (warp < kTaEpWarp0) {
-    // ------------------------------ weights --------------------------------------------
+    // (one instruction for the whole warpgroup, ahead of its roles)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTaIssueRegs));
-    if (warp == kTaWeightWarp && lane == 0) {
-      uint32_t b_it = 0;
-      for (uint32_t st = blockIdx.x; st < n_super && !timed_out; st += gridDim.x) {
-        uint32_t todo = 0;
+    if (warp == kTaMmaWarp) {
+      // ------------------------------ MMA issuer -----------------------------------------
+      // Warp-uniform code, one elected lane issues. B descriptors differ only in the start address field. Masks of a plan
+      // come through a warp vote (the ballot of "bit `lane` of the mask" is the mask itself), whose result is warp-uniform
+      // by construction, so that branches on it keep the loop on the uniform datapath.
+      constexpr uint32_t IDESC = instr_desc(kTileM, CC, true);
+      constexpr uint64_t B_DESC0 = smem_desc_sw_const(KB * SWB, 8 * SWB, SWB == 128 ? 2u : 4u);
+      constexpr uint32_t B_DESC_HI = (uint32_t)(B_DESC0 >> 32);
+      uint32_t cnts = 0;  // stages taken from each group so far, modulo 8 (one byte per group)
+      uint32_t b_it = 0, tile_iter = 0;
+      for (uint32_t st = blockIdx.x; st < n_super && !timed_out; st += gridDim.x, ++tile_iter) {
+        const uint32_t buf = tile_iter % C::ACC_BUFS, acc_ph = (tile_iter / C::ACC_BUFS) & 1u;
+        uint32_t m[T], todo = 0;
         if constexpr (kPlan) {
-#pragma unroll
-          for (int t = 0; t < T; ++t) todo |= __ldg(tile_mask + (size_t)st * T + t);
+  #pragma unroll
+          for (int t = 0; t < T; ++t) {
+            m[t] = __ballot_sync(0xFFFFFFFFu, (__ldg(tile_mask + (size_t)st * T + t) >> lane) & 1u);
+            todo |= m[t];
+          }
         }
-        for (int k = 0; (kPlan ? todo != 0 : k < n_off) && !timed_out; ++k) {
+        uint32_t started = 0, odd = 0;  // per tile: an MMA has been issued; parity of its offset count
+        for (int k = 0; kPlan ? todo != 0 : k < n_off; ++k) {
           if constexpr (kPlan) {
             k = __ffs(todo) - 1;
             todo &= todo - 1u;
           }
+  #pragma unroll
           for (int kb = 0; kb < NKB; ++kb, ++b_it) {
-            const uint32_t s = b_it % BST;
-            if (!mbar_wait(&b_empty[s], ((b_it / BST) & 1u) ^ 1u)) { timed_out = true; break; }
-            bulk_load(smem_base + s * C::B_BYTES, image + ((size_t)(k * NKB + kb) * n_cols + col0) * (KB * 2), C::B_BYTES,
-                      smem_u32(&b_full[s]));
+            const uint32_t bs = b_it % BST;
+            if (!mbar_wait(&b_full[bs], (b_it / BST) & 1u)) { timed_out = true; goto mma_done; }
+            const uint32_t b_lo = ((smem_base + bs * C::B_BYTES) >> 4) + (uint32_t)(B_DESC0 & 0xFFFFFFFFu);
+  #pragma unroll
+            for (int t = 0; t < T; ++t) {
+              if constexpr (kPlan) {
+                if (!((m[t] >> k) & 1u)) continue;
+              }
+              const uint32_t g = t + T * (KSTEP > 1 ? (kPlan ? (odd >> t) & 1u : (uint32_t)k % KSTEP) * NKB + kb : kb % PH);
+              const uint32_t c = (cnts >> (8 * g)) & 7u, s = c % SLOTS;
+              const uint32_t begun = (started >> t) & 1u;
+              if (!mbar_wait(&a_full[g * SLOTS + s], (c / SLOTS) & 1u)) { timed_out = true; goto mma_done; }
+              if (!begun && !mbar_wait(&acc_empty[buf * T + t], acc_ph ^ 1u)) { timed_out = true; goto mma_done; }
+              tc_fence_after();
+              const uint32_t d_tmem = tmem_base + (buf * T + t) * CC;
+              const uint32_t a_tmem = tmem_base + C::ACC_COLS + (g * SLOTS + s) * C::A_COLS;
+  #pragma unroll
+              for (int j = 0; j < KB / 16; ++j) {
+                // MN-major B: 8-row K groups 8 * SWB apart (SBO), 64-column atoms KB * SWB apart (LBO), a K step is 16 lines
+                const uint64_t b_desc = ((uint64_t)B_DESC_HI << 32) | (b_lo + (uint32_t)((j * 16 * SWB) >> 4));
+                tc_mma_bf16_ta_elect(d_tmem, a_tmem + j * 8, b_desc, IDESC, j > 0 ? 1u : begun);
+              }
+              tc_commit_elect(&a_empty[g * SLOTS + s]);
+              cnts = (cnts + (1u << (8 * g))) & 0x07070707u;
+              started |= 1u << t;
+              if (kPlan && KSTEP > 1 && kb == NKB - 1) odd ^= 1u << t;
+            }
+            tc_commit_elect(&b_empty[bs]);
           }
         }
+  #pragma unroll
+        for (int t = 0; t < T; ++t) {
+          if (!((started >> t) & 1u) && !mbar_wait(&acc_empty[buf * T + t], acc_ph ^ 1u)) { timed_out = true; goto mma_done; }
+          tc_commit_elect(&acc_full[buf * T + t]);
+        }
       }
-      // no copy may be in flight when the CTA exits: wait for the last round of the ring
-      for (uint32_t i = b_it > BST ? b_it - BST : 0; i < b_it; ++i)
-        if (!mbar_wait(&b_full[i % BST], (i / BST) & 1u)) timed_out = true;
+    mma_done:;
+    } else {
+      // ------------------------------ weights --------------------------------------------
+      if (warp == kTaWeightWarp && lane == 0) {
+        uint32_t b_it = 0;
+        for (uint32_t st = blockIdx.x; st < n_super && !timed_out; st += gridDim.x) {
+          uint32_t todo = 0;
+          if constexpr (kPlan) {
+  #pragma unroll
+            for (int t = 0; t < T; ++t) todo |= __ldg(tile_mask + (size_t)st * T + t);
+          }
+          for (int k = 0; (kPlan ? todo != 0 : k < n_off) && !timed_out; ++k) {
+            if constexpr (kPlan) {
+              k = __ffs(todo) - 1;
+              todo &= todo - 1u;
+            }
+            for (int kb = 0; kb < NKB; ++kb, ++b_it) {
+              const uint32_t s = b_it % BST;
+              if (!mbar_wait(&b_empty[s], ((b_it / BST) & 1u) ^ 1u)) { timed_out = true; break; }
+              bulk_load(smem_base + s * C::B_BYTES, image + ((size_t)(k * NKB + kb) * n_cols + col0) * (KB * 2), C::B_BYTES,
+                        smem_u32(&b_full[s]));
+            }
+          }
+        }
+        // no copy may be in flight when the CTA exits: wait for the last round of the ring
+        for (uint32_t i = b_it > BST ? b_it - BST : 0; i < b_it; ++i)
+          if (!mbar_wait(&b_full[i % BST], (i / BST) & 1u)) timed_out = true;
+      }
     }
   } else {
     // ------------------------------ epilogue -------------------------------------------

@@ -26,3 +26,14 @@ def test_the_next_kernel_is_released_behind_the_allocation_of_tensor_memory(file
     for release in ("after_previous_kernel()", "release_next_kernel()", "griddepcontrol.launch_dependents"):
         for m in re.finditer(re.escape(release), text):
             assert m.start() > barrier, (file, kernel, release)
+
+
+@pytest.mark.parametrize("file,kernel,text", [pytest.param(*k, id=k[1]) for k in _kernels() if "setmaxnreg" in k[2]])
+def test_register_splits_are_executed_by_whole_warpgroups(file, kernel, text):
+    """setmaxnreg is one instruction for the four warps of a warpgroup: the branch it opens has to hold for all or none."""
+    with open(os.path.join(CSRC, file)) as f:
+        constants = dict(re.findall(r"\b(k\w+) = (\d+)\b", f.read()))
+    for m in re.finditer("setmaxnreg", text):
+        branch = text[text.rindex("if (", 0, m.start()):m.start()]
+        limit = re.match(r"if \(warp < (\w+)\) \{", branch)
+        assert limit and int(constants[limit.group(1)]) % 4 == 0, (file, kernel, branch)
