@@ -226,6 +226,12 @@ cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_
   return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
 }
 #ifdef __CUDACC__
+// max(v, 0) that keeps a NaN, as torch's relu does (fmaxf would turn it into 0): a diverged network shows in its output.
+__device__ __forceinline__ float relu_f32(float v) {
+  float r;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));
+  return r;
+}
 // The next kernel may be launched once every block has come here (or ended). One thread of a block is enough, so a block that
 // takes something which a block of the next kernel could take first, and which that one would hold while it waits for this kernel
 // - tensor memory - comes here behind a barrier that follows the taking.

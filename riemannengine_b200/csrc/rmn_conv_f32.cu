@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256)
     for (int q = 0; q < 4; ++q) {
       if (ep_scale) f[q] *= __ldg(ep_scale + n + q);
       if (ep_shift) f[q] += __ldg(ep_shift + n + q);
-      if (ep_relu) f[q] = fmaxf(f[q], 0.f);
+      if (ep_relu) f[q] = relu_f32(f[q]);
     }
     *reinterpret_cast<float4*>(out + (size_t)row * c_col + n) = make_float4(f[0], f[1], f[2], f[3]);
   }

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) k_conv_gather_gemm(
         float f = acc[i][j];
         if (ep_scale) f *= __ldg(ep_scale + n);
         if (ep_shift) f += __ldg(ep_shift + n);
-        if (ep_relu) f = fmaxf(f, 0.f);
+        if (ep_relu) f = relu_f32(f);
         out[(size_t)row * c_col + n] = from_f32<T>(f);
       }
     }

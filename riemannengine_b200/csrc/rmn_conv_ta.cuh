@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
                   }
                   if (ep_relu) {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) f[v] = fmaxf(f[v], 0.f);
+                    for (int v = 0; v < 4; ++v) f[v] = relu_f32(f[v]);
                   }
                 }
                 const __nv_bfloat162 p0 = __floats2bfloat162_rn(f[0], f[1]), p1 = __floats2bfloat162_rn(f[2], f[3]);

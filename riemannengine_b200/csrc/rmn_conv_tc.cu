@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(Cfg<CR, CC>::THREADS, 1) k_conv_tc(const __nv_
 #pragma unroll
             for (int v = 0; v < 32; ++v) {
               float f = fmaf(__uint_as_float(r[v]), s_ep[c0 + v], s_ep[CC + c0 + v]);
-              if (ep_relu) f = fmaxf(f, 0.f);
+              if (ep_relu) f = relu_f32(f);
               r[v] = __float_as_uint(f);
             }
           }

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) k_affine_act(const T* __restrict__ x, siz
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int c = (int)(i % C);
     float v = ld_f32(x + i) * (scale ? __ldg(scale + c) : 1.f) + (shift ? __ldg(shift + c) : 0.f);
-    if (relu) v = fmaxf(v, 0.f);
+    if (relu) v = relu_f32(v);
     if constexpr (sizeof(T) == 4) out[i] = v;
     else out[i] = __float2bfloat16_rn(v);
   }
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256) k_affine_act_bf16x8(const uint4* __restri
       const int c = c0 + 2 * j;
       f.x = f.x * (scale ? __ldg(scale + c) : 1.f) + (shift ? __ldg(shift + c) : 0.f);
       f.y = f.y * (scale ? __ldg(scale + c + 1) : 1.f) + (shift ? __ldg(shift + c + 1) : 0.f);
-      if (relu) { f.x = fmaxf(f.x, 0.f); f.y = fmaxf(f.y, 0.f); }
+      if (relu) { f.x = relu_f32(f.x); f.y = relu_f32(f.y); }
       const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
       o[j] = *reinterpret_cast<const uint32_t*>(&b);
     }
