@@ -2,6 +2,8 @@
 // autograd, the C ABI of librmn_b200.so for every coordinate / convolution operation.
 #include "riemann_b200.hpp"
 
+#include <ATen/TensorSubclassLikeUtils.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -876,7 +878,8 @@ at::Tensor pad_channels(const at::Tensor& x, int64_t channels) {
 at::Tensor contiguous_rows(const at::Tensor& x) { return x.dim() == 2 ? pad_channels(x, x.size(1)) : x.contiguous(); }
 
 // Concatenation of the channels of two matrices with the same rows (a skip connection). The gradient of a part is made
-// contiguous here: as a view into the whole gradient it would be read with strides by every kernel behind it.
+// contiguous here: as a view into the whole gradient it would be read with strides by every kernel behind it. The copy is a raw
+// kernel, so where the gradient is itself differentiated, or is a wrapper (vmap), the parts stay views as torch::cat gives them.
 class ChannelCatAutograd : public torch::autograd::Function<ChannelCatAutograd> {
 public:
   static at::Tensor forward(torch::autograd::AutogradContext* ctx, at::Tensor a, at::Tensor b) {
@@ -887,12 +890,23 @@ public:
                                                  torch::autograd::variable_list grad_outputs) {
     const auto& grad = grad_outputs[0];
     const int64_t split = ctx->saved_data["split"].toInt();
+    const bool copy = !at::GradMode::is_enabled() && !at::isTensorSubclassLike(grad);
+    auto part = [&](int64_t first, int64_t channels) {
+      auto view = grad.narrow(1, first, channels);
+      return copy ? contiguous_rows(view) : view;
+    };
     at::Tensor ga, gb;
-    if (ctx->needs_input_grad(0)) ga = contiguous_rows(grad.narrow(1, 0, split));
-    if (ctx->needs_input_grad(1)) gb = contiguous_rows(grad.narrow(1, split, grad.size(1) - split));
+    if (ctx->needs_input_grad(0)) ga = part(0, split);
+    if (ctx->needs_input_grad(1)) gb = part(split, grad.size(1) - split);
     return {ga, gb};
   }
 };
+
+// autograd functions of the C++ API know neither forward-mode derivatives nor function transforms
+bool plain_autograd(const at::Tensor& x) {
+  return !at::isTensorSubclassLike(x) && !x._fw_grad(/*level=*/0).defined() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
 }  // namespace
 
 SparseTensor cat(const std::vector<SparseTensor>& tensors) {
@@ -902,7 +916,8 @@ SparseTensor cat(const std::vector<SparseTensor>& tensors) {
   for (auto const& t : tensors) {
     features.push_back(t.F());
     grad = grad || t.F().requires_grad();
-    same = same && t.F().is_cuda() && t.F().dim() == 2 && t.F().scalar_type() == tensors.front().F().scalar_type();
+    same = same && t.F().is_cuda() && t.F().dim() == 2 && t.F().scalar_type() == tensors.front().F().scalar_type() &&
+           plain_autograd(t.F());
   }
   auto joined = grad && same && features.size() == 2 && at::GradMode::is_enabled()
                     ? ChannelCatAutograd::apply(features[0], features[1])

@@ -141,3 +141,41 @@ def test_channel_cat_splits_its_gradient():
         y.F.backward(g)
         assert torch.equal(y.F, torch.cat([a, b], 1))
         assert torch.equal(a.grad, g[:, :32]) and torch.equal(b.grad, g[:, 32:])
+
+
+def _cat_inputs():
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    coords = torch.tensor([[0, i, 0, 0] for i in range(40)], dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, b, w = (torch.randn((40, c), generator=g, device="cuda") for c in (12, 8, 20))
+    base = C.SparseTensor(a, coords)
+    on_map = lambda t: C.SparseTensor(t, base.coordinate_map_key, base.coordinate_manager)  # noqa: E731
+    return a, b, w, lambda x, y: C.cat([on_map(x), on_map(y)]).F
+
+
+def test_channel_cat_is_twice_differentiable():
+    a, b, w, cat = _cat_inputs()
+    second = []
+    for join in (cat, lambda x, y: torch.cat([x, y], 1)):
+        x, y = a.clone().requires_grad_(True), b.clone().requires_grad_(True)
+        first = torch.autograd.grad((join(x, y) ** 3 * w).sum(), (x, y), create_graph=True)
+        second.append(torch.autograd.grad(sum((f ** 2).sum() for f in first), (x, y)))
+    for got, want in zip(*second):
+        assert torch.equal(got, want)
+
+
+def test_channel_cat_takes_forward_mode_batched_gradients_and_function_transforms():
+    import torch.autograd.forward_ad as fwd
+    a, b, w, cat = _cat_inputs()
+    with fwd.dual_level():
+        x = fwd.make_dual(a.clone().requires_grad_(True), torch.ones_like(a))
+        y = fwd.make_dual(b.clone().requires_grad_(True), 2 * torch.ones_like(b))
+        tangent = fwd.unpack_dual(cat(x, y)).tangent
+    assert torch.equal(tangent, torch.cat([torch.ones_like(a), 2 * torch.ones_like(b)], 1))
+    x, y = a.clone().requires_grad_(True), b.clone().requires_grad_(True)
+    seeds = torch.stack([w, 2 * w, -w])
+    ga, gb = torch.autograd.grad(cat(x, y), (x, y), seeds, is_grads_batched=True)
+    assert torch.equal(ga, seeds[:, :, :12]) and torch.equal(gb, seeds[:, :, 12:])
+    ga, gb = torch.func.grad(lambda x, y: (cat(x, y) * w).sum(), argnums=(0, 1))(a, b)
+    assert torch.equal(ga, w[:, :12]) and torch.equal(gb, w[:, 12:])
