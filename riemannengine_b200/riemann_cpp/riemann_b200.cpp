@@ -609,6 +609,13 @@ std::map<int64_t, at::Tensor> CoordinateManager::kernel_map_th(
 // SparseTensor (engine/tensor/sparse_tensor.cpp:62-120, 447-481)
 // ---------------------------------------------------------------------------------------------
 namespace {
+// whether x may go to a raw kernel or to an autograd function of the C++ API, which know neither forward-mode derivatives nor
+// function transforms
+bool plain_autograd(const at::Tensor& x) {
+  return !at::isTensorSubclassLike(x) && !x._fw_grad(/*level=*/0).defined() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
 at::Tensor quantize_features(const at::Tensor& features, const at::Tensor& first_rows,
                              const at::Tensor& row_to_unique, int64_t unique_count,
                              SparseTensorQuantizationMode::Type mode) {
@@ -621,9 +628,10 @@ at::Tensor quantize_features(const at::Tensor& features, const at::Tensor& first
       return features;
     case SparseTensorQuantizationMode::UNWEIGHTED_SUM:
     case SparseTensorQuantizationMode::UNWEIGHTED_AVERAGE: {
-      const bool grad = at::GradMode::is_enabled() && features.requires_grad();
+      // (rmn_segment_reduce adds the rows of a voxel in no fixed order and hands no derivative on)
+      const bool grad = (at::GradMode::is_enabled() && features.requires_grad()) || !plain_autograd(features);
       if (features.is_cuda() && features.scalar_type() == at::kFloat && !grad && features.size(0) > 0 &&
-          features.size(1) > 0) {
+          features.size(1) > 0 && !at::globalContext().deterministicAlgorithms()) {
         c10::cuda::CUDAGuard guard(features.device());
         auto rows = features.contiguous();
         auto out = at::empty({unique_count, features.size(1)}, features.options());
@@ -901,12 +909,6 @@ public:
     return {ga, gb};
   }
 };
-
-// autograd functions of the C++ API know neither forward-mode derivatives nor function transforms
-bool plain_autograd(const at::Tensor& x) {
-  return !at::isTensorSubclassLike(x) && !x._fw_grad(/*level=*/0).defined() &&
-         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
-}
 }  // namespace
 
 SparseTensor cat(const std::vector<SparseTensor>& tensors) {
@@ -1489,7 +1491,8 @@ SparseTensor fused_conv_bn_relu(const SparseTensor& input, RiemannConvolutionBas
 SparseTensor conv_norm_relu(const SparseTensor& input, RiemannConvolutionBaseImpl& conv, RiemannBatchNormImpl& norm,
                             const SparseTensor* residual) {
   auto bn = norm.normalization();
-  bool fuse = !at::GradMode::is_enabled() && !bn->is_training() && folds_batch_norm(conv, input, *bn);
+  bool fuse = !at::GradMode::is_enabled() && !bn->is_training() && plain_autograd(input.F()) &&
+              folds_batch_norm(conv, input, *bn);
   if (fuse && residual) {  // (a stride-1 layer: the output lies on the input's map)
     auto const& r = residual->F();
     fuse = conv.kernel_generator_.kernel_stride() == stride_type(conv.dimension_, 1) && !conv.is_transpose_ &&

@@ -102,3 +102,34 @@ def test_segment_reduce_matches_float64(n, channels, extent, mean):
         want /= per
     assert float((out.double() - want).abs().max()) <= 1e-5 * max(1.0, float(want.abs().max()))
     assert n == m or torch.equal(counts.double(), per[:, 0])
+
+
+def test_voxel_averages_are_fixed_where_determinism_is_asked_for():
+    """With torch.use_deterministic_algorithms every sum has torch's fixed order; without it the order is the atomics'."""
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    n = 200_000
+    points = _coords(n, 3, 6, 9).float()
+    x = torch.randn((n, 5), device="cuda", generator=torch.Generator(device="cuda").manual_seed(9)) * 1e3
+    voxels, inverse = torch.unique(points, dim=0, return_inverse=True)
+    torch.use_deterministic_algorithms(True)
+    try:
+        want = torch.zeros((voxels.size(0), 5), device="cuda").index_add_(0, inverse, x)
+        want /= torch.zeros(voxels.size(0), device="cuda").index_add_(0, inverse, torch.ones(n, device="cuda"))[:, None]
+        for _ in range(3):
+            y = C.TensorField(x, points).sparse()
+            row = (y.C.float()[:, None] == voxels[None]).all(2).int().argmax(1)
+            assert torch.equal(y.F, want[row])
+    finally:
+        torch.use_deterministic_algorithms(False)
+
+
+def test_voxel_averages_hand_forward_derivatives_on():
+    import torch.autograd.forward_ad as fwd
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    points = _coords(500, 3, 3, 2).float()
+    with fwd.dual_level():
+        x = fwd.make_dual(torch.randn((500, 4), device="cuda"), torch.full((500, 4), 3.0, device="cuda"))
+        tangent = fwd.unpack_dual(C.TensorField(x, points).sparse().F).tangent
+    assert tangent is not None and torch.allclose(tangent, torch.full_like(tangent, 3.0))
