@@ -149,8 +149,9 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots,
     const int32_t* __restrict__ coords, uint32_t n, const int32_t* __restrict__ offsets, int K,
     int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks,
-    uint32_t* __restrict__ scan_ticket) {
+    uint32_t* __restrict__ scan_ticket, const uint32_t* __restrict__ index_state) {
   after_previous_kernel();
+  if (index_state && *index_state == ~0u) return;  // kIndexInUse: k_kmap_blocks_self has written the map
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int D = W - 1;
   const int half = K / 2;
@@ -386,10 +387,11 @@ __global__ void __launch_bounds__(256) k_kmap_transpose(const int32_t* __restric
 
 inline uint32_t kmap_blocks(uint32_t n_query) { return (n_query + kKmapBlock - 1) / kKmapBlock; }
 
-// Self maps whose hash table does not fit the 126 MB L2 go over the occupancy index (rmn_kmap_blocks.cuh); below that a
-// probe of the table is an L2 hit and the index saves nothing (1.2 M rows x 27 offsets: 137 us by probing, 240 us with it).
-inline bool use_block_index(uint32_t n, int K) {
-  return (size_t)n * 64 > ((size_t)120 << 20) && (K & 1) && K >= 9 && K <= 2048;
+// Self maps of three and more dimensions whose hash table takes most of the 126 MB L2 (94 MB from 1.97 M rows on, see
+// table_capacity) may go over the occupancy index, see k_block_choose; below that a probe of the table is an L2 hit in any order
+// of the rows (1.2 M shuffled rows x 27 offsets: 137 us by probing, 240 us with the index).
+inline bool may_use_block_index(uint32_t n, int W, int K) {
+  return W >= 4 && (size_t)n * 64 > ((size_t)120 << 20) && (K & 1) && K >= 9 && K <= 2048;
 }
 
 // counts per (offset, 256 query rows), totals, flags
@@ -458,7 +460,7 @@ extern "C" int rmn_region_offsets(int region_type, int D, const int32_t* kernel_
 
 extern "C" size_t rmn_kmap_workspace_bytes(uint32_t n_query, int K) {
   if (K < 1) K = 1;
-  return kmap_counts_bytes(n_query, K) + (use_block_index(n_query, K) ? block_index_bytes(n_query) : 0);
+  return kmap_counts_bytes(n_query, K) + (may_use_block_index(n_query, RMN_MAX_W, K) ? block_index_bytes(n_query) : 0);
 }
 
 // Blocks that share the offsets of a row block (gridDim.y): about four blocks per SM in all, three offsets each at least.
@@ -495,26 +497,40 @@ static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_qu
   auto* slots =
       reinterpret_cast<const Slot*>(reinterpret_cast<const char*>(d_table) + sizeof(TableHeader));
   const int half = self ? K / 2 : 0;
-  if (self && use_block_index(n_query, K) && ((uintptr_t)d_workspace & 15) == 0) {
+  const int hs = half > 0 ? half : 1;
+  const size_t self_smem = (size_t)hs * 8 + (size_t)hs * (W - 1) * 4 + (size_t)hs * 4;
+  if (self && may_use_block_index(n_query, W, K) && ((uintptr_t)d_workspace & 15) == 0) {
     const BlockIndex ix = block_index(static_cast<char*>(d_workspace) + kmap_counts_bytes(n_query, K), n_query);
-    RMN_CUDA_TRY(cudaMemsetAsync(ix.slots, 0xFF, (size_t)ix.capacity * sizeof(BlockSlot) + 32, stream));
-    RMN_DISPATCH_W(W, k_block_insert<kW><<<nb, 256, 0, stream>>>(h, d_query, n_query, ix));
-    RMN_LAUNCH_CHECK();
-    k_block_bases<<<(ix.capacity + 255) / 256, 256, 0, stream>>>(ix);
-    RMN_LAUNCH_CHECK();
-    RMN_DISPATCH_W(W, k_block_scatter<kW><<<nb, 256, 0, stream>>>(h, d_query, n_query, ix));
-    RMN_LAUNCH_CHECK();
+    const dim3 grid(148 * 8), block(256);
     const size_t smem = (size_t)8 * kKmapBlock * 12 + (size_t)K * 4 + (size_t)half * 4;
-    RMN_DISPATCH_W(W, k_kmap_blocks_self<kW><<<nb, kKmapBlock, smem, stream>>>(h, slots, d_query, n_query, d_offsets, K,
-                                                                              d_nbr, block_counts, nb, ticket, ix));
+    RMN_DISPATCH_W(W, if constexpr (kW >= 4) {
+      BlockSample* sample = reinterpret_cast<BlockSample*>(ix.perm);
+      RMN_CUDA_TRY(launch_overlapped(k_block_sample<kW>, dim3(kChooseRows / 256), block, 0, stream, h, slots, d_query, n_query,
+                                     sample));
+      RMN_LAUNCH_CHECK();
+      RMN_CUDA_TRY(launch_overlapped(k_block_choose, dim3(148 * 2), dim3(1024), 0, stream, h, n_query, sample, ix,
+                                     d_nbr + (size_t)(half + 1) * n_query, (size_t)half * n_query));
+      RMN_LAUNCH_CHECK();
+      RMN_CUDA_TRY(launch_overlapped(k_block_insert<kW>, grid, block, 0, stream, h, d_query, n_query, ix));
+      RMN_LAUNCH_CHECK();
+      RMN_CUDA_TRY(launch_overlapped(k_block_bases, dim3((ix.capacity + 255) / 256), block, 0, stream, ix));
+      RMN_LAUNCH_CHECK();
+      RMN_CUDA_TRY(launch_overlapped(k_block_scatter<kW>, grid, block, 0, stream, h, d_query, n_query, ix));
+      RMN_LAUNCH_CHECK();
+      RMN_CUDA_TRY(launch_overlapped(k_kmap_blocks_self<kW>, dim3(148 * 6), dim3(kKmapBlock), smem, stream, h, slots, d_query,
+                                     n_query, d_offsets, K, d_nbr, block_counts, nb, ticket, ix));
+      RMN_LAUNCH_CHECK();
+      RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock), self_smem,
+                                     stream, h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket,
+                                     ix.state));
+    });
   } else if (self) {
     if (half > 0)  // the mirrored half starts as "no neighbour"
       RMN_CUDA_TRY(cudaMemsetAsync(d_nbr + (size_t)(half + 1) * n_query, 0xFF, (size_t)half * n_query * sizeof(int32_t),
                                    stream));
-    const int hs = half > 0 ? half : 1;
-    const size_t smem = (size_t)hs * 8 + (size_t)hs * (W - 1) * 4 + (size_t)hs * 4;
-    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(
-                        k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock), smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket)));
+    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock),
+                                                     self_smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr,
+                                                     block_counts, nb, ticket, nullptr)));
   } else {
     const size_t smem = (size_t)K * 8 + (size_t)K * (W - 1) * 4 + (size_t)K * 4;
     RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(

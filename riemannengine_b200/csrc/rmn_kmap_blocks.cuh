@@ -1,13 +1,16 @@
 // Self map over an occupancy index: the rows of a map grouped into 4 x 4 x 4 blocks of voxels, one 64-bit mask per block.
 //
-// What bounds k_kmap_probe_self on a large map is random access: a hash-table line per (row, x-triple of offsets), and
-// for every hit a scattered 4-byte store of the mirror entry into a table that no cache holds; once the hash table
-// exceeds the L2 the probes go to DRAM as well (4.8 M rows x 81 offsets: 3740 us). Here a row looks up the blocks that its
-// neighbourhood can touch (at most 8 per position on the axes behind the third; the slots of all blocks stay in L2), and
-// every offset is a bit test; a hit ranks its bit in the mask and reads the row number from `perm`, where the rows of a
-// block lie next to one another. All K offsets are computed, nothing is mirrored, and the table is written once,
-// coalesced: 2180 us for that map, still bound by the row numbers' random reads (26 per row; more registers or wider
-// shared entries leave less L1 and are slower: 2030 and 2350 us against 1980 us for the kernel alone).
+// What bounds k_kmap_probe_self on a large map whose rows come in no spatial order is random access: a hash-table line per
+// (row, x-triple of offsets), and for every hit a scattered 4-byte store of the mirror entry into a table that no cache holds;
+// once the table lines that the rows of a stretch touch exceed the L2 the probes go to DRAM as well. Here a row looks up the
+// blocks that its neighbourhood can touch (at most 8 per position on the axes behind the third; the slots of all blocks stay
+// in L2), and every offset is a bit test; a hit ranks its bit in the mask and reads the row number from `perm`, where the rows
+// of a block lie next to one another. All K offsets are computed, nothing is mirrored, and the table is written once,
+// coalesced. 4.8 M rows of four shuffled clips x 81 offsets: 3650 us by probing, 2324 with the index, still bound by the row
+// numbers' random reads (26 per row; more registers or wider shared entries leave less L1 and are slower: 2030 and 2350 us
+// against 1980 us for the kernel alone). Rows that do come in spatial order are probed in 1480 us and take 2240 with the index,
+// and thin clouds 290 and 1080: k_block_choose decides on the device, and where the index does not serve, its kernels end at
+// once and k_kmap_probe_self runs behind them (25 - 30 us later than it would by itself).
 //
 // Included by rmn_kmap.cu.
 #pragma once
@@ -22,16 +25,16 @@ struct __align__(32) BlockSlot {  // one 32-byte sector: a lookup is one access
 };
 
 // Index in a workspace of block_index_bytes(n). One slot per eight rows, so that the slots fit the L2 where the hash table
-// does not: a surface fills a block with about twenty rows. Rows that lie too thinly for that (a lidar sweep) overflow
-// the index; its user then falls back to the hash table.
+// does not: a surface fills a block with about twenty rows. Rows that lie too thinly for that (a lidar sweep) do not fit.
 struct BlockIndex {
   BlockSlot* slots;
   uint32_t* counter;      // rows numbered so far, minus one
-  uint32_t* overflow;     // all ones; 0: the blocks did not fit
+  uint32_t* state;        // one of the three below
   int32_t* perm;          // row numbers, block by block
   uint32_t* slot_of_row;  // build scratch
   uint32_t capacity;
 };
+constexpr uint32_t kIndexInUse = ~0u, kIndexNotChosen = 0u, kIndexFull = 1u;  // full: the blocks did not fit
 // (a surface loads two slots in five: runs of 32 taken slots occur, runs of 128 do not; 4.8 M clip rows overflowed at 32 in
 // some scenes, and took 3.0 ms by the hash table)
 constexpr uint32_t kBlockMaxProbes = 128;
@@ -43,8 +46,8 @@ inline BlockIndex block_index(void* workspace, uint32_t n) {
   BlockIndex b;
   b.capacity = block_index_capacity(n);
   b.slots = static_cast<BlockSlot*>(workspace);
-  b.counter = reinterpret_cast<uint32_t*>(b.slots + b.capacity);  // (filled together with the slots)
-  b.overflow = b.counter + 1;
+  b.counter = reinterpret_cast<uint32_t*>(b.slots + b.capacity);
+  b.state = b.counter + 1;
   b.perm = reinterpret_cast<int32_t*>(b.counter + 8);
   b.slot_of_row = reinterpret_cast<uint32_t*>(b.perm + n);
   return b;
@@ -59,11 +62,13 @@ __device__ __forceinline__ uint32_t block_hash(unsigned long long key, uint32_t 
   return __umulhi(h, capacity);
 }
 
-// Coordinates of a row relative to the box, split into block and position. The first three spatial columns (fewer in
-// two or one dimensions) are the block's axes; the low bits that all rows share (tensor stride) are left out of them.
+// Coordinates of a row relative to the box, split into block and position. The first three spatial columns are the block's
+// axes (in fewer dimensions a block has too few rows for the index); the low bits that all rows share (tensor stride) are left
+// out of them.
 template <int W>
 struct BlockCoords {
-  static constexpr int NA = W - 1 < 3 ? W - 1 : 3;
+  static_assert(W >= 4, "three spatial columns");
+  static constexpr int NA = 3;
   uint32_t local;           // 2 bits per block axis, in nibbles
   uint32_t block[NA];       // block coordinate per block axis
   unsigned long long key;   // packed block coordinates with the remaining columns
@@ -90,40 +95,162 @@ struct BlockCoords {
   }
 };
 
+// Whether the index serves this map, by two samples of its rows.
+// Working set: the part of the hash table that the rows of a stretch touch goes with the part of the map's space which the
+// stretch covers. Of 8192 rows in sequence every other one marks its coarse cell (eight per block axis, four on the other
+// axes); the part of 8192 rows spread over the map that lie in marked cells, by the same part of the stretch's other rows (the
+// marks do not reach every cell), is the part covered. Measured, by (part x table): 27 offsets, 41 MiB 650 us probed and 801
+// with the index, 48 MiB 413 and 501, 55 MiB 1064 and 1037, 61 MiB 606 and 621, 82 MiB 902 and 803, 219 MiB 1601 and 1058;
+// 81 offsets, 14 MiB 1394 and 1822, 55 MiB 2585 and 1832.
+// Density: 64 rows count the rows of their blocks in the hash table; the mean of 1 / count is blocks per row. With more than
+// 0.6 of the slots taken, the runs of taken slots grow towards kBlockMaxProbes.
+// k_block_sample reads the rows (a single SM would wait 50 us for these random reads); in k_block_choose every block counts and
+// decides, then all clear the slots or, where k_kmap_probe_self will run, fill the mirrored half of the table with "no
+// neighbour" - work that hides the launches of the kernels behind it.
+constexpr uint32_t kChooseRows = 8192, kChooseCells = 47 * 1024, kChooseBlocks = 64;
+constexpr float kChooseBytes = 51.f * (1 << 20), kChooseLoad = 0.6f;
+
+struct BlockSample {                            // lies in perm, which is not needed before the choice
+  uint16_t sequence[kChooseRows];               // coarse cells of rows in sequence
+  uint16_t spread[kChooseRows];                 // and of rows spread over the map
+  uint32_t rows[kChooseBlocks * 64 / 32];       // rows found by every 32 lookups of voxels, 64 per sampled block
+};
+
+template <int W>
+__global__ void __launch_bounds__(256) k_block_sample(const TableHeader* __restrict__ h, const Slot* __restrict__ slots,
+                                                      const int32_t* __restrict__ coords, uint32_t n,
+                                                      BlockSample* __restrict__ sample) {
+  after_previous_kernel();
+  const uint32_t t = blockIdx.x * 256 + threadIdx.x;  // kChooseRows in all
+  auto cell = [&](uint32_t row) {
+    int32_t c[W];
+    load_row<W>(coords, row, c);
+    unsigned long long key = (uint32_t)c[0] - (uint32_t)h->mn[0];
+#pragma unroll
+    for (int a = 1; a < W; ++a) {
+      const int width = 32 - __clz((int)((uint32_t)h->mx[a] - (uint32_t)h->mn[a])), bits = a <= 3 ? 3 : 2;
+      key = key * 8 + (((uint32_t)c[a] - (uint32_t)h->mn[a]) >> (width > bits ? width - bits : 0));
+    }
+    return (uint16_t)block_hash(key, kChooseCells);
+  };
+  sample->sequence[t] = cell(n / 8 * 3 + t);
+  sample->spread[t] = cell((uint32_t)((uint64_t)t * n / kChooseRows));
+  if (t >= kChooseBlocks * 64) return;
+  int32_t c[W];
+  load_row<W>(coords, (uint32_t)((uint64_t)(t / 64) * n / kChooseBlocks), c);
+  unsigned long long key = 0;
+  bool in_box = true;
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    uint32_t d = (uint32_t)c[i] - (uint32_t)h->mn[i];
+    if (i >= 1 && i <= 3) {
+      const uint32_t s = h->low_shift(i - 1);
+      d = (((d >> s) & ~3u) | ((t >> (2 * (i - 1))) & 3u)) << s;
+      in_box = in_box && d <= (uint32_t)h->mx[i] - (uint32_t)h->mn[i];
+    }
+    key |= (unsigned long long)d << h->shift[i];
+  }
+  const bool found = in_box && table_find(slots, h->capacity, h->pos_shift, key) != 0xFFFFFFFFu;
+  const uint32_t votes = __ballot_sync(0xFFFFFFFFu, found);
+  if ((t & 31) == 0) sample->rows[t / 32] = (uint32_t)__popc(votes);
+}
+
+__global__ void __launch_bounds__(1024) k_block_choose(const TableHeader* __restrict__ h, uint32_t n,
+                                                       const BlockSample* __restrict__ sample, BlockIndex ix,
+                                                       int32_t* __restrict__ mirrored, size_t n_mirrored) {
+  after_previous_kernel();
+  __shared__ __align__(16) uint8_t s_marked[kChooseCells];
+  __shared__ uint32_t s_inside[2], s_serves;
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid; i < kChooseCells / 16; i += 1024) reinterpret_cast<uint4*>(s_marked)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid < 2) s_inside[tid] = 0u;
+  static_assert(kChooseRows == 8 * 1024, "rows of a thread");
+  __align__(16) uint16_t sequence[8], spread[8];
+  *reinterpret_cast<uint4*>(sequence) = reinterpret_cast<const uint4*>(sample->sequence)[tid];
+  *reinterpret_cast<uint4*>(spread) = reinterpret_cast<const uint4*>(sample->spread)[tid];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) s_marked[sequence[i]] = 1;
+  __syncthreads();
+  uint32_t near = 0, far = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (i & 1) near += s_marked[sequence[i]];
+    far += s_marked[spread[i]];
+  }
+  near = __reduce_add_sync(0xFFFFFFFFu, near);
+  far = __reduce_add_sync(0xFFFFFFFFu, far);
+  if ((tid & 31) == 0) {
+    atomicAdd(&s_inside[0], near);
+    atomicAdd(&s_inside[1], far);
+  }
+  __syncthreads();
+  if (tid < 32) {
+    float blocks = 0.f;
+#pragma unroll
+    for (uint32_t j = tid; j < kChooseBlocks; j += 32) blocks += 1.f / (float)(sample->rows[2 * j] + sample->rows[2 * j + 1]);
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) blocks += __shfl_xor_sync(0xFFFFFFFFu, blocks, d);
+    const float part = fminf(1.f, 0.5f * (float)s_inside[1] / (float)s_inside[0]);
+    const float set = part * ((float)h->capacity * sizeof(Slot));
+    if (tid == 0)
+      s_serves = set > kChooseBytes && blocks / kChooseBlocks * (float)n <= kChooseLoad * (float)ix.capacity ? 1u : 0u;
+  }
+  __syncthreads();
+  const bool serves = s_serves != 0u;
+  const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+  const size_t first = blockIdx.x * 1024 + tid, step = gridDim.x * 1024;
+  if (first == 0) {
+    *ix.state = serves ? kIndexInUse : kIndexNotChosen;
+    *ix.counter = ~0u;
+  }
+  if (serves) {
+    for (size_t i = first; i < 2 * (size_t)ix.capacity; i += step) reinterpret_cast<uint4*>(ix.slots)[i] = ones;
+  } else {  // single words up to the first 16-byte boundary and behind the last one
+    const size_t head = ((16 - ((uintptr_t)mirrored & 15)) & 15) / 4, vecs = (n_mirrored - head) / 4;
+    const size_t tail = head + 4 * vecs;
+    for (size_t i = first; i < vecs; i += step) __stcs(reinterpret_cast<uint4*>(mirrored + head) + i, ones);
+    if (first < head) mirrored[first] = -1;
+    if (tail + first < n_mirrored) mirrored[tail + first] = -1;
+  }
+}
+
 template <int W>
 __global__ void __launch_bounds__(256) k_block_insert(const TableHeader* __restrict__ h, const int32_t* __restrict__ coords,
                                                       uint32_t n, BlockIndex ix) {
-  const uint32_t row = blockIdx.x * 256 + threadIdx.x;
-  if (row >= n) return;
-  int32_t c[W];
-  load_row<W>(coords, row, c);
-  BlockCoords<W> b;
-  b.load(h, c);
-  if (*(volatile uint32_t*)ix.overflow == 0) return;
-  uint32_t s = block_hash(b.key, ix.capacity);
-  bool placed = false;
-  for (uint32_t probe = 0; probe < kBlockMaxProbes; ++probe) {
-    unsigned long long cur = *(volatile unsigned long long*)&ix.slots[s].key;
-    if (cur == kEmptyKey) cur = atomicCAS(&ix.slots[s].key, kEmptyKey, b.key);
-    if (cur == kEmptyKey || cur == b.key) {
-      placed = true;
-      break;
+  after_previous_kernel();
+  for (uint32_t row = blockIdx.x * 256 + threadIdx.x; row < n; row += gridDim.x * 256) {
+    if (*(volatile uint32_t*)ix.state != kIndexInUse) return;
+    int32_t c[W];
+    load_row<W>(coords, row, c);
+    BlockCoords<W> b;
+    b.load(h, c);
+    uint32_t s = block_hash(b.key, ix.capacity);
+    bool placed = false;
+    for (uint32_t probe = 0; probe < kBlockMaxProbes; ++probe) {
+      unsigned long long cur = *(volatile unsigned long long*)&ix.slots[s].key;
+      if (cur == kEmptyKey) cur = atomicCAS(&ix.slots[s].key, kEmptyKey, b.key);
+      if (cur == kEmptyKey || cur == b.key) {
+        placed = true;
+        break;
+      }
+      if (++s == ix.capacity) s = 0;
     }
-    if (++s == ix.capacity) s = 0;
+    if (!placed) {
+      *(volatile uint32_t*)ix.state = kIndexFull;
+      return;
+    }
+    atomicAnd(&ix.slots[s].free, ~(1ull << b.bit(b.local)));
+    ix.slot_of_row[row] = s;
   }
-  if (!placed) {
-    *(volatile uint32_t*)ix.overflow = 0;
-    return;
-  }
-  atomicAnd(&ix.slots[s].free, ~(1ull << b.bit(b.local)));
-  ix.slot_of_row[row] = s;
 }
 
 // Gives every block its range of perm. Which range a block gets depends on the order of the atomics; what the index
 // returns does not.
 __global__ void __launch_bounds__(256) k_block_bases(BlockIndex ix) {
+  after_previous_kernel();
   __shared__ uint32_t s_warp[8], s_base;
-  if (__ldg(ix.overflow) == 0) return;
+  if (*ix.state != kIndexInUse) return;
   const uint32_t s = blockIdx.x * 256 + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t count = s < ix.capacity ? (uint32_t)__popcll(~__ldg(&ix.slots[s].free)) : 0u;
@@ -152,25 +279,35 @@ __global__ void __launch_bounds__(256) k_block_bases(BlockIndex ix) {
 template <int W>
 __global__ void __launch_bounds__(256) k_block_scatter(const TableHeader* __restrict__ h, const int32_t* __restrict__ coords,
                                                        uint32_t n, BlockIndex ix) {
-  const uint32_t row = blockIdx.x * 256 + threadIdx.x;
-  if (row >= n) return;
-  if (__ldg(ix.overflow) == 0) return;
-  const uint32_t s = ix.slot_of_row[row];
-  int32_t c[W];
-  load_row<W>(coords, row, c);
-  BlockCoords<W> b;
-  b.load(h, c);
-  const unsigned long long below = (1ull << b.bit(b.local)) - 1ull;
-  ix.perm[__ldg(&ix.slots[s].base) + (uint32_t)__popcll(~__ldg(&ix.slots[s].free) & below)] = (int32_t)row;
+  after_previous_kernel();
+  if (*ix.state != kIndexInUse) return;
+  for (uint32_t row = blockIdx.x * 256 + threadIdx.x; row < n; row += gridDim.x * 256) {
+    const uint32_t s = ix.slot_of_row[row];
+    int32_t c[W];
+    load_row<W>(coords, row, c);
+    BlockCoords<W> b;
+    b.load(h, c);
+    const unsigned long long below = (1ull << b.bit(b.local)) - 1ull;
+    ix.perm[__ldg(&ix.slots[s].base) + (uint32_t)__popcll(~__ldg(&ix.slots[s].free) & below)] = (int32_t)row;
+  }
 }
 
-// One thread per row, as in k_kmap_probe. Offsets that reach further than two voxels (in units of the map's grid) along
-// a block axis look their row up in the hash table instead.
+// One thread per row, as in k_kmap_probe, in blocks that stay (one setup each, and few to launch where the index is not in
+// use: 2450 -> 2324 us for the four clips). Offsets that reach further than two voxels (in units of the map's grid) along a
+// block axis look their row up in the hash table instead. Where the blocks did not fit, the mirrored half of the table is
+// filled with "no neighbour" for k_kmap_probe_self, which follows.
 template <int W>
 __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots, const int32_t* __restrict__ coords, uint32_t n,
     const int32_t* __restrict__ offsets, int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts,
     uint32_t n_blocks, uint32_t* __restrict__ scan_ticket, BlockIndex ix) {
+  after_previous_kernel();
+  if (*ix.state != kIndexInUse) {
+    if (*ix.state == kIndexFull)
+      for (uint32_t row = blockIdx.x * kKmapBlock + threadIdx.x; row < n; row += gridDim.x * kKmapBlock)
+        for (int k = K / 2 + 1; k < K; ++k) __stcs(nbr + (size_t)k * n + row, -1);
+    return;
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) *scan_ticket = 0;
   using B = BlockCoords<W>;
   constexpr int D = W - 1, NA = B::NA, CELLS = 1 << NA;
@@ -182,7 +319,6 @@ __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
   uint32_t* s_cnt = s_off + K;                                                  // [half]
   __shared__ uint32_t s_reach[2 * NA];  // largest step down / up per block axis
   const int half = K / 2;
-  const bool overflow = __ldg(ix.overflow) == 0;
   if (threadIdx.x < 2 * NA) s_reach[threadIdx.x] = 0;
   __syncthreads();
   for (int k = threadIdx.x; k < K; k += kKmapBlock) {
@@ -208,112 +344,115 @@ __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
         if (step[a] > 0) atomicMax(&s_reach[2 * a + 1], (uint32_t)step[a]);
       }
     }
-    if (overflow) e |= kFar;
     s_off[k] = e;
-    if (k < half) s_cnt[k] = 0;
   }
-  __syncthreads();
 
-  const uint32_t q = blockIdx.x * kKmapBlock + threadIdx.x;
-  const bool active = q < n;
-  const int lane = threadIdx.x & 31;
-  int32_t c[W];
+  for (uint32_t row_block = blockIdx.x; row_block < n_blocks; row_block += gridDim.x) {
+    __syncthreads();  // (the offsets are there, the counts of the block before are written)
+    for (int k = threadIdx.x; k < half; k += kKmapBlock) s_cnt[k] = 0;
+    __syncthreads();
+    const uint32_t q = row_block * kKmapBlock + threadIdx.x;
+    const bool active = q < n;
+    const int lane = threadIdx.x & 31;
+    int32_t c[W];
 #pragma unroll
-  for (int i = 0; i < W; ++i) c[i] = h->mn[i];
-  if (active) load_row<W>(coords, q, c);
-  B b;
-  b.load(h, c);
-  // per block axis: the neighbouring block on the side of the row's half of its block, if any offset reaches it
-  long long side[NA];
-  uint32_t reach = 0;
+    for (int i = 0; i < W; ++i) c[i] = h->mn[i];
+    if (active) load_row<W>(coords, q, c);
+    B b;
+    b.load(h, c);
+    // per block axis: the neighbouring block on the side of the row's half of its block, if any offset reaches it
+    long long side[NA];
+    uint32_t reach = 0;
 #pragma unroll
-  for (int a = 0; a < NA; ++a) {
-    const uint32_t l = (b.local >> (4 * a)) & 3u;
-    const uint32_t last = (((uint32_t)(h->mx[a + 1] - h->mn[a + 1])) >> h->low_shift(a)) >> 2;
-    const bool up = l >= 2;
-    if (up ? (l + s_reach[2 * a + 1] > 3 && b.block[a] < last) : (s_reach[2 * a] > l && b.block[a] > 0)) reach |= 1u << a;
-    side[a] = (up ? 1ll : -1ll) * (1ll << h->shift[a + 1]);
-  }
-  unsigned long long* occ = s_occ + threadIdx.x;
-  uint32_t* base = s_base + threadIdx.x;
-  int32_t* dst = nbr + q;
-  for (int k = 0; k < K; ++k, dst += n) {
-    const uint32_t e = s_off[k];
-    if (!overflow && (e & kNewOuter)) {  // (same for the whole block) look up the blocks around the row
-      unsigned long long key0 = b.key;
-      bool in_box = active;
+    for (int a = 0; a < NA; ++a) {
+      const uint32_t l = (b.local >> (4 * a)) & 3u;
+      const uint32_t last = (((uint32_t)(h->mx[a + 1] - h->mn[a + 1])) >> h->low_shift(a)) >> 2;
+      const bool up = l >= 2;
+      if (up ? (l + s_reach[2 * a + 1] > 3 && b.block[a] < last) : (s_reach[2 * a] > l && b.block[a] > 0)) reach |= 1u << a;
+      side[a] = (up ? 1ll : -1ll) * (1ll << h->shift[a + 1]);
+    }
+    unsigned long long* occ = s_occ + threadIdx.x;
+    uint32_t* base = s_base + threadIdx.x;
+    int32_t* dst = nbr + q;
+    for (int k = 0; k < K; ++k, dst += n) {
+      const uint32_t e = s_off[k];
+      if (e & kNewOuter) {  // (same for the whole block) look up the blocks around the row
+        unsigned long long key0 = b.key;
+        bool in_box = active;
 #pragma unroll
-      for (int a = NA; a < D; ++a) {
-        const int32_t o = __ldg(offsets + k * D + a);
-        in_box = in_box && b.dist[a + 1] + (uint32_t)o <= (uint32_t)(h->mx[a + 1] - h->mn[a + 1]);
-        key0 += (unsigned long long)((long long)o << h->shift[a + 1]);
-      }
-      constexpr int BATCH = CELLS < 4 ? CELLS : 4;  // independent lookups in flight
+        for (int a = NA; a < D; ++a) {
+          const int32_t o = __ldg(offsets + k * D + a);
+          in_box = in_box && b.dist[a + 1] + (uint32_t)o <= (uint32_t)(h->mx[a + 1] - h->mn[a + 1]);
+          key0 += (unsigned long long)((long long)o << h->shift[a + 1]);
+        }
+        constexpr int BATCH = CELLS < 4 ? CELLS : 4;  // independent lookups in flight
 #pragma unroll
-      for (int i0 = 0; i0 < CELLS; i0 += BATCH) {
-        ulonglong2 v[BATCH];
-        uint32_t at[BATCH];
+        for (int i0 = 0; i0 < CELLS; i0 += BATCH) {
+          ulonglong2 v[BATCH];
+          uint32_t at[BATCH];
 #pragma unroll
-        for (int j = 0; j < BATCH; ++j) {
-          const int i = i0 + j;
-          v[j] = make_ulonglong2(kEmptyKey, ~0ull);
-          at[j] = 0;
-          if (in_box && (i & ~reach) == 0) {
+          for (int j = 0; j < BATCH; ++j) {
+            const int i = i0 + j;
+            v[j] = make_ulonglong2(kEmptyKey, ~0ull);
+            at[j] = 0;
+            if (in_box && (i & ~reach) == 0) {
+              unsigned long long key = key0;
+#pragma unroll
+              for (int a = 0; a < NA; ++a)
+                if ((i >> a) & 1) key += (unsigned long long)side[a];
+              at[j] = block_hash(key, ix.capacity);
+              v[j] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[j]));
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < BATCH; ++j) {
+            const int i = i0 + j;
             unsigned long long key = key0;
 #pragma unroll
             for (int a = 0; a < NA; ++a)
               if ((i >> a) & 1) key += (unsigned long long)side[a];
-            at[j] = block_hash(key, ix.capacity);
-            v[j] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[j]));
+            for (uint32_t probe = 1; v[j].x != key && v[j].x != kEmptyKey && probe < kBlockMaxProbes; ++probe) {
+              if (++at[j] == ix.capacity) at[j] = 0;
+              v[j] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[j]));
+            }
+            const bool found = v[j].x == key;
+            occ[i * kKmapBlock] = found ? ~v[j].y : 0ull;
+            if (found) base[i * kKmapBlock] = __ldg(&ix.slots[at[j]].base);
           }
         }
+      }
+      uint32_t uid = 0xFFFFFFFFu;
+      bool hit = false;
+      if (!(e & (kNever | kFar))) {
+        const uint32_t p = b.local + (e & 0xFFFu), bit = B::bit(p);
+        // bits 2, 6 and 10: is the voxel in the row's own block or in the next one along the axis
+        const uint32_t cell = ((((p & 0x444u) * 0x124u) >> 10) & 7u) * kKmapBlock;
+        const unsigned long long m = occ[cell];
+        hit = (m >> bit) & 1ull;
+        if (hit) uid = (uint32_t)__ldg(ix.perm + base[cell] + __popcll(m & ((1ull << bit) - 1ull)));
+      } else if (e & kFar && !(e & kNever)) {
+        bool in_box = active;
+        unsigned long long key = 0;
 #pragma unroll
-        for (int j = 0; j < BATCH; ++j) {
-          const int i = i0 + j;
-          unsigned long long key = key0;
-#pragma unroll
-          for (int a = 0; a < NA; ++a)
-            if ((i >> a) & 1) key += (unsigned long long)side[a];
-          for (uint32_t probe = 1; v[j].x != key && v[j].x != kEmptyKey && probe < kBlockMaxProbes; ++probe) {
-            if (++at[j] == ix.capacity) at[j] = 0;
-            v[j] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[j]));
-          }
-          const bool found = v[j].x == key;
-          occ[i * kKmapBlock] = found ? ~v[j].y : 0ull;
-          if (found) base[i * kKmapBlock] = __ldg(&ix.slots[at[j]].base);
+        for (int i = 0; i < W; ++i) {
+          const uint32_t d = b.dist[i] + (i > 0 ? (uint32_t)__ldg(offsets + k * D + i - 1) : 0u);
+          in_box = in_box && d <= (uint32_t)(h->mx[i] - h->mn[i]);
+          key |= (unsigned long long)d << h->shift[i];
         }
+        if (in_box) uid = table_find(slots, h->capacity, h->pos_shift, key);
+        hit = uid != 0xFFFFFFFFu;
+      }
+      if (active) __stcs(dst, (int32_t)uid);
+      if (k < half) {  // (the other half has the same counts, see k_kmap_scan)
+        const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+        if (lane == 0) atomicAdd(&s_cnt[k], (uint32_t)__popc(hits));
       }
     }
-    uint32_t uid = 0xFFFFFFFFu;
-    bool hit = false;
-    if (!(e & (kNever | kFar))) {
-      const uint32_t p = b.local + (e & 0xFFFu), bit = B::bit(p);
-      // bits 2, 6 and 10: is the voxel in the row's own block or in the next one along the axis
-      const uint32_t cell = ((((p & 0x444u) * 0x124u) >> 10) & 7u) * kKmapBlock;
-      const unsigned long long m = occ[cell];
-      hit = (m >> bit) & 1ull;
-      if (hit) uid = (uint32_t)__ldg(ix.perm + base[cell] + __popcll(m & ((1ull << bit) - 1ull)));
-    } else if (e & kFar && !(e & kNever)) {
-      bool in_box = active;
-      unsigned long long key = 0;
-#pragma unroll
-      for (int i = 0; i < W; ++i) {
-        const uint32_t d = b.dist[i] + (i > 0 ? (uint32_t)__ldg(offsets + k * D + i - 1) : 0u);
-        in_box = in_box && d <= (uint32_t)(h->mx[i] - h->mn[i]);
-        key |= (unsigned long long)d << h->shift[i];
-      }
-      if (in_box) uid = table_find(slots, h->capacity, h->pos_shift, key);
-      hit = uid != 0xFFFFFFFFu;
-    }
-    if (active) __stcs(dst, (int32_t)uid);
-    if (k < half) {  // (the other half has the same counts, see k_kmap_scan)
-      const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
-      if (lane == 0) atomicAdd(&s_cnt[k], (uint32_t)__popc(hits));
-    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < half; k += kKmapBlock) block_counts[(size_t)k * n_blocks + row_block] = s_cnt[k];
+    if (threadIdx.x == 0)
+      block_counts[(size_t)half * n_blocks + row_block] = min((uint32_t)kKmapBlock, n - row_block * kKmapBlock);
   }
-  __syncthreads();
-  for (int k = threadIdx.x; k < half; k += kKmapBlock) block_counts[(size_t)k * n_blocks + blockIdx.x] = s_cnt[k];
-  if (threadIdx.x == 0) block_counts[(size_t)half * n_blocks + blockIdx.x] = min((uint32_t)kKmapBlock, n - blockIdx.x * kKmapBlock);
 }
 
 }  // namespace rmn

@@ -1,30 +1,48 @@
-"""Self maps whose hash table exceeds the L2, which go over the occupancy index, against the general builder (which the
-oracle covers): dimensions, tensor strides, offsets inside and beyond the reach of the index, negative coordinates, clouds
-dense enough for the index and clouds that overflow it."""
+"""Self maps whose hash table takes most of the L2, which may go over the occupancy index, against the general builder
+(which the oracle covers): dimensions, tensor strides, offsets inside and beyond the reach of the index, negative coordinates,
+clouds dense enough for the index and too thin for it, rows in random and in spatial order - and which way they went."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("D,n,extent,kernel,dilation,stride", [
-    (3, 1_970_000, 110, 3, 1, 1), (3, 2_000_001, 5000, 3, 1, 1), (3, 1_970_000, 110, 5, 1, 1), (3, 1_970_000, 100, 3, 3, 1),
-    (3, 1_980_000, 100, 3, 1, 4), (3, 1_980_000, 100, 3, 2, 6), (2, 1_970_000, 1100, 3, 1, 2), (4, 2_100_003, 36, 3, 1, 1),
-    (5, 1_970_000, 16, 3, 1, 2), (1, 1_970_000, 1_500_000, 9, 1, 1),
+IN_USE, NOT_CHOSEN, FULL = -1, 0, 1
+
+
+def _index_state(kmap):
+    """The word of the build's workspace that says what became of the index (csrc/rmn_kmap_blocks.cuh)."""
+    n, K = kmap.n_query, kmap.K
+    counts = ((K * ((n + 255) // 256) + K + 64) * 4 + 255) // 256 * 256
+    at = counts + (n // 8 + 64) * 32 + 4
+    return kmap.workspace[at:at + 4].cpu().view(torch.int32).item()
+
+
+# (a stride that is no power of two leaves the blocks thin; order: "random", or "sorted" by coordinates; index: what
+# becomes of it, None below three dimensions, where there is none)
+@pytest.mark.parametrize("D,n,extent,kernel,dilation,stride,order,index", [
+    (3, 1_970_000, 110, 3, 1, 1, "random", IN_USE), (3, 2_000_001, 5000, 3, 1, 1, "random", NOT_CHOSEN),
+    (3, 1_970_000, 110, 5, 1, 1, "random", IN_USE), (3, 1_970_000, 100, 3, 3, 1, "random", IN_USE),
+    (3, 1_980_000, 100, 3, 1, 4, "random", IN_USE), (3, 1_980_000, 100, 3, 2, 6, "random", NOT_CHOSEN),
+    (2, 1_970_000, 1100, 3, 1, 2, "random", None), (4, 2_100_003, 36, 3, 1, 1, "random", IN_USE),
+    (5, 1_970_000, 16, 3, 1, 2, "random", IN_USE), (1, 1_970_000, 1_500_000, 9, 1, 1, "random", None),
+    (3, 2_600_001, 110, 3, 1, 1, "sorted", NOT_CHOSEN), (3, 1_970_003, 250, 3, 1, 1, "random", NOT_CHOSEN),
 ])
-def test_large_self_map_equals_general_builder(D, n, extent, kernel, dilation, stride):
+def test_large_self_map_equals_general_builder(D, n, extent, kernel, dilation, stride, order, index):
     from riemannengine_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(D * 1000 + n)
     c = torch.cat([torch.randint(0, 3, (3 * n, 1), generator=g, device="cuda"),
                    torch.randint(-extent // 2, extent - extent // 2, (3 * n, D), generator=g, device="cuda") * stride], 1)
     c = torch.unique(c, dim=0)
-    c = c[torch.randperm(c.size(0), generator=g, device="cuda")][:n].int().contiguous()
+    c = c[torch.randperm(c.size(0), generator=g, device="cuda")][:n]
+    c = (torch.unique(c, dim=0) if order == "sorted" else c).int().contiguous()
     assert c.size(0) == n
     table = ops.table_build(c)
     off = ops.region_offsets(0, [kernel] * D, [dilation] * D, [stride] * D)
     a = ops.kmap_build(table, table.coords, off)
     b = ops.kmap_build(table, table.coords, off, self_map=True)
     assert torch.equal(a.nbr, b.nbr) and torch.equal(a.offset_ptr, b.offset_ptr)
+    assert index is None or _index_state(b) == index
     if kernel > 3 or D > 4:
         return
     (pa, xa, ya), (pb, xb, yb) = a.pairs(), b.pairs()
@@ -33,3 +51,28 @@ def test_large_self_map_equals_general_builder(D, n, extent, kernel, dilation, s
         lo, hi = int(a.offset_ptr[k]), int(a.offset_ptr[k + 1])
         order_a, order_b = ya[lo:hi].argsort(), yb[lo:hi].argsort()
         assert torch.equal(xa[lo:hi][order_a], xb[lo:hi][order_b]) and torch.equal(ya[lo:hi][order_a], yb[lo:hi][order_b])
+
+
+def test_index_that_turns_out_too_small_gives_way_to_the_table():
+    """Rows that the choice samples lie in full blocks, all others thinly: chosen, then full."""
+    from riemannengine_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n = 2_000_003
+    thin = torch.randint(16, 4000, (n + 200_000, 3), generator=g, device="cuda")
+    thin = torch.unique(thin, dim=0)
+    c = thin[torch.randperm(thin.size(0), generator=g, device="cuda")][:n]
+    dense = torch.cartesian_prod(*[torch.arange(16, device="cuda")] * 3)   # 64 blocks of 64 voxels
+    by_block = dense[((dense // 4) * torch.tensor([16, 4, 1], device="cuda")).sum(1).argsort(stable=True)]
+    at = torch.arange(64, device="cuda") * n // 64                         # one voxel of every block where the choice looks
+    c[at] = by_block[::64]
+    rest = torch.ones(4096, dtype=torch.bool, device="cuda")
+    rest[::64] = False
+    free = torch.arange(n, device="cuda")[~torch.isin(torch.arange(n, device="cuda"), at)]
+    c[free[torch.randperm(free.numel(), generator=g, device="cuda")[:4032]]] = by_block[rest]
+    coords = torch.cat([torch.zeros((n, 1), dtype=torch.long, device="cuda"), c], 1).int().contiguous()
+    table = ops.table_build(coords)
+    assert table.n_unique == n
+    off = ops.region_offsets(0, [3] * 3, [1] * 3, [1] * 3)
+    a, b = ops.kmap_build(table, table.coords, off), ops.kmap_build(table, table.coords, off, self_map=True)
+    assert _index_state(b) == FULL
+    assert torch.equal(a.nbr, b.nbr) and torch.equal(a.offset_ptr, b.offset_ptr)
