@@ -468,6 +468,7 @@ int f32_conv_backward_weight(const float* feats, const float* grad_out, uint32_t
   const uint32_t rows = f32_wgrad_chunk_rows(n_dst, K, c_in, c_out), chunks = (n_dst + rows - 1) / rows;
   const int cot = c_out <= 32 ? 32 : 64, tiles_co = (c_out + cot - 1) / cot;
   dim3 grid(chunks, K, (c_in + 31) / 32 * tiles_co);
+  if (grid.z > 65535u) return RMN_ERR_UNSUPPORTED;  // (a launch takes no more)
   if (cot == 32) {
     static SmemOptIn opt_in;
     RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_wgrad_f32<32>), F32WgCfg<32>::SMEM));

@@ -47,6 +47,16 @@ def test_f32_passes_match_float64(n, c_in, c_out, K, fill):
     close(ops.conv_backward_weight(d(feats), d(grad), d(nbr)), want_w)
 
 
+def test_weight_gradient_of_more_channel_tiles_than_a_launch_takes():
+    from riemannengine_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(1)
+    feats, grad = torch.randn((3, 16384), generator=g, device="cuda"), torch.randn((3, 8192), generator=g, device="cuda")
+    nbr = torch.tensor([[2, -1, 0]], dtype=torch.int32, device="cuda")
+    got = ops.conv_backward_weight(feats, grad, nbr)[0]
+    want = feats[2][:, None] * grad[0] + feats[0][:, None] * grad[2]
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
 def test_transpose_weights_reverses_the_offsets():
     from riemannengine_b200 import capi, ops
     for dtype, code in ((torch.float32, capi.F32), (torch.bfloat16, capi.BF16)):
