@@ -141,20 +141,22 @@ class KernelMap:
 
     # Convolution plans (ops.conv_plan_build), built lazily under the same rule as the C++ host layer
     # (KernelMap::plan_out in riemann_cpp): passes of 128 x 128 channels or more count, by c_in * c_out, and
-    # the one that brings the sum to two 128 x 128 layers' worth builds the plan; narrower ones gain nothing.
-    plan_policy = 0  # 0 automatic, 1 always, 2 never
+    # the one that brings the sum to two 128 x 128 layers' worth builds the plan; narrower ones and maps of up
+    # to 74 row tiles take none.
+    plan_policy = 0  # 0 automatic, 1 always (the first wide pass), 2 never
     _WIDE_PASS = 128 * 128
+    _PLAN_MIN_ROWS = 74 * 128 + 1
 
     @staticmethod
     def _want_plan(weight_sum: int, rows: int) -> bool:
-        if KernelMap.plan_policy == 2 or rows < 8192:
+        if KernelMap.plan_policy == 2 or rows < KernelMap._PLAN_MIN_ROWS:
             return False
         return KernelMap.plan_policy == 1 or weight_sum >= 2 * KernelMap._WIDE_PASS
 
     def plan_out(self, weight: int):
         if self._parent is not None:
             return self._parent.plan_in(weight)
-        if weight < self._WIDE_PASS and KernelMap.plan_policy == 0:
+        if weight < self._WIDE_PASS:
             return None
         self._uses_out += weight
         if (self._plan_out is None and self.region_offsets is not None
@@ -167,7 +169,7 @@ class KernelMap:
             return self._parent.plan_out(weight)
         if self.self_symmetric:
             return self.plan_out(weight)
-        if weight < self._WIDE_PASS and KernelMap.plan_policy == 0:
+        if weight < self._WIDE_PASS:
             return None
         self._uses_in += weight
         if (self._plan_in is None and self.region_offsets is not None

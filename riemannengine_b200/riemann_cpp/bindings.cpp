@@ -172,8 +172,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("__truediv__", [](const SparseTensor& a, const SparseTensor& b) { return a / b; })
       .def("__add__", [](const SparseTensor& a, double s) { return a + at::Scalar(s); })
       .def("__mul__", [](const SparseTensor& a, double s) { return a * at::Scalar(s); });
-  // 0 = automatic (plan a kernel map from its second convolution pass on, or at once for wide layers),
-  // 1 = always, 2 = never
+  // 0 = automatic (plan a kernel map at its second pass of 128 x 128 channels), 1 = always (at the first such pass), 2 = never
   m.def("set_convolution_plan_policy", [](int policy) { set_convolution_plan_policy(PlanPolicy::Type(policy)); },
         py::arg("policy"));
   m.def("convolution_plan_policy", []() { return int(convolution_plan_policy()); });

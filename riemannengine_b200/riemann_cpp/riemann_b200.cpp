@@ -155,18 +155,19 @@ namespace {
 // AUTO: a plan costs about two passes over the table (0.12 ms for 1.2 M rows x 27 offsets) and saves some 10 % of a
 // tensor-core pass of 128 x 128 channels or more; narrower passes are bound by their gather and gain nothing. Only the
 // wide passes over a table are therefore counted, by c_in * c_out, and the plan is built by the one that brings the sum
-// to two 128 x 128 layers' worth.
-constexpr int64_t kWidePass = 128 * 128;
+// to two 128 x 128 layers' worth. Up to 74 row tiles of 128 the convolution runs single tiles, which take no plan.
+// (ALWAYS: the first wide pass builds the plan.)
+constexpr int64_t kWidePass = 128 * 128, kPlanMinRows = 74 * 128 + 1;
 bool want_plan(int64_t weight_sum, int64_t rows) {
   const int policy = g_plan_policy.load();
-  if (policy == PlanPolicy::NEVER || rows < 8192) return false;
+  if (policy == PlanPolicy::NEVER || rows < kPlanMinRows) return false;
   return policy == PlanPolicy::ALWAYS || weight_sum >= 2 * kWidePass;
 }
 }  // namespace
 
 at::Tensor KernelMap::plan_out(int64_t weight) {
   if (parent) return parent->plan_in(weight);  // a swapped view: its output table is the parent's input table
-  if (weight < kWidePass && g_plan_policy.load() == PlanPolicy::AUTO) return at::Tensor();
+  if (weight < kWidePass) return at::Tensor();
   weight_out_ += weight;
   if (!plan_out_.defined() && want_plan(weight_out_, n_out)) plan_out_ = build_plan(nbr_out, false);
   return plan_out_;
@@ -175,7 +176,7 @@ at::Tensor KernelMap::plan_out(int64_t weight) {
 at::Tensor KernelMap::plan_in(int64_t weight) {
   if (parent) return parent->plan_out(weight);
   if (self_symmetric) return plan_out(weight);  // the input gradient of a self map runs over the same table
-  if (weight < kWidePass && g_plan_policy.load() == PlanPolicy::AUTO) return at::Tensor();
+  if (weight < kWidePass) return at::Tensor();
   weight_in_ += weight;
   if (!plan_in_.defined() && want_plan(weight_in_, n_in)) plan_in_ = build_plan(nbr_in(), true);
   return plan_in_;

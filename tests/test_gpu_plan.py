@@ -68,7 +68,19 @@ def test_plan_buffer_is_a_stable_class_sort_of_the_table(n, D, ksize, stride):
         assert (((tmask[:, k // 32] >> (k % 32)) & 1).astype(bool) == any_hit).all(), k
 
 
-@pytest.mark.parametrize("c_in,c_out", [(32, 32), (64, 64), (64, 128), (128, 128), (32, 64), (128, 64), (256, 128)])
+def _assert_plan_is_used(feats, w, nbr, offsets):
+    """A plan holds its own copy of the table: with the plan of another table the planned kernel computes that table's
+    result, a kernel that drops the plan computes this one's."""
+    from riemannengine_b200 import ops
+    other = nbr.clone()
+    other[0] = -1
+    want = ops.conv_forward(feats, w, other)
+    assert not torch.equal(want, ops.conv_forward(feats, w, nbr))
+    assert torch.equal(want, ops.conv_forward(feats, w, nbr, plan=ops.conv_plan_build(other, offsets)))
+
+
+# (the pairs that the kernels on prepared weights plan; the others, which drop a plan, are in test_gpu_plain_conv.py)
+@pytest.mark.parametrize("c_in,c_out", [(128, 128), (128, 256), (256, 128), (256, 256)])
 def test_planned_forward_and_input_gradient_are_bit_identical(c_in, c_out):
     from riemannengine_b200 import ops
     table, nbr, offsets = _cloud_table(50 + c_in + c_out, 40000, 3, -25, 25, 3)
@@ -77,6 +89,7 @@ def test_planned_forward_and_input_gradient_are_bit_identical(c_in, c_out):
     feats = torch.randn(n, c_in, device="cuda", generator=g).bfloat16()
     w = (torch.randn(27, c_in, c_out, device="cuda", generator=g) / (27 * c_in) ** 0.5).bfloat16()
     plan = ops.conv_plan_build(nbr, offsets)
+    _assert_plan_is_used(feats, w, nbr, offsets)
     plain = ops.conv_forward(feats, w, nbr)
     planned = ops.conv_forward(feats, w, nbr, plan=plan)
     assert torch.equal(plain, planned)
@@ -98,12 +111,13 @@ def test_planned_forward_and_input_gradient_are_bit_identical(c_in, c_out):
 def test_planned_strided_4d_and_2d_tables_are_bit_identical():
     from riemannengine_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(2)
-    for n, D, ksize, stride, c_in, c_out in ((60000, 3, 2, 2, 64, 128), (15000, 4, 2, 1, 32, 32), (20000, 2, 5, 1, 32, 64)):
+    for n, D, ksize, stride, c_in, c_out in ((60000, 3, 2, 2, 128, 256), (15000, 4, 2, 1, 128, 128), (20000, 2, 5, 1, 256, 128)):
         table, nbr, offsets = _cloud_table(90 + D + ksize, n, D, -10 if D == 4 else -40, 10 if D == 4 else 40, ksize, stride)
         K, n_dst = int(nbr.size(0)), int(nbr.size(1))
         feats = torch.randn(table.n_unique, c_in, device="cuda", generator=g).bfloat16()
         w = (torch.randn(K, c_in, c_out, device="cuda", generator=g) / (K * c_in) ** 0.5).bfloat16()
         plan = ops.conv_plan_build(nbr, offsets)
+        _assert_plan_is_used(feats, w, nbr, offsets)
         assert torch.equal(ops.conv_forward(feats, w, nbr), ops.conv_forward(feats, w, nbr, plan=plan))
         # the input gradient of a strided map runs over the inverse table, which gets a plan of its own
         nbr_t = ops.kmap_transpose(nbr, table.n_unique)
@@ -117,7 +131,7 @@ def test_planned_rows_without_any_neighbour_store_the_epilogue_of_zero():
     offset and must still store act(0 * scale + shift)."""
     from riemannengine_b200 import capi, ops
     rng = np.random.default_rng(5)
-    c = np.concatenate([np.zeros((3000, 1)), rng.integers(-8, 9, (3000, 3))], 1).astype(np.int32)
+    c = np.concatenate([np.zeros((30000, 1)), rng.integers(-14, 15, (30000, 3))], 1).astype(np.int32)
     table = ops.table_build(torch.from_numpy(c).cuda())
     far = table.coords.clone()
     far[:, 1] += 1000
@@ -126,13 +140,14 @@ def test_planned_rows_without_any_neighbour_store_the_epilogue_of_zero():
     nbr = ops.kmap_build(table, query, offsets).nbr
     plan = ops.conv_plan_build(nbr, offsets)
     g = torch.Generator(device="cuda").manual_seed(3)
-    feats = torch.randn(table.n_unique, 64, device="cuda", generator=g).bfloat16()
-    w = (torch.randn(27, 64, 64, device="cuda", generator=g) / 40).bfloat16()
-    shift = torch.randn(64, device="cuda", generator=g)
+    feats = torch.randn(table.n_unique, 128, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(27, 128, 128, device="cuda", generator=g) / 60).bfloat16()
+    shift = torch.randn(128, device="cuda", generator=g)
+    _assert_plan_is_used(feats, w, nbr, offsets)
     a = ops.conv_forward(feats, w, nbr, None, shift, False)
     b = ops.conv_forward(feats, w, nbr, None, shift, False, plan=plan)
     assert torch.equal(a, b)
-    assert torch.equal(b[table.n_unique:].float(), shift.bfloat16().float().expand(2 * table.n_unique, 64))
+    assert torch.equal(b[table.n_unique:].float(), shift.bfloat16().float().expand(2 * table.n_unique, 128))
 
 
 def test_plan_falls_back_for_fp32_and_large_kernels():
@@ -152,12 +167,12 @@ def _host_network(make_tensor, make_conv, coords, feats, seed_weights):
     the transposed 2^3 back up; returns the output features and every gradient."""
     f = feats.clone().requires_grad_(True)
     x = make_tensor(f, coords)
-    layers = [make_conv(32, 32, 3, 1, False), make_conv(32, 32, 3, 1, False), make_conv(32, 64, 2, 2, False),
-              make_conv(64, 32, 2, 2, True)]
+    layers = [make_conv(128, 128, 3, 1, False), make_conv(128, 128, 3, 1, False), make_conv(128, 256, 2, 2, False),
+              make_conv(256, 128, 2, 2, True)]
     g = torch.Generator(device="cuda").manual_seed(seed_weights)
     with torch.no_grad():
         for layer in layers:
-            layer.kernel.copy_((torch.randn(layer.kernel.shape, device="cuda", generator=g) * 0.05).to(layer.kernel.dtype))
+            layer.kernel.copy_((torch.randn(layer.kernel.shape, device="cuda", generator=g) * 0.02).to(layer.kernel.dtype))
     y = x
     for layer in layers:
         y = layer(y)
@@ -173,7 +188,7 @@ def test_hosts_plan_shared_maps_and_keep_results(host):
     rng = np.random.default_rng(9)
     c = np.concatenate([rng.integers(0, 2, (40000, 1)), rng.integers(-30, 31, (40000, 3))], 1).astype(np.int32)
     coords = torch.from_numpy(c).cuda()
-    feats = torch.randn(len(c), 32, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).bfloat16()
+    feats = torch.randn(len(c), 128, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).bfloat16()
     if host == "cpp":
         from riemannengine_b200 import cpp
         C = cpp.load()
@@ -195,14 +210,37 @@ def test_hosts_plan_shared_maps_and_keep_results(host):
             E.KernelMap.plan_policy = p
 
         make_tensor = E.SparseTensor
-    results = {}
+    results, launches = {}, {}
     try:
         for policy in (2, 1, 0):   # never, always, automatic
             set_policy(policy)
+            before = capi.lib().rmn_launch_count()
             results[policy] = _host_network(make_tensor, make_conv, coords, feats, 17)
+            launches[policy] = capi.lib().rmn_launch_count() - before
     finally:
         set_policy(0)
+    assert launches[1] > launches[2] and launches[0] > launches[2]   # plans were built
     for policy in (1, 0):
         for a, b in zip(results[policy], results[2]):
             assert torch.equal(a, b)
     assert capi.lib().rmn_device_status(None) == capi.OK
+
+
+def test_no_host_builds_a_plan_that_its_kernels_would_drop():
+    """Narrow passes, and wide ones over maps of few row tiles, run unplanned kernels under every policy."""
+    from riemannengine_b200 import engine as E
+    rng = np.random.default_rng(9)
+    for rows, channels in ((40000, 64), (9000, 128)):
+        c = np.concatenate([np.zeros((rows, 1)), rng.integers(-40, 41, (rows, 3))], 1).astype(np.int32)
+        built = []
+        try:
+            for E.KernelMap.plan_policy in (1, 2):
+                x = E.SparseTensor(torch.ones((rows, channels), device="cuda", dtype=torch.bfloat16), torch.from_numpy(c).cuda())
+                layer = E.RiemannConvolution(channels, channels, kernel_size=3, dimension=3).cuda().bfloat16()
+                from riemannengine_b200 import capi
+                before = capi.lib().rmn_launch_count()
+                layer(layer(x))
+                built.append(capi.lib().rmn_launch_count() - before)
+        finally:
+            E.KernelMap.plan_policy = 0
+        assert built[0] == built[1], (rows, channels)
