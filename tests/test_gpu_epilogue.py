@@ -1,4 +1,6 @@
 """What the kernels do behind the sum: ReLU, residual and folded batch norm of the convolutions and the affine pass."""
+import ctypes
+
 import pytest
 import torch
 
@@ -61,3 +63,57 @@ def test_network_shows_a_nan_in_its_input_with_and_without_gradients():
     with torch.no_grad():
         got = net(C.SparseTensor(feats, coords)).F.isnan()
     assert bool(want.any()) and torch.equal(got, want)
+
+
+class _Fold(ctypes.Structure):   # rmn_bn_fold of include/rmn_b200.h
+    _fields_ = [(n, ctypes.c_void_p) for n in ("mean", "var", "gamma", "beta", "conv_bias")] + [
+        ("param_dtype", ctypes.c_int), ("eps", ctypes.c_float), ("scale", ctypes.c_void_p), ("shift", ctypes.c_void_p)]
+
+
+# single 64-column blocks (up to 74 row tiles; the second and fourth block of the columns among them) and super-tiles, rows
+# around a tile's edge, narrower weights, every absent parameter, both parameter types
+@pytest.mark.parametrize("n,w_in,w_out,c_in,c_out,params,dtype,relu", [
+    (1, 64, 64, 64, 64, "mvgbc", torch.float32, 1), (127, 64, 128, 64, 128, "mvgbc", torch.bfloat16, 1),
+    (129, 100, 250, 128, 256, "mv", torch.float32, 0), (257, 128, 256, 128, 256, "mvg", torch.bfloat16, 1),
+    (20_003, 128, 128, 128, 128, "mvb", torch.float32, 1), (20_003, 33, 20, 64, 32, "mvgbc", torch.bfloat16, 0),
+    (60_001, 256, 256, 256, 256, "mvgbc", torch.float32, 1), (100_003, 32, 64, 32, 64, "mvc", torch.float32, 1),
+])
+def test_folded_batch_norm_and_residual_match_float64(n, w_in, w_out, c_in, c_out, params, dtype, relu):
+    from riemannengine_b200 import capi, ops
+    K = 3
+    g = torch.Generator(device="cuda").manual_seed(n)
+    nbr = torch.randint(0, n, (K, n), generator=g, dtype=torch.int32, device="cuda")
+    nbr[torch.rand((K, n), generator=g, device="cuda") >= 0.6] = -1
+    feats = torch.zeros((n, c_in), device="cuda", dtype=torch.bfloat16)
+    feats[:, :w_in] = torch.randn((n, w_in), generator=g, device="cuda")
+    w = (torch.randn((K, w_in, w_out), generator=g, device="cuda") / w_in ** 0.5).bfloat16()
+    add = torch.randn((n, c_out), generator=g, device="cuda").bfloat16()
+    values = {"m": torch.randn(w_out, generator=g, device="cuda").to(dtype), "v": torch.rand(w_out, generator=g, device="cuda").add(0.5).to(dtype),
+              "g": torch.randn(w_out, generator=g, device="cuda").to(dtype), "b": torch.randn(w_out, generator=g, device="cuda").to(dtype),
+              "c": torch.randn(w_out, generator=g, device="cuda").to(dtype)}
+    given = [values[p].data_ptr() if p in params else None for p in "mvgbc"]
+    vectors = torch.full((2, c_out), 7.0, device="cuda")
+    fold = _Fold(*given, capi.F32 if dtype == torch.float32 else capi.BF16, 1e-5, vectors[0].data_ptr(), vectors[1].data_ptr())
+    lib = capi.lib()
+    image = torch.empty(lib.rmn_conv_weight_image_bytes(K, c_in, c_out, capi.BF16), dtype=torch.uint8, device="cuda")
+    capi.check(lib.rmn_conv_weight_image(ops._ptr(w), K, w_in, w_out, c_in, c_out, capi.BF16, 0, 0, ctypes.byref(fold),
+                                         ops._ptr(image), ops._stream()), "rmn_conv_weight_image")
+    out = torch.empty((n, c_out), dtype=torch.bfloat16, device="cuda")
+    capi.check(lib.rmn_conv_forward_image(ops._ptr(feats), n, c_in, ops._ptr(image), K, c_out, ops._ptr(nbr), None, n,
+                                          ops._ptr(out), vectors[0].data_ptr(), vectors[1].data_ptr(), ops._ptr(add), relu,
+                                          ops._stream()), "rmn_conv_forward_image")
+    d = {p: values[p].double() if p in params else torch.full((w_out,), 1.0 if p == "g" else 0.0, device="cuda").double()
+         for p in "mvgbc"}
+    scale = d["g"] / torch.sqrt(d["v"] + 1e-5)
+    shift = d["b"] + (d["c"] - d["m"]) * scale
+    assert torch.allclose(vectors[0, :w_out].double(), scale, rtol=1e-5, atol=1e-6)
+    assert torch.allclose(vectors[1, :w_out].double(), shift, rtol=1e-5, atol=1e-5)
+    want = torch.zeros((n, w_out), dtype=torch.float64, device="cuda")
+    for k in range(K):
+        hit = nbr[k] >= 0
+        want[hit] += feats[nbr[k][hit].long()][:, :w_in].double() @ w[k].double()
+    want = want * scale + shift + add[:, :w_out].double()
+    if relu:
+        want = torch.relu(want)
+    # fp32 sums rounded to bf16 once: 2^-9 of a value, and the sum's own error
+    assert bool(((out[:, :w_out].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4 * want.abs().max()).all())

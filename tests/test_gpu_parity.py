@@ -314,7 +314,8 @@ def test_self_map_builder_equals_general_builder(gpu, D, ks, dil, n):
 def test_tma_gather4_producers_match_cp_async(gpu, monkeypatch):
     """The optional TMA (tile::gather4) producers of the tensor-core kernel give the same
     output as the default cp.async producers, bit for bit (same MMA order)."""
-    from riemannengine_b200 import ops, synthetic
+    from riemannengine_b200 import capi, ops, synthetic
+    from tests.test_gpu_plain_conv import _forward, _input_gradient
     from tests.gpu_backend import dev_coords
     c = synthetic.indoor_scene(91, 30000)
     c = np.concatenate([np.zeros((len(c), 1), np.int32), c], 1)
@@ -325,11 +326,11 @@ def test_tma_gather4_producers_match_cp_async(gpu, monkeypatch):
         x = torch.randn(len(c), c_in, device="cuda", generator=g).bfloat16()
         w = (torch.randn(27, c_in, c_out, device="cuda", generator=g) * 0.05).bfloat16()
         monkeypatch.delenv("RMN_B200_CONV_TMA", raising=False)
-        y0 = ops.conv_forward(x, w, nbr)
-        d0 = ops.conv_backward_input(y0, w, ops.kmap_transpose(nbr, len(c)))
+        y0 = _forward(x, w, nbr, capi.BF16)
+        d0 = _input_gradient(y0, w, ops.kmap_transpose(nbr, len(c)), capi.BF16)
         monkeypatch.setenv("RMN_B200_CONV_TMA", "1")
-        y1 = ops.conv_forward(x, w, nbr)
-        d1 = ops.conv_backward_input(y0, w, ops.kmap_transpose(nbr, len(c)))
+        y1 = _forward(x, w, nbr, capi.BF16)
+        d1 = _input_gradient(y0, w, ops.kmap_transpose(nbr, len(c)), capi.BF16)
         assert torch.equal(y0, y1) and torch.equal(d0, d1)
     monkeypatch.delenv("RMN_B200_CONV_TMA", raising=False)
     assert capi_status_ok()
