@@ -33,6 +33,7 @@ UNIT = "Mvoxels/s"
 N_SCENES, N_VOXELS = 8, 150_000
 C_IN, C_OUT, KSIZE = 64, 64, 3
 K_VOL = KSIZE ** 3
+WIDE = 128   # channels of the layer on which convolution plans are measured
 CPU_SAMPLE_SCENES = N_SCENES  # the reference arm runs the whole batch of one rank
 
 
@@ -318,10 +319,9 @@ def run_extras(args, C, dev, rank, world, coords, feats, weights_np, res, xf, co
     # the phases alone, on the cached map (device events, no host synchronisation in between)
     gy = grad_out
     wk = conv.kernel.detach()
-    plan = ops.conv_plan_build(res.nbr, ops.region_offsets(0, [KSIZE] * 3, [1] * 3, [1] * 3))
     dw = ops.conv_backward_weight(xf, gy, res.nbr)
-    fns = [lambda: ops.conv_forward(xf, wk, res.nbr, plan=plan),
-           lambda: ops.conv_backward_input(gy, wk.flip(0), res.nbr, plan=plan),
+    fns = [lambda: ops.conv_forward(xf, wk, res.nbr),
+           lambda: ops.conv_backward_input(gy, wk.flip(0), res.nbr),
            lambda: ops.conv_backward_weight(xf, gy, res.nbr),
            lambda: C.allreduce_gradients([dw])]
     marks = [[torch.cuda.Event(enable_timing=True) for _ in range(len(fns) + 1)] for _ in range(8)]
@@ -336,15 +336,14 @@ def run_extras(args, C, dev, rank, world, coords, feats, weights_np, res, xf, co
         "workload": "headline batch, 3^3 64->64 bf16: hash insert + kernel map + forward + backward (dX, dW) + "
                     "weight-gradient all-reduce, fresh manager every step, C++ host layer",
         "ms_per_step": ms_all, "mvoxels_per_s": vox_all / (ms_all / 1e3) / 1e6, "steps": steps,
-        "phases_ms": {"forward_planned": med[0], "input_gradient_planned": med[1], "weight_gradient": med[2],
+        "phases_ms": {"forward": med[0], "input_gradient": med[1], "weight_gradient": med[2],
                       "allreduce_alone": med[3] if world > 1 else 0.0},
-        "phases_note": "each phase timed alone on a cached map with a convolution plan; the step builds a fresh map, "
-                       "for which the plan policy (two passes of one 64->64 layer) builds no plan",
+        "phases_note": "each phase timed alone on a cached map; layers of 64 channels take no convolution plan",
         "allreduce_bytes": int(dw.numel() * 4) if world > 1 else 0,
         "allreduce": ("one ncclAllReduce per layer on a second stream behind the weight-gradient kernel, "
                       "overlapping the input-gradient kernel") if world > 1 else "single rank: none",
     }
-    del tfeats, grad_out, dw, plan
+    del tfeats, grad_out, dw
 
     # ---- the other configurations ---------------------------------------------------------------------
     configs = {}
@@ -663,25 +662,29 @@ def run_product(args) -> None:
         barrier()
         e2e_ms = g0.elapsed_time(g1)
 
-        # ---- convolution plan: build time and the planned (cached-map) forward ---------------------
-        plan_marks = [[torch.cuda.Event(enable_timing=True) for _ in range(3)] for _ in range(reps + 2)]
+        # ---- convolution plan: build time and what it saves a layer wide enough to use one --------------
+        plan_marks = [[torch.cuda.Event(enable_timing=True) for _ in range(4)] for _ in range(reps + 2)]
         plan = ops.conv_plan_build(res.nbr, offsets)
+        wide_x = torch.randn((n_unique, WIDE), device=dev).bfloat16()
+        wide_w = (torch.randn((K_VOL, WIDE, WIDE), device=dev) / (K_VOL * WIDE) ** 0.5).bfloat16()
         for rep in plan_marks:
             rep[0].record()
             ops.conv_plan_build(res.nbr, offsets)
             rep[1].record()
-            ops.conv_forward(xf, conv.kernel, res.nbr, plan=plan)
+            planned = ops.conv_forward(wide_x, wide_w, res.nbr, plan=plan)
             rep[2].record()
+            plain = ops.conv_forward(wide_x, wide_w, res.nbr)
+            rep[3].record()
         torch.cuda.synchronize()
-        t_plan = statistics.median(rep[0].elapsed_time(rep[1]) for rep in plan_marks[2:])
-        t_fwd_planned = statistics.median(rep[1].elapsed_time(rep[2]) for rep in plan_marks[2:])
-        assert torch.equal(ops.conv_forward(xf, conv.kernel, res.nbr, plan=plan), ops.conv_forward(xf, conv.kernel, res.nbr))
-        # fraction of (512-row super-tile, offset) stages the planned kernel skips
+        t_plan, t_fwd_planned, t_fwd_wide = (
+            statistics.median(rep[i].elapsed_time(rep[i + 1]) for rep in plan_marks[2:]) for i in range(3))
+        assert torch.equal(planned, plain)
+        del wide_x, planned, plain
+        # (128-row tile, offset) pairs with any neighbour: the planned kernel runs no others
         n_pos = (n_unique + 511) // 512 * 512
-        tile_masks = plan[256 + ((n_pos * 4 + 255) & ~255):][:n_pos // 128 * 4].view(torch.int32).view(-1, 4)
-        st_mask = tile_masks[:, 0] | tile_masks[:, 1] | tile_masks[:, 2] | tile_masks[:, 3]
-        stages_run = int(sum(int(((st_mask >> k) & 1).sum()) for k in range(K_VOL)))
-        stage_fraction = stages_run / float(st_mask.numel() * K_VOL)
+        tile_masks = plan[256 + ((n_pos * 4 + 255) & ~255):][:n_pos // 128 * 4].view(torch.int32)
+        stages_run = int(sum(int(((tile_masks >> k) & 1).sum()) for k in range(K_VOL)))
+        stage_fraction = stages_run / float(tile_masks.numel() * K_VOL)
 
     extras = run_extras(args, cpp_host, dev, rank, world, coords, feats, weights_np, res, xf, conv) \
         if cpp_host is not None and not args.no_extras else {}
@@ -719,8 +722,8 @@ def run_product(args) -> None:
     bytes_kmap = n_unique * 4 * W + n_unique * K_VOL * 32 + 8 * total_pairs
     phases = {"hash_insert_ms": t_hash, "kmap_probe_ms": t_kmap, "kmap_probe_general_ms": t_kmap_general,
               "kmap_pairs_ms": t_pairs, "conv_fwd_ms": t_fwd, "conv_plan_build_ms": t_plan,
-              "conv_fwd_planned_ms": t_fwd_planned}
-    planned_tflops = flops / (t_fwd_planned / 1e3) / 1e12
+              f"conv{WIDE}_fwd_ms": t_fwd_wide, f"conv{WIDE}_fwd_planned_ms": t_fwd_planned}
+    planned_tflops = 2.0 * total_pairs * WIDE * WIDE / (t_fwd_planned / 1e3) / 1e12
     fwd_tflops = flops / (t_fwd / 1e3) / 1e12
     kmap_gbs = bytes_kmap / ((t_kmap + t_pairs) / 1e3) / 1e9
     hash_gbs = bytes_hash / (t_hash / 1e3) / 1e9
@@ -775,15 +778,16 @@ def run_product(args) -> None:
                                     / peaks["hbm_gbs"]},
             "conv_forward": {"bound": "tensor", "achieved": fwd_tflops, "peak": peaks["bf16_tflops"],
                              "unit": "TFLOP/s", "frac": fwd_tflops / peaks["bf16_tflops"],
-                             "note": "first use of a kernel map (what the timed step runs): no plan"},
-            # the same layer on a map that has a convolution plan (second and later layers on a map, the
-            # input-gradient pass): offsets at which no row of a 512-row super-tile has a neighbour are skipped
+                             "note": "what the timed step runs; layers of 64 channels take no convolution plan"},
+            # a layer of WIDE -> WIDE channels on the same map with its plan: (128-row tile, offset) pairs without
+            # any neighbour are skipped
             "conv_forward_planned": {"bound": "tensor", "achieved": planned_tflops, "peak": peaks["bf16_tflops"],
                                      "unit": "TFLOP/s", "frac": planned_tflops / peaks["bf16_tflops"],
                                      "traffic": captured_traffic("conv_forward_planned"),
+                                     "layer": f"{WIDE}->{WIDE}", "unplanned_ms": t_fwd_wide,
                                      "stages_run_fraction": stage_fraction,
                                      # MMAs issued (zero rows included) against the measured peak
-                                     "executed_frac": (2.0 * stages_run * 512 * C_IN * C_OUT)
+                                     "executed_frac": (2.0 * stages_run * 128 * WIDE * WIDE)
                                      / (t_fwd_planned / 1e3) / 1e12 / peaks["bf16_tflops"],
                                      "plan_build_ms": t_plan},
         },
@@ -888,7 +892,7 @@ def run_train(args) -> None:
 def run_kernels(args) -> None:
     """One pass over the kernels of the headline workload (for profilers: `ncu -k regex:<kernel> ...
     python bench.py --mode kernels`): table build, both kernel-map builders, pair lists, plan build, forward
-    (plain and planned), input gradient, weight gradient - `--steps` times each after one warm-up, no timing."""
+    (and a wide one with its plan), input gradient, weight gradient - `--steps` times each after one warm-up, no timing."""
     import torch
 
     from riemannengine_b200 import capi, ops
@@ -901,6 +905,8 @@ def run_kernels(args) -> None:
     w = torch.from_numpy(weights_np).to(dev).bfloat16()
     offsets = ops.region_offsets(capi.HYPER_CUBE, [KSIZE] * 3, [1] * 3, [1] * 3)
     gy = torch.randn(len(coords_np), C_OUT, device=dev).bfloat16()
+    wide_x = torch.randn((len(coords_np), WIDE), device=dev).bfloat16()
+    wide_w = (torch.randn((K_VOL, WIDE, WIDE), device=dev) / (K_VOL * WIDE) ** 0.5).bfloat16()
     for _ in range(1 + max(args.steps, 1)):
         table = ops.table_build(coords)
         res = ops.kmap_build(table, table.coords, offsets, self_map=True)
@@ -908,8 +914,8 @@ def run_kernels(args) -> None:
         res.pairs()
         plan = ops.conv_plan_build(res.nbr, offsets)
         ops.conv_forward(feats, w, res.nbr)
-        ops.conv_forward(feats, w, res.nbr, plan=plan)
-        ops.conv_backward_input(gy, w.flip(0), res.nbr, plan=plan)
+        ops.conv_forward(wide_x, wide_w, res.nbr, plan=plan)
+        ops.conv_backward_input(gy, w.flip(0), res.nbr)
         ops.conv_backward_weight(feats, gy, res.nbr)
     torch.cuda.synchronize()
     print(json.dumps({"mode": "kernels", "voxels": len(coords_np), "passes": 1 + max(args.steps, 1)}))

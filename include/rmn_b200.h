@@ -142,7 +142,7 @@ int rmn_segment_reduce(const float *d_feats, uint32_t n_rows, int channels, cons
  * rmn_table_build for callers that cannot allocate device memory. It has no
  * counterpart in the reference. Same inputs, outputs and results as
  * rmn_table_build, but there is no workspace argument: the build's scratch is
- * a fixed device array inside the library (4 MiB per GPU, held from the moment
+ * a fixed device array inside the library (4.2 MiB per GPU, held from the moment
  * the library is loaded on that GPU until the process exits).
  * Meant for hosts with a frozen memory plan (real-time loops where cudaMalloc
  * is banned because it synchronises the device and may fail mid-run) and for

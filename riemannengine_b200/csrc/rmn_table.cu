@@ -935,7 +935,7 @@ extern "C" int rmn_table_build(const int32_t* d_coords, uint32_t n_rows, int W, 
 // nowhere to put the build's scratch (slot-of-row array + block counters).
 // Here that scratch lives in a file-scope device array of fixed size, so the
 // call needs nothing beyond its inputs and outputs. The price is a hard row
-// limit and 4 MiB of device memory held by every GPU that loads the library.
+// limit and 4.2 MiB of device memory held by every GPU that loads the library.
 //
 // The host symbol below is only a handle: kernels must be given the device
 // address obtained with cudaGetSymbolAddress, which is looked up once per
