@@ -14,8 +14,14 @@
 // tcgen05.ld gives every lane 32 contiguous bytes of an output row; and W[k] arrives by one bulk copy per stage.
 //
 // Persistent CTAs, one per SM, over super-tiles of T x 128 output rows. 24 warps: 16 gather (four groups of four: group g
-// serves tile g % T), 1 MMA, 1 weights, 2 idle, 4 epilogue. Waits are bounded (g_tc_status), results are
-// bit-reproducible: every output row adds its offsets in ascending order, planned or not.
+// serves tile g % T), 2 MMA, 1 weights, 1 idle, 4 epilogue. A (tile, offset) stage costs the warp that issues its MMAs some 150
+// cycles of barrier, fence and commit latency beside 128 of math at 64 columns, and one such warp is what bound tables of few
+// entries. So two issue, each for half of the tiles; where a super-tile is a single tile of up to 64 columns, one takes its even
+// stages and one its odd ones, into accumulators of their own that the epilogue adds (SPLIT). Rows are fetched past the L1: a
+// hit there passes the load/store pipe in twice the wavefronts of a miss. us before and after both: 1.2 M rows of rooms 64 -> 64
+// 281 and 271, sorted by blocks 300 and 274, 32 -> 32 154 and 149; 240 000 lidar voxels 64 -> 64 57 and 51; 850 rows 256 -> 256
+// 21.5 and 19.6. Waits are bounded (g_tc_status), results are bit-reproducible: every accumulator adds its offsets in ascending
+// order, planned or not.
 //
 // Included by rmn_conv_tc.cu.
 #pragma once
@@ -32,8 +38,11 @@ struct TaCfg {
   static constexpr int T = T_;
   static constexpr int GROUPS = 4, PHASES = GROUPS / T;         // the PHASES groups of a tile take its stages in turn
   static constexpr int A_COLS = KB / 2;                         // tensor-memory columns of one A slot
-  static constexpr int ACC_BUFS = T * CC * 2 + GROUPS * 2 * A_COLS <= 512 ? 2 : 1;
-  static constexpr int ACC_COLS = T * CC * ACC_BUFS;
+  static constexpr int SPLIT = T == 1 && CC <= 64 ? 2 : 1;      // sums of a tile: even and odd stages apart, see the issuers
+  static constexpr int ISSUERS = T > 1 ? 2 : SPLIT;
+  static constexpr int SUM_COLS = T * SPLIT * CC;
+  static constexpr int ACC_BUFS = SUM_COLS * 2 + GROUPS * 2 * A_COLS <= 512 ? 2 : 1;
+  static constexpr int ACC_COLS = SUM_COLS * ACC_BUFS;
   static constexpr int FIT = (512 - ACC_COLS) / (GROUPS * A_COLS);
   static constexpr int SLOTS = FIT >= 4 ? 4 : 2;                // A slots per group
   static constexpr uint32_t B_BYTES = KB * CC * 2;
@@ -48,7 +57,7 @@ struct TaCfg {
 };
 
 // Registers: 768 threads x 80 at launch = 512 x 88 (gather) + 128 x 48 (MMA, weights) + 128 x 80 (epilogue)
-constexpr int kTaGatherWarps = 16, kTaMmaWarp = 16, kTaWeightWarp = 17, kTaEpWarp0 = 20;
+constexpr int kTaGatherWarps = 16, kTaMmaWarp = 16, kTaWeightWarp = 18, kTaEpWarp0 = 20;  // MMA: 16 and 17
 constexpr int kTaThreads = (kTaEpWarp0 + 4) * 32;
 constexpr int kTaGatherRegs = 88, kTaIssueRegs = 48;
 
@@ -159,6 +168,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
               const int32_t* __restrict__ perm, const uint32_t* __restrict__ tile_mask) {
   using C = TaCfg<CR, CC, T_>;
   constexpr int KB = C::KB, NKB = C::NKB, OPS = C::OPS, T = C::T, G = C::GROUPS, PH = C::PHASES, SLOTS = C::SLOTS, BST = C::B_STAGES;
+  constexpr int NI = C::ISSUERS, SPLIT = C::SPLIT, NT = T > 1 ? T / NI : 1;  // NT: tiles of an issuer
   constexpr int KSTEP = PH > NKB ? PH / NKB : 1;  // every KSTEP-th offset belongs to one group of a tile ...
   constexpr int NB = NKB > PH ? NKB / PH : 1;     // ... with NB of its channel blocks, PH apart
   constexpr int NBLK = CC < 64 ? CC : 64;         // columns of one atom
@@ -184,14 +194,14 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   if (tid == 0) {
     for (int s = 0; s < BST; ++s) {
       mbar_init(&b_full[s], 1);
-      mbar_init(&b_empty[s], 1);
+      mbar_init(&b_empty[s], NI / SPLIT);
     }
     for (int s = 0; s < G * SLOTS; ++s) {
       mbar_init(&a_full[s], 4);
       mbar_init(&a_empty[s], 1);
     }
     for (int a = 0; a < C::ACC_BUFS * T; ++a) {
-      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_full[a], SPLIT);
       mbar_init(&acc_empty[a], 128);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -340,11 +350,12 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   } else if (warp < kTaEpWarp0) {
     // (one instruction for the whole warpgroup, ahead of its roles)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTaIssueRegs));
-    if (warp == kTaMmaWarp) {
+    if (warp < kTaMmaWarp + NI) {
       // ------------------------------ MMA issuer -----------------------------------------
-      // Warp-uniform code, one elected lane issues. B descriptors differ only in the start address field. Masks of a plan
-      // come through a warp vote (the ballot of "bit `lane` of the mask" is the mask itself), whose result is warp-uniform
-      // by construction, so that branches on it keep the loop on the uniform datapath.
+      // The warp's tiles are t0 .. t0 + T / NI - 1. Warp-uniform code, one elected lane issues. B descriptors differ only in the
+      // start address field. Masks of a plan come through a warp vote (the ballot of "bit `lane` of the mask" is the mask
+      // itself), whose result is warp-uniform by construction, so that branches on it keep the loop on the uniform datapath.
+      const int issuer = warp - kTaMmaWarp, t0 = SPLIT > 1 ? 0 : issuer * NT;
       constexpr uint32_t IDESC = instr_desc(kTileM, CC, true);
       constexpr uint64_t B_DESC0 = smem_desc_sw_const(KB * SWB, 8 * SWB, SWB == 128 ? 2u : 4u);
       constexpr uint32_t B_DESC_HI = (uint32_t)(B_DESC0 >> 32);
@@ -352,12 +363,15 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       uint32_t b_it = 0, tile_iter = 0;
       for (uint32_t st = blockIdx.x; st < n_super && !timed_out; st += gridDim.x, ++tile_iter) {
         const uint32_t buf = tile_iter % C::ACC_BUFS, acc_ph = (tile_iter / C::ACC_BUFS) & 1u;
-        uint32_t m[T], todo = 0;
+        uint32_t m[NT] = {}, todo = 0;
         if constexpr (kPlan) {
   #pragma unroll
           for (int t = 0; t < T; ++t) {
-            m[t] = __ballot_sync(0xFFFFFFFFu, (__ldg(tile_mask + (size_t)st * T + t) >> lane) & 1u);
-            todo |= m[t];
+            const uint32_t v = __ballot_sync(0xFFFFFFFFu, (__ldg(tile_mask + (size_t)st * T + t) >> lane) & 1u);
+            todo |= v;
+  #pragma unroll
+            for (int i = 0; i < NT; ++i)
+              if (t == t0 + i) m[i] = v;
           }
         }
         uint32_t started = 0, odd = 0;  // per tile: an MMA has been issued; parity of its offset count
@@ -368,13 +382,15 @@ __global__ void __launch_bounds__(kTaThreads, 1)
           }
   #pragma unroll
           for (int kb = 0; kb < NKB; ++kb, ++b_it) {
+            if (SPLIT > 1 && ((k * NKB + kb) & 1) != issuer) continue;
             const uint32_t bs = b_it % BST;
             if (!mbar_wait(&b_full[bs], (b_it / BST) & 1u)) { timed_out = true; goto mma_done; }
             const uint32_t b_lo = ((smem_base + bs * C::B_BYTES) >> 4) + (uint32_t)(B_DESC0 & 0xFFFFFFFFu);
   #pragma unroll
-            for (int t = 0; t < T; ++t) {
+            for (int i = 0; i < NT; ++i) {
+              const int t = t0 + i;
               if constexpr (kPlan) {
-                if (!((m[t] >> k) & 1u)) continue;
+                if (!((m[i] >> k) & 1u)) continue;
               }
               const uint32_t g = t + T * (KSTEP > 1 ? (kPlan ? (odd >> t) & 1u : (uint32_t)k % KSTEP) * NKB + kb : kb % PH);
               const uint32_t c = (cnts >> (8 * g)) & 7u, s = c % SLOTS;
@@ -382,7 +398,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
               if (!mbar_wait(&a_full[g * SLOTS + s], (c / SLOTS) & 1u)) { timed_out = true; goto mma_done; }
               if (!begun && !mbar_wait(&acc_empty[buf * T + t], acc_ph ^ 1u)) { timed_out = true; goto mma_done; }
               tc_fence_after();
-              const uint32_t d_tmem = tmem_base + (buf * T + t) * CC;
+              const uint32_t d_tmem = tmem_base + (SPLIT > 1 ? buf * 2 + issuer : buf * T + t) * CC;
               const uint32_t a_tmem = tmem_base + C::ACC_COLS + (g * SLOTS + s) * C::A_COLS;
   #pragma unroll
               for (int j = 0; j < KB / 16; ++j) {
@@ -399,7 +415,8 @@ __global__ void __launch_bounds__(kTaThreads, 1)
           }
         }
   #pragma unroll
-        for (int t = 0; t < T; ++t) {
+        for (int i = 0; i < NT; ++i) {
+          const int t = t0 + i;
           if (!((started >> t) & 1u) && !mbar_wait(&acc_empty[buf * T + t], acc_ph ^ 1u)) { timed_out = true; goto mma_done; }
           tc_commit_elect(&acc_full[buf * T + t]);
         }
@@ -467,7 +484,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
           const int ch = nb * NBLK + u * (NBLK / 4);  // this lane's first channel
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const uint32_t taddr = tmem_base + ((quad * 32u + h * 16u) << 16) + (buf * T + t) * CC + nb * NBLK;
+            const uint32_t taddr = tmem_base + ((quad * 32u + h * 16u) << 16) + (buf * T + t) * SPLIT * CC + nb * NBLK;
             uint32_t w0[NW], w1[NW];  // rows 2 h and 2 h + 1: first what is added to them, then the result
             if (ep_add) {
               auto fetch = [&](uint32_t row, uint32_t (&w)[NW]) {
@@ -486,7 +503,15 @@ __global__ void __launch_bounds__(kTaThreads, 1)
               uint32_t r[16];
               if (tile_any) {
                 tc_ld16x256b(taddr + q * 32, r);
-                tc_wait_ld();
+                if (SPLIT > 1 && n_off * NKB > 1) {  // the odd stages' sum
+                  uint32_t odd[16];
+                  tc_ld16x256b(taddr + CC + q * 32, odd);
+                  tc_wait_ld();
+#pragma unroll
+                  for (int v = 0; v < 16; ++v) r[v] = __float_as_uint(__uint_as_float(r[v]) + __uint_as_float(odd[v]));
+                } else {
+                  tc_wait_ld();
+                }
               } else {
 #pragma unroll
                 for (int v = 0; v < 16; ++v) r[v] = 0u;

@@ -45,7 +45,7 @@ namespace rmn {
 // lets a host or a test tell that a convolution ran on the tensor cores rather than on the SIMT kernels.
 static std::atomic<unsigned long long> g_tc_launches{0};
 unsigned long long tc_launch_count() { return g_tc_launches.load(std::memory_order_relaxed); }
-static inline void count_tc_launch() { g_tc_launches.fetch_add(1, std::memory_order_relaxed); }
+void count_tc_launch() { g_tc_launches.fetch_add(1, std::memory_order_relaxed); }
 
 // Sticky status word of the tensor-core kernels, one per device (not per stream): a kernel whose
 // bounded wait ran out stores RMN_ERR_TIMEOUT here and returns early. Hosts read it (and clear it)
@@ -53,15 +53,6 @@ static inline void count_tc_launch() { g_tc_launches.fetch_add(1, std::memory_or
 __device__ uint32_t g_tc_status = 0;
 
 namespace tc {
-
-constexpr int kTileM = 128;
-
-// chunk position of 16-byte chunk c in row r of a swizzled image with SW-byte lines
-template <int SW>
-__device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t c) {
-  if constexpr (SW == 128) return c ^ (r & 7u);
-  else return c ^ ((r >> 1) & 3u);
-}
 
 template <int CR, int CC>
 struct Cfg {

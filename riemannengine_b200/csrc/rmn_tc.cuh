@@ -179,14 +179,14 @@ __device__ __forceinline__ void tc_st16x64b(uint32_t taddr, const uint32_t (&r)[
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // 32 bytes of global memory into r[FIRST .. FIRST + 7], zeros where `ok` is false. volatile keeps the loads where they
-// are issued.
+// are issued. (Past the L1, see rmn_conv_ta.cuh.)
 template <int FIRST, int N>
 __device__ __forceinline__ void ldg32_or_zero(const void* p, bool ok, uint32_t (&r)[N]) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %9, 0;\n\t"
       "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
       "mov.b32 %4, 0;\n\tmov.b32 %5, 0;\n\tmov.b32 %6, 0;\n\tmov.b32 %7, 0;\n\t"
-      "@p ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+      "@p ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
       : "=r"(r[FIRST]), "=r"(r[FIRST + 1]), "=r"(r[FIRST + 2]), "=r"(r[FIRST + 3]), "=r"(r[FIRST + 4]), "=r"(r[FIRST + 5]),
         "=r"(r[FIRST + 6]), "=r"(r[FIRST + 7])
       : "l"(p), "r"((int)ok));
@@ -210,6 +210,15 @@ __device__ __forceinline__ void tc_ld16x256b(uint32_t taddr, uint32_t (&r)[16]) 
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+constexpr int kTileM = 128;
+
+// chunk position of 16-byte chunk c in row r of a swizzled image with SW-byte lines
+template <int SW>
+__device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t c) {
+  if constexpr (SW == 128) return c ^ (r & 7u);
+  else return c ^ ((r >> 1) & 3u);
+}
 
 // Shared-memory matrix descriptor, no swizzle: start address, leading-dimension and
 // stride-dimension byte offsets (all >> 4), descriptor version 1.
