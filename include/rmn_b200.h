@@ -405,6 +405,22 @@ int rmn_conv_transpose_weights(const void *d_weights, int K, int c_in, int c_out
                                void *d_out, void *stream);
 
 /*
+ * fp32 convolution on the tensor cores: every number as three bf16 parts, products of parts whose error is that of fp32,
+ * sums in fp32 (results that are not finite, or below 2^-90, are computed with fp32 multiply-adds). Bytes of scratch (the
+ * prepared weights) of rmn_conv_forward_f32, 0 where it does not serve (use rmn_conv_forward): c_in a multiple of 8 from 16
+ * on, c_out a multiple of 4.
+ * rmn_conv_forward_f32: rmn_conv_forward_fused for fp32 (d_feats 32-byte aligned, d_weights, d_out and d_scratch 16-byte
+ * aligned: RMN_ERR_UNSUPPORTED otherwise). transpose: d_weights is [K, c_out, c_in], each offset's matrix used transposed;
+ * reverse: offset k uses d_weights[K - 1 - k]. With both, the input gradient of a point-symmetric self map is this call on
+ * grad_out over the forward table.
+ */
+size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, int c_out);
+int rmn_conv_forward_f32(const float *d_feats, uint32_t n_src, int c_in, const float *d_weights, int K, int c_out,
+                         int transpose, int reverse, const int32_t *d_nbr, uint32_t n_dst, float *d_out,
+                         const float *d_scale, const float *d_shift, int relu, void *d_scratch,
+                         size_t scratch_bytes, void *stream);
+
+/*
  * Prepared weights for the fastest bf16 kernels. rmn_conv_weight_image_bytes: size of the image of [K, c_in, c_out]
  * weights, 0 when no such kernel covers the dtype and channel counts (use the plain entry points then).
  * rmn_conv_weight_image builds it (one small kernel) from [K, w_in, w_out] weights, w_in <= c_in and w_out <= c_out: the

@@ -1,0 +1,576 @@
+// fp32 convolution on the tensor cores (sm_100a): the forward pass, and the input gradient on transposed weights.
+//   out[j] = sum_k F[nbr[k][j]] . W[k]
+//
+// An fp32 number is the sum of three bf16 numbers x0 + x1 + x2 of eight significant bits each, every one the nearest to what the
+// ones before it leave. Of the nine products of the parts of two numbers the six with i + j <= 2 are multiplied, the smallest
+// first; the others lie below 2^-24 of the product. Tensor memory adds with truncation, so no sum stays there for long: after
+// every stage (32 channels of an offset) it is read back and added, rounded to nearest, to sums in registers. Error against 64
+// bits (2-norm) here / by k_conv_f32, whose sums of an offset are chains of multiply-adds: 101 930 rows of a shell, 32 -> 32
+// 0.99e-7 / 1.19e-7, 64 -> 64 1.25e-7 / 1.56e-7; rooms at 46 %, 32 -> 64 0.90e-7 / 1.19e-7; lidar at 4 % 0.57e-7 / 1.04e-7.
+// (Read back every other stage, it is 2.7e-7.)
+//
+// Sums that are not finite are computed again with fp32 multiply-adds (exact_row): infinities and NaN do not survive the
+// split (inf - inf), nor do numbers that round to infinity in bf16. So are sums below 2^-90, where the third parts leave the
+// range of bf16.
+//
+// The kernel is built like k_conv_ta (rmn_conv_ta.cuh): gather warps fetch rows into registers, split them there and store the
+// parts into tensor memory as the A operand; W[k] comes as a prepared image by bulk copies. 20 warps: 8 gather (two groups of
+// four), 2 MMA, 1 weights, 1 idle, 8 drain. Group g, issuer g and accumulators g make up stream g: one of the two row tiles of a
+// super-tile (T = 2), or every other stage of a single one (T = 1). Waits are bounded, results bit-reproducible.
+//
+// What bounds it is the gather warps' chain of fetching, splitting (eleven instructions per two numbers) and storing a stage,
+// some 600 cycles, against 12 MMAs of 16 to 32 cycles. us with the weight image / k_conv_f32: 101 930 rows at 66 %, 32 -> 32
+// 59 / 164, 64 -> 64 124 / 519; 48 503 rows at 45 %, 32 -> 64 41 / 117, 64 -> 32 59 / 140; 119 755 lidar voxels, 32 -> 32 53 / 51,
+// 64 -> 64 118 / 110 (k_conv_f32 goes with the rows that exist; blocks of 32 rows none of which exists are not split here: 66
+// and 140 without).
+#include "rmn_common.cuh"
+#include "rmn_tc.cuh"
+
+#include <cuda_bf16.h>
+
+namespace rmn {
+
+const uint32_t* tc_status_device_address();  // rmn_conv_tc.cu
+void count_tc_launch();
+
+namespace tc {
+
+template <int CC, int T_>
+struct F3Cfg {
+  static constexpr int T = T_, STREAMS = 2, PARTS = 3;
+  static constexpr int KB = 32;                         // reduction channels of a stage
+  static constexpr int A_COLS = PARTS * KB / 2;         // tensor-memory columns of one A slot
+  static constexpr int ACC_BUFS = 2, ACC_COLS = STREAMS * ACC_BUFS * CC;
+  static constexpr int FIT = (512 - ACC_COLS) / (STREAMS * A_COLS);
+  static constexpr int SLOTS = FIT >= 4 ? 4 : 2;        // A slots per stream
+  static constexpr uint32_t PART_BYTES = KB * CC * 2, B_BYTES = PARTS * PART_BYTES;
+  static constexpr int B_STAGES = 8;
+  static constexpr uint32_t BAR_OFFSET = B_STAGES * B_BYTES;
+  static constexpr int BARRIERS = 2 * B_STAGES + 2 * STREAMS * SLOTS + 2 * STREAMS * ACC_BUFS;
+  static constexpr uint32_t EP_OFFSET = BAR_OFFSET + 1024;  // 2 * CC floats of epilogue scale / shift
+  static constexpr uint32_t SMEM = EP_OFFSET + 2 * CC * 4;
+  static_assert(FIT >= 2 && BARRIERS * 8 + 4 <= 1024 && (CC == 32 || CC == 64), "tensor / shared memory");
+};
+
+constexpr int kF3MmaWarp = 8, kF3WeightWarp = 10, kF3DrainWarp0 = 12, kF3Warps = 20, kF3Threads = kF3Warps * 32;
+// Registers: 640 threads x 96 at launch = 256 x 112 (gather) + 128 x 48 (MMA, weights) + 256 x 104 (drain)
+constexpr int kF3GatherRegs = 112, kF3IssueRegs = 48, kF3DrainRegs = 104;
+
+struct F3Args {
+  const float* src;      // [*, c_red]
+  const uint8_t* image;  // k_f3_image of w
+  const float* w;        // [K][c_red][c_col], transpose: [K][c_col][c_red]
+  const int32_t* nbr;
+  float* out;            // [n_dst, c_col]
+  const float* ep_scale;
+  const float* ep_shift;
+  uint32_t* status;
+  uint32_t n_dst, n_super;
+  int K, c_red, c_col, n_kb, transpose, reverse, relu;
+};
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t p;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(hi), "f"(lo));
+  return p;
+}
+// bf16 pair nearest to (lo, hi), which keep what is left
+__device__ __forceinline__ uint32_t take_part(float& lo, float& hi) {
+  const uint32_t p = pack_bf16(lo, hi);
+  asm("{\n\t.reg .b64 v, q;\n\t"
+      "mov.b64 v, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\t"
+      "sub.rn.f32x2 v, v, q;\n\tmov.b64 {%0, %1}, v;\n\t}"
+      : "+f"(lo), "+f"(hi)
+      : "f"(__uint_as_float(p << 16)), "f"(__uint_as_float(p & 0xFFFF0000u)));
+  return p;
+}
+
+// Order of the 32 channels of a stage along K (what the gather's loads and stores make of them), and of the CC columns of an
+// image (for the drain's loads, see n_channel in rmn_conv_ta.cuh).
+__device__ __forceinline__ constexpr uint32_t f3_k_channel(uint32_t p) {
+  return 16 * (p >> 4) + 8 * ((p >> 1) & 1u) + 2 * ((p >> 2) & 3u) + (p & 1u);
+}
+template <int CC>
+__device__ __forceinline__ constexpr uint32_t f3_n_channel(uint32_t p) {
+  return (CC / 4) * ((p >> 1) & 3u) + 2 * (p >> 3) + (p & 1u);
+}
+
+// Image of the weights: per stage (offset, 32-channel block) and block of CC columns the three parts, each the MN-major swizzled
+// operand of 32 lines. One thread per line and eight columns. reverse: offset k of the image is W[K - 1 - k].
+template <int CC>
+__global__ void __launch_bounds__(256) k_f3_image(const float* __restrict__ w, int K, int c_red, int c_col, int n_kb, int blocks,
+                                                  int transpose, int reverse, uint4* __restrict__ image) {
+  after_previous_kernel();
+  constexpr uint32_t CPL = CC / 8, CHUNKS = 32 * CPL;
+  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= (uint32_t)(K * n_kb * blocks) * CHUNKS) return;
+  const uint32_t block = i / CHUNKS, p = i % CHUNKS / CPL, c = i % CPL;
+  const int stage = (int)block / blocks, k = stage / n_kb, col0 = ((int)block % blocks) * CC;
+  const int ci = stage % n_kb * 32 + (int)f3_k_channel(p);
+  const float* wk = w + (size_t)(reverse ? K - 1 - k : k) * c_red * c_col;
+  float v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int co = col0 + (int)f3_n_channel<CC>(c * 8 + q);
+    v[q] = ci >= c_red || co >= c_col ? 0.f : __ldg(wk + (transpose ? (size_t)co * c_red + ci : (size_t)ci * c_col + co));
+  }
+  uint4* dst = image + (size_t)block * 3 * CHUNKS + p * CPL + swz<CC * 2>(p, c);
+#pragma unroll
+  for (int part = 0; part < 3; ++part)
+    dst[part * CHUNKS] = make_uint4(take_part(v[0], v[1]), take_part(v[2], v[3]), take_part(v[4], v[5]), take_part(v[6], v[7]));
+}
+
+// 32 channels of a gather warp's 32 rows: lane t holds channels 8 c .. 8 c + 7 and 16 + 8 c .. 16 + 8 c + 7 (c = t / 2 & 1) of row
+// t / 4 + 8 (t & 1) of each half of 16, see RowBlock in rmn_conv_ta.cuh. The registers keep their place until they are split.
+struct F3Rows {
+  uint32_t v[2][16];
+  bool any;  // (the same in all lanes) one of the rows exists
+  __device__ __forceinline__ void load(const float* __restrict__ src_lane, int c_red, int32_t idx, int kb, int lane) {
+    const int mine = (lane >> 2) + 8 * (lane & 1), ch = kb * 32 + 8 * ((lane >> 1) & 1);
+    any = __any_sync(0xFFFFFFFFu, idx >= 0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int32_t row = __shfl_sync(0xFFFFFFFFu, idx, h * 16 + mine);
+      const float* p = src_lane + (size_t)(uint32_t)row * (uint32_t)c_red + kb * 32;
+      ldg32_or_zero<0>(p, row >= 0 && ch < c_red, v[h]);
+      ldg32_or_zero<8>(p + 16, row >= 0 && ch + 16 < c_red, v[h]);
+    }
+  }
+  __device__ __forceinline__ void store_zeros(uint32_t taddr) const {  // (of rows none of which exists: v is zero)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      {
+        tc_st16x64b(taddr + ((uint32_t)(h * 16) << 16), v[h]);  // 32 columns, and the 16 behind them
+        uint32_t p[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p[i] = v[h][i];
+        tc_st16x64b(taddr + ((uint32_t)(h * 16) << 16) + 32, p);
+      }
+  }
+  __device__ __forceinline__ void split_store(uint32_t taddr) const {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[h][i]);
+#pragma unroll
+      for (int part = 0; part < 3; ++part) {
+        uint32_t p[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p[i] = take_part(x[2 * i], x[2 * i + 1]);
+        tc_st16x64b(taddr + ((uint32_t)(h * 16) << 16) + part * 16, p);
+      }
+    }
+  }
+};
+
+__device__ __forceinline__ float f3_finish(float v, float scale, float shift, int relu) {
+  v = fmaf(v, scale, shift);
+  return relu ? relu_f32(v) : v;
+}
+
+// One output row (columns col0 .. col0 + width - 1) by fp32 multiply-adds, by a whole warp
+__device__ __noinline__ void exact_row(const F3Args& a, uint32_t row, int col0, int width, const float* s_ep, int lane) {
+  for (int c = lane; c < width && col0 + c < a.c_col; c += 32) {
+    float sum = 0.f;
+    for (int k = 0; k < a.K; ++k) {
+      const int32_t idx = __ldg(a.nbr + (size_t)k * a.n_dst + row);
+      if (idx < 0) continue;
+      const float* x = a.src + (size_t)idx * a.c_red;
+      const float* w = a.w + (size_t)(a.reverse ? a.K - 1 - k : k) * a.c_red * a.c_col;
+      w += a.transpose ? (size_t)(col0 + c) * a.c_red : (size_t)(col0 + c);
+      const int step = a.transpose ? 1 : a.c_col;
+      float part = 0.f;
+      for (int ci = 0; ci < a.c_red; ++ci) part = fmaf(__ldg(x + ci), __ldg(w + (size_t)ci * step), part);
+      sum += part;
+    }
+    a.out[(size_t)row * a.c_col + col0 + c] = f3_finish(sum, s_ep[c], s_ep[width + c], a.relu);
+  }
+}
+
+// blockIdx.y: block of CC columns
+template <int CC, int T_>
+__global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant__ F3Args a) {
+  using C = F3Cfg<CC, T_>;
+  constexpr int T = T_, SLOTS = C::SLOTS, BST = C::B_STAGES, SWB = CC * 2;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* b_full = reinterpret_cast<uint64_t*>(smem + C::BAR_OFFSET);
+  uint64_t* b_empty = b_full + BST;
+  uint64_t* a_full = b_empty + BST;              // [stream][slot]
+  uint64_t* a_empty = a_full + 2 * SLOTS;        // [stream][slot]
+  uint64_t* acc_full = a_empty + 2 * SLOTS;      // [stream][buffer]
+  uint64_t* acc_empty = acc_full + 4;            // [stream][buffer]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 4);
+  float* s_ep = reinterpret_cast<float*>(smem + C::EP_OFFSET);  // scale | shift
+
+  // (uniform for the compiler, see k_conv_ta)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < BST; ++s) {
+      mbar_init(&b_full[s], 1);
+      mbar_init(&b_empty[s], T > 1 ? 2 : 1);
+    }
+    for (int s = 0; s < 2 * SLOTS; ++s) {
+      mbar_init(&a_full[s], 4);
+      mbar_init(&a_empty[s], 1);
+    }
+    for (int s = 0; s < 4; ++s) {
+      mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_empty[s], T > 1 ? 4 : 8);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+  }
+  // (tensor memory is taken behind the kernels before this one and ahead of the next: see release_next_kernel)
+  wait_previous_kernels();
+  if (warp == kF3MmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  const int col0 = (int)blockIdx.y * CC;
+  if (tid < CC) {
+    const bool in = col0 + tid < a.c_col;
+    s_ep[tid] = a.ep_scale && in ? __ldg(a.ep_scale + col0 + tid) : 1.f;
+    s_ep[CC + tid] = a.ep_shift && in ? __ldg(a.ep_shift + col0 + tid) : 0.f;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  release_next_kernel();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+  const uint32_t smem_base = smem_u32(smem);
+  const int n_stages = a.K * a.n_kb;
+  // stages of a stream per super-tile
+  auto stages_of = [&](int stream) { return T > 1 ? n_stages : (n_stages + 1 - stream) / 2; };
+  bool timed_out = false;
+
+  if (warp < kF3MmaWarp) {
+    // ------------------------------ gather ---------------------------------------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kF3GatherRegs));
+    constexpr int STEP = T > 1 ? 1 : 2;
+    const int g = warp >> 2, t = T > 1 ? g : 0;
+    const float* src_lane = a.src + 8 * ((lane >> 1) & 1);
+    const uint32_t a_base = tmem_base + C::ACC_COLS + g * SLOTS * C::A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t bars = smem_u32(a_full + g * SLOTS);  // full barriers; the empty ones lie 2 * SLOTS further
+
+    // Cursor over the table entries of this lane's rows and the channel blocks that go with them; kEnd behind the last one
+    constexpr int32_t kEnd = INT32_MIN;
+    uint32_t st = blockIdx.x;
+    int k = a.K, kb = 0, kb_next = 0;
+    const int32_t* entry = a.nbr;
+    bool row_ok = false, fresh = true;
+    auto next = [&]() -> int32_t {
+      for (;;) {
+        if (k < a.K) {
+          const int32_t v = row_ok ? __ldg(entry) : -1;
+          kb = kb_next;
+          kb_next += STEP;
+          while (kb_next >= a.n_kb) {
+            kb_next -= a.n_kb;
+            ++k;
+            entry += a.n_dst;
+          }
+          return v;
+        }
+        if (!fresh) st += gridDim.x;
+        fresh = false;
+        if (st >= a.n_super) {
+          fresh = true;  // stay here
+          return kEnd;
+        }
+        const uint32_t row = st * (kTileM * T) + t * kTileM + (warp & 3) * 32 + lane;
+        row_ok = row < a.n_dst;
+        entry = a.nbr + row;
+        k = 0;
+        kb_next = T > 1 ? 0 : g;
+        while (kb_next >= a.n_kb) {
+          kb_next -= a.n_kb;
+          ++k;
+          entry += a.n_dst;
+        }
+      }
+    };
+    // (entries are fetched four stages ahead, rows two, in windows unrolled by hand: see k_conv_ta)
+    uint32_t cnt = 0, zero = 0;  // zero: slots whose rows of this warp are zeros already
+    F3Rows b0, b1;
+    auto load = [&](F3Rows& b, int32_t idx, int block) { b.load(src_lane, a.c_red, idx, block, lane); };
+    auto arrive = [&]() {  // the block stored last has reached tensor memory
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + ((cnt - 1u) % SLOTS) * 8);
+    };
+    auto put = [&](const F3Rows& b) {
+      if (cnt) arrive();
+      const uint32_t s = cnt % SLOTS, ph = (cnt / SLOTS) & 1u;
+      ++cnt;
+      if (!mbar_wait(bars + (2 * SLOTS + s) * 8, ph ^ 1u)) timed_out = true;
+      tc_fence_after();
+      __syncwarp();
+      if (b.any) {
+        b.split_store(a_base + s * C::A_COLS);
+        zero &= ~(1u << s);
+      } else if (!((zero >> s) & 1u)) {
+        b.store_zeros(a_base + s * C::A_COLS);
+        zero |= 1u << s;
+      }
+    };
+    int32_t w0, w1, w2, w3;
+    int x0, x1, x2, x3;
+    w0 = next(), x0 = kb;
+    w1 = next(), x1 = kb;
+    load(b0, w0, x0);
+    load(b1, w1, x1);
+    bool live0 = w0 != kEnd, live1 = w1 != kEnd;
+    w2 = next(), x2 = kb;
+    w3 = next(), x3 = kb;
+    w0 = next(), x0 = kb;
+    w1 = next(), x1 = kb;
+    while (live0) {
+      put(b0);
+      load(b0, w2, x2);
+      live0 = w2 != kEnd;
+      w2 = next(), x2 = kb;
+      if (!live1) break;
+      put(b1);
+      load(b1, w3, x3);
+      live1 = w3 != kEnd;
+      w3 = next(), x3 = kb;
+      if (!live0) break;
+      put(b0);
+      load(b0, w0, x0);
+      live0 = w0 != kEnd;
+      w0 = next(), x0 = kb;
+      if (!live1) break;
+      put(b1);
+      load(b1, w1, x1);
+      live1 = w1 != kEnd;
+      w1 = next(), x1 = kb;
+      if (__any_sync(0xFFFFFFFFu, timed_out)) break;
+    }
+    if (cnt) arrive();
+  } else if (warp < kF3DrainWarp0) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kF3IssueRegs));
+    if (warp < kF3MmaWarp + 2) {
+      // ------------------------------ MMA issuers ----------------------------------------
+      constexpr uint32_t IDESC = instr_desc(kTileM, CC, true);
+      constexpr uint64_t B_DESC0 = smem_desc_sw_const(C::PART_BYTES, 8 * SWB, SWB == 128 ? 2u : 4u);
+      constexpr uint32_t B_DESC_HI = (uint32_t)(B_DESC0 >> 32);
+      const int stream = warp - kF3MmaWarp, mine = stages_of(stream);
+      uint32_t cnt = 0, b_base = 0;
+      for (uint32_t st = blockIdx.x; st < a.n_super && !timed_out; st += gridDim.x, b_base += (uint32_t)n_stages) {
+        for (int i = 0; i < mine; ++i, ++cnt) {
+          const uint32_t b_it = b_base + (T > 1 ? i : 2 * i + stream), bs = b_it % BST, s = cnt % SLOTS;
+          const uint32_t buf = cnt & 1u;
+          if (!mbar_wait(&b_full[bs], (b_it / BST) & 1u)) { timed_out = true; goto mma_done; }
+          if (!mbar_wait(&a_full[stream * SLOTS + s], (cnt / SLOTS) & 1u)) { timed_out = true; goto mma_done; }
+          if (!mbar_wait(&acc_empty[stream * 2 + buf], ((cnt >> 1) & 1u) ^ 1u)) {
+            timed_out = true;
+            goto mma_done;
+          }
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + (stream * 2 + buf) * CC;
+          const uint32_t a_tmem = tmem_base + C::ACC_COLS + (stream * SLOTS + s) * C::A_COLS;
+          const uint32_t b_lo = ((smem_base + bs * C::B_BYTES) >> 4) + (uint32_t)(B_DESC0 & 0xFFFFFFFFu);
+          static_for<12>([&](auto xc) {
+            constexpr int x = decltype(xc)::value, j = x & 1;
+            constexpr int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};
+            const uint64_t b_desc = ((uint64_t)B_DESC_HI << 32) | (b_lo + ((pb[x / 2] * C::PART_BYTES + j * 16 * SWB) >> 4));
+            tc_mma_bf16_ta_elect(d_tmem, a_tmem + pa[x / 2] * 16 + j * 8, b_desc, IDESC, x > 0 ? 1u : 0u);
+          });
+          tc_commit_elect(&a_empty[stream * SLOTS + s]);
+          tc_commit_elect(&b_empty[bs]);
+          tc_commit_elect(&acc_full[stream * 2 + buf]);
+        }
+      }
+    mma_done:;
+    } else if (warp == kF3WeightWarp && lane == 0) {
+      // ------------------------------ weights --------------------------------------------
+      const uint8_t* image = a.image + (size_t)blockIdx.y * C::B_BYTES;
+      uint32_t b_it = 0;
+      for (uint32_t st = blockIdx.x; st < a.n_super && !timed_out; st += gridDim.x) {
+        for (int i = 0; i < n_stages; ++i, ++b_it) {
+          const uint32_t s = b_it % BST;
+          if (!mbar_wait(&b_empty[s], ((b_it / BST) & 1u) ^ 1u)) { timed_out = true; break; }
+          bulk_load(smem_base + s * C::B_BYTES, image + (size_t)i * gridDim.y * C::B_BYTES, C::B_BYTES, smem_u32(&b_full[s]));
+        }
+      }
+      // no copy may be in flight when the CTA exits: wait for the last round of the ring
+      for (uint32_t i = b_it > BST ? b_it - BST : 0; i < b_it; ++i)
+        if (!mbar_wait(&b_full[i % BST], (i / BST) & 1u)) timed_out = true;
+    }
+  } else if (warp < kF3Warps) {
+    // ------------------------------ drain ----------------------------------------------
+    // Four warps per set, one per 32 rows. T = 2: set d adds up stream d; T = 1: set d half d of the rows, of both streams.
+    // Lane t holds, of rows t / 4 and t / 4 + 8 of a half, CC / 4 channels from (t % 4) * CC / 4 on.
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kF3DrainRegs));
+    constexpr int HALVES = T > 1 ? 2 : 1;
+    const int set = (warp - kF3DrainWarp0) >> 2, u = lane & 3;
+    const uint32_t quad = warp & 3;
+    const int longest = stages_of(0);
+    uint32_t cnt[2] = {0, 0};
+    for (uint32_t st = blockIdx.x; st < a.n_super && !timed_out; st += gridDim.x) {
+      float sum[HALVES][CC / 8][4];
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+        for (int v = 0; v < CC / 8; ++v)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sum[h][v][e] = 0.f;
+#pragma unroll 1
+      for (int d = 0; d < longest && !timed_out; ++d) {
+#pragma unroll
+        for (int x = 0; x < (T > 1 ? 1 : 2); ++x) {
+          const int stream = T > 1 ? set : x;
+          if (d >= stages_of(stream)) continue;
+          const uint32_t acc = stream * 2 + (cnt[x] & 1u), ph = (cnt[x] >> 1) & 1u;
+          ++cnt[x];
+          if (!mbar_wait(&acc_full[acc], ph)) timed_out = true;
+          timed_out = __any_sync(0xFFFFFFFFu, timed_out);
+          if (timed_out) break;
+          tc_fence_after();
+#pragma unroll
+          for (int h = 0; h < HALVES; ++h) {
+            const uint32_t taddr = tmem_base + ((quad * 32u + (T > 1 ? h : set) * 16u) << 16) + acc * CC;
+            uint32_t r[CC / 32][16];
+#pragma unroll
+            for (int q = 0; q < CC / 32; ++q) tc_ld16x256b(taddr + q * 32, r[q]);
+            tc_wait_ld();
+#pragma unroll
+            for (int v = 0; v < CC / 2; ++v) sum[h][v / 4][v % 4] += __uint_as_float(r[v / 16][v % 16]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[acc]);
+        }
+      }
+      if (timed_out) break;
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t tile_row0 = st * (kTileM * T) + (T > 1 ? set : 0) * kTileM + quad * 32 + (T > 1 ? h : set) * 16 + i * 8;
+          const uint32_t row = tile_row0 + (lane >> 2);
+          // magnitudes outside [2^-90, the largest number], zero apart
+          bool again = false;
+#pragma unroll
+          for (int v = 0; v < CC / 8; ++v)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const uint32_t bits = __float_as_uint(sum[h][v][2 * i + e]) << 1;
+              again = again || (bits != 0u && bits - (37u << 24) >= (255u - 37u) << 24);
+            }
+          uint32_t votes = __ballot_sync(0xFFFFFFFFu, again && row < a.n_dst);
+          if (row < a.n_dst && !((votes >> (lane & 28)) & 0xFu)) {
+            float* dst = a.out + (size_t)row * a.c_col;
+#pragma unroll
+            for (int v = 0; v < CC / 8; v += 2) {
+              const int c = u * (CC / 4) + v * 2;
+              if (col0 + c < a.c_col) {
+                float4 f;
+                f.x = f3_finish(sum[h][v][2 * i], s_ep[c], s_ep[CC + c], a.relu);
+                f.y = f3_finish(sum[h][v][2 * i + 1], s_ep[c + 1], s_ep[CC + c + 1], a.relu);
+                f.z = f3_finish(sum[h][v + 1][2 * i], s_ep[c + 2], s_ep[CC + c + 2], a.relu);
+                f.w = f3_finish(sum[h][v + 1][2 * i + 1], s_ep[c + 3], s_ep[CC + c + 3], a.relu);
+                *reinterpret_cast<float4*>(dst + col0 + c) = f;
+              }
+            }
+          }
+          while (votes) {
+            const int r = (__ffs(votes) - 1) >> 2;
+            votes &= ~(0xFu << (4 * r));
+            exact_row(a, tile_row0 + r, col0, CC, s_ep, lane);
+          }
+        }
+      }
+    }
+  }
+
+  if (timed_out) atomicExch(a.status, (uint32_t)RMN_ERR_TIMEOUT);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kF3MmaWarp) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+  }
+}
+
+template <int CC, int T>
+int launch_f3(F3Args a, uint32_t blocks, uint32_t fit, cudaStream_t stream) {
+  using C = F3Cfg<CC, T>;
+  static SmemOptIn opt_in;
+  RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_conv_f3<CC, T>), C::SMEM));
+  a.n_super = (a.n_dst + kTileM * T - 1) / (kTileM * T);
+  RMN_CUDA_TRY(launch_overlapped(k_conv_f3<CC, T>, dim3(fit < a.n_super ? fit : a.n_super, blocks), dim3(kF3Threads), C::SMEM,
+                                 stream, a));
+  RMN_LAUNCH_CHECK();
+  count_tc_launch();
+  return RMN_OK;
+}
+
+template <int CC>
+int run_f3(F3Args a, uint8_t* image, cudaStream_t stream) {
+  int dev = 0, sms = 148;
+  RMN_CUDA_TRY(cudaGetDevice(&dev));
+  RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const uint32_t blocks = (uint32_t)(a.c_col + CC - 1) / CC, fit = (uint32_t)sms > blocks ? (uint32_t)sms / blocks : 1u;
+  const uint32_t lines = (uint32_t)(a.K * a.n_kb) * blocks * 32 * (CC / 8);
+  RMN_CUDA_TRY(launch_overlapped(k_f3_image<CC>, dim3((lines + 255) / 256), dim3(256), 0, stream, a.w, a.K, a.c_red, a.c_col,
+                                 a.n_kb, (int)blocks, a.transpose, a.reverse, reinterpret_cast<uint4*>(image)));
+  RMN_LAUNCH_CHECK();
+  a.image = image;
+  // row tiles of the busiest SM: pairs of them share their weights, single ones leave fewer SMs idle at the end
+  const uint32_t tiles = (a.n_dst + kTileM - 1) / kTileM, pairs = (tiles + 1) / 2;
+  const uint32_t rounds2 = (pairs + fit - 1) / fit * 2, rounds1 = (tiles + fit - 1) / fit;
+  return rounds2 <= rounds1 ? launch_f3<CC, 2>(a, blocks, fit, stream) : launch_f3<CC, 1>(a, blocks, fit, stream);
+}
+
+}  // namespace tc
+}  // namespace rmn
+
+using namespace rmn;
+
+extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, int c_out) {
+  // Few rows leave most SMs idle here, where every row tile walks all offsets in turn, and k_conv_f32 deals the offsets of a row
+  // to several warps; 64 columns cost it twice the time and these kernels little more. 27 offsets, half of them present, us
+  // there / here: 1000 rows 32 -> 32 12.4 / 14.2, 64 -> 32 20.7 / 22.8, 32 -> 64 20.5 / 16.3; 4000 rows 16.1 / 14.7, 27.3 / 23.0,
+  // 26.0 / 16.5, 16 -> 16 11.3 / 13.9; 100 rows 32 -> 64 19.8 / 15.7
+  if (c_out <= 32 && n_dst < (c_in < 32 ? 8192u : 3072u)) return 0;
+  if (n_dst == 0 || K < 1 || K > 4096 || c_in < 16 || c_in > 1024 || c_in % 8 || c_out < 4 || c_out > 1024 || c_out % 4) return 0;
+  const size_t cc = c_out <= 32 ? 32 : 64, columns = (c_out + cc - 1) / cc * cc;
+  return (size_t)K * ((c_in + 31) / 32) * 32 * columns * 3 * 2;
+}
+
+extern "C" int rmn_conv_forward_f32(const float* d_feats, uint32_t n_src, int c_in, const float* d_weights, int K, int c_out,
+                                    int transpose, int reverse, const int32_t* d_nbr, uint32_t n_dst, float* d_out,
+                                    const float* d_scale, const float* d_shift, int relu, void* d_scratch, size_t scratch_bytes,
+                                    void* stream_) {
+  if (n_dst == 0) return RMN_OK;
+  const size_t need = rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out);
+  if (need == 0) return RMN_ERR_UNSUPPORTED;
+  // (with no source rows every table entry is -1 and nothing is read through d_feats)
+  if (!d_weights || !d_nbr || !d_out || !d_scratch || (n_src > 0 && !d_feats)) return RMN_ERR_BAD_ARG;
+  if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_weights & 15) || ((uintptr_t)d_out & 15) || ((uintptr_t)d_scratch & 15))
+    return RMN_ERR_UNSUPPORTED;
+  if (scratch_bytes < need) return RMN_ERR_ALLOC;
+  tc::F3Args a = {};
+  a.src = d_feats;
+  a.w = d_weights;
+  a.nbr = d_nbr;
+  a.out = d_out;
+  a.ep_scale = d_scale;
+  a.ep_shift = d_shift;
+  a.status = const_cast<uint32_t*>(tc_status_device_address());
+  a.n_dst = n_dst;
+  a.K = K;
+  a.c_red = c_in;
+  a.c_col = c_out;
+  a.n_kb = (c_in + 31) / 32;
+  a.transpose = transpose;
+  a.reverse = reverse;
+  a.relu = relu;
+  if (!a.status) return RMN_ERR_CUDA;
+  return c_out <= 32 ? tc::run_f3<32>(a, static_cast<uint8_t*>(d_scratch), (cudaStream_t)stream_)
+                     : tc::run_f3<64>(a, static_cast<uint8_t*>(d_scratch), (cudaStream_t)stream_);
+}

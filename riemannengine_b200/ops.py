@@ -265,6 +265,24 @@ def _weight_image(weights: torch.Tensor, transpose: bool, feats: torch.Tensor,
     return image
 
 
+def _conv_f32(feats: torch.Tensor, weights: torch.Tensor, transpose: bool, nbr: torch.Tensor, out: torch.Tensor,
+              scale: Optional[torch.Tensor] = None, shift: Optional[torch.Tensor] = None, relu: bool = False) -> bool:
+    """fp32 on the tensor cores (rmn_conv_forward_f32) into ``out``; False where that does not serve. The current device is
+    the tensors'."""
+    n_dst, n_src, K = int(nbr.size(1)), int(feats.size(0)), int(weights.size(0))
+    if feats.dtype != torch.float32 or not n_dst or not n_src or feats.data_ptr() % 32:
+        return False
+    c_in, c_out = int(feats.size(1)), int(out.size(1))
+    nbytes = capi.lib().rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out)
+    if nbytes == 0:
+        return False
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=feats.device)
+    capi.check(capi.lib().rmn_conv_forward_f32(_ptr(feats), n_src, c_in, _ptr(weights), K, c_out, int(transpose), 0, _ptr(nbr),
+                                               n_dst, _ptr(out), _ptr(scale), _ptr(shift), int(bool(relu)), _ptr(scratch),
+                                               nbytes, _stream()), "rmn_conv_forward_f32")
+    return True
+
+
 def conv_forward(feats: torch.Tensor, weights: torch.Tensor, nbr: torch.Tensor,
                  scale: Optional[torch.Tensor] = None, shift: Optional[torch.Tensor] = None,
                  relu: bool = False, plan: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -295,6 +313,8 @@ def conv_forward(feats: torch.Tensor, weights: torch.Tensor, nbr: torch.Tensor,
                                                          _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _ptr(sc), _ptr(sh),
                                                          None, int(bool(relu)), _stream()), "rmn_conv_forward_image")
             return out
+        if _conv_f32(feats, weights, False, nbr, out, sc, sh, relu):
+            return out
         capi.check(capi.lib().rmn_conv_forward_planned(_ptr(feats), int(feats.size(0)), c_in, _ptr(weights), K, c_out,
                                                        _ptr(nbr), _ptr(plan), n_dst, _ptr(out), _dtype_code(feats),
                                                        _ptr(sc), _ptr(sh), int(bool(relu)), _stream()),
@@ -313,7 +333,9 @@ def conv_backward_input(grad_out: torch.Tensor, weights: torch.Tensor, nbr_t: to
     out = torch.empty((n_src, c_in), dtype=grad_out.dtype, device=grad_out.device)
     with torch.cuda.device(grad_out.device):
         if grad_out.dtype == torch.float32 and n_src and grad_out.size(0):
-            # fp32: the forward pass on transposed weights (rmn_conv_transpose_weights)
+            # fp32: the forward pass on transposed weights
+            if _conv_f32(grad_out, weights, True, nbr_t, out):
+                return out
             wt = torch.empty((K, c_out, c_in), dtype=weights.dtype, device=weights.device)
             capi.check(capi.lib().rmn_conv_transpose_weights(_ptr(weights), K, c_in, c_out, capi.F32, 0, _ptr(wt),
                                                              _stream()), "rmn_conv_transpose_weights")

@@ -1115,6 +1115,29 @@ at::Tensor weight_image(const at::Tensor& kernel, std::pair<int64_t, int64_t> sh
   return image;
 }
 
+// fp32 features on the tensor cores (rmn_conv_forward_f32); undefined where that does not serve. transpose: kernel is
+// [K, c_out, c_in].
+at::Tensor conv_f32(const at::Tensor& feats, const at::Tensor& kernel, bool transpose, bool reverse, const at::Tensor& nbr,
+                    const at::Tensor& scale = at::Tensor(), const at::Tensor& shift = at::Tensor(), bool relu = false) {
+  if (feats.scalar_type() != at::kFloat || feats.size(0) == 0 || nbr.size(1) == 0 ||
+      reinterpret_cast<uintptr_t>(feats.data_ptr()) % 32 != 0 || reinterpret_cast<uintptr_t>(kernel.data_ptr()) % 16 != 0)
+    return at::Tensor();
+  const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(feats.size(1)),
+            c_out = static_cast<int>(kernel.size(transpose ? 1 : 2));
+  const uint32_t n_dst = static_cast<uint32_t>(nbr.size(1));
+  const size_t bytes = rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out);
+  if (bytes == 0) return at::Tensor();
+  auto scratch = at::empty({static_cast<int64_t>(bytes)}, kernel.options().dtype(at::kByte));
+  auto out = at::empty({nbr.size(1), c_out}, feats.options());
+  check(rmn_conv_forward_f32(static_cast<const float*>(ptr(feats)), static_cast<uint32_t>(feats.size(0)), c_in,
+                             static_cast<const float*>(ptr(kernel)), K, c_out, transpose ? 1 : 0, reverse ? 1 : 0,
+                             static_cast<const int32_t*>(ptr(nbr)), n_dst, static_cast<float*>(ptr(out)),
+                             static_cast<const float*>(ptr(scale)), static_cast<const float*>(ptr(shift)), relu ? 1 : 0,
+                             ptr(scratch), bytes, current_stream()),
+        "rmn_conv_forward_f32");
+  return out;
+}
+
 // Epilogue of a convolution: out = act(conv * scale + shift + add). The vectors are per output channel; with a batch norm
 // (evaluation mode) they are made by the kernel that prepares the weights.
 struct ConvEpilogue {
@@ -1168,6 +1191,7 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
     TORCH_CHECK(!bn && !ep.add.defined(), "no kernel folds this layer's batch norm");
   }
   auto shift = vector(ep.shift, "bias"), scale = vector(ep.scale, "scale");
+  if (auto out = conv_f32(feats, kernel, false, false, nbr, scale, shift, ep.relu); out.defined()) return out;
   auto out = at::empty({nbr.size(1), c_out}, feats.options());
   check(rmn_conv_forward_planned(ptr(feats), static_cast<uint32_t>(feats.size(0)), c_in, ptr(kernel), K, c_out,
                                  static_cast<const int32_t*>(ptr(nbr)), ptr(plan), static_cast<uint32_t>(nbr.size(1)),
@@ -1185,6 +1209,7 @@ at::Tensor conv_backward_input(const at::Tensor& grad_in, const at::Tensor& kern
   if (grad.scalar_type() == at::kFloat && grad.size(0) > 0 && nbr_t.size(1) > 0) {
     // fp32: the forward pass on transposed weights
     auto w = kernel_in.contiguous();
+    if (auto out = conv_f32(grad, w, true, reverse, nbr_t); out.defined()) return out;
     auto wt = at::empty({w.size(0), w.size(2), w.size(1)}, w.options());
     check(rmn_conv_transpose_weights(ptr(w), static_cast<int>(w.size(0)), static_cast<int>(w.size(1)),
                                      static_cast<int>(w.size(2)), RMN_F32, reverse ? 1 : 0, ptr(wt), current_stream()),

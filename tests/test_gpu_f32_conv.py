@@ -47,6 +47,75 @@ def test_f32_passes_match_float64(n, c_in, c_out, K, fill):
     close(ops.conv_backward_weight(d(feats), d(grad), d(nbr)), want_w)
 
 
+# Row counts around a row tile, a pair of them and the size from which few columns take this path; channel counts that fill a
+# 32-channel stage or a block of 32 or 64 columns or not; one stage, an odd number, two blocks of channels per offset.
+@pytest.mark.parametrize("n,c_in,c_out,K,fill", [
+    (1, 16, 36, 1, 1.0), (127, 32, 64, 2, 0.5), (129, 64, 64, 27, 0.0), (257, 40, 36, 27, 0.6), (3071, 32, 64, 5, 0.02),
+    (3072, 32, 32, 27, 0.5), (8192, 16, 4, 8, 1.0), (19_073, 96, 100, 3, 0.4), (40_003, 48, 64, 27, 0.3), (1000, 64, 200, 27, 0.5),
+])
+@pytest.mark.parametrize("transpose,reverse", [(0, 0), (1, 0), (1, 1)])
+def test_f32_on_tensor_cores_matches_float64(n, c_in, c_out, K, fill, transpose, reverse):
+    from riemannengine_b200 import capi, ops
+    g = torch.Generator(device="cuda").manual_seed(n + c_in)
+    n_src = n + 5
+    nbr = torch.randint(0, n_src, (K, n), generator=g, dtype=torch.int32, device="cuda")
+    nbr[torch.rand((K, n), generator=g, device="cuda") >= fill] = -1
+    feats = torch.randn((n_src, c_in), generator=g, device="cuda")
+    w = torch.randn((K, c_in, c_out), generator=g, device="cuda")
+    scale, shift = (torch.randn(c_out, generator=g, device="cuda") for _ in range(2))
+    given = w.flip(0) if reverse else w
+    given = (given.transpose(1, 2) if transpose else given).contiguous()
+    lib = capi.lib()
+    size = lib.rmn_conv_f32_scratch_bytes(n, K, c_in, c_out)
+    scratch, out = torch.empty(size, dtype=torch.uint8, device="cuda"), torch.empty((n, c_out), device="cuda")
+    want, most = (torch.zeros((n, c_out), dtype=torch.float64, device="cuda") for _ in range(2))
+    for k in range(K):
+        hit = nbr[k] >= 0
+        x, y = feats[nbr[k][hit].long()].double(), w[k].double()
+        want[hit] += x @ y
+        most[hit] += x.abs() @ y.abs()
+
+    def run(relu, *epilogue):
+        capi.check(lib.rmn_conv_forward_f32(ops._ptr(feats), n_src, c_in, ops._ptr(given), K, c_out, transpose, reverse,
+                                            ops._ptr(nbr), n, ops._ptr(out), *epilogue, relu, ops._ptr(scratch), size,
+                                            ops._stream()), "rmn_conv_forward_f32")
+        return out.double()
+
+    # Each product within 2^-23 (parts left out, and the last ones rounded); 32 of them and the parts' sums truncated to the
+    # largest, 2^-23 of it at most in each of four steps; sums of K stages rounded, 2^-24 each. 2^-20 of the magnitudes covers it.
+    assert size > 0 and bool(((run(0, None, None) - want).abs() <= 2.0 ** -20 * most).all())
+    got = run(1, ops._ptr(scale), ops._ptr(shift))
+    limit = 2.0 ** -20 * (most * scale.abs() + shift.abs())
+    assert bool(((got - torch.relu(want * scale.double() + shift.double())).abs() <= limit).all())
+
+
+def test_f32_on_tensor_cores_keeps_what_bf16_parts_cannot_hold():
+    """Infinities, NaN, numbers next to the largest one and tiny ones: as the fp32 multiply-adds give them."""
+    from riemannengine_b200 import capi, ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n, K, c = 700, 3, 64
+    nbr = torch.arange(n, dtype=torch.int32, device="cuda").repeat(K, 1)
+    nbr[1:][torch.rand((K - 1, n), generator=g, device="cuda") < 0.5] = -1
+    feats = torch.randn((n, c), generator=g, device="cuda")
+    most = torch.finfo(torch.float32).max
+    for row, value in ((3, float("inf")), (40, float("-inf")), (200, float("nan")), (301, most), (333, -most), (420, 3.39e38)):
+        feats[row, row % c] = value
+    feats[500:600] *= 1e-34   # their third parts lie below the smallest bf16 number
+    feats[600:610] = 0
+    w = torch.randn((K, c, c), generator=g, device="cuda") * 0.01
+    w[:, 5] = 0               # infinity times zero
+    feats[650, 5] = float("inf")
+    out, again = torch.empty((n, c), device="cuda"), torch.empty((n, c), device="cuda")
+    assert ops._conv_f32(feats, w, False, nbr, out)
+    capi.check(capi.lib().rmn_conv_forward(ops._ptr(feats), n, c, ops._ptr(w), K, c, ops._ptr(nbr), n, ops._ptr(again),
+                                           capi.F32, ops._stream()), "rmn_conv_forward")
+    assert torch.equal(out.isnan(), again.isnan()) and torch.equal(out.isposinf(), again.isposinf())
+    assert torch.equal(out.isneginf(), again.isneginf()) and bool(out.isnan().any()) and bool(out.isinf().any())
+    finite = again.isfinite()
+    size = torch.where(finite, again, 0).abs().amax(1, keepdim=True).expand_as(out)[finite]   # (sums of 64 products and more)
+    assert bool(((out[finite].double() - again[finite].double()).abs() <= 1e-5 * size.double()).all())
+
+
 def test_weight_gradient_of_more_channel_tiles_than_a_launch_takes():
     from riemannengine_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(1)
