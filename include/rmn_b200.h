@@ -319,6 +319,18 @@ int rmn_kmap_build_host(const void *d_table, const int32_t *d_query, uint32_t n_
                         void *d_workspace, size_t workspace_bytes, void *stream);
 
 /*
+ * Self map of rmn_kmap_build_self in an internal order of the rows, for rmn_conv_forward_ordered: d_order[p] [n_rows] is the row
+ * at position p, d_nbr[k][p] [K, n_rows] the row of the table at offset k from it, or -1. The rows lie block by block of the
+ * map's space, which spares a large map of shuffled rows the random accesses of the public order; a map too thin for that keeps
+ * the order of its rows. rmn_kmap_ordered_workspace_bytes: scratch (16-byte aligned), 0 where there is no such build (three
+ * dimensions and more, from 1.97 M rows on, K odd from 9 to 2048). The order may differ from call to call; what a convolution
+ * makes of it does not.
+ */
+size_t rmn_kmap_ordered_workspace_bytes(uint32_t n_rows, int W, int K);
+int rmn_kmap_build_ordered(const void *d_table, const int32_t *d_coords, uint32_t n_rows, int W, const int32_t *d_offsets,
+                           int K, int32_t *d_order, int32_t *d_nbr, void *d_workspace, size_t workspace_bytes, void *stream);
+
+/*
  * Materialise the pair lists of the last rmn_kmap_build (same d_nbr,
  * d_offset_ptr and d_workspace): d_a_idx[p], d_q_idx[p] for p < ptr[K],
  * pairs of one offset sorted by query row (for a map built by
@@ -446,6 +458,10 @@ int rmn_conv_weight_image(const void *d_weights, int K, int w_in, int w_out, int
 int rmn_conv_forward_image(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
                            const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out, const float *d_scale,
                            const float *d_shift, const void *d_add, int relu, void *stream);
+/* rmn_conv_forward_image over an ordered map: row d_order[p] of d_out (and of d_add) belongs to entry p of every offset. */
+int rmn_conv_forward_ordered(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
+                             const int32_t *d_nbr, const int32_t *d_order, uint32_t n_dst, void *d_out, const float *d_scale,
+                             const float *d_shift, const void *d_add, int relu, void *stream);
 /* d_dst [n_rows, c_dst] = the first c_src elements of rows ld_src apart in d_src, with c_dst - c_src zeros behind (2-byte
  * elements; fp32 as pairs of them). */
 int rmn_pad_channels(const void *d_src, uint32_t n_rows, int c_src, int ld_src, void *d_dst, int c_dst, void *stream);

@@ -21,7 +21,7 @@ int ta_weight_image(const void* w, int K, int w_red, int w_col, int c_red, int c
                     const rmn_bn_fold& fold, void* image, cudaStream_t stream);
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial,
-            uint32_t* n_partials, cudaStream_t stream, const void* plan);
+            uint32_t* n_partials, cudaStream_t stream, const void* plan, const int32_t* order);
 int tc_read_status(cudaStream_t stream, uint32_t* status);
 unsigned long long tc_launch_count();
 int tc_conv_wgrad(const void* feats, const void* grad_out, const int32_t* nbr, uint32_t n_dst, int K, int c_in,
@@ -136,7 +136,19 @@ extern "C" int rmn_conv_forward_image(const void* d_feats, uint32_t n_src, int c
   if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_image & 15) || ((uintptr_t)d_out & 15) || ((uintptr_t)d_add & 15))
     return RMN_ERR_BAD_ARG;
   return ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, d_add, relu, nullptr, nullptr,
-                 (cudaStream_t)stream_, d_plan);
+                 (cudaStream_t)stream_, d_plan, nullptr);
+}
+
+extern "C" int rmn_conv_forward_ordered(const void* d_feats, uint32_t n_src, int c_in, const void* d_image, int K, int c_out,
+                                        const int32_t* d_nbr, const int32_t* d_order, uint32_t n_dst, void* d_out,
+                                        const float* d_scale, const float* d_shift, const void* d_add, int relu,
+                                        void* stream_) {
+  if (n_dst == 0) return RMN_OK;
+  if (!d_image || !d_nbr || !d_order || !d_out || (n_src > 0 && !d_feats) || K < 1 || K > 65535) return RMN_ERR_BAD_ARG;
+  if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_image & 15) || ((uintptr_t)d_out & 15) || ((uintptr_t)d_add & 15))
+    return RMN_ERR_BAD_ARG;
+  return ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, d_add, relu, nullptr, nullptr,
+                 (cudaStream_t)stream_, nullptr, d_order);
 }
 
 extern "C" int rmn_conv_backward_input(const void* d_grad_out, uint32_t n_dst, int c_out,

@@ -157,6 +157,7 @@ struct RowBlock {
 // table [K][n_dst] (n_dst = the padded position count), `perm` maps a position to the output row it is stored to (-1:
 // padding) and `tile_mask` holds, per 128-row tile, the offsets at which any row of the tile has a neighbour: other
 // (tile, offset) pairs take no gather, no slot and no MMA, offsets that no tile of the super-tile has no copy of W[k].
+// Without a plan `perm` may be the order of an ordered map (rmn_kmap_build_ordered), or NULL.
 // kStats: the epilogue also accumulates, per output channel, the sum and the sum of squares of the values it stores
 // and writes them to stats_partial[blockIdx.x][2][CC].
 // The columns [CC * blockIdx.y, CC * (blockIdx.y + 1)) of n_cols are computed.
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
         for (int i = 0; i < 4; ++i) {
           const uint32_t pos = st * (kTileM * T) + t * kTileM + quad * 32 + i * 8 + (lane >> 2);
           rows[i] = pos < n_dst ? pos : 0xFFFFFFFFu;
-          if constexpr (kPlan) rows[i] = (uint32_t)__ldg(perm + pos);  // (-1: padding)
+          if (kPlan || (perm && pos < n_dst)) rows[i] = (uint32_t)__ldg(perm + pos);  // (-1: padding of a plan)
         }
 #pragma unroll 1
         for (int nb = 0; nb < CC / NBLK; ++nb) {
@@ -601,10 +602,10 @@ __global__ void __launch_bounds__(kTaThreads, 1)
 template <int CR, int CC, int T, bool kStats, bool kPlan>
 int launch_ta(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, void* out, const float* ep_scale,
               const float* ep_shift, const void* ep_add, int ep_relu, uint32_t n_cols, int sms, cudaStream_t stream, float* stats_partial,
-              uint32_t* grid_out, const void* plan) {
+              uint32_t* grid_out, const void* plan, const int32_t* order) {
   using C = TaCfg<CR, CC, T>;
   auto kern = k_conv_ta<CR, CC, T, kStats, kPlan>;
-  const int32_t* perm = nullptr;
+  const int32_t* perm = order;
   const uint32_t* tile_mask = nullptr;
   if constexpr (kPlan) {
     const PlanLayout L = plan_layout(n_dst, K);
@@ -685,13 +686,13 @@ bool ta_small(uint32_t n_dst, int c_col, int sms) {
 // stats_partial != nullptr: also leave per-CTA channel statistics ([*n_partials][2][c_col] floats)
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial, uint32_t* n_partials,
-            cudaStream_t stream, const void* plan) {
+            cudaStream_t stream, const void* plan, const int32_t* order) {
   if (ta_image_bytes(K, c_red, c_col) == 0) return RMN_ERR_UNSUPPORTED;  // (the cases below match blocks of columns)
   int dev = 0, sms = 148;
   RMN_CUDA_TRY(cudaGetDevice(&dev));
   RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 #define RMN_TA_ARGS \
-  src, image, nbr, n_dst, K, out, ep_scale, ep_shift, ep_add, ep_relu, (uint32_t)c_col, sms, stream, stats_partial, n_partials, plan
+  src, image, nbr, n_dst, K, out, ep_scale, ep_shift, ep_add, ep_relu, (uint32_t)c_col, sms, stream, stats_partial, n_partials, plan, order
   if (ta_small(n_dst, c_col, sms)) {
     plan = nullptr;
 #define RMN_TA_CASE(R, Cc)                                                                   \

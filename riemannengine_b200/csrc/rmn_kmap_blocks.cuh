@@ -32,8 +32,10 @@ struct BlockIndex {
   uint32_t* state;        // one of the three below
   int32_t* perm;          // row numbers, block by block
   uint32_t* slot_of_row;  // build scratch
+  uint32_t* buckets;      // of an ordered map (k_block_assign), NULL otherwise
   uint32_t capacity;
 };
+constexpr uint32_t kBlockBucketBits = 13, kBlockBuckets = 1u << kBlockBucketBits;
 constexpr uint32_t kIndexInUse = ~0u, kIndexNotChosen = 0u, kIndexFull = 1u;  // full: the blocks did not fit
 // (a surface loads two slots in five: runs of 32 taken slots occur, runs of 128 do not; 4.8 M clip rows overflowed at 32 in
 // some scenes, and took 3.0 ms by the hash table)
@@ -50,6 +52,7 @@ inline BlockIndex block_index(void* workspace, uint32_t n) {
   b.state = b.counter + 1;
   b.perm = reinterpret_cast<int32_t*>(b.counter + 8);
   b.slot_of_row = reinterpret_cast<uint32_t*>(b.perm + n);
+  b.buckets = nullptr;
   return b;
 }
 
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(1024) k_block_choose(const TableHeader* __rest
     const float part = fminf(1.f, 0.5f * (float)s_inside[1] / (float)s_inside[0]);
     const float set = part * ((float)h->capacity * sizeof(Slot));
     if (tid == 0)
-      s_serves = set > kChooseBytes && blocks / kChooseBlocks * (float)n <= kChooseLoad * (float)ix.capacity ? 1u : 0u;
+      s_serves = (ix.buckets || set > kChooseBytes) && blocks / kChooseBlocks * (float)n <= kChooseLoad * (float)ix.capacity ? 1u : 0u;
   }
   __syncthreads();
   const bool serves = s_serves != 0u;
@@ -206,6 +209,8 @@ __global__ void __launch_bounds__(1024) k_block_choose(const TableHeader* __rest
   }
   if (serves) {
     for (size_t i = first; i < 2 * (size_t)ix.capacity; i += step) reinterpret_cast<uint4*>(ix.slots)[i] = ones;
+    if (ix.buckets)
+      for (size_t i = first; i < kBlockBuckets; i += step) ix.buckets[i] = 0u;
   } else {  // single words up to the first 16-byte boundary and behind the last one
     const size_t head = ((16 - ((uintptr_t)mirrored & 15)) & 15) / 4, vecs = (n_mirrored - head) / 4;
     const size_t tail = head + 4 * vecs;
@@ -242,6 +247,50 @@ __global__ void __launch_bounds__(256) k_block_insert(const TableHeader* __restr
     }
     atomicAnd(&ix.slots[s].free, ~(1ull << b.bit(b.local)));
     ix.slot_of_row[row] = s;
+  }
+}
+
+// The ranges of perm in an ordered map: blocks that share the highest bits of their key - batch, further axes, layers of blocks along
+// the third axis - lie together, so that the rows which a stretch of the convolution gathers stay in the L2. Rows per bucket,
+// their exclusive sums (one block), and a range for every block.
+__device__ __forceinline__ uint32_t block_bucket(const TableHeader* h, unsigned long long key) {
+  return (uint32_t)(key >> (h->total_bits > kBlockBucketBits ? h->total_bits - kBlockBucketBits : 0u));
+}
+template <bool kAssign>
+__global__ void __launch_bounds__(256) k_block_assign(const TableHeader* __restrict__ h, BlockIndex ix) {
+  after_previous_kernel();
+  if (*ix.state != kIndexInUse) return;
+  const uint32_t s = blockIdx.x * 256 + threadIdx.x;
+  if (s >= ix.capacity || ix.slots[s].key == kEmptyKey) return;
+  const uint32_t first = atomicAdd(ix.buckets + block_bucket(h, ix.slots[s].key), (uint32_t)__popcll(~ix.slots[s].free));
+  if constexpr (kAssign) ix.slots[s].base = first;
+}
+__global__ void __launch_bounds__(1024) k_block_bucket_sums(BlockIndex ix) {
+  after_previous_kernel();
+  if (*ix.state != kIndexInUse) return;
+  __shared__ uint32_t s_warp[32];
+  constexpr uint32_t PER = kBlockBuckets / 1024;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t v[PER], sum = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < PER; ++i) {
+    v[i] = ix.buckets[threadIdx.x * PER + i];
+    sum += v[i];
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+    if (lane >= (uint32_t)d) incl += t;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  uint32_t run = incl - sum;
+  for (uint32_t w = 0; w < warp; ++w) run += s_warp[w];
+#pragma unroll
+  for (uint32_t i = 0; i < PER; ++i) {
+    ix.buckets[threadIdx.x * PER + i] = run;
+    run += v[i];
   }
 }
 
@@ -296,19 +345,24 @@ __global__ void __launch_bounds__(256) k_block_scatter(const TableHeader* __rest
 // use: 2450 -> 2324 us for the four clips). Offsets that reach further than two voxels (in units of the map's grid) along a
 // block axis look their row up in the hash table instead. Where the blocks did not fit, the mirrored half of the table is
 // filled with "no neighbour" for k_kmap_probe_self, which follows.
-template <int W>
+// kOrdered: the map is written in the order of perm, block by block: position p is row perm[p], entries are row numbers. The rows
+// of a warp then share their blocks, and what they read of the index comes from the L1. Nothing is counted; where the index is
+// not in use perm becomes the identity.
+template <int W, bool kOrdered>
 __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots, const int32_t* __restrict__ coords, uint32_t n,
     const int32_t* __restrict__ offsets, int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts,
     uint32_t n_blocks, uint32_t* __restrict__ scan_ticket, BlockIndex ix) {
   after_previous_kernel();
   if (*ix.state != kIndexInUse) {
+    if constexpr (kOrdered)
+      for (uint32_t row = blockIdx.x * kKmapBlock + threadIdx.x; row < n; row += gridDim.x * kKmapBlock) ix.perm[row] = (int32_t)row;
     if (*ix.state == kIndexFull)
       for (uint32_t row = blockIdx.x * kKmapBlock + threadIdx.x; row < n; row += gridDim.x * kKmapBlock)
         for (int k = K / 2 + 1; k < K; ++k) __stcs(nbr + (size_t)k * n + row, -1);
     return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *scan_ticket = 0;
+  if (!kOrdered && blockIdx.x == 0 && threadIdx.x == 0) *scan_ticket = 0;
   using B = BlockCoords<W>;
   constexpr int D = W - 1, NA = B::NA, CELLS = 1 << NA;
   constexpr uint32_t kNever = 1u << 28, kFar = 1u << 29, kNewOuter = 1u << 30;
@@ -357,7 +411,7 @@ __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
     int32_t c[W];
 #pragma unroll
     for (int i = 0; i < W; ++i) c[i] = h->mn[i];
-    if (active) load_row<W>(coords, q, c);
+    if (active) load_row<W>(coords, kOrdered ? (uint32_t)ix.perm[q] : q, c);
     B b;
     b.load(h, c);
     // per block axis: the neighbouring block on the side of the row's half of its block, if any offset reaches it
@@ -443,11 +497,12 @@ __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
         hit = uid != 0xFFFFFFFFu;
       }
       if (active) __stcs(dst, (int32_t)uid);
-      if (k < half) {  // (the other half has the same counts, see k_kmap_scan)
+      if (!kOrdered && k < half) {  // (the other half has the same counts, see k_kmap_scan)
         const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
         if (lane == 0) atomicAdd(&s_cnt[k], (uint32_t)__popc(hits));
       }
     }
+    if constexpr (kOrdered) continue;
     __syncthreads();
     for (int k = threadIdx.x; k < half; k += kKmapBlock) block_counts[(size_t)k * n_blocks + row_block] = s_cnt[k];
     if (threadIdx.x == 0)

@@ -18,7 +18,7 @@ int tc_conv_stats(const void* src, uint32_t n_src, const void* w, const int32_t*
 
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial,
-            uint32_t* n_partials, cudaStream_t stream, const void* plan);
+            uint32_t* n_partials, cudaStream_t stream, const void* plan, const int32_t* order);
 
 constexpr uint32_t kMaxStatPartials = 1024;
 
@@ -200,7 +200,7 @@ extern "C" int rmn_conv_forward_image_stats(const void* d_feats, uint32_t n_src,
   if (workspace_bytes < rmn_channel_stats_workspace_bytes(c_out)) return RMN_ERR_ALLOC;
   uint32_t n_partials = 0;
   const int st = ta_conv(d_feats, d_image, d_nbr, n_dst, K, c_in, c_out, d_out, d_scale, d_shift, nullptr, relu,
-                         (float*)d_workspace, &n_partials, stream, d_plan);
+                         (float*)d_workspace, &n_partials, stream, d_plan, nullptr);
   if (st != RMN_OK) return st;
   RMN_CUDA_TRY(launch_overlapped(k_stats_reduce, dim3((2 * c_out + 127) / 128), dim3(128), 0, stream,
                                  (const float*)d_workspace, n_partials, c_out, d_stats));

@@ -508,6 +508,23 @@ std::shared_ptr<KernelMap> CoordinateManager::kernel_map(const CoordinateMapKey&
                                                          const stride_type& kernel_dilation,
                                                          RegionType::Type region_type, const at::Tensor& offsets,
                                                          bool is_transpose, bool is_pool) {
+  return find_or_build(in_key, out_key, kernel_size, kernel_stride, kernel_dilation, region_type, offsets, is_transpose, is_pool,
+                       false);
+}
+
+std::shared_ptr<KernelMap> CoordinateManager::layer_map(const CoordinateMapKey& in_key, const CoordinateMapKey& out_key,
+                                                        const stride_type& kernel_size, const stride_type& kernel_stride,
+                                                        const stride_type& kernel_dilation, RegionType::Type region_type,
+                                                        const at::Tensor& offsets, bool is_transpose) {
+  return find_or_build(in_key, out_key, kernel_size, kernel_stride, kernel_dilation, region_type, offsets, is_transpose, false,
+                       true);
+}
+
+std::shared_ptr<KernelMap> CoordinateManager::find_or_build(const CoordinateMapKey& in_key, const CoordinateMapKey& out_key,
+                                                            const stride_type& kernel_size, const stride_type& kernel_stride,
+                                                            const stride_type& kernel_dilation, RegionType::Type region_type,
+                                                            const at::Tensor& offsets, bool is_transpose, bool is_pool,
+                                                            bool may_order) {
   const size_t kernel_dim = kernel_size.size();
   if (kernel_dim != kernel_stride.size() || kernel_dim != kernel_dilation.size())
     throw std::runtime_error("kernel size mismatch");
@@ -529,6 +546,8 @@ std::shared_ptr<KernelMap> CoordinateManager::kernel_map(const CoordinateMapKey&
   };
   const std::string key = cache_key(in_key, out_key, is_transpose);
   if (auto it = kernel_maps_.find(key); it != kernel_maps_.end()) return it->second;
+  if (may_order)
+    if (auto it = ordered_maps_.find(key); it != ordered_maps_.end()) return it->second;
 
   auto const& in_map = find(in_key, "in_map");
   auto const& out_map = find(out_key, "out_map");
@@ -566,9 +585,6 @@ std::shared_ptr<KernelMap> CoordinateManager::kernel_map(const CoordinateMapKey&
     result->n_in = in_map.size;
     result->n_out = out_map.size;
     result->nbr_out = at::empty({K, static_cast<int64_t>(out_map.size)}, ints);
-    result->offset_ptr = at::empty({K + 1}, ints.dtype(at::kLong));
-    const size_t ws_bytes = rmn_kmap_workspace_bytes(out_map.size, K);
-    result->workspace = at::empty({static_cast<int64_t>(ws_bytes)}, ints.dtype(at::kByte));
     // self map (stride-1 convolution) with a point-symmetric region: half the probes
     bool self_symmetric = !is_transpose && in_key.get_key() == out_key.get_key() && (K % 2 == 1);
     for (int k = 0; self_symmetric && k < K; ++k)
@@ -576,6 +592,19 @@ std::shared_ptr<KernelMap> CoordinateManager::kernel_map(const CoordinateMapKey&
         if (off[static_cast<size_t>(k) * D + a] != -off[static_cast<size_t>(K - 1 - k) * D + a]) self_symmetric = false;
     result->self_symmetric = self_symmetric;
     result->region_offsets = off;
+    if (const size_t bytes = may_order && self_symmetric ? rmn_kmap_ordered_workspace_bytes(out_map.size, W, K) : 0; bytes) {
+      result->order = at::empty({static_cast<int64_t>(out_map.size)}, ints);
+      auto scratch = at::empty({static_cast<int64_t>(bytes)}, ints.dtype(at::kByte));
+      check(rmn_kmap_build_ordered(ptr(in_map.table), static_cast<const int32_t*>(ptr(out_map.coords)), out_map.size, W,
+                                   static_cast<const int32_t*>(ptr(d_off)), K, static_cast<int32_t*>(ptr(result->order)),
+                                   static_cast<int32_t*>(ptr(result->nbr_out)), ptr(scratch), bytes, current_stream()),
+            "rmn_kmap_build_ordered");
+      ordered_maps_[key] = result;
+      return result;
+    }
+    result->offset_ptr = at::empty({K + 1}, ints.dtype(at::kLong));
+    const size_t ws_bytes = rmn_kmap_workspace_bytes(out_map.size, K);
+    result->workspace = at::empty({static_cast<int64_t>(ws_bytes)}, ints.dtype(at::kByte));
     // stored by the build's last kernel, not a copy engine: behind a large device-to-host copy of the caller's (the
     // previous step's result) an engine copy of these few bytes would wait for all of it
     result->host_offset_ptr = at::empty({K + 1}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
@@ -1146,7 +1175,8 @@ struct ConvEpilogue {
 };
 
 at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in, const at::Tensor& nbr,
-                        const ConvEpilogue& ep = {}, const at::Tensor& plan = at::Tensor(), torch::nn::BatchNorm1dImpl* bn = nullptr) {
+                        const ConvEpilogue& ep = {}, const at::Tensor& plan = at::Tensor(), torch::nn::BatchNorm1dImpl* bn = nullptr,
+                        const at::Tensor& order = at::Tensor()) {
   TORCH_CHECK(feats_in.is_cuda() && kernel_in.is_cuda(), "features and kernel must be CUDA tensors");
   TORCH_CHECK(feats_in.scalar_type() == kernel_in.scalar_type(), "expected features and kernel to have the same dtype");
   auto feats = contiguous_rows(feats_in), kernel = kernel_in.contiguous();
@@ -1181,6 +1211,15 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
     if (auto image = weight_image(kernel, shape, false, false, feats, bn ? &fold : nullptr); image.defined()) {
       TORCH_CHECK(!padded || !ep.add.defined(), "a padded convolution adds nothing");
       auto out = at::empty({nbr.size(1), shape.second}, feats.options());
+      if (order.defined()) {
+        check(rmn_conv_forward_ordered(ptr(feats), static_cast<uint32_t>(feats.size(0)), static_cast<int>(shape.first), ptr(image),
+                                       K, static_cast<int>(shape.second), static_cast<const int32_t*>(ptr(nbr)),
+                                       static_cast<const int32_t*>(ptr(order)), static_cast<uint32_t>(nbr.size(1)), ptr(out),
+                                       static_cast<const float*>(ptr(scale)), static_cast<const float*>(ptr(shift)), ptr(ep.add),
+                                       ep.relu ? 1 : 0, current_stream()),
+              "rmn_conv_forward_ordered");
+        return contiguous_rows(out.narrow(1, 0, c_out));
+      }
       check(rmn_conv_forward_image(ptr(feats), static_cast<uint32_t>(feats.size(0)), static_cast<int>(shape.first), ptr(image),
                                    K, static_cast<int>(shape.second), static_cast<const int32_t*>(ptr(nbr)), ptr(plan),
                                    static_cast<uint32_t>(nbr.size(1)), ptr(out), static_cast<const float*>(ptr(scale)),
@@ -1188,6 +1227,7 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
             "rmn_conv_forward_image");
       return contiguous_rows(out.narrow(1, 0, c_out));
     }
+    TORCH_CHECK(!order.defined(), "an ordered map serves the kernels of prepared weights");
     TORCH_CHECK(!bn && !ep.add.defined(), "no kernel folds this layer's batch norm");
   }
   auto shift = vector(ep.shift, "bias"), scale = vector(ep.scale, "scale");
@@ -1434,9 +1474,23 @@ bool folds_batch_norm(const RiemannConvolutionBaseImpl& conv, const SparseTensor
                                      static_cast<int>(shape.second), RMN_BF16) > 0 &&
          (shape.first != x.size(1) || !x.is_contiguous() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 == 0);
 }
+
+// whether a layer that only runs forward may take an ordered map: its pass goes to the kernels of prepared weights
+bool takes_ordered_map(const RiemannConvolutionBaseImpl& conv, const SparseTensor& input) {
+  auto const& kernel = conv.kernel_;
+  auto const& x = input.F();
+  if (at::GradMode::is_enabled() || !plain_autograd(x) || !plain_autograd(kernel) || !x.is_cuda() || x.size(0) == 0 ||
+      x.scalar_type() != at::kBFloat16 || kernel.scalar_type() != at::kBFloat16 || conv.is_transpose_)
+    return false;
+  const auto shape = run_shape(kernel);
+  return rmn_conv_weight_image_bytes(static_cast<int>(kernel.size(0)), static_cast<int>(shape.first),
+                                     static_cast<int>(shape.second), RMN_BF16) > 0 &&
+         (shape.first != x.size(1) || (x.is_contiguous() && reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 == 0));
+}
 }  // namespace
 
-std::pair<std::shared_ptr<KernelMap>, CoordinateMapKey> RiemannConvolutionBaseImpl::kernel_map(const SparseTensor& input) {
+std::pair<std::shared_ptr<KernelMap>, CoordinateMapKey> RiemannConvolutionBaseImpl::kernel_map(const SparseTensor& input,
+                                                                                               bool may_order) {
   TORCH_CHECK(input.dimension() == dimension_, "Input dimension mismatch");
   TORCH_CHECK(input.F().size(1) == in_channels_, "Input channel count does not match convolution");
   const auto params = kernel_generator_.get_kernel(input.tensor_stride(), is_transpose_);
@@ -1465,25 +1519,30 @@ std::pair<std::shared_ptr<KernelMap>, CoordinateMapKey> RiemannConvolutionBaseIm
   if (is_transpose_ && kernel_generator_.expand_coordinates())
     output_key = manager->stride_region(input.coordinate_map_key(), params.kernel_size, params.kernel_dilation,
                                         output_stride, params.region_type, params.region_offsets);
-  auto kmap = manager->kernel_map(input.coordinate_map_key(), output_key, params.kernel_size, params.kernel_stride,
-                                  params.kernel_dilation, params.region_type, params.region_offsets, is_transpose_,
-                                  false);
+  auto kmap = may_order ? manager->layer_map(input.coordinate_map_key(), output_key, params.kernel_size, params.kernel_stride,
+                                             params.kernel_dilation, params.region_type, params.region_offsets, is_transpose_)
+                        : manager->kernel_map(input.coordinate_map_key(), output_key, params.kernel_size,
+                                              params.kernel_stride, params.kernel_dilation, params.region_type,
+                                              params.region_offsets, is_transpose_, false);
   return {std::move(kmap), output_key};
 }
 
 SparseTensor RiemannConvolutionBaseImpl::forward(const SparseTensor& input) {
-  auto [kmap, output_key] = kernel_map(input);
-  auto result = sparse_convolution(input.F(), kernel_, kmap, bias_);  // the bias add is fused into the epilogue
+  auto [kmap, output_key] = kernel_map(input, takes_ordered_map(*this, input));
+  // (the bias add is fused into the epilogue)
+  auto result = kmap->order.defined() ? conv_forward(input.F(), kernel_, kmap->nbr_out, ConvEpilogue{at::Tensor(), bias_},
+                                                     at::Tensor(), nullptr, kmap->order)
+                                      : sparse_convolution(input.F(), kernel_, kmap, bias_);
   return SparseTensor(std::move(result), output_key, input.coordinate_manager());
 }
 
 SparseTensor RiemannConvolutionBaseImpl::forward_fused(const SparseTensor& input, torch::nn::BatchNorm1d bn, bool relu,
                                                        const at::Tensor& add) {
   torch::NoGradGuard guard;
-  auto [kmap, output_key] = kernel_map(input);
+  auto [kmap, output_key] = kernel_map(input, takes_ordered_map(*this, input));
   const auto shape = run_shape(kernel_);
   at::Tensor plan;
-  if (input.F().scalar_type() == at::kBFloat16) plan = kmap->plan_out(shape.first * shape.second);
+  if (!kmap->order.defined() && input.F().scalar_type() == at::kBFloat16) plan = kmap->plan_out(shape.first * shape.second);
   ConvEpilogue ep;
   ep.shift = bias_;
   ep.add = add;
@@ -1500,7 +1559,7 @@ SparseTensor RiemannConvolutionBaseImpl::forward_fused(const SparseTensor& input
       if (bias_.defined()) ep.shift = ep.shift + bias_.reshape({-1}).to(at::kFloat) * ep.scale;
     }
   }
-  auto result = conv_forward(input.F(), kernel_, kmap->nbr_out, ep, plan, folded);
+  auto result = conv_forward(input.F(), kernel_, kmap->nbr_out, ep, plan, folded, kmap->order);
   return SparseTensor(std::move(result), output_key, input.coordinate_manager());
 }
 

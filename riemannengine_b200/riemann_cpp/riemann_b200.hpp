@@ -95,6 +95,7 @@ private:
 // reference's representation (engine/grid/maps.hpp:19-79).
 struct KernelMap {
   at::Tensor nbr_out;
+  at::Tensor order;  // of an ordered map (CoordinateManager::layer_map): the row at each position of nbr_out; undefined otherwise
   int64_t n_in = 0, n_out = 0;
   at::Tensor offset_ptr;  // int64 [K+1] device, of the probe that produced nbr_out (undefined on a swapped view)
   at::Tensor workspace;
@@ -198,6 +199,12 @@ public:
                                         const stride_type& kernel_size, const stride_type& kernel_stride,
                                         const stride_type& kernel_dilation, RegionType::Type region_type,
                                         const at::Tensor& offsets, bool is_transpose, bool is_pool);
+  // kernel_map for a convolution that only runs forward: a large self map may come in an internal order of its rows
+  // (rmn_kmap_build_ordered; `order` is defined then), unless the public map exists already. Cached apart from the public maps.
+  std::shared_ptr<KernelMap> layer_map(const CoordinateMapKey& in_key, const CoordinateMapKey& out_key,
+                                       const stride_type& kernel_size, const stride_type& kernel_stride,
+                                       const stride_type& kernel_dilation, RegionType::Type region_type,
+                                       const at::Tensor& offsets, bool is_transpose);
   // {offset index -> int32 [2, P_k]} (engine/grid/space.cpp:202-228)
   std::map<int64_t, at::Tensor> kernel_map_th(const CoordinateMapKey& in_key, const CoordinateMapKey& out_key,
                                               const stride_type& kernel_size, const stride_type& kernel_stride,
@@ -215,13 +222,17 @@ private:
     uint32_t size = 0;
   };
   Map const& find(const CoordinateMapKey& key, const char* what = "") const;
+  std::shared_ptr<KernelMap> find_or_build(const CoordinateMapKey& in_key, const CoordinateMapKey& out_key,
+                                           const stride_type& kernel_size, const stride_type& kernel_stride,
+                                           const stride_type& kernel_dilation, RegionType::Type region_type,
+                                           const at::Tensor& offsets, bool is_transpose, bool is_pool, bool may_order);
   Map build(const at::Tensor& coords, const stride_type& tensor_stride, at::Tensor* mapping, at::Tensor* inverse,
             bool expect_duplicates);
 
   int D_;
   CoordinateMapBackend::Type map_type_;
   std::map<coordinate_map_key_type, Map> maps_;
-  std::map<std::string, std::shared_ptr<KernelMap>> kernel_maps_;
+  std::map<std::string, std::shared_ptr<KernelMap>> kernel_maps_, ordered_maps_;
   std::map<coordinate_map_key_type, at::Tensor> fields_;
 };
 
@@ -400,7 +411,7 @@ public:
 
 private:
   // input map -> (kernel map, output key), building or reusing the output map
-  std::pair<std::shared_ptr<KernelMap>, CoordinateMapKey> kernel_map(const SparseTensor& input);
+  std::pair<std::shared_ptr<KernelMap>, CoordinateMapKey> kernel_map(const SparseTensor& input, bool may_order = false);
 };
 
 // RiemannBatchNormImpl (engine/nn/normalization.hpp:11-34): torch's BatchNorm1d over the feature matrix.

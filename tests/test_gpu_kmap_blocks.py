@@ -76,3 +76,64 @@ def test_index_that_turns_out_too_small_gives_way_to_the_table():
     a, b = ops.kmap_build(table, table.coords, off), ops.kmap_build(table, table.coords, off, self_map=True)
     assert _index_state(b) == FULL
     assert torch.equal(a.nbr, b.nbr) and torch.equal(a.offset_ptr, b.offset_ptr)
+
+
+def _cloud(D, n, extent, stride, order, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    c = torch.cat([torch.randint(0, 3, (3 * n, 1), generator=g, device="cuda"),
+                   torch.randint(-extent // 2, extent - extent // 2, (3 * n, D), generator=g, device="cuda") * stride], 1)
+    c = torch.unique(c, dim=0)
+    c = c[torch.randperm(c.size(0), generator=g, device="cuda")][:n]
+    return (torch.unique(c, dim=0) if order == "sorted" else c).int().contiguous()
+
+
+# the index used and (thin clouds) not used, rows in spatial order, further offsets, one voxel of key bits and many
+@pytest.mark.parametrize("D,n,extent,kernel,dilation,stride,order,in_use", [
+    (3, 1_970_000, 110, 3, 1, 1, "random", True), (3, 2_000_001, 5000, 3, 1, 1, "random", False),
+    (3, 1_970_001, 100, 3, 3, 4, "sorted", True), (4, 2_100_003, 36, 3, 1, 1, "random", True),
+    (5, 1_970_000, 16, 3, 1, 2, "random", True),
+])
+def test_ordered_map_is_the_self_map_in_another_order(D, n, extent, kernel, dilation, stride, order, in_use):
+    from riemannengine_b200 import capi, ops
+    c = _cloud(D, n, extent, stride, order, D * 1000 + n)
+    table = ops.table_build(c)
+    off = ops.region_offsets(0, [kernel] * D, [dilation] * D, [stride] * D)
+    K = off.shape[0]
+    want = ops.kmap_build(table, table.coords, off).nbr
+    lib = capi.lib()
+    size = lib.rmn_kmap_ordered_workspace_bytes(n, D + 1, K)
+    assert size > 0 and lib.rmn_kmap_ordered_workspace_bytes(1_900_000, D + 1, K) == 0
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    rows, nbr = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty((K, n), dtype=torch.int32, device="cuda")
+    offsets = torch.as_tensor(off, dtype=torch.int32, device="cuda").contiguous()
+    capi.check(lib.rmn_kmap_build_ordered(ops._ptr(table.buffer), ops._ptr(table.coords), n, D + 1, ops._ptr(offsets), K,
+                                          ops._ptr(rows), ops._ptr(nbr), ops._ptr(scratch), size, ops._stream()), "ordered")
+    identity = torch.arange(n, dtype=torch.int32, device="cuda")
+    assert torch.equal(rows.sort().values, identity) and torch.equal(rows, identity) == (not in_use)
+    for k in range(K):
+        assert torch.equal(nbr[k], want[k][rows.long()])
+
+
+def test_layers_that_only_run_forward_give_the_same_rows_over_an_ordered_map():
+    """The C++ host takes an ordered map where no gradient is wanted, the public map otherwise: same bits, bias, residual and
+    padded channels included; pair lists asked for afterwards are those of the public map."""
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    n = 1_980_000
+    c = _cloud(3, n, 110, 1, "random", 7)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    for c_in, c_out in ((32, 32), (4, 20)):
+        layer = C.RiemannConvolution(c_in, c_out, kernel_size=3, stride=1, bias=True, dimension=3)
+        layer.to("cuda:0")
+        layer.to(torch.bfloat16)
+        feats = torch.randn((n, c_in), generator=g, device="cuda").bfloat16()
+        want = layer(C.SparseTensor(feats, c)).F.detach()
+        with torch.no_grad():
+            x = C.SparseTensor(feats, c)
+            got, again = layer(x), layer(x)
+        assert torch.equal(got.F, want) and torch.equal(again.F, want)
+    key = x.coordinate_map_key
+    pairs = x.coordinate_manager.kernel_map_pairs(key, got.coordinate_map_key, [3] * 3, [1] * 3, [1] * 3)
+    y = C.SparseTensor(feats, c)
+    public = y.coordinate_manager.kernel_map_pairs(y.coordinate_map_key, y.coordinate_map_key, [3] * 3, [1] * 3, [1] * 3)
+    assert all(torch.equal(torch.as_tensor(a), torch.as_tensor(b)) for a, b in zip(pairs, public))
