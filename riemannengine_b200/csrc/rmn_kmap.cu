@@ -516,7 +516,7 @@ static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_qu
       RMN_LAUNCH_CHECK();
       RMN_CUDA_TRY(launch_overlapped(k_block_scatter<kW>, grid, block, 0, stream, h, d_query, n_query, ix));
       RMN_LAUNCH_CHECK();
-      RMN_CUDA_TRY(launch_overlapped(k_kmap_blocks_self<kW, false>, dim3(148 * 6), dim3(kKmapBlock), smem, stream, h, slots, d_query,
+      RMN_CUDA_TRY(launch_overlapped(k_kmap_blocks_self<kW>, dim3(148 * 6), dim3(kKmapBlock), smem, stream, h, slots, d_query,
                                      n_query, d_offsets, K, d_nbr, block_counts, nb, ticket, ix));
       RMN_LAUNCH_CHECK();
       RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock), self_smem,
@@ -544,7 +544,7 @@ static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_qu
 
 extern "C" size_t rmn_kmap_ordered_workspace_bytes(uint32_t n_rows, int W, int K) {
   if (W > RMN_MAX_W || !may_use_block_index(n_rows, W, K)) return 0;
-  return kmap_counts_bytes(n_rows, K) + block_index_bytes(n_rows) + kBlockBuckets * sizeof(uint32_t) + 32;
+  return kmap_counts_bytes(n_rows, K) + block_index_bytes(n_rows, true) + kBlockBuckets * sizeof(uint32_t) + 32;
 }
 
 extern "C" int rmn_kmap_build_ordered(const void* d_table, const int32_t* d_coords, uint32_t n_rows, int W,
@@ -563,13 +563,12 @@ extern "C" int rmn_kmap_build_ordered(const void* d_table, const int32_t* d_coor
   uint32_t* counts = static_cast<uint32_t*>(d_workspace);
   const uint32_t nb = kmap_blocks(n_rows);
   char* index = static_cast<char*>(d_workspace) + kmap_counts_bytes(n_rows, K);
-  BlockIndex ix = block_index(index, n_rows);
+  BlockIndex ix = block_index(index, n_rows, true);
   BlockSample* sample = reinterpret_cast<BlockSample*>(ix.perm);
   ix.perm = d_order;
-  ix.buckets = reinterpret_cast<uint32_t*>(index + ((block_index_bytes(n_rows) + 15) & ~(size_t)15));
+  ix.buckets = reinterpret_cast<uint32_t*>(index + ((block_index_bytes(n_rows, true) + 15) & ~(size_t)15));
   const int half = K / 2;
   const dim3 grid(148 * 8), block(256), slot_grid((ix.capacity + 255) / 256);
-  const size_t smem = (size_t)8 * kKmapBlock * 12 + (size_t)K * 4 + (size_t)half * 4;
   const size_t self_smem = (size_t)half * 8 + (size_t)half * (W - 1) * 4 + (size_t)half * 4;
   RMN_DISPATCH_W(W, if constexpr (kW >= 4) {
     RMN_CUDA_TRY(launch_overlapped(k_block_sample<kW>, dim3(kChooseRows / 256), block, 0, stream, h, slots, d_coords, n_rows,
@@ -588,8 +587,8 @@ extern "C" int rmn_kmap_build_ordered(const void* d_table, const int32_t* d_coor
     RMN_LAUNCH_CHECK();
     RMN_CUDA_TRY(launch_overlapped(k_block_scatter<kW>, grid, block, 0, stream, h, d_coords, n_rows, ix));
     RMN_LAUNCH_CHECK();
-    RMN_CUDA_TRY(launch_overlapped(k_kmap_blocks_self<kW, true>, dim3(148 * 6), dim3(kKmapBlock), smem, stream, h, slots,
-                                   d_coords, n_rows, d_offsets, K, d_nbr, counts, nb, counts, ix));
+    RMN_CUDA_TRY(launch_overlapped(k_kmap_ordered<kW>, dim3(148 * 4), dim3(kKmapBlock), ordered_smem(K), stream, h, slots,
+                                   d_coords, n_rows, d_offsets, K, d_nbr, ix));
     RMN_LAUNCH_CHECK();
     RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock), self_smem, stream,
                                    h, slots, d_coords, n_rows, d_offsets, K, d_nbr, counts, nb,

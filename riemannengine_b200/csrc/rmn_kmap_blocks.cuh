@@ -40,13 +40,14 @@ constexpr uint32_t kIndexInUse = ~0u, kIndexNotChosen = 0u, kIndexFull = 1u;  //
 // (a surface loads two slots in five: runs of 32 taken slots occur, runs of 128 do not; 4.8 M clip rows overflowed at 32 in
 // some scenes, and took 3.0 ms by the hash table)
 constexpr uint32_t kBlockMaxProbes = 128;
-inline uint32_t block_index_capacity(uint32_t n) { return n / 8 + 64; }
-inline size_t block_index_bytes(uint32_t n) {
-  return (size_t)block_index_capacity(n) * sizeof(BlockSlot) + 32 + (size_t)n * 8;
+// (For an ordered map, whose lookups wait for the longest of 27, it is one per four: 1141 -> 1004 us.)
+inline uint32_t block_index_capacity(uint32_t n, bool ordered = false) { return n / (ordered ? 4 : 8) + 64; }
+inline size_t block_index_bytes(uint32_t n, bool ordered = false) {
+  return (size_t)block_index_capacity(n, ordered) * sizeof(BlockSlot) + 32 + (size_t)n * 8;
 }
-inline BlockIndex block_index(void* workspace, uint32_t n) {
+inline BlockIndex block_index(void* workspace, uint32_t n, bool ordered = false) {
   BlockIndex b;
-  b.capacity = block_index_capacity(n);
+  b.capacity = block_index_capacity(n, ordered);
   b.slots = static_cast<BlockSlot*>(workspace);
   b.counter = reinterpret_cast<uint32_t*>(b.slots + b.capacity);
   b.state = b.counter + 1;
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(1024) k_block_choose(const TableHeader* __rest
     const float part = fminf(1.f, 0.5f * (float)s_inside[1] / (float)s_inside[0]);
     const float set = part * ((float)h->capacity * sizeof(Slot));
     if (tid == 0)
-      s_serves = (ix.buckets || set > kChooseBytes) && blocks / kChooseBlocks * (float)n <= kChooseLoad * (float)ix.capacity ? 1u : 0u;
+      s_serves = (ix.buckets || set > kChooseBytes) && blocks / kChooseBlocks * (float)n <= kChooseLoad * (float)(n / 8) ? 1u : 0u;
   }
   __syncthreads();
   const bool serves = s_serves != 0u;
@@ -251,8 +252,9 @@ __global__ void __launch_bounds__(256) k_block_insert(const TableHeader* __restr
 }
 
 // The ranges of perm in an ordered map: blocks that share the highest bits of their key - batch, further axes, layers of blocks along
-// the third axis - lie together, so that the rows which a stretch of the convolution gathers stay in the L2. Rows per bucket,
-// their exclusive sums (one block), and a range for every block.
+// the third axis - lie together, so that the rows which a stretch of the convolution gathers stay in the L2. (Rows of blocks
+// along the second axis, too: 1004 -> 992 us, and more to add up.) Rows per bucket, their exclusive sums (one block), and a
+// range for every block.
 __device__ __forceinline__ uint32_t block_bucket(const TableHeader* h, unsigned long long key) {
   return (uint32_t)(key >> (h->total_bits > kBlockBucketBits ? h->total_bits - kBlockBucketBits : 0u));
 }
@@ -271,11 +273,11 @@ __global__ void __launch_bounds__(1024) k_block_bucket_sums(BlockIndex ix) {
   __shared__ uint32_t s_warp[32];
   constexpr uint32_t PER = kBlockBuckets / 1024;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t v[PER], sum = 0;
-#pragma unroll
-  for (uint32_t i = 0; i < PER; ++i) {
-    v[i] = ix.buckets[threadIdx.x * PER + i];
-    sum += v[i];
+  uint4* mine = reinterpret_cast<uint4*>(ix.buckets + threadIdx.x * PER);
+  uint32_t sum = 0;
+  for (uint32_t i = 0; i < PER / 4; ++i) {
+    const uint4 v = mine[i];
+    sum += v.x + v.y + v.z + v.w;
   }
   uint32_t incl = sum;
 #pragma unroll
@@ -287,10 +289,10 @@ __global__ void __launch_bounds__(1024) k_block_bucket_sums(BlockIndex ix) {
   __syncthreads();
   uint32_t run = incl - sum;
   for (uint32_t w = 0; w < warp; ++w) run += s_warp[w];
-#pragma unroll
-  for (uint32_t i = 0; i < PER; ++i) {
-    ix.buckets[threadIdx.x * PER + i] = run;
-    run += v[i];
+  for (uint32_t i = 0; i < PER / 4; ++i) {
+    const uint4 v = mine[i];
+    mine[i] = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+    run += v.x + v.y + v.z + v.w;
   }
 }
 
@@ -345,24 +347,19 @@ __global__ void __launch_bounds__(256) k_block_scatter(const TableHeader* __rest
 // use: 2450 -> 2324 us for the four clips). Offsets that reach further than two voxels (in units of the map's grid) along a
 // block axis look their row up in the hash table instead. Where the blocks did not fit, the mirrored half of the table is
 // filled with "no neighbour" for k_kmap_probe_self, which follows.
-// kOrdered: the map is written in the order of perm, block by block: position p is row perm[p], entries are row numbers. The rows
-// of a warp then share their blocks, and what they read of the index comes from the L1. Nothing is counted; where the index is
-// not in use perm becomes the identity.
-template <int W, bool kOrdered>
+template <int W>
 __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots, const int32_t* __restrict__ coords, uint32_t n,
     const int32_t* __restrict__ offsets, int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts,
     uint32_t n_blocks, uint32_t* __restrict__ scan_ticket, BlockIndex ix) {
   after_previous_kernel();
   if (*ix.state != kIndexInUse) {
-    if constexpr (kOrdered)
-      for (uint32_t row = blockIdx.x * kKmapBlock + threadIdx.x; row < n; row += gridDim.x * kKmapBlock) ix.perm[row] = (int32_t)row;
     if (*ix.state == kIndexFull)
       for (uint32_t row = blockIdx.x * kKmapBlock + threadIdx.x; row < n; row += gridDim.x * kKmapBlock)
         for (int k = K / 2 + 1; k < K; ++k) __stcs(nbr + (size_t)k * n + row, -1);
     return;
   }
-  if (!kOrdered && blockIdx.x == 0 && threadIdx.x == 0) *scan_ticket = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scan_ticket = 0;
   using B = BlockCoords<W>;
   constexpr int D = W - 1, NA = B::NA, CELLS = 1 << NA;
   constexpr uint32_t kNever = 1u << 28, kFar = 1u << 29, kNewOuter = 1u << 30;
@@ -411,7 +408,7 @@ __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
     int32_t c[W];
 #pragma unroll
     for (int i = 0; i < W; ++i) c[i] = h->mn[i];
-    if (active) load_row<W>(coords, kOrdered ? (uint32_t)ix.perm[q] : q, c);
+    if (active) load_row<W>(coords, q, c);
     B b;
     b.load(h, c);
     // per block axis: the neighbouring block on the side of the row's half of its block, if any offset reaches it
@@ -497,16 +494,232 @@ __global__ void __launch_bounds__(kKmapBlock, 6) k_kmap_blocks_self(
         hit = uid != 0xFFFFFFFFu;
       }
       if (active) __stcs(dst, (int32_t)uid);
-      if (!kOrdered && k < half) {  // (the other half has the same counts, see k_kmap_scan)
+      if (k < half) {  // (the other half has the same counts, see k_kmap_scan)
         const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
         if (lane == 0) atomicAdd(&s_cnt[k], (uint32_t)__popc(hits));
       }
     }
-    if constexpr (kOrdered) continue;
     __syncthreads();
     for (int k = threadIdx.x; k < half; k += kKmapBlock) block_counts[(size_t)k * n_blocks + row_block] = s_cnt[k];
     if (threadIdx.x == 0)
       block_counts[(size_t)half * n_blocks + row_block] = min((uint32_t)kKmapBlock, n - row_block * kKmapBlock);
+  }
+}
+
+// The map in the order of perm, block by block (rmn_kmap_build_ordered): position p is row perm[p], entries are row numbers,
+// nothing is counted. The positions of a CUDA block lie in a dozen or two blocks of the index, so these are looked up with the
+// 26 around them once for all their rows, a warp per block and a lane per cell; rows test bits in shared memory, and the row
+// numbers that they read lie next to one another. What
+// bounds it is issued instructions: 4.8 M clip rows x 81 offsets with the index 2250 us by k_kmap_blocks_self, 1700 by the same
+// kernel walking perm, 1200 here (270 the index, 260 looking blocks up, 550 the rows, of them 160 the stores).
+// Where the index is not in use perm becomes the identity, and k_kmap_probe_self follows.
+constexpr int kOrderedCells = 27, kOrderedChunk = 32;  // blocks in shared memory at a time
+struct OrderedHalf {  // half of a block's mask (32 voxels) and the position in perm of its first row
+  uint32_t mask, base;
+};
+inline size_t ordered_smem(int K) { return (size_t)kOrderedChunk * kOrderedCells * 2 * sizeof(OrderedHalf) + (size_t)K * 4; }
+
+template <int W>
+__global__ void __launch_bounds__(kKmapBlock, 4) k_kmap_ordered(
+    const TableHeader* __restrict__ h, const Slot* __restrict__ slots, const int32_t* __restrict__ coords, uint32_t n,
+    const int32_t* __restrict__ offsets, int K, int32_t* __restrict__ nbr, BlockIndex ix) {
+  after_previous_kernel();
+  if (*ix.state != kIndexInUse) {
+    for (uint32_t row = blockIdx.x * kKmapBlock + threadIdx.x; row < n; row += gridDim.x * kKmapBlock) {
+      ix.perm[row] = (int32_t)row;
+      if (*ix.state == kIndexFull)
+        for (int k = K / 2 + 1; k < K; ++k) __stcs(nbr + (size_t)k * n + row, -1);
+    }
+    return;
+  }
+  using B = BlockCoords<W>;
+  constexpr int D = W - 1, NA = B::NA;
+  constexpr uint32_t kCube = 1u << 27, kNever = 1u << 28, kFar = 1u << 29, kNewOuter = 1u << 30;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  OrderedHalf* s_half = reinterpret_cast<OrderedHalf*>(smem_raw);                               // [chunk][cell][half]
+  uint32_t* s_off = reinterpret_cast<uint32_t*>(s_half + kOrderedChunk * kOrderedCells * 2);  // [K] nibbles modulo 8, flags
+  __shared__ unsigned long long s_key[kKmapBlock];  // of the blocks of this CUDA block, moved along the outer axes
+  __shared__ uint8_t s_sides[kKmapBlock];           // bit 2 a (+ 1): the box goes on below (above) the block along axis a
+  __shared__ uint32_t s_slot[kKmapBlock], s_heads[kKmapBlock / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int k = tid; k < K; k += kKmapBlock) {
+    uint32_t e = 0;
+    int32_t step[NA];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+      const int32_t o = __ldg(offsets + k * D + a);
+      const uint32_t s = h->low_shift(a);
+      if (o & ((1 << s) - 1)) e |= kNever;  // off the map's grid
+      step[a] = o >> s;
+      if (step[a] < -2 || step[a] > 2) e |= kFar;
+      e |= ((uint32_t)step[a] & 7u) << (4 * a);
+    }
+    bool new_outer = k == 0;
+#pragma unroll
+    for (int a = NA; a < D; ++a) new_outer |= k > 0 && __ldg(offsets + k * D + a) != __ldg(offsets + (k - 1) * D + a);
+    if (new_outer) e |= kNewOuter;
+    bool cube = new_outer && k + kOrderedCells <= K;  // the 27 steps of -1, 0, 1, the first axis fastest
+    for (int j = 0; cube && j < kOrderedCells; ++j)
+      for (int a = 0, c = j; a < D; ++a, c /= 3)
+        cube = cube && __ldg(offsets + (k + j) * D + a) == (a < NA ? (c % 3 - 1) * (1 << h->low_shift(a)) : __ldg(offsets + k * D + a));
+    if (cube) e |= kCube;
+    s_off[k] = e;
+  }
+  // this lane's cell: its distance in keys, and the sides of a block on which the box has to go on
+  unsigned long long cell_step = 0;
+  uint32_t cell_sides = 0;
+#pragma unroll
+  for (int a = 0, c = (int)lane; a < NA; ++a, c /= 3) {
+    const int d = c % 3 - 1;
+    cell_step += (unsigned long long)((long long)d * (1ll << h->shift[a + 1]));
+    if (d) cell_sides |= 1u << (2 * a + (d > 0 ? 1 : 0));
+  }
+  const uint32_t n_blocks = (n + kKmapBlock - 1) / kKmapBlock;
+  for (uint32_t row_block = blockIdx.x; row_block < n_blocks; row_block += gridDim.x) {
+    const uint32_t q = row_block * kKmapBlock + tid;
+    const bool active = q < n;
+    const uint32_t row = active ? (uint32_t)__ldg(ix.perm + q) : 0u;
+    int32_t c[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) c[i] = h->mn[i];
+    if (active) load_row<W>(coords, row, c);
+    B b;
+    b.load(h, c);
+    // number the blocks of these positions
+    __syncthreads();  // (the lists of the positions before have been read)
+    s_slot[tid] = active ? __ldg(ix.slot_of_row + row) : ~0u;
+    __syncthreads();
+    const bool head = active && (tid == 0 || s_slot[tid] != s_slot[tid - 1]);
+    const uint32_t heads = __ballot_sync(0xFFFFFFFFu, head);
+    if (lane == 0) s_heads[warp] = __popc(heads);
+    __syncthreads();
+    uint32_t mine = __popc(heads & ((2u << lane) - 1u)) - 1u, n_own = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kKmapBlock / 32; ++w) {
+      if (w < warp) mine += s_heads[w];
+      n_own += s_heads[w];
+    }
+    if (head) {
+      uint32_t sides = 0;
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        const uint32_t last = (((uint32_t)(h->mx[a + 1] - h->mn[a + 1])) >> h->low_shift(a)) >> 2;
+        sides |= (b.block[a] > 0 ? 1u : 0u) << (2 * a) | (b.block[a] < last ? 2u : 0u) << (2 * a);
+      }
+      s_sides[mine] = (uint8_t)sides;
+    }
+    int32_t* dst = nbr + q;
+    for (int k0 = 0, k1; k0 < K; k0 = k1) {  // the offsets that share their steps along the outer axes
+      for (k1 = k0 + 1; k1 < K && !(s_off[k1] & kNewOuter);) ++k1;
+      if (head) {
+        unsigned long long key = b.key;
+        bool in_box = true;
+#pragma unroll
+        for (int a = NA; a < D; ++a) {
+          const int32_t o = __ldg(offsets + k0 * D + a);
+          in_box = in_box && b.dist[a + 1] + (uint32_t)o <= (uint32_t)(h->mx[a + 1] - h->mn[a + 1]);
+          key += (unsigned long long)((long long)o << h->shift[a + 1]);
+        }
+        s_key[mine] = in_box ? key : kEmptyKey;
+      }
+      for (uint32_t chunk = 0; chunk < n_own; chunk += kOrderedChunk) {
+        __syncthreads();  // (the keys are there, the cells before have been read)
+        constexpr uint32_t WARPS = kKmapBlock / 32;
+        for (uint32_t j = warp; j < kOrderedChunk && chunk + j < n_own; j += 2 * WARPS) {  // two lookups in flight
+          unsigned long long key[2];
+          uint32_t at[2];
+          ulonglong2 v[2];
+#pragma unroll
+          for (uint32_t i = 0; i < 2; ++i) {
+            const uint32_t own = j + i * WARPS;
+            const unsigned long long origin = own < kOrderedChunk && chunk + own < n_own ? s_key[chunk + own] : kEmptyKey;
+            key[i] = origin + cell_step;
+            at[i] = block_hash(key[i], ix.capacity);
+            v[i] = make_ulonglong2(kEmptyKey, ~0ull);
+            if (lane < kOrderedCells && origin != kEmptyKey && !(cell_sides & ~s_sides[chunk + own]))
+              v[i] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[i]));
+          }
+#pragma unroll
+          for (uint32_t i = 0; i < 2; ++i) {
+            const uint32_t own = j + i * WARPS;
+            for (uint32_t probe = 1; v[i].x != key[i] && v[i].x != kEmptyKey && probe < kBlockMaxProbes; ++probe) {
+              if (++at[i] == ix.capacity) at[i] = 0;
+              v[i] = __ldg(reinterpret_cast<const ulonglong2*>(ix.slots + at[i]));
+            }
+            const bool found = v[i].x == key[i];
+            const uint32_t lo = found ? (uint32_t)~v[i].y : 0u, hi = found ? (uint32_t)(~v[i].y >> 32) : 0u;
+            const uint32_t base = found ? __ldg(&ix.slots[at[i]].base) : 0u;
+            if (lane < kOrderedCells && own < kOrderedChunk)
+              *reinterpret_cast<uint4*>(s_half + (own * kOrderedCells + lane) * 2) = make_uint4(lo, base, hi, base + __popc(lo));
+          }
+        }
+        __syncthreads();
+        if (!active || mine - chunk >= (uint32_t)kOrderedChunk) continue;
+        const OrderedHalf* half_of = s_half + (mine - chunk) * kOrderedCells * 2;
+        // cell beside the block along an axis, from the nibble of a position: 0..3 the block itself, 4, 5 above, 6, 7 below
+        auto beside = [](uint32_t nibble) { return nibble & 4u ? (nibble & 2u ? 0u : 2u) : 1u; };
+        int32_t* out = dst + (size_t)k0 * n;
+        int k = k0;
+        if (s_off[k0] & kCube) {
+          // Steps -1, 0, 1 along the first axis are neighbouring bits of a row of four, whose ranks differ by the bits between
+          // them, and at the block's edge one bit of the block beside it.
+          const uint32_t x = b.local & 3u, edge_x = x ? 0u : 3u;
+          const int edge_cell = x < 2u ? -2 : 2;
+          uint32_t cell_y[3], shift_y[3];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const uint32_t y = (((b.local >> 4) & 3u) + (uint32_t)i - 1u) & 7u;
+            cell_y[i] = beside(y) * 6u;
+            shift_y[i] = 4u * (y & 3u);
+          }
+#pragma unroll
+          for (int iz = 0; iz < 3; ++iz) {
+            const uint32_t z = (((b.local >> 8) & 3u) + (uint32_t)iz - 1u) & 7u;
+            const OrderedHalf* plane = half_of + beside(z) * 18u + 2u + ((z >> 1) & 1u);
+            const uint32_t shift_z = 16u * (z & 1u);
+#pragma unroll
+            for (int iy = 0; iy < 3; ++iy) {
+              const OrderedHalf* cell = plane + cell_y[iy];
+              const uint2 own = *reinterpret_cast<const uint2*>(cell), edge = *reinterpret_cast<const uint2*>(cell + edge_cell);
+              const uint32_t shift = shift_y[iy] + shift_z, at = shift + x, edge_at = shift + edge_x;
+              const uint32_t edge_bit = (edge.x >> edge_at) & 1u;
+              const uint32_t window = ((own.x >> shift) & 15u) << 1 | (x == 0u ? edge_bit : 0u) | (x == 3u ? edge_bit << 5 : 0u);
+              const uint32_t hits = window >> x;
+              const uint32_t centre = own.y + __popc(own.x & ((1u << at) - 1u));
+              const uint32_t other = edge.y + __popc(edge.x & ((1u << edge_at) - 1u));
+              int32_t v[3] = {-1, -1, -1};
+              if (hits & 1u) v[0] = __ldg(ix.perm + (x ? centre - 1u : other));
+              if (hits & 2u) v[1] = __ldg(ix.perm + centre);
+              if (hits & 4u) v[2] = __ldg(ix.perm + (x < 3u ? centre + ((hits >> 1) & 1u) : other));
+#pragma unroll
+              for (int i = 0; i < 3; ++i, out += n) __stcs(out, v[i]);
+            }
+          }
+          k += kOrderedCells;
+        }
+        for (; k < k1; ++k, out += n) {
+          const uint32_t e = s_off[k];
+          uint32_t uid = 0xFFFFFFFFu;
+          if (!(e & (kNever | kFar))) {
+            const uint32_t p = b.local + (e & 0xFFFu), bit = B::bit(p);
+            const uint32_t cell = 9 * beside((p >> 8) & 7u) + 3 * beside((p >> 4) & 7u) + beside(p & 7u);
+            const OrderedHalf m = half_of[cell * 2 + (bit >> 5)];
+            if ((m.mask >> (bit & 31u)) & 1u) uid = (uint32_t)__ldg(ix.perm + m.base + __popc(m.mask & ((1u << (bit & 31u)) - 1u)));
+          } else if (!(e & kNever)) {
+            bool in_box = true;
+            unsigned long long key = 0;
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+              const uint32_t d = b.dist[i] + (i > 0 ? (uint32_t)__ldg(offsets + k * D + i - 1) : 0u);
+              in_box = in_box && d <= (uint32_t)(h->mx[i] - h->mn[i]);
+              key |= (unsigned long long)d << h->shift[i];
+            }
+            if (in_box) uid = table_find(slots, h->capacity, h->pos_shift, key);
+          }
+          __stcs(out, (int32_t)uid);
+        }
+      }
+    }
   }
 }
 
