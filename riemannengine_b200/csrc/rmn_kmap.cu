@@ -372,9 +372,27 @@ __global__ void __maxnreg__(32) k_kmap_pairs_background(
   kmap_pairs_body(nbr, n_query, K, offset_ptr, block_prefix, n_blocks, a_idx, q_idx, capacity, overflow);
 }
 
+// n entries "no neighbour" (a launch that overlaps its neighbours, where a memset would not)
+__global__ void __launch_bounds__(256) k_kmap_clear(int32_t* __restrict__ nbr, size_t n) {
+  after_previous_kernel();
+  // single words up to the first 16-byte boundary and behind the last one
+  const size_t head = min(n, (size_t)(((16 - ((uintptr_t)nbr & 15)) & 15) / 4)), vecs = (n - head) / 4, tail = head + 4 * vecs;
+  const size_t first = (size_t)blockIdx.x * 256 + threadIdx.x, step = (size_t)gridDim.x * 256;
+  const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (size_t i = first; i < vecs; i += step) reinterpret_cast<uint4*>(nbr + head)[i] = ones;
+  if (first < head) nbr[first] = -1;
+  if (tail + first < n) nbr[tail + first] = -1;
+}
+inline cudaError_t clear_entries(int32_t* nbr, size_t n, cudaStream_t stream) {
+  const size_t blocks = (n / 4 + 255) / 256 + 1;
+  count_launch();
+  return launch_overlapped(k_kmap_clear, dim3((uint32_t)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, nbr, n);
+}
+
 __global__ void __launch_bounds__(256) k_kmap_transpose(const int32_t* __restrict__ nbr,
                                                         uint32_t n_query, int K, uint32_t n_a,
                                                         int32_t* __restrict__ nbr_t) {
+  after_previous_kernel();
   const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= (uint64_t)K * n_query) return;
   const int32_t a = __ldg(nbr + i);
@@ -525,8 +543,7 @@ static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_qu
     });
   } else if (self) {
     if (half > 0)  // the mirrored half starts as "no neighbour"
-      RMN_CUDA_TRY(cudaMemsetAsync(d_nbr + (size_t)(half + 1) * n_query, 0xFF, (size_t)half * n_query * sizeof(int32_t),
-                                   stream));
+      RMN_CUDA_TRY(clear_entries(d_nbr + (size_t)(half + 1) * n_query, (size_t)half * n_query, stream));
     RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock),
                                                      self_smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr,
                                                      block_counts, nb, ticket, nullptr)));
@@ -683,12 +700,12 @@ extern "C" int rmn_kmap_transpose(const int32_t* d_nbr, uint32_t n_query, int K,
   if (K < 1) return RMN_ERR_BAD_ARG;
   if (n_a == 0) return RMN_OK;
   if (!d_nbr_t) return RMN_ERR_BAD_ARG;
-  RMN_CUDA_TRY(cudaMemsetAsync(d_nbr_t, 0xFF, (size_t)K * n_a * sizeof(int32_t), stream));
+  RMN_CUDA_TRY(clear_entries(d_nbr_t, (size_t)K * n_a, stream));
   if (n_query == 0) return RMN_OK;
   if (!d_nbr) return RMN_ERR_BAD_ARG;
   const uint64_t total = (uint64_t)K * n_query;
-  k_kmap_transpose<<<(uint32_t)((total + 255) / 256), 256, 0, stream>>>(d_nbr, n_query, K, n_a,
-                                                                       d_nbr_t);
+  RMN_CUDA_TRY(launch_overlapped(k_kmap_transpose, dim3((uint32_t)((total + 255) / 256)), dim3(256), 0, stream, d_nbr, n_query, K,
+                                 n_a, d_nbr_t));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }

@@ -2,12 +2,11 @@
 // stride alignment. Integer work bound by HBM/L2 bandwidth.
 //
 // Build pipeline (all on the caller's stream, no host synchronisation):
-//   256-byte memset of the header
+//   header cleared
 //   -> fill + range (slots to the empty pattern, column min/max; the last block plans the bit packing)
-//   -> insert (one 16-byte CAS on the packed key, atomicMin on the first row)
-//   -> count (first rows per 256-row block, from the bits of the others; the last block scans the counts and, where the
-//      caller waits for them, stores the header's words into the host's memory)
-//   -> finalize (unique ids, mapping, unique coordinates; identity inverse when nothing was a duplicate)
+//   -> insert (one 16-byte CAS on the packed key, atomicMin on the first row; marks and counts the repeated rows)
+//   -> finalize (number of unique rows, stored into the host's memory first where the caller waits for it; unique ids, mapping,
+//      unique coordinates; identity inverse when nothing was a duplicate)
 //   -> inverse (only does work when there were duplicates)
 // Up to kSmallRows rows one block does all of it in one launch.
 // Numbering unique rows by first occurrence reproduces the reference CPU map
@@ -34,25 +33,29 @@ const uint32_t* tc_status_device_address();
 constexpr int kRowsPerBlock = 256;
 constexpr uint32_t kGrid = 148 * 8;  // blocks of the passes that may have nothing to do
 
-// Scratch of a build of n rows: slot of every row, rows that are the first of their key per 256-row block (then the
-// blocks' offsets), and one bit per row that is not the first of its key
+// Scratch of a build of n rows: slot of every row, one bit per row that is not the first of its key, and how many of these
+// every kSuperBlocks blocks of 256 rows hold (with them and the bits of its own super-block a block of k_finalize numbers its
+// rows without a scan: 5 to 8 us less than a pass that counts and scans)
 struct Scratch {
   uint32_t* slot_of_row;
-  uint32_t* block_counts;
+  uint32_t* super_repeats;
   uint32_t* repeat_bits;
 };
+constexpr uint32_t kSuperBlocks = 64, kSuperRows = kSuperBlocks * kRowsPerBlock;
+// Counted by k_insert, or where many duplicates are expected by k_super_repeats from the bits: there the atomics would serialise
+// (1.2 M rows on 0.27 M strided cells: insert 33 us without them, 60 with sixteen counters per super-block, 80 with one).
+constexpr size_t super_words(size_t n) { return ((n + kSuperRows - 1) / kSuperRows + 3) / 4 * 4; }
 constexpr size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 constexpr size_t scratch_bytes(size_t n) {
   const size_t nb = (n + kRowsPerBlock - 1) / kRowsPerBlock;
-  return align16(n * 4) + align16((nb + 1) * 4) + nb * (kRowsPerBlock / 8) + 256;
+  return align16(n * 4) + super_words(n) * 4 + nb * (kRowsPerBlock / 8) + 256;
 }
 inline Scratch scratch(void* workspace, uint32_t n) {
-  const size_t nb = (n + kRowsPerBlock - 1) / kRowsPerBlock;
   char* p = reinterpret_cast<char*>(((uintptr_t)workspace + 15) & ~(uintptr_t)15);
   Scratch s;
   s.slot_of_row = reinterpret_cast<uint32_t*>(p);
-  s.block_counts = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4));
-  s.repeat_bits = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4) + align16((nb + 1) * 4));
+  s.super_repeats = reinterpret_cast<uint32_t*>(p + align16((size_t)n * 4));
+  s.repeat_bits = s.super_repeats + super_words(n);
   return s;
 }
 
@@ -95,14 +98,19 @@ __device__ void write_header(TableHeader* h, uint32_t W, uint32_t n, uint32_t ca
   plan_packing(h);
 }
 
-// First kernel of a build, on a header that a 256-byte memset has zeroed: fills the slots with the empty
+// (a launch that overlaps its neighbours, where a memset would not)
+__global__ void __launch_bounds__(64) k_clear_header(uint32_t* __restrict__ words) {
+  after_previous_kernel();
+  words[threadIdx.x] = 0u;
+}
+
+// First pass of a build, on a cleared header: fills the slots with the empty
 // pattern (all ones) and reduces the column bounds of the rows in the same pass (the fill writes, the
 // reduction reads: one launch moves both at HBM speed). The last block to finish writes the header's
 // constants, decodes the bounds and plans the key packing.
 template <int W>
 __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ coords, uint32_t n,
-                                                    TableHeader* h, uint4* __restrict__ slots, uint32_t capacity,
-                                                    uint32_t* __restrict__ repeat_bits) {
+                                                    TableHeader* h, uint4* __restrict__ slots, uint32_t capacity, Scratch sc) {
   after_previous_kernel();
   __shared__ int32_t s_mn[8][W], s_mx[8][W];
   constexpr int NA = W - 1 < 3 ? W - 1 : 3;
@@ -111,7 +119,8 @@ __global__ void __launch_bounds__(256) k_fill_range(const int32_t* __restrict__ 
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < capacity; i += gridDim.x * blockDim.x)
     slots[i] = ones;
   const uint32_t bit_words = (n + kRowsPerBlock - 1) / kRowsPerBlock * (kRowsPerBlock / 32);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < bit_words; i += gridDim.x * blockDim.x) repeat_bits[i] = 0u;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < bit_words; i += gridDim.x * blockDim.x) sc.repeat_bits[i] = 0u;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < super_words(n); i += gridDim.x * blockDim.x) sc.super_repeats[i] = 0u;
   int32_t mn[W], mx[W];
 #pragma unroll
   for (int c = 0; c < W; ++c) { mn[c] = INT_MAX; mx[c] = INT_MIN; }
@@ -261,104 +270,53 @@ __global__ void __launch_bounds__(256) k_insert(const int32_t* __restrict__ coor
   }
   const uint32_t own = __ballot_sync(0xFFFFFFFFu, repeat == row);  // (rows of a warp share a word)
   if ((threadIdx.x & 31) == 0 && own) atomicOr(sc.repeat_bits + (row >> 5), own);
-  if (repeat != kNoRow && repeat != row) atomicOr(sc.repeat_bits + (repeat >> 5), 1u << (repeat & 31));
-  const int dups = __syncthreads_count(repeat != kNoRow);  // one atomic per block: the rows' own would serialise on the word
-  if (threadIdx.x == 0 && dups) atomicAdd(&h->n_dups, (uint32_t)dups);
-}
-
-// In-place exclusive scan of counts[n] by ONE block (any multiple of 32 threads up to 1024), sixteen counts per thread and
-// step; returns the total. Reads bypass the L1: the counts may have been written by other blocks of the same launch.
-// counts is 16-byte aligned and may be read up to the next multiple of four.
-__device__ __forceinline__ uint32_t scan_u32_block(uint32_t* __restrict__ counts, uint32_t n) {
-  __shared__ uint32_t warp_sums[33];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  uint32_t carry = 0;
-  for (uint32_t base = 0; base < n; base += blockDim.x * 16u) {
-    const uint32_t i0 = base + threadIdx.x * 16u;
-    uint32_t v[16];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint4 x = make_uint4(0u, 0u, 0u, 0u);
-      if (i0 + 4 * q < n) x = __ldcg(reinterpret_cast<const uint4*>(counts + i0) + q);
-      v[4 * q] = x.x, v[4 * q + 1] = x.y, v[4 * q + 2] = x.z, v[4 * q + 3] = x.w;
-    }
-    uint32_t sum = 0;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const uint32_t x = i0 + i < n ? v[i] : 0u;
-      v[i] = sum;
-      sum += x;
-    }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-      if (lane >= (uint32_t)d) incl += t;
-    }
-    __syncthreads();  // (the sums of the step before have been read)
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      const uint32_t w = lane < nwarps ? warp_sums[lane] : 0u;
-      uint32_t wi = w;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wi, d);
-        if (lane >= (uint32_t)d) wi += t;
-      }
-      warp_sums[lane] = wi - w;  // exclusive
-      if (lane == 31) warp_sums[32] = wi;
-    }
-    __syncthreads();
-    const uint32_t before = carry + warp_sums[warp] + incl - sum;
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (i0 + i < n) counts[i0 + i] = before + v[i];
-    carry += warp_sums[32];
+  if (repeat != kNoRow && repeat != row) {
+    atomicOr(sc.repeat_bits + (repeat >> 5), 1u << (repeat & 31));
+    if (!look_first) atomicAdd(sc.super_repeats + repeat / kSuperRows, 1u);
   }
-  return carry;
-}
-
-// Rows that are the first of their key, counted per 256-row block from the bits of those that are not (one thread per
-// block); the last CUDA block to finish turns the numbers into block offsets (exclusive scan) and writes n_unique. Nothing
-// to do when the insert pass met no duplicate: nothing is compacted then (see k_finalize).
-__global__ void __launch_bounds__(256) k_count_first(uint32_t n, TableHeader* h, Scratch sc, HostPost post) {
-  after_previous_kernel();
-  const bool failed = h->status != RMN_OK;
-  if (failed || h->n_dups == 0) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      if (!failed) h->n_unique = n;
-      post.store(h, failed ? 0u : n);
-    }
-    return;
-  }
-  __shared__ uint32_t s_last;
-  const uint32_t nb = (n + kRowsPerBlock - 1) / kRowsPerBlock;
-  const uint32_t block = blockIdx.x * 256 + threadIdx.x;
-  if (block < nb) {
-    uint32_t repeats = 0;
-#pragma unroll
-    for (int w = 0; w < kRowsPerBlock / 32; ++w) repeats += __popc(__ldg(sc.repeat_bits + block * (kRowsPerBlock / 32) + w));
-    sc.block_counts[block] = min((uint32_t)kRowsPerBlock, n - block * kRowsPerBlock) - repeats;
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&h->count_blocks_done, 1u) == gridDim.x - 1 ? 1u : 0u;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const uint32_t n_unique = scan_u32_block(sc.block_counts, nb);
+  // one atomic per block: the rows' own would serialise on the words
+  const int dups = __syncthreads_count(repeat != kNoRow);
+  const int dups_here = dups && !look_first ? __syncthreads_count(repeat == row) : 0;
   if (threadIdx.x == 0) {
-    h->n_unique = n_unique;
-    post.store(h, n_unique);
+    if (dups_here) atomicAdd(sc.super_repeats + blockIdx.x / kSuperBlocks, (uint32_t)dups_here);
+    if (dups) atomicAdd(&h->n_dups, (uint32_t)dups);
   }
+}
+
+__global__ void __launch_bounds__(256) k_super_repeats(uint32_t n, const TableHeader* __restrict__ h, Scratch sc) {
+  after_previous_kernel();
+  if (h->status != RMN_OK || h->n_dups == 0) return;
+  const uint32_t words = (n + kRowsPerBlock - 1) / kRowsPerBlock * (kRowsPerBlock / 32);
+  const uint32_t super = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  uint32_t count = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < kSuperRows / 32; i += 32) {
+    const uint32_t at = super * (kSuperRows / 32) + i + lane;
+    if (at < words) count += __popc(__ldg(sc.repeat_bits + at));
+  }
+  count = __reduce_add_sync(0xFFFFFFFFu, count);
+  if (lane == 0 && super * (kSuperRows / 32) < words) sc.super_repeats[super] = count;
+}
+
+// (one thread, behind k_insert) the number of unique rows: every row but the first of its key has lost once
+__device__ __forceinline__ void publish_unique(TableHeader* h, uint32_t n, const HostPost& post) {
+  const bool ok = h->status == RMN_OK;
+  const uint32_t n_unique = ok ? n - h->n_dups : 0u;
+  if (ok) h->n_unique = n_unique;
+  post.store(h, n_unique);
+}
+__global__ void k_publish_unique(uint32_t n, TableHeader* h) {
+  after_previous_kernel();
+  publish_unique(h, n, HostPost{});
 }
 
 template <int W>
 __global__ void __launch_bounds__(kRowsPerBlock) k_finalize(
-    const int32_t* __restrict__ coords, uint32_t n, const TableHeader* h, Slot* slots,
-    Scratch sc, int64_t* __restrict__ mapping, int32_t* __restrict__ unique_coords, int64_t* __restrict__ inverse) {
+    const int32_t* __restrict__ coords, uint32_t n, TableHeader* h, Slot* slots,
+    Scratch sc, int64_t* __restrict__ mapping, int32_t* __restrict__ unique_coords, int64_t* __restrict__ inverse,
+    HostPost post) {
   after_previous_kernel();
+  if (blockIdx.x == 0 && threadIdx.x == 0) publish_unique(h, n, post);
   if (h->status != RMN_OK) return;
   const uint32_t row = blockIdx.x * kRowsPerBlock + threadIdx.x;
   if (h->n_dups == 0) {
@@ -374,14 +332,26 @@ __global__ void __launch_bounds__(kRowsPerBlock) k_finalize(
         for (int i = 0; i < W; ++i) unique_coords[(size_t)row * W + i] = c[i];
       }
     }
-    if (row == 0) const_cast<TableHeader*>(h)->n_unique = n;
     return;
   }
-  if (row >= n) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // repeated rows before this block
+  __shared__ uint32_t s_before[kRowsPerBlock / 32];
+  uint32_t before = 0;
+  const uint32_t super = blockIdx.x / kSuperBlocks;
+  for (uint32_t i = threadIdx.x; i < super; i += kRowsPerBlock) before += __ldg(sc.super_repeats + i);
+  for (uint32_t i = super * (kSuperRows / 32) + threadIdx.x; i < blockIdx.x * (kRowsPerBlock / 32); i += kRowsPerBlock)
+    before += __popc(__ldg(sc.repeat_bits + i));
+  before = __reduce_add_sync(0xFFFFFFFFu, before);
+  if (lane == 0) s_before[warp] = before;
+  __syncthreads();
+  if (row >= n) return;
+  before = 0;
+#pragma unroll
+  for (int w = 0; w < kRowsPerBlock / 32; ++w) before += s_before[w];
   const uint32_t* bits = sc.repeat_bits + blockIdx.x * (kRowsPerBlock / 32);
   if ((__ldg(bits + warp) >> lane) & 1u) return;
-  uint32_t uid = sc.block_counts[blockIdx.x] + __popc(~__ldg(bits + warp) & ((1u << lane) - 1u));
+  uint32_t uid = blockIdx.x * kRowsPerBlock - before + __popc(~__ldg(bits + warp) & ((1u << lane) - 1u));
   for (int w = 0; w < warp; ++w) uid += __popc(~__ldg(bits + w));
   const uint32_t s = sc.slot_of_row[row];
   slots[s].uid = uid | (slots[s].uid & kPassedBit);
@@ -567,6 +537,7 @@ __device__ __forceinline__ int32_t floor_to(int32_t c, int32_t s) {
 template <int W, bool kVec>
 __global__ void __launch_bounds__(256) k_stride(const int32_t* __restrict__ coords, uint32_t n, StrideArg st,
                                                 int32_t* __restrict__ out) {
+  after_previous_kernel();
   const uint32_t row = blockIdx.x * 256 + threadIdx.x;
   if (row >= n) return;
   int32_t c[W];
@@ -628,6 +599,7 @@ __global__ void __launch_bounds__(256) k_segment_divide(uint32_t m, int C, const
 template <int W, bool kVec>
 __global__ void __launch_bounds__(256) k_field_quantize(const float* __restrict__ field, uint32_t n, StrideArg st,
                                                         int32_t* __restrict__ out) {
+  after_previous_kernel();
   const uint32_t row = blockIdx.x * 256 + threadIdx.x;
   if (row >= n) return;
   float v[W];
@@ -737,9 +709,10 @@ extern "C" int rmn_field_quantize(const float* d_field, uint32_t n_rows, int W, 
   }
   const uint32_t nb = (n_rows + 255) / 256;
   if (W == 4 && !((uintptr_t)d_field & 15) && !((uintptr_t)d_out & 15))
-    k_field_quantize<4, true><<<nb, 256, 0, stream>>>(d_field, n_rows, st, d_out);
+    RMN_CUDA_TRY(launch_overlapped(k_field_quantize<4, true>, dim3(nb), dim3(256), 0, stream, d_field, n_rows, st, d_out));
   else
-    RMN_DISPATCH_W(W, k_field_quantize<kW, false><<<nb, 256, 0, stream>>>(d_field, n_rows, st, d_out));
+    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_field_quantize<kW, false>, dim3(nb), dim3(256), 0, stream, d_field, n_rows,
+                                                     st, d_out)));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -831,17 +804,19 @@ static int table_build_args(const int32_t* d_coords, uint32_t n_rows, int W, con
 }
 
 static int table_build_begin(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table, void* d_workspace,
-                             int look_first, const HostPost& post, cudaStream_t stream) {
+                             int look_first, cudaStream_t stream) {
   auto* h = reinterpret_cast<TableHeader*>(d_table);
   auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
   const uint32_t capacity = table_capacity(n_rows);
   const Scratch sc = scratch(d_workspace, n_rows);
-  RMN_CUDA_TRY(cudaMemsetAsync(h, 0, sizeof(TableHeader), stream));
+  static_assert(sizeof(TableHeader) == 64 * 4, "a thread per word");
+  RMN_CUDA_TRY(launch_overlapped(k_clear_header, dim3(1), dim3(64), 0, stream, reinterpret_cast<uint32_t*>(h)));
+  RMN_LAUNCH_CHECK();
   {
     const uint32_t fill_blocks = (capacity + 255u) / 256u;
     const uint32_t blocks = fill_blocks < kGrid ? fill_blocks : kGrid;
     RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_fill_range<kW>, dim3(blocks), dim3(256), 0, stream,
-                        d_coords, n_rows, h, reinterpret_cast<uint4*>(slots), capacity, sc.repeat_bits)));
+                        d_coords, n_rows, h, reinterpret_cast<uint4*>(slots), capacity, sc)));
     RMN_LAUNCH_CHECK();
   }
   if (n_rows == 0) return RMN_OK;
@@ -849,20 +824,23 @@ static int table_build_begin(const int32_t* d_coords, uint32_t n_rows, int W, vo
   RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_insert<kW>, dim3(nb), dim3(256), 0, stream,
                         d_coords, n_rows, h, slots, sc, look_first)));
   RMN_LAUNCH_CHECK();
-  RMN_CUDA_TRY(launch_overlapped(k_count_first, dim3((nb + 255) / 256), dim3(256), 0, stream,
-                        n_rows, h, sc, post));
-  RMN_LAUNCH_CHECK();
+  if (look_first) {
+    const uint32_t supers = (n_rows + kSuperRows - 1) / kSuperRows;
+    RMN_CUDA_TRY(launch_overlapped(k_super_repeats, dim3((supers + 7) / 8), dim3(256), 0, stream, n_rows, h, sc));
+    RMN_LAUNCH_CHECK();
+  }
   return RMN_OK;
 }
 
 static int table_build_finish(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table, int64_t* d_mapping,
-                              int64_t* d_inverse, int32_t* d_unique_coords, void* d_workspace, cudaStream_t stream) {
+                              int64_t* d_inverse, int32_t* d_unique_coords, void* d_workspace, const HostPost& post,
+                              cudaStream_t stream) {
   auto* h = reinterpret_cast<TableHeader*>(d_table);
   auto* slots = reinterpret_cast<Slot*>(reinterpret_cast<char*>(d_table) + sizeof(TableHeader));
   const Scratch sc = scratch(d_workspace, n_rows);
   const uint32_t nb = (n_rows + kRowsPerBlock - 1) / kRowsPerBlock;
   RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_finalize<kW>, dim3(nb), dim3(kRowsPerBlock), 0, stream,
-                        d_coords, n_rows, h, slots, sc, d_mapping, d_unique_coords, d_inverse)));
+                        d_coords, n_rows, h, slots, sc, d_mapping, d_unique_coords, d_inverse, post)));
   RMN_LAUNCH_CHECK();
   if (d_inverse) {  // optional: only the quantisation modes that average or sample features read it
     RMN_CUDA_TRY(launch_overlapped(k_inverse, dim3(nb < kGrid ? nb : kGrid), dim3(256), 0, stream,
@@ -884,9 +862,9 @@ static int table_build(const int32_t* d_coords, uint32_t n_rows, int W, void* d_
     RMN_LAUNCH_CHECK();
     return RMN_OK;
   }
-  const int rc = table_build_begin(d_coords, n_rows, W, d_table, d_workspace, look_first, post, stream);
+  const int rc = table_build_begin(d_coords, n_rows, W, d_table, d_workspace, look_first, stream);
   if (rc != RMN_OK || n_rows == 0) return rc;
-  return table_build_finish(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace, stream);
+  return table_build_finish(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace, post, stream);
 }
 
 // First half of a build: header, slot fill + bounding box, insert, first-occurrence counts. When it has
@@ -897,7 +875,12 @@ extern "C" int rmn_table_build_begin(const int32_t* d_coords, uint32_t n_rows, i
                                      void* stream_) {
   const int rc = table_build_args(d_coords, n_rows, W, d_table, table_bytes, d_workspace, workspace_bytes);
   if (rc != RMN_OK) return rc;
-  return table_build_begin(d_coords, n_rows, W, d_table, d_workspace, 0, HostPost{}, (cudaStream_t)stream_);
+  const int st = table_build_begin(d_coords, n_rows, W, d_table, d_workspace, 0, (cudaStream_t)stream_);
+  if (st != RMN_OK || n_rows == 0) return st;
+  RMN_CUDA_TRY(launch_overlapped(k_publish_unique, dim3(1), dim3(1), 0, (cudaStream_t)stream_, n_rows,
+                                 reinterpret_cast<TableHeader*>(d_table)));
+  RMN_LAUNCH_CHECK();
+  return RMN_OK;
 }
 
 // Second half: unique ids, mapping, unique coordinates, inverse. Same table, coordinates and workspace as
@@ -909,7 +892,7 @@ extern "C" int rmn_table_build_finish(const int32_t* d_coords, uint32_t n_rows, 
   if (n_rows == 0) return RMN_OK;
   if (!d_coords || !d_mapping || !d_workspace) return RMN_ERR_BAD_ARG;
   return table_build_finish(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace,
-                            (cudaStream_t)stream_);
+                            HostPost{}, (cudaStream_t)stream_);
 }
 
 extern "C" int rmn_table_build(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table,
@@ -1173,9 +1156,10 @@ extern "C" int rmn_coords_stride(const int32_t* d_coords, uint32_t n_rows, int W
   }
   const uint32_t nb = (n_rows + 255) / 256;
   if (W == 4 && !((uintptr_t)d_coords & 15) && !((uintptr_t)d_out & 15))
-    k_stride<4, true><<<nb, 256, 0, stream>>>(d_coords, n_rows, st, d_out);
+    RMN_CUDA_TRY(launch_overlapped(k_stride<4, true>, dim3(nb), dim3(256), 0, stream, d_coords, n_rows, st, d_out));
   else
-    RMN_DISPATCH_W(W, k_stride<kW, false><<<nb, 256, 0, stream>>>(d_coords, n_rows, st, d_out));
+    RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_stride<kW, false>, dim3(nb), dim3(256), 0, stream, d_coords, n_rows, st,
+                                                     d_out)));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
