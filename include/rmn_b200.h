@@ -455,6 +455,14 @@ typedef struct {
 } rmn_bn_fold;
 int rmn_conv_weight_image(const void *d_weights, int K, int w_in, int w_out, int c_in, int c_out, int dtype, int transpose,
                           int reverse, const rmn_bn_fold *fold, void *d_image, void *stream);
+/* rmn_conv_weight_image (bf16, not transposed, not reversed) of several layers at once; fold.scale NULL: no batch norm. */
+typedef struct {
+  const void *weights;
+  void *image;
+  int K, w_in, w_out, c_in, c_out;
+  rmn_bn_fold fold;
+} rmn_weight_job;
+int rmn_conv_weight_images(const rmn_weight_job *jobs, int n_jobs, void *stream);
 int rmn_conv_forward_image(const void *d_feats, uint32_t n_src, int c_in, const void *d_image, int K, int c_out,
                            const int32_t *d_nbr, const void *d_plan, uint32_t n_dst, void *d_out, const float *d_scale,
                            const float *d_shift, const void *d_add, int relu, void *stream);

@@ -74,6 +74,7 @@ SIGNATURES = {
     "rmn_conv_weight_image_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "rmn_conv_weight_image": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                       c_void_p]),
+    "rmn_conv_weight_images": (c_int, [c_void_p, c_int, c_void_p]),
     "rmn_pad_channels": (c_int, [c_void_p, c_uint32, c_int, c_int, c_void_p, c_int, c_void_p]),
     "rmn_conv_forward_image": (c_int, [c_void_p, c_uint32, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_uint32,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),

@@ -22,6 +22,7 @@ int ta_weight_image(const void* w, int K, int w_red, int w_col, int c_red, int c
 int ta_conv(const void* src, const void* image, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, void* out,
             const float* ep_scale, const float* ep_shift, const void* ep_add, int ep_relu, float* stats_partial,
             uint32_t* n_partials, cudaStream_t stream, const void* plan, const int32_t* order);
+int ta_weight_images(const rmn_weight_job* jobs, int n_jobs, cudaStream_t stream);
 int tc_read_status(cudaStream_t stream, uint32_t* status);
 unsigned long long tc_launch_count();
 int tc_conv_wgrad(const void* feats, const void* grad_out, const int32_t* nbr, uint32_t n_dst, int K, int c_in,
@@ -124,6 +125,18 @@ extern "C" int rmn_conv_weight_image(const void* d_weights, int K, int w_in, int
   if (rmn_conv_weight_image_bytes(K, c_in, c_out, dtype) == 0) return RMN_ERR_UNSUPPORTED;
   return transpose ? ta_weight_image(d_weights, K, w_out, w_in, c_out, c_in, 1, reverse, f, d_image, (cudaStream_t)stream_)
                    : ta_weight_image(d_weights, K, w_in, w_out, c_in, c_out, 0, reverse, f, d_image, (cudaStream_t)stream_);
+}
+
+extern "C" int rmn_conv_weight_images(const rmn_weight_job* jobs, int n_jobs, void* stream_) {
+  if (n_jobs < 0 || (n_jobs > 0 && !jobs)) return RMN_ERR_BAD_ARG;
+  for (int j = 0; j < n_jobs; ++j) {
+    const rmn_weight_job& a = jobs[j];
+    if (!a.weights || !a.image || a.K < 1 || a.K > 65535 || ((uintptr_t)a.image & 15)) return RMN_ERR_BAD_ARG;
+    if (a.w_in < 1 || a.w_in > a.c_in || a.w_out < 1 || a.w_out > a.c_out) return RMN_ERR_BAD_ARG;
+    if (a.fold.scale && (!a.fold.shift || (a.fold.param_dtype != RMN_F32 && a.fold.param_dtype != RMN_BF16))) return RMN_ERR_BAD_ARG;
+    if (rmn_conv_weight_image_bytes(a.K, a.c_in, a.c_out, RMN_BF16) == 0) return RMN_ERR_UNSUPPORTED;
+  }
+  return ta_weight_images(jobs, n_jobs, (cudaStream_t)stream_);
 }
 
 extern "C" int rmn_conv_forward_image(const void* d_feats, uint32_t n_src, int c_in, const void* d_image, int K, int c_out,

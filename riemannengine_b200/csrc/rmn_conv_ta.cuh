@@ -80,27 +80,23 @@ __device__ __forceinline__ constexpr uint32_t n_channel(uint32_t p) {
 template <int CC>
 constexpr int ta_tiles() { return CC <= 64 ? 4 : (CC <= 128 ? 2 : 1); }
 
-template <int CR, int CC>
-__global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, uint32_t w_red,
-                                                      uint32_t w_col, int transpose, int reverse, rmn_bn_fold fold,
-                                                      uint4* __restrict__ image) {
-  after_previous_kernel();
-  if (fold.scale && blockIdx.x == gridDim.x - 1) {
-    for (uint32_t c = threadIdx.x; c < CC; c += 256) {
-      auto param = [&](const void* p, float absent) {
-        if (!p || c >= w_col) return absent;
-        return fold.param_dtype == RMN_F32 ? static_cast<const float*>(p)[c]
-                                           : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[c]);
-      };
-      const float s = param(fold.gamma, 1.f) / sqrtf(param(fold.var, 1.f) + fold.eps);
-      fold.scale[c] = s;
-      fold.shift[c] = param(fold.beta, 0.f) + (param(fold.conv_bias, 0.f) - param(fold.mean, 0.f)) * s;
-    }
-    return;
+__device__ __forceinline__ void fold_batch_norm(const rmn_bn_fold& fold, uint32_t w_col, uint32_t c_col) {
+  for (uint32_t c = threadIdx.x; c < c_col; c += 256) {
+    auto param = [&](const void* p, float absent) {
+      if (!p || c >= w_col) return absent;
+      return fold.param_dtype == RMN_F32 ? static_cast<const float*>(p)[c]
+                                         : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[c]);
+    };
+    const float s = param(fold.gamma, 1.f) / sqrtf(param(fold.var, 1.f) + fold.eps);
+    fold.scale[c] = s;
+    fold.shift[c] = param(fold.beta, 0.f) + (param(fold.conv_bias, 0.f) - param(fold.mean, 0.f)) * s;
   }
+}
+template <int CR, int CC>
+__device__ __forceinline__ void image_chunk(const __nv_bfloat16* __restrict__ w, int K, uint32_t w_red, uint32_t w_col,
+                                            int transpose, int reverse, uint4* __restrict__ image, uint32_t i) {
   using C = TaCfg<CR, CC, ta_tiles<CC>()>;
   constexpr int KB = C::KB, NBLK = CC < 64 ? CC : 64, CPL = NBLK / 8, CHUNKS = KB * CC / 8;
-  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (i >= (uint32_t)((K + C::OPS - 1) / C::OPS) * C::NKB * CHUNKS) return;
   const uint32_t stage = i / CHUNKS, r = i % CHUNKS;
   const uint32_t atom = r / (KB * CPL), p = (r / CPL) % KB, c = r % CPL;
@@ -121,6 +117,15 @@ __global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __res
     v[q] = e[0] | ((uint32_t)e[1] << 16);
   }
   image[stage * CHUNKS + atom * (KB * CPL) + p * CPL + swz<NBLK * 2>(p, c)] = make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+template <int CR, int CC>
+__global__ void __launch_bounds__(256) k_weight_image(const __nv_bfloat16* __restrict__ w, int K, uint32_t w_red,
+                                                      uint32_t w_col, int transpose, int reverse, rmn_bn_fold fold,
+                                                      uint4* __restrict__ image) {
+  after_previous_kernel();
+  if (fold.scale && blockIdx.x == gridDim.x - 1) return fold_batch_norm(fold, w_col, CC);
+  image_chunk<CR, CC>(w, K, w_red, w_col, transpose, reverse, image, blockIdx.x * 256 + threadIdx.x);
 }
 
 // The 32 rows of a gather warp on their way from global to tensor memory: 64 channels of one row each, or the 32 channels
@@ -651,6 +656,46 @@ int launch_image(const void* w, int K, int w_red, int w_col, int transpose, int 
 
 #define RMN_TA_SHAPES(CASE) \
   CASE(32, 32) CASE(32, 64) CASE(64, 32) CASE(64, 64) CASE(64, 128) CASE(128, 64) CASE(128, 128) CASE(128, 256) CASE(256, 128) CASE(256, 256)
+
+size_t ta_image_bytes(int K, int c_red, int c_col);
+
+// The images of up to kImageJobs layers in one launch: what one of them costs a network of small layers is the launch between two
+// convolutions (3 to 4 us each: 113 us of a network of thirty layers, 24 like this; the pass, which the host bounds, 877 to 866).
+constexpr int kImageJobs = 24;
+struct ImageJobs {
+  int n;
+  uint32_t first[kImageJobs + 1];  // block range of every job; its last block folds the batch norm, if there is one
+  rmn_weight_job job[kImageJobs];
+};
+__global__ void __launch_bounds__(256) k_weight_images(const __grid_constant__ ImageJobs jobs) {
+  after_previous_kernel();
+  int j = 0;
+  while (blockIdx.x >= jobs.first[j + 1]) ++j;
+  const rmn_weight_job& job = jobs.job[j];
+  if (job.fold.scale && blockIdx.x + 1 == jobs.first[j + 1]) return tc::fold_batch_norm(job.fold, (uint32_t)job.w_out, (uint32_t)job.c_out);
+  const uint32_t i = (blockIdx.x - jobs.first[j]) * 256 + threadIdx.x;
+#define RMN_TA_CASE(R, Cc)                                                                                             \
+  if (job.c_in == R && job.c_out == Cc)                                                                                \
+    return tc::image_chunk<R, Cc>(static_cast<const __nv_bfloat16*>(job.weights), job.K, (uint32_t)job.w_in,           \
+                                  (uint32_t)job.w_out, 0, 0, static_cast<uint4*>(job.image), i);
+  RMN_TA_SHAPES(RMN_TA_CASE)
+#undef RMN_TA_CASE
+}
+
+int ta_weight_images(const rmn_weight_job* jobs, int n_jobs, cudaStream_t stream) {
+  for (int done = 0; done < n_jobs; done += kImageJobs) {
+    ImageJobs a = {};
+    a.n = n_jobs - done < kImageJobs ? n_jobs - done : kImageJobs;
+    for (int j = 0; j < a.n; ++j) {
+      a.job[j] = jobs[done + j];
+      const size_t chunks = ta_image_bytes(a.job[j].K, a.job[j].c_in, a.job[j].c_out) / 16;
+      a.first[j + 1] = a.first[j] + (uint32_t)((chunks + 255) / 256) + (a.job[j].fold.scale ? 1u : 0u);
+    }
+    RMN_CUDA_TRY(launch_overlapped(k_weight_images, dim3(a.first[a.n]), dim3(256), 0, stream, a));
+    RMN_LAUNCH_CHECK();
+  }
+  return RMN_OK;
+}
 
 constexpr int kPlanMinWeight = 128 * 128;
 

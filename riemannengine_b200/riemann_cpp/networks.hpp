@@ -22,7 +22,9 @@ struct ConvNormActImpl : torch::nn::Module {
     norm = register_module("norm", RiemannBatchNorm(c_out));
     act = register_module("act", RiemannReLU());
   }
-  SparseTensor forward(SparseTensor x) { return conv_norm_relu(x, *conv->base(), *norm); }
+  SparseTensor forward(SparseTensor x, const PreparedWeights* prepared = nullptr) {
+    return conv_norm_relu(x, *conv->base(), *norm, nullptr, prepared);
+  }
 };
 TORCH_MODULE(ConvNormAct);
 
@@ -38,7 +40,9 @@ struct UpNormActImpl : torch::nn::Module {
     norm = register_module("norm", RiemannBatchNorm(c_out));
     act = register_module("act", RiemannReLU());
   }
-  SparseTensor forward(SparseTensor x) { return conv_norm_relu(x, *conv->base(), *norm); }
+  SparseTensor forward(SparseTensor x, const PreparedWeights* prepared = nullptr) {
+    return conv_norm_relu(x, *conv->base(), *norm, nullptr, prepared);
+  }
 };
 TORCH_MODULE(UpNormAct);
 
@@ -57,8 +61,9 @@ struct BasicBlockImpl : torch::nn::Module {
     norm = register_module("norm", RiemannBatchNorm(channels));
     act = register_module("act", RiemannReLU());
   }
-  SparseTensor forward(SparseTensor x) {
-    return conv_norm_relu(first->forward(x), *conv->base(), *norm, &x);
+  // prepared: of the first and of the second layer, or nullptr
+  SparseTensor forward(SparseTensor x, const PreparedWeights* prepared = nullptr) {
+    return conv_norm_relu(first->forward(x, prepared), *conv->base(), *norm, &x, prepared ? prepared + 1 : nullptr);
   }
 };
 TORCH_MODULE(BasicBlock);
@@ -95,16 +100,42 @@ struct MinkUNetImpl : torch::nn::Module {
   }
 
   SparseTensor forward(SparseTensor x) {
-    std::vector<SparseTensor> skips;
-    auto y = stem->forward(x);
+    // the weights of all layers in the order of their use (serving: prepared together; training: every layer its own)
+    std::vector<std::pair<RiemannConvolutionBaseImpl*, RiemannBatchNormImpl*>> layers;
+    auto block = [&](BasicBlock& b) {
+      layers.emplace_back(b->first->conv->base().get(), b->first->norm.get());
+      layers.emplace_back(b->conv->base().get(), b->norm.get());
+    };
+    layers.emplace_back(stem->conv->base().get(), stem->norm.get());
     for (int s = 0; s < 4; ++s) {
-      if (s > 0) y = down[s - 1]->forward(y);
-      y = enc_b[s]->forward(enc_a[s]->forward(y));
+      if (s > 0) layers.emplace_back(down[s - 1]->conv->base().get(), down[s - 1]->norm.get());
+      block(enc_a[s]);
+      block(enc_b[s]);
+    }
+    for (int i = 0; i < 3; ++i) {
+      layers.emplace_back(up[i]->conv->base().get(), up[i]->norm.get());
+      layers.emplace_back(fuse[i]->conv->base().get(), fuse[i]->norm.get());
+      block(dec[i]);
+    }
+    const auto weights = prepare_layers(layers);
+    const PreparedWeights* w = weights.empty() ? nullptr : weights.data();
+    auto next = [&](int n) {
+      auto p = w;
+      if (w) w += n;
+      return p;
+    };
+    std::vector<SparseTensor> skips;
+    auto y = stem->forward(x, next(1));
+    for (int s = 0; s < 4; ++s) {
+      if (s > 0) y = down[s - 1]->forward(y, next(1));
+      y = enc_a[s]->forward(y, next(2));
+      y = enc_b[s]->forward(y, next(2));
       if (s < 3) skips.push_back(y);
     }
     for (int i = 0; i < 3; ++i) {
-      auto u = up[i]->forward(y);
-      y = dec[i]->forward(fuse[i]->forward(cat({u, skips[2 - i]})));
+      auto u = up[i]->forward(y, next(1));
+      y = fuse[i]->forward(cat({u, skips[2 - i]}), next(1));
+      y = dec[i]->forward(y, next(2));
     }
     return head->forward(y);
   }

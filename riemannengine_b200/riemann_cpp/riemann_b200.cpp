@@ -1176,7 +1176,7 @@ struct ConvEpilogue {
 
 at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in, const at::Tensor& nbr,
                         const ConvEpilogue& ep = {}, const at::Tensor& plan = at::Tensor(), torch::nn::BatchNorm1dImpl* bn = nullptr,
-                        const at::Tensor& order = at::Tensor()) {
+                        const at::Tensor& order = at::Tensor(), const PreparedWeights* prepared = nullptr) {
   TORCH_CHECK(feats_in.is_cuda() && kernel_in.is_cuda(), "features and kernel must be CUDA tensors");
   TORCH_CHECK(feats_in.scalar_type() == kernel_in.scalar_type(), "expected features and kernel to have the same dtype");
   auto feats = contiguous_rows(feats_in), kernel = kernel_in.contiguous();
@@ -1195,7 +1195,11 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
     const bool padded = shape.second != c_out;
     at::Tensor shift, scale;
     rmn_bn_fold fold{};
-    if (bn) {
+    const bool ready = bn && prepared && prepared->image.defined();
+    if (ready) {
+      scale = prepared->scale;
+      shift = scale[1];
+    } else if (bn) {
       auto data = [](const at::Tensor& t) { return t.defined() ? ptr(t) : nullptr; };
       scale = at::empty({2, shape.second}, feats.options().dtype(at::kFloat));
       shift = scale[1];
@@ -1208,7 +1212,8 @@ at::Tensor conv_forward(const at::Tensor& feats_in, const at::Tensor& kernel_in,
       if (padded && shift.defined()) shift = at::constant_pad_nd(shift, {0, shape.second - c_out});
       if (padded && scale.defined()) scale = at::constant_pad_nd(scale, {0, shape.second - c_out});
     }
-    if (auto image = weight_image(kernel, shape, false, false, feats, bn ? &fold : nullptr); image.defined()) {
+    if (auto image = ready ? prepared->image : weight_image(kernel, shape, false, false, feats, bn ? &fold : nullptr);
+        image.defined()) {
       TORCH_CHECK(!padded || !ep.add.defined(), "a padded convolution adds nothing");
       auto out = at::empty({nbr.size(1), shape.second}, feats.options());
       if (order.defined()) {
@@ -1457,22 +1462,27 @@ void RiemannConvolutionBaseImpl::reset_parameters(bool is_transpose) {
 
 namespace {
 // whether the kernel that prepares a layer's weights also folds this batch norm (bf16 on tensor cores, parameters of one type)
-bool folds_batch_norm(const RiemannConvolutionBaseImpl& conv, const SparseTensor& input, const torch::nn::BatchNorm1dImpl& bn) {
+bool folds_parameters(const RiemannConvolutionBaseImpl& conv, const torch::nn::BatchNorm1dImpl& bn) {
   auto const& kernel = conv.kernel_;
   auto const& mean = bn.running_mean;
-  if (!mean.defined() || !bn.running_var.defined() || input.F().scalar_type() != at::kBFloat16 ||
-      kernel.scalar_type() != at::kBFloat16 || !input.F().is_cuda() || input.F().size(0) == 0)
-    return false;
+  if (!mean.defined() || !bn.running_var.defined() || kernel.scalar_type() != at::kBFloat16 || !kernel.is_cuda()) return false;
   if (mean.scalar_type() != at::kBFloat16 && mean.scalar_type() != at::kFloat) return false;
   for (auto const& p : {bn.running_var, bn.weight, bn.bias, conv.bias_, mean})
     if (p.defined() && (p.scalar_type() != mean.scalar_type() || !p.is_contiguous() || p.numel() != conv.out_channels_ ||
-                        p.device() != input.F().device()))
+                        p.device() != kernel.device()))
       return false;
   const auto shape = run_shape(kernel);
-  auto x = input.F();
   return rmn_conv_weight_image_bytes(static_cast<int>(kernel.size(0)), static_cast<int>(shape.first),
-                                     static_cast<int>(shape.second), RMN_BF16) > 0 &&
-         (shape.first != x.size(1) || !x.is_contiguous() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 == 0);
+                                     static_cast<int>(shape.second), RMN_BF16) > 0;
+}
+// ... for this input
+bool folds_batch_norm(const RiemannConvolutionBaseImpl& conv, const SparseTensor& input, const torch::nn::BatchNorm1dImpl& bn) {
+  auto x = input.F();
+  if (!folds_parameters(conv, bn) || x.scalar_type() != at::kBFloat16 || !x.is_cuda() || x.size(0) == 0 ||
+      x.device() != conv.kernel_.device())
+    return false;
+  const auto shape = run_shape(conv.kernel_);
+  return (shape.first != x.size(1) || !x.is_contiguous() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 == 0);
 }
 
 // whether a layer that only runs forward may take an ordered map: its pass goes to the kernels of prepared weights
@@ -1537,7 +1547,7 @@ SparseTensor RiemannConvolutionBaseImpl::forward(const SparseTensor& input) {
 }
 
 SparseTensor RiemannConvolutionBaseImpl::forward_fused(const SparseTensor& input, torch::nn::BatchNorm1d bn, bool relu,
-                                                       const at::Tensor& add) {
+                                                       const at::Tensor& add, const PreparedWeights* prepared) {
   torch::NoGradGuard guard;
   auto [kmap, output_key] = kernel_map(input, takes_ordered_map(*this, input));
   const auto shape = run_shape(kernel_);
@@ -1559,7 +1569,7 @@ SparseTensor RiemannConvolutionBaseImpl::forward_fused(const SparseTensor& input
       if (bias_.defined()) ep.shift = ep.shift + bias_.reshape({-1}).to(at::kFloat) * ep.scale;
     }
   }
-  auto result = conv_forward(input.F(), kernel_, kmap->nbr_out, ep, plan, folded, kmap->order);
+  auto result = conv_forward(input.F(), kernel_, kmap->nbr_out, ep, plan, folded, kmap->order, prepared);
   return SparseTensor(std::move(result), output_key, input.coordinate_manager());
 }
 
@@ -1574,8 +1584,60 @@ SparseTensor fused_conv_bn_relu(const SparseTensor& input, RiemannConvolutionBas
   return conv.forward_fused(input, bn, relu);
 }
 
+std::vector<PreparedWeights> prepare_layers(
+    const std::vector<std::pair<RiemannConvolutionBaseImpl*, RiemannBatchNormImpl*>>& layers) {
+  if (at::GradMode::is_enabled() || layers.empty()) return {};
+  std::vector<PreparedWeights> out(layers.size());
+  auto const device = layers.front().first->kernel_.device();
+  std::vector<rmn_weight_job> jobs;
+  std::vector<size_t> index;
+  std::vector<int64_t> offset;
+  int64_t bytes = 0, columns = 0;
+  for (size_t i = 0; i < layers.size(); ++i) {
+    auto const& conv = *layers[i].first;
+    auto bn = layers[i].second->normalization();
+    auto const& kernel = conv.kernel_;
+    if (bn->is_training() || !plain_autograd(kernel) || kernel.device() != device || !kernel.is_contiguous() ||
+        !folds_parameters(conv, *bn))
+      continue;
+    const auto shape = run_shape(kernel);
+    auto data = [](const at::Tensor& t) { return t.defined() ? ptr(t) : nullptr; };
+    rmn_weight_job job{};
+    job.weights = ptr(kernel);
+    job.K = static_cast<int>(kernel.size(0));
+    job.w_in = static_cast<int>(kernel.size(1));
+    job.w_out = static_cast<int>(kernel.size(2));
+    job.c_in = static_cast<int>(shape.first);
+    job.c_out = static_cast<int>(shape.second);
+    job.fold = rmn_bn_fold{data(bn->running_mean), data(bn->running_var), data(bn->weight), data(bn->bias), data(conv.bias_),
+                           dtype_code(bn->running_mean), static_cast<float>(bn->options.eps()), nullptr, nullptr};
+    jobs.push_back(job);
+    index.push_back(i);
+    offset.push_back(bytes);
+    bytes += (static_cast<int64_t>(rmn_conv_weight_image_bytes(job.K, job.c_in, job.c_out, RMN_BF16)) + 255) / 256 * 256;
+    columns += 2 * shape.second;
+  }
+  if (jobs.empty()) return out;
+  c10::cuda::CUDAGuard guard(device);
+  auto images = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(device));
+  auto scales = at::empty({columns}, at::TensorOptions().dtype(at::kFloat).device(device));
+  int64_t column = 0;
+  for (size_t j = 0; j < jobs.size(); ++j) {
+    auto& w = out[index[j]];
+    const int64_t end = j + 1 < jobs.size() ? offset[j + 1] : bytes;
+    w.image = images.narrow(0, offset[j], end - offset[j]);
+    w.scale = scales.narrow(0, column, 2 * jobs[j].c_out).view({2, jobs[j].c_out});
+    column += 2 * jobs[j].c_out;
+    jobs[j].image = ptr(w.image);
+    jobs[j].fold.scale = static_cast<float*>(ptr(w.scale));
+    jobs[j].fold.shift = jobs[j].fold.scale + jobs[j].c_out;
+  }
+  check(rmn_conv_weight_images(jobs.data(), static_cast<int>(jobs.size()), current_stream()), "rmn_conv_weight_images");
+  return out;
+}
+
 SparseTensor conv_norm_relu(const SparseTensor& input, RiemannConvolutionBaseImpl& conv, RiemannBatchNormImpl& norm,
-                            const SparseTensor* residual) {
+                            const SparseTensor* residual, const PreparedWeights* prepared) {
   auto bn = norm.normalization();
   bool fuse = !at::GradMode::is_enabled() && !bn->is_training() && plain_autograd(input.F()) &&
               folds_batch_norm(conv, input, *bn);
@@ -1588,7 +1650,7 @@ SparseTensor conv_norm_relu(const SparseTensor& input, RiemannConvolutionBaseImp
            r.device() == input.F().device() && reinterpret_cast<uintptr_t>(r.data_ptr()) % 16 == 0 &&
            run_shape(conv.kernel_).second == conv.out_channels_;
   }
-  if (fuse) return conv.forward_fused(input, bn, true, residual ? residual->F() : at::Tensor());
+  if (fuse) return conv.forward_fused(input, bn, true, residual ? residual->F() : at::Tensor(), prepared);
   auto y = norm.forward(conv.forward(input));
   if (residual) y = y + *residual;
   return SparseTensor(at::relu(y.F()), y.coordinate_map_key(), y.coordinate_manager());

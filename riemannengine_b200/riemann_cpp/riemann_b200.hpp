@@ -387,6 +387,13 @@ struct ConvolutionTransposeFunction {
                           std::shared_ptr<CoordinateManager> manager);
 };
 
+// Weights of a layer in the form that its kernel reads, with the epilogue's scale and shift of its batch norm [2, c]: made for
+// several layers at once by prepare_layers, for the pass at hand. Undefined where the layer prepares its own.
+struct PreparedWeights {
+  at::Tensor image, scale;
+};
+
+
 class RiemannConvolutionBaseImpl : public torch::nn::Cloneable<RiemannConvolutionBaseImpl> {
 public:
   RiemannConvolutionBaseImpl(int in_channels, int out_channels, int kernel_size = 3, int stride = 1,
@@ -407,7 +414,8 @@ public:
   torch::Tensor bias_{nullptr};
   // out = act(conv(input) (+ bias) * scale + shift + add) with the batch norm's running statistics as scale and shift
   // (a missing holder: bias only); inference only
-  SparseTensor forward_fused(const SparseTensor& input, torch::nn::BatchNorm1d bn, bool relu, const at::Tensor& add = {});
+  SparseTensor forward_fused(const SparseTensor& input, torch::nn::BatchNorm1d bn, bool relu, const at::Tensor& add = {},
+                             const PreparedWeights* prepared = nullptr);
 
 private:
   // input map -> (kernel map, output key), building or reusing the output map
@@ -436,7 +444,12 @@ SparseTensor fused_conv_bn_relu(const SparseTensor& input, RiemannConvolutionBas
 // relu(norm(conv(input)) [+ residual]): one kernel in evaluation mode without gradients, where bf16 kernels cover the layer;
 // otherwise (training, fp32, a residual on other coordinates) the layers one after the other.
 SparseTensor conv_norm_relu(const SparseTensor& input, RiemannConvolutionBaseImpl& conv, RiemannBatchNormImpl& norm,
-                            const SparseTensor* residual = nullptr);
+                            const SparseTensor* residual = nullptr, const PreparedWeights* prepared = nullptr);
+
+// For a network that runs conv_norm_relu on all these layers in evaluation mode without gradients: their weights prepared by one
+// kernel instead of one between every two convolutions. An entry per layer, or none at all where gradients are enabled.
+std::vector<PreparedWeights> prepare_layers(
+    const std::vector<std::pair<RiemannConvolutionBaseImpl*, RiemannBatchNormImpl*>>& layers);
 
 #define RIEMANN_B200_CONV_WRAPPER(Name)                                                                   \
   class Name##Impl : public torch::nn::Cloneable<Name##Impl> {                                            \

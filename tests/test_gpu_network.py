@@ -192,3 +192,26 @@ def test_cpp_host_network_on_a_whole_room_matches_cpu_reference_arithmetic():
     for bn, g, b in zip(bns, G, B):
         assert rel(bn.weight.grad, g.grad) <= 1e-4 and rel(bn.bias.grad, b.grad) <= 1e-4
     assert rel(convs[5].bias.grad, head_bias.grad) <= 1e-4
+
+
+def test_layers_prepared_together_run_as_prepared_alone():
+    """The serving network (weights of all layers by one kernel) against its layers without gradients one by one: more layers
+    than one launch takes, padded stem, batch norms of both parameter types; enabled gradients prepare nothing."""
+    import torch
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    xyz = torch.unique(torch.randint(0, 40, (6000, 3), generator=g, device="cuda"), dim=0)
+    coords = torch.cat([torch.zeros((xyz.size(0), 1), dtype=xyz.dtype, device="cuda"), xyz], 1).int().contiguous()
+    torch.manual_seed(3)
+    net = C.MinkUNet(4, 20, width=32, dimension=3)
+    net.to("cuda:0")
+    net.to(torch.bfloat16)
+    net.train(False)
+    feats = torch.randn((coords.size(0), 4), generator=g, device="cuda").bfloat16()
+    with torch.no_grad():
+        together = net(C.SparseTensor(feats, coords)).F
+    alone = net(C.SparseTensor(feats, coords)).F.detach()   # gradients enabled: conv, norm and ReLU one after the other
+    scale = float(alone.float().pow(2).mean().sqrt())
+    # every layer rounds to bf16 (2^-9) once instead of three times: some thirty layers' worth of it
+    assert float((together.float() - alone.float()).pow(2).mean().sqrt()) <= 30 * 2.0 ** -9 * scale
