@@ -25,6 +25,85 @@ namespace rmn {
 
 constexpr int kKmapBlock = 256;
 
+// The scan of pass 2 by the last block of the probing kernel, on maps of up to kTailCounts counts: a launch of its own takes
+// longer there (900 rows x 27 offsets: 6.4 us of a pass of 53). Warp w takes the counted offsets w, w + 8, ...
+constexpr uint32_t kTailCounts = 4096;
+struct TailScan {
+  uint32_t* ticket;  // NULL: k_kmap_scan does it
+  uint32_t* totals;
+  int64_t* offset_ptr;
+  volatile int64_t* host_ptr;
+};
+__device__ __forceinline__ void scan_counts_in_last_block(const TailScan& tail, uint32_t* block_counts, uint32_t n_blocks, int K,
+                                                          int mirror_half) {
+  __shared__ uint32_t s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(tail.ticket, 1u) == gridDim.x * gridDim.y - 1 ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto scan = [&](auto v) {  // inclusive, over the warp
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const auto t = __shfl_up_sync(0xFFFFFFFFu, v, d);
+      if (lane >= d) v += t;
+    }
+    return v;
+  };
+  for (int k = warp; k < K - mirror_half; k += kKmapBlock / 32) {
+    uint32_t* counts = block_counts + (size_t)k * n_blocks;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < n_blocks; base += 128) {
+      uint32_t v[4], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t i = base + lane * 4 + j;
+        v[j] = i < n_blocks ? __ldcg(counts + i) : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t x = v[j];
+        v[j] = sum;
+        sum += x;
+      }
+      const uint32_t incl = scan(sum), before = carry + incl - sum;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t i = base + lane * 4 + j;
+        if (i < n_blocks) counts[i] = before + v[j];
+      }
+      carry += __shfl_sync(0xFFFFFFFFu, incl, 31);
+    }
+    if (lane == 0) {
+      tail.totals[k] = carry;
+      if (k < mirror_half) tail.totals[K - 1 - k] = carry;
+    }
+  }
+  __syncthreads();
+  uint32_t* flags = tail.totals + K;  // [0] "pair lists did not fit", [1] half
+  if (threadIdx.x == 0) {
+    flags[0] = 0;
+    flags[1] = (uint32_t)mirror_half;
+  }
+  if (warp) return;
+  int64_t carry = 0;
+  for (int base = 0; base < K; base += 32) {
+    const int k = base + lane;
+    const int64_t t = k < K ? (int64_t)__ldcg(tail.totals + k) : 0, incl = scan(t);
+    if (k < K) {
+      tail.offset_ptr[k] = carry + incl - t;
+      if (tail.host_ptr) tail.host_ptr[k] = carry + incl - t;
+    }
+    carry += __shfl_sync(0xFFFFFFFFu, incl, 31);
+  }
+  if (lane == 0) {
+    tail.offset_ptr[K] = carry;
+    if (tail.host_ptr) tail.host_ptr[K] = carry;
+  }
+}
+
 // The packed key is linear in the coordinates: key(c + off) = key(c) + sum_i (off_i << shift_i)
 // in 64-bit modular arithmetic, so each probe costs one 64-bit add on top of the range test
 // (a neighbour outside the table's bounding box is a miss without touching memory).
@@ -33,12 +112,12 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots,
     const int32_t* __restrict__ query, uint32_t n_query, const int32_t* __restrict__ offsets,
     int K, int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks,
-    uint32_t* __restrict__ scan_ticket) {
+    uint32_t* __restrict__ scan_ticket, TailScan tail) {
   after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int D = W - 1;
   const int k_begin = (int)((uint32_t)K * blockIdx.y / gridDim.y), k_end = (int)((uint32_t)K * (blockIdx.y + 1) / gridDim.y);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scan_ticket = 0;
+  if (!tail.ticket && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scan_ticket = 0;
   long long* s_delta = reinterpret_cast<long long*>(smem_raw);           // [K]
   int32_t* s_off = reinterpret_cast<int32_t*>(s_delta + K);              // [K][D]
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_off + K * D);          // [K]
@@ -137,6 +216,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe(
   __syncthreads();
   for (int k = k_begin + threadIdx.x; k < k_end; k += kKmapBlock)
     block_counts[(size_t)k * n_blocks + blockIdx.x] = s_cnt[k];
+  if (tail.ticket) scan_counts_in_last_block(tail, block_counts, n_blocks, K, 0);
 }
 
 // Self map with a point-symmetric region (stride-1 convolution: the query rows ARE the table's
@@ -149,7 +229,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
     const TableHeader* __restrict__ h, const Slot* __restrict__ slots,
     const int32_t* __restrict__ coords, uint32_t n, const int32_t* __restrict__ offsets, int K,
     int32_t* __restrict__ nbr, uint32_t* __restrict__ block_counts, uint32_t n_blocks,
-    uint32_t* __restrict__ scan_ticket, const uint32_t* __restrict__ index_state) {
+    uint32_t* __restrict__ scan_ticket, const uint32_t* __restrict__ index_state, TailScan tail) {
   after_previous_kernel();
   if (index_state && *index_state == ~0u) return;  // kIndexInUse: k_kmap_blocks_self has written the map
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -157,7 +237,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
   const int half = K / 2;
   const int k_begin = (int)((uint32_t)half * blockIdx.y / gridDim.y);
   const int k_end = (int)((uint32_t)half * (blockIdx.y + 1) / gridDim.y);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scan_ticket = 0;
+  if (!tail.ticket && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scan_ticket = 0;
   long long* s_delta = reinterpret_cast<long long*>(smem_raw);   // [half]
   int32_t* s_off = reinterpret_cast<int32_t*>(s_delta + (half > 0 ? half : 1));  // [half][D]
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_off + (half > 0 ? half : 1) * D);  // [half]
@@ -214,6 +294,7 @@ __global__ void __launch_bounds__(kKmapBlock) k_kmap_probe_self(
     const uint32_t row0 = blockIdx.x * kKmapBlock;
     block_counts[(size_t)half * n_blocks + blockIdx.x] = row0 < n ? min((uint32_t)kKmapBlock, n - row0) : 0u;
   }
+  if (tail.ticket) scan_counts_in_last_block(tail, block_counts, n_blocks, K, half);
 }
 
 // One block of 1024 threads per counted offset: exclusive scan of block_counts[k][0..n_blocks) in place, totals[k] = number
@@ -373,8 +454,9 @@ __global__ void __maxnreg__(32) k_kmap_pairs_background(
 }
 
 // n entries "no neighbour" (a launch that overlaps its neighbours, where a memset would not)
-__global__ void __launch_bounds__(256) k_kmap_clear(int32_t* __restrict__ nbr, size_t n) {
+__global__ void __launch_bounds__(256) k_kmap_clear(int32_t* __restrict__ nbr, size_t n, uint32_t* __restrict__ ticket) {
   after_previous_kernel();
+  if (ticket && blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
   // single words up to the first 16-byte boundary and behind the last one
   const size_t head = min(n, (size_t)(((16 - ((uintptr_t)nbr & 15)) & 15) / 4)), vecs = (n - head) / 4, tail = head + 4 * vecs;
   const size_t first = (size_t)blockIdx.x * 256 + threadIdx.x, step = (size_t)gridDim.x * 256;
@@ -383,10 +465,10 @@ __global__ void __launch_bounds__(256) k_kmap_clear(int32_t* __restrict__ nbr, s
   if (first < head) nbr[first] = -1;
   if (tail + first < n) nbr[tail + first] = -1;
 }
-inline cudaError_t clear_entries(int32_t* nbr, size_t n, cudaStream_t stream) {
+inline cudaError_t clear_entries(int32_t* nbr, size_t n, uint32_t* ticket, cudaStream_t stream) {
   const size_t blocks = (n / 4 + 255) / 256 + 1;
   count_launch();
-  return launch_overlapped(k_kmap_clear, dim3((uint32_t)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, nbr, n);
+  return launch_overlapped(k_kmap_clear, dim3((uint32_t)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, nbr, n, ticket);
 }
 
 __global__ void __launch_bounds__(256) k_kmap_transpose(const int32_t* __restrict__ nbr,
@@ -515,6 +597,7 @@ static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_qu
       reinterpret_cast<const Slot*>(reinterpret_cast<const char*>(d_table) + sizeof(TableHeader));
   const int half = self ? K / 2 : 0;
   const int hs = half > 0 ? half : 1;
+  const TailScan tail{(uint64_t)(K - half) * nb <= kTailCounts ? ticket : nullptr, totals, d_offset_ptr, host_alias};
   const size_t self_smem = (size_t)hs * 8 + (size_t)hs * (W - 1) * 4 + (size_t)hs * 4;
   if (self && may_use_block_index(n_query, W, K) && ((uintptr_t)d_workspace & 15) == 0) {
     const BlockIndex ix = block_index(static_cast<char*>(d_workspace) + kmap_counts_bytes(n_query, K), n_query);
@@ -539,20 +622,22 @@ static int kmap_build(const void* d_table, const int32_t* d_query, uint32_t n_qu
       RMN_LAUNCH_CHECK();
       RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock), self_smem,
                                      stream, h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket,
-                                     ix.state));
+                                     ix.state, TailScan{}));
     });
   } else if (self) {
-    if (half > 0)  // the mirrored half starts as "no neighbour"
-      RMN_CUDA_TRY(clear_entries(d_nbr + (size_t)(half + 1) * n_query, (size_t)half * n_query, stream));
+    if (half > 0 || tail.ticket)  // the mirrored half starts as "no neighbour"
+      RMN_CUDA_TRY(clear_entries(d_nbr + (size_t)(half + 1) * n_query, (size_t)half * n_query, tail.ticket, stream));
     RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock),
                                                      self_smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr,
-                                                     block_counts, nb, ticket, nullptr)));
+                                                     block_counts, nb, ticket, nullptr, tail)));
   } else {
+    if (tail.ticket) RMN_CUDA_TRY(clear_entries(d_nbr, 0, tail.ticket, stream));
     const size_t smem = (size_t)K * 8 + (size_t)K * (W - 1) * 4 + (size_t)K * 4;
     RMN_DISPATCH_W(W, RMN_CUDA_TRY(launch_overlapped(
-                        k_kmap_probe<kW>, dim3(nb, offset_split(nb, K)), dim3(kKmapBlock), smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket)));
+                        k_kmap_probe<kW>, dim3(nb, offset_split(nb, K)), dim3(kKmapBlock), smem, stream, h, slots, d_query, n_query, d_offsets, K, d_nbr, block_counts, nb, ticket, tail)));
   }
   RMN_LAUNCH_CHECK();
+  if (tail.ticket) return RMN_OK;
   RMN_CUDA_TRY(launch_overlapped(k_kmap_scan, dim3(self ? half + 1 : K), dim3(1024), 0, stream,
                         block_counts, nb, K, half, totals, d_offset_ptr, host_alias));
   RMN_LAUNCH_CHECK();
@@ -609,7 +694,7 @@ extern "C" int rmn_kmap_build_ordered(const void* d_table, const int32_t* d_coor
     RMN_LAUNCH_CHECK();
     RMN_CUDA_TRY(launch_overlapped(k_kmap_probe_self<kW>, dim3(nb, offset_split(nb, half)), dim3(kKmapBlock), self_smem, stream,
                                    h, slots, d_coords, n_rows, d_offsets, K, d_nbr, counts, nb,
-                                   counts + (size_t)K * nb + K + 2, ix.state));
+                                   counts + (size_t)K * nb + K + 2, ix.state, TailScan{}));
     RMN_LAUNCH_CHECK();
   });
   return RMN_OK;
@@ -700,7 +785,7 @@ extern "C" int rmn_kmap_transpose(const int32_t* d_nbr, uint32_t n_query, int K,
   if (K < 1) return RMN_ERR_BAD_ARG;
   if (n_a == 0) return RMN_OK;
   if (!d_nbr_t) return RMN_ERR_BAD_ARG;
-  RMN_CUDA_TRY(clear_entries(d_nbr_t, (size_t)K * n_a, stream));
+  RMN_CUDA_TRY(clear_entries(d_nbr_t, (size_t)K * n_a, nullptr, stream));
   if (n_query == 0) return RMN_OK;
   if (!d_nbr) return RMN_ERR_BAD_ARG;
   const uint64_t total = (uint64_t)K * n_query;

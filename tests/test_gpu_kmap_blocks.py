@@ -137,3 +137,22 @@ def test_layers_that_only_run_forward_give_the_same_rows_over_an_ordered_map():
     y = C.SparseTensor(feats, c)
     public = y.coordinate_manager.kernel_map_pairs(y.coordinate_map_key, y.coordinate_map_key, [3] * 3, [1] * 3, [1] * 3)
     assert all(torch.equal(torch.as_tensor(a), torch.as_tensor(b)) for a, b in zip(pairs, public))
+
+
+# up to 4096 counts (offsets x blocks of 256 rows) the last block of the probing kernel adds them up, beyond a kernel of its own
+@pytest.mark.parametrize("n,self_map,kernel", [(1, True, 3), (300, True, 1), (5000, True, 3), (74_752, True, 3), (74_753, True, 3),
+                                               (300, False, 2), (131_072, False, 2), (131_073, False, 2)])
+def test_offset_pointers_and_pair_lists_of_small_maps(n, self_map, kernel):
+    from riemannengine_b200 import ops
+    c = _cloud(3, n, 60, 1, "random", n)
+    table = ops.table_build(c)
+    off = ops.region_offsets(0, [kernel] * 3, [1] * 3, [1] * 3)
+    m = ops.kmap_build(table, table.coords, off, self_map=self_map)
+    counts = (m.nbr >= 0).sum(1)
+    assert torch.equal(m.offset_ptr[1:], counts.cumsum(0)) and int(m.offset_ptr[0]) == 0
+    ptr, a, q = m.pairs()
+    for k in range(off.shape[0]):
+        lo, hi = int(m.offset_ptr[k]), int(m.offset_ptr[k + 1])
+        want = (m.nbr[k] >= 0).nonzero().flatten()
+        order = q[lo:hi].argsort()
+        assert torch.equal(q[lo:hi][order].long(), want) and torch.equal(a[lo:hi][order], m.nbr[k][want])
