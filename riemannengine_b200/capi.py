@@ -69,6 +69,7 @@ SIGNATURES = {
     "rmn_conv_forward_ordered": (c_int, [c_void_p, c_uint32, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_uint32,
                                          c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "rmn_conv_f32_scratch_bytes": (c_size_t, [c_uint32, c_int, c_int, c_int]),
+    "rmn_conv_f32_pays": (c_int, [c_uint32, c_int, c_int, c_int]),
     "rmn_conv_forward_f32": (c_int, [c_void_p, c_uint32, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_uint32,
                                      c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_size_t, c_void_p]),
     "rmn_conv_weight_image_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),

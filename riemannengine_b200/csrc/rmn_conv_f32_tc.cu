@@ -532,14 +532,18 @@ int run_f3(F3Args a, uint8_t* image, cudaStream_t stream) {
 using namespace rmn;
 
 extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, int c_out) {
-  // Few rows leave most SMs idle here, where every row tile walks all offsets in turn, and k_conv_f32 deals the offsets of a row
-  // to several warps; 64 columns cost it twice the time and these kernels little more. 27 offsets, half of them present, us
-  // there / here: 1000 rows 32 -> 32 12.4 / 14.2, 64 -> 32 20.7 / 22.8, 32 -> 64 20.5 / 16.3; 4000 rows 16.1 / 14.7, 27.3 / 23.0,
-  // 26.0 / 16.5, 16 -> 16 11.3 / 13.9; 100 rows 32 -> 64 19.8 / 15.7
-  if (c_out <= 32 && n_dst < (c_in < 32 ? 8192u : 3072u)) return 0;
   if (n_dst == 0 || K < 1 || K > 4096 || c_in < 16 || c_in > 1024 || c_in % 8 || c_out < 4 || c_out > 1024 || c_out % 4) return 0;
   const size_t cc = c_out <= 32 ? 32 : 64, columns = (c_out + cc - 1) / cc * cc;
   return (size_t)K * ((c_in + 31) / 32) * 32 * columns * 3 * 2;
+}
+
+// Little work is the multiply-add kernel's: these kernels need the weights prepared by a launch of their own, which a host that
+// waits for nothing else pays for, and few rows leave most SMs idle while every row tile walks all offsets in turn. Passes of
+// one layer, us there / here, forward alone and with its gradients, by the rows x offsets x channels in x out of the layer, in
+// millions: 221 (8000 rows 32 -> 32) 69 / 66 and 168 / 173; 442 (32 -> 64) 75 / 67 and 168 / 172; 553 (20 000 rows 32 -> 32)
+// 91 / 72 and 175 / 172; 663 (8000 rows 64 -> 48) 94 / 75 and 181 / 169; 90 (strided, 11 000 rows, 8 offsets) 94 / 99.
+extern "C" int rmn_conv_f32_pays(uint32_t n_dst, int K, int c_in, int c_out) {
+  return rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out) > 0 && (double)n_dst * K * c_in * c_out >= 500e6;
 }
 
 extern "C" int rmn_conv_forward_f32(const float* d_feats, uint32_t n_src, int c_in, const float* d_weights, int K, int c_out,

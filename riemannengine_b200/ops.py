@@ -266,15 +266,16 @@ def _weight_image(weights: torch.Tensor, transpose: bool, feats: torch.Tensor,
 
 
 def _conv_f32(feats: torch.Tensor, weights: torch.Tensor, transpose: bool, nbr: torch.Tensor, out: torch.Tensor,
-              scale: Optional[torch.Tensor] = None, shift: Optional[torch.Tensor] = None, relu: bool = False) -> bool:
-    """fp32 on the tensor cores (rmn_conv_forward_f32) into ``out``; False where that does not serve. The current device is
-    the tensors'."""
+              scale: Optional[torch.Tensor] = None, shift: Optional[torch.Tensor] = None, relu: bool = False,
+              always: bool = False) -> bool:
+    """fp32 on the tensor cores (rmn_conv_forward_f32) into ``out``; False where that does not serve or (unless ``always``)
+    does not pay. The current device is the tensors'."""
     n_dst, n_src, K = int(nbr.size(1)), int(feats.size(0)), int(weights.size(0))
     if feats.dtype != torch.float32 or not n_dst or not n_src or feats.data_ptr() % 32:
         return False
     c_in, c_out = int(feats.size(1)), int(out.size(1))
     nbytes = capi.lib().rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out)
-    if nbytes == 0:
+    if nbytes == 0 or not (always or capi.lib().rmn_conv_f32_pays(n_dst, K, c_in, c_out)):
         return False
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=feats.device)
     capi.check(capi.lib().rmn_conv_forward_f32(_ptr(feats), n_src, c_in, _ptr(weights), K, c_out, int(transpose), 0, _ptr(nbr),

@@ -1144,7 +1144,7 @@ at::Tensor weight_image(const at::Tensor& kernel, std::pair<int64_t, int64_t> sh
   return image;
 }
 
-// fp32 features on the tensor cores (rmn_conv_forward_f32); undefined where that does not serve. transpose: kernel is
+// fp32 features on the tensor cores (rmn_conv_forward_f32); undefined where that does not serve or pay. transpose: kernel is
 // [K, c_out, c_in].
 at::Tensor conv_f32(const at::Tensor& feats, const at::Tensor& kernel, bool transpose, bool reverse, const at::Tensor& nbr,
                     const at::Tensor& scale = at::Tensor(), const at::Tensor& shift = at::Tensor(), bool relu = false) {
@@ -1154,8 +1154,8 @@ at::Tensor conv_f32(const at::Tensor& feats, const at::Tensor& kernel, bool tran
   const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(feats.size(1)),
             c_out = static_cast<int>(kernel.size(transpose ? 1 : 2));
   const uint32_t n_dst = static_cast<uint32_t>(nbr.size(1));
+  if (!rmn_conv_f32_pays(n_dst, K, c_in, c_out)) return at::Tensor();
   const size_t bytes = rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out);
-  if (bytes == 0) return at::Tensor();
   auto scratch = at::empty({static_cast<int64_t>(bytes)}, kernel.options().dtype(at::kByte));
   auto out = at::empty({nbr.size(1), c_out}, feats.options());
   check(rmn_conv_forward_f32(static_cast<const float*>(ptr(feats)), static_cast<uint32_t>(feats.size(0)), c_in,
