@@ -110,7 +110,7 @@ int rmn_table_build(const int32_t *d_coords, uint32_t n_rows, int W, void *d_tab
 
 /*
  * rmn_table_build in two calls on one stream, for hosts that want the number of unique rows as early as
- * possible: after rmn_table_build_begin (header, slot fill, insert, first-occurrence counts) the header is
+ * possible: after rmn_table_build_begin (header, slot fill, insert) the header is
  * final, so an event recorded between the two calls lets a second stream run rmn_table_info while
  * rmn_table_build_finish (unique ids, mapping, unique coordinates, inverse) still runs on the first.
  * Arguments as in rmn_table_build; both calls take the same table, coordinates and workspace.

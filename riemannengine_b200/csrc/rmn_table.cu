@@ -867,7 +867,7 @@ static int table_build(const int32_t* d_coords, uint32_t n_rows, int W, void* d_
   return table_build_finish(d_coords, n_rows, W, d_table, d_mapping, d_inverse, d_unique_coords, d_workspace, post, stream);
 }
 
-// First half of a build: header, slot fill + bounding box, insert, first-occurrence counts. When it has
+// First half of a build: header, slot fill + bounding box, insert, number of unique rows. When it has
 // run, the header is final (number of unique rows, status): a caller may read it back while the second
 // half is still running.
 extern "C" int rmn_table_build_begin(const int32_t* d_coords, uint32_t n_rows, int W, void* d_table,
