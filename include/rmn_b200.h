@@ -411,7 +411,7 @@ int rmn_conv_backward_input(const void *d_grad_out, uint32_t n_dst, int c_out,
 
 /* d_out[reverse ? K - 1 - k : k] = d_weights[k]^T, [K, c_in, c_out] -> [K, c_out, c_in]. The input gradient is
  * rmn_conv_forward of grad_out with the transposed weights over d_nbr_t, which is the faster way to run it for fp32
- * features (rmn_conv_backward_input has no scratch to transpose into); `reverse` serves point-symmetric self maps,
+ * features where rmn_conv_forward_f32 does not pay (rmn_conv_backward_input has no scratch to transpose into); `reverse` serves point-symmetric self maps,
  * whose d_nbr_t is the forward table with its offsets in reverse order. */
 int rmn_conv_transpose_weights(const void *d_weights, int K, int c_in, int c_out, int dtype, int reverse,
                                void *d_out, void *stream);

@@ -8,6 +8,8 @@
 // Half or more of a table's entries are empty (35 % of a shell's, 54 % of a room's, 95 % of a lidar sweep's), and a
 // row-stationary register tile multiplies them as zeros. Both kernels compact the rows that have a neighbour at
 // an offset first and multiply only those. All sums run in a fixed order: no atomics, bit-reproducible.
+// The hosts run the forward pass and the input gradient here where little is to be done or the channel counts do not suit the
+// tensor cores (rmn_conv_f32_pays), elsewhere by rmn_conv_f32_tc.cu.
 #include "rmn_common.cuh"
 #include "rmn_tc.cuh"
 
