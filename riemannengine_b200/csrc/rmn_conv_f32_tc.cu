@@ -555,7 +555,8 @@ extern "C" int rmn_conv_forward_f32(const float* d_feats, uint32_t n_src, int c_
   if (need == 0) return RMN_ERR_UNSUPPORTED;
   // (with no source rows every table entry is -1 and nothing is read through d_feats)
   if (!d_weights || !d_nbr || !d_out || !d_scratch || (n_src > 0 && !d_feats)) return RMN_ERR_BAD_ARG;
-  if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_weights & 15) || ((uintptr_t)d_out & 15) || ((uintptr_t)d_scratch & 15))
+  // (weights are read by single elements: a view into a larger buffer of parameters need not be aligned)
+  if (((uintptr_t)d_feats & 31) || ((uintptr_t)d_out & 15) || ((uintptr_t)d_scratch & 15))
     return RMN_ERR_UNSUPPORTED;
   if (scratch_bytes < need) return RMN_ERR_ALLOC;
   tc::F3Args a = {};

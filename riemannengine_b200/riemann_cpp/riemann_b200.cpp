@@ -1149,7 +1149,7 @@ at::Tensor weight_image(const at::Tensor& kernel, std::pair<int64_t, int64_t> sh
 at::Tensor conv_f32(const at::Tensor& feats, const at::Tensor& kernel, bool transpose, bool reverse, const at::Tensor& nbr,
                     const at::Tensor& scale = at::Tensor(), const at::Tensor& shift = at::Tensor(), bool relu = false) {
   if (feats.scalar_type() != at::kFloat || feats.size(0) == 0 || nbr.size(1) == 0 ||
-      reinterpret_cast<uintptr_t>(feats.data_ptr()) % 32 != 0 || reinterpret_cast<uintptr_t>(kernel.data_ptr()) % 16 != 0)
+      reinterpret_cast<uintptr_t>(feats.data_ptr()) % 32 != 0)
     return at::Tensor();
   const int K = static_cast<int>(kernel.size(0)), c_in = static_cast<int>(feats.size(1)),
             c_out = static_cast<int>(kernel.size(transpose ? 1 : 2));

@@ -136,3 +136,19 @@ def test_transpose_weights_reverses_the_offsets():
                                                              ops._stream()), "rmn_conv_transpose_weights")
             want = w.transpose(1, 2)
             assert torch.equal(out, (want.flip(0) if reverse else want).contiguous())
+
+
+def test_weights_in_the_middle_of_a_buffer():
+    """Parameters flattened into one buffer start at any element: the same results as aligned ones, in every pass."""
+    from riemannengine_b200 import capi, ops
+    g = torch.Generator(device="cuda").manual_seed(4)
+    n, c, K = 20_000, 32, 27
+    assert capi.lib().rmn_conv_f32_pays(n, K, c, c)
+    nbr = torch.randint(-n, n, (K, n), generator=g, dtype=torch.int32, device="cuda").clamp_(min=-1)
+    feats = torch.randn((n, c), generator=g, device="cuda")
+    w = torch.randn((K, c, c), generator=g, device="cuda")
+    for first in (1, 2, 3):
+        inside = torch.zeros(w.numel() + 4, device="cuda")[first:first + w.numel()].view(w.shape).copy_(w)
+        assert inside.is_contiguous() and inside.data_ptr() % 16
+        assert torch.equal(ops.conv_forward(feats, inside, nbr), ops.conv_forward(feats, w, nbr))
+        assert torch.equal(ops.conv_backward_input(feats, inside, nbr), ops.conv_backward_input(feats, w, nbr))
