@@ -1461,15 +1461,18 @@ void RiemannConvolutionBaseImpl::reset_parameters(bool is_transpose) {
 }
 
 namespace {
-// whether the kernel that prepares a layer's weights also folds this batch norm (bf16 on tensor cores, parameters of one type)
+// whether the kernel that prepares a layer's weights also folds this batch norm (bf16 on tensor cores, parameters of one type,
+// none with a tangent or under a transform)
 bool folds_parameters(const RiemannConvolutionBaseImpl& conv, const torch::nn::BatchNorm1dImpl& bn) {
   auto const& kernel = conv.kernel_;
   auto const& mean = bn.running_mean;
-  if (!mean.defined() || !bn.running_var.defined() || kernel.scalar_type() != at::kBFloat16 || !kernel.is_cuda()) return false;
+  if (!mean.defined() || !bn.running_var.defined() || kernel.scalar_type() != at::kBFloat16 || !kernel.is_cuda() ||
+      !plain_autograd(kernel))
+    return false;
   if (mean.scalar_type() != at::kBFloat16 && mean.scalar_type() != at::kFloat) return false;
   for (auto const& p : {bn.running_var, bn.weight, bn.bias, conv.bias_, mean})
     if (p.defined() && (p.scalar_type() != mean.scalar_type() || !p.is_contiguous() || p.numel() != conv.out_channels_ ||
-                        p.device() != kernel.device()))
+                        p.device() != kernel.device() || !plain_autograd(p)))
       return false;
   const auto shape = run_shape(kernel);
   return rmn_conv_weight_image_bytes(static_cast<int>(kernel.size(0)), static_cast<int>(shape.first),
@@ -1489,7 +1492,8 @@ bool folds_batch_norm(const RiemannConvolutionBaseImpl& conv, const SparseTensor
 bool takes_ordered_map(const RiemannConvolutionBaseImpl& conv, const SparseTensor& input) {
   auto const& kernel = conv.kernel_;
   auto const& x = input.F();
-  if (at::GradMode::is_enabled() || !plain_autograd(x) || !plain_autograd(kernel) || !x.is_cuda() || x.size(0) == 0 ||
+  if (at::GradMode::is_enabled() || !plain_autograd(x) || !plain_autograd(kernel) ||
+      (conv.bias_.defined() && !plain_autograd(conv.bias_)) || !x.is_cuda() || x.size(0) == 0 ||
       x.scalar_type() != at::kBFloat16 || kernel.scalar_type() != at::kBFloat16 || conv.is_transpose_)
     return false;
   const auto shape = run_shape(kernel);
@@ -1597,8 +1601,7 @@ std::vector<PreparedWeights> prepare_layers(
     auto const& conv = *layers[i].first;
     auto bn = layers[i].second->normalization();
     auto const& kernel = conv.kernel_;
-    if (bn->is_training() || !plain_autograd(kernel) || kernel.device() != device || !kernel.is_contiguous() ||
-        !folds_parameters(conv, *bn))
+    if (bn->is_training() || kernel.device() != device || !kernel.is_contiguous() || !folds_parameters(conv, *bn))
       continue;
     const auto shape = run_shape(kernel);
     auto data = [](const at::Tensor& t) { return t.defined() ? ptr(t) : nullptr; };
@@ -1643,7 +1646,7 @@ SparseTensor conv_norm_relu(const SparseTensor& input, RiemannConvolutionBaseImp
               folds_batch_norm(conv, input, *bn);
   if (fuse && residual) {  // (a stride-1 layer: the output lies on the input's map)
     auto const& r = residual->F();
-    fuse = conv.kernel_generator_.kernel_stride() == stride_type(conv.dimension_, 1) && !conv.is_transpose_ &&
+    fuse = plain_autograd(r) && conv.kernel_generator_.kernel_stride() == stride_type(conv.dimension_, 1) && !conv.is_transpose_ &&
            residual->coordinate_manager() == input.coordinate_manager() &&
            residual->coordinate_map_key() == input.coordinate_map_key() && r.size(0) == input.F().size(0) &&
            r.size(1) == conv.out_channels_ && r.scalar_type() == at::kBFloat16 && r.is_contiguous() &&

@@ -215,3 +215,46 @@ def test_layers_prepared_together_run_as_prepared_alone():
     scale = float(alone.float().pow(2).mean().sqrt())
     # every layer rounds to bf16 (2^-9) once instead of three times: some thirty layers' worth of it
     assert float((together.float() - alone.float()).pow(2).mean().sqrt()) <= 30 * 2.0 ** -9 * scale
+
+
+def test_parameters_with_tangents_are_not_dropped():
+    """Forward-mode derivatives do not depend on no_grad: a layer that fuses its parameters into a kernel of its own must not
+    return a result without the tangent. The convolutions have no forward-mode formula, so such a call raises."""
+    import torch
+    import torch.autograd.forward_ad as fwd
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    g = torch.Generator(device="cuda").manual_seed(6)
+
+    def give_tangent(p):
+        p.copy_(fwd.make_dual(p.detach().clone(), torch.ones_like(p)))
+
+    # a map large enough for an internal row order
+    c = torch.unique(torch.randint(0, 38, (3_600_000, 4), generator=g, device="cuda"), dim=0)
+    coords = torch.cat([torch.arange(c.size(0), device="cuda")[:, None] % 2, c], 1)[:1_500_000]
+    coords = torch.cat([coords, coords + torch.tensor([2, 0, 0, 0, 0], device="cuda")])[:1_980_000].int().contiguous()
+    layer = C.RiemannConvolution(32, 32, kernel_size=3, bias=True, dimension=4)
+    layer.to("cuda:0")
+    layer.to(torch.bfloat16)
+    x = torch.randn((coords.size(0), 32), generator=g, device="cuda").bfloat16()
+    with torch.no_grad():
+        layer(C.SparseTensor(x, coords))
+        with fwd.dual_level():
+            give_tangent(layer.bias)
+            with pytest.raises(RuntimeError, match="jvp"):
+                layer(C.SparseTensor(x, coords))
+    # a network whose layers fold their batch norms
+    xyz = torch.unique(torch.randint(0, 30, (4000, 3), generator=g, device="cuda"), dim=0)
+    small = torch.cat([torch.zeros((xyz.size(0), 1), dtype=xyz.dtype, device="cuda"), xyz], 1).int().contiguous()
+    feats = torch.randn((small.size(0), 4), generator=g, device="cuda").bfloat16()
+    for part in ("norm", "kernel"):
+        net = C.MinkUNet(4, 20, width=32, dimension=3)
+        net.to("cuda:0")
+        net.to(torch.bfloat16)
+        net.train(False)
+        with torch.no_grad():
+            net(C.SparseTensor(feats, small))
+            with fwd.dual_level():
+                give_tangent(next(p for name, p in net.named_parameters().items() if part in name))
+                with pytest.raises(RuntimeError, match="jvp"):
+                    net(C.SparseTensor(feats, small))
