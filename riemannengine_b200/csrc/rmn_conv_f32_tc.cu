@@ -9,9 +9,11 @@
 // 0.99e-7 / 1.19e-7, 64 -> 64 1.25e-7 / 1.56e-7; rooms at 46 %, 32 -> 64 0.90e-7 / 1.19e-7; lidar at 4 % 0.57e-7 / 1.04e-7.
 // (Read back every other stage, it is 2.7e-7.)
 //
-// Sums that are not finite are computed again with fp32 multiply-adds (exact_row): infinities and NaN do not survive the
-// split (inf - inf), nor do numbers that round to infinity in bf16. So are sums below 2^-90, where the third parts leave the
-// range of bf16.
+// Sums that are not finite are computed again with fp32 multiply-adds: infinities and NaN do not survive the split (inf - inf),
+// nor do numbers that round to infinity in bf16. So are sums below 2^-90, where the third parts leave the range of bf16. The
+// drain only marks their rows, and when the pipeline has ended sixteen of the CTA's warps take the marked ones (exact_rows):
+// nothing in the pipeline waits for them, however many they are. 40 003 rows of infinities, 64 -> 64: 0.88 ms, 5.2 ms
+// where the drain computed each row itself.
 //
 // The kernel is built like k_conv_ta (rmn_conv_ta.cuh): gather warps fetch rows into registers, split them there and store the
 // parts into tensor memory as the A operand; W[k] comes as a prepared image by bulk copies. 20 warps: 8 gather (two groups of
@@ -45,28 +47,30 @@ struct F3Cfg {
   static constexpr int SLOTS = FIT >= 4 ? 4 : 2;        // A slots per stream
   static constexpr uint32_t PART_BYTES = KB * CC * 2, B_BYTES = PARTS * PART_BYTES;
   static constexpr int B_STAGES = 8;
-  static constexpr uint32_t BAR_OFFSET = B_STAGES * B_BYTES;
   static constexpr int BARRIERS = 2 * B_STAGES + 2 * STREAMS * SLOTS + 2 * STREAMS * ACC_BUFS;
-  static constexpr uint32_t EP_OFFSET = BAR_OFFSET + 1024;  // 2 * CC floats of epilogue scale / shift
-  static constexpr uint32_t SMEM = EP_OFFSET + 2 * CC * 4;
+  static constexpr uint32_t EP_OFFSET = 1024;  // behind the barriers: 2 * CC floats of epilogue scale / shift
+  static constexpr uint32_t RING_OFFSET = 2048;  // W[k]
+  static constexpr uint32_t SMEM = RING_OFFSET + B_STAGES * B_BYTES;
   static_assert(FIT >= 2 && BARRIERS * 8 + 4 <= 1024 && (CC == 32 || CC == 64), "tensor / shared memory");
 };
+// Marks of a CTA's rows that are computed again, one bit each; rows beyond this many share them.
+constexpr uint32_t kF3Marks = 8192;
 
 constexpr int kF3MmaWarp = 8, kF3WeightWarp = 10, kF3DrainWarp0 = 12, kF3Warps = 20, kF3Threads = kF3Warps * 32;
 // Registers: 640 threads x 96 at launch = 256 x 112 (gather) + 128 x 48 (MMA, weights) + 256 x 104 (drain)
-constexpr int kF3GatherRegs = 112, kF3IssueRegs = 48, kF3DrainRegs = 104;
+constexpr int kF3GatherRegs = 112, kF3IssueRegs = 48, kF3DrainRegs = 104, kF3ExactRegs = 96;
 
 struct F3Args {
   const float* src;      // [*, c_red]
   const uint8_t* image;  // k_f3_image of w
-  const float* w;        // [K][c_red][c_col], transpose: [K][c_col][c_red]
+  const float* w;        // [K][c_red][c_col]
   const int32_t* nbr;
   float* out;            // [n_dst, c_col]
   const float* ep_scale;
   const float* ep_shift;
   uint32_t* status;
   uint32_t n_dst, n_super;
-  int K, c_red, c_col, n_kb, transpose, reverse, relu;
+  int K, c_red, c_col, n_kb, relu;
 };
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -96,10 +100,12 @@ __device__ __forceinline__ constexpr uint32_t f3_n_channel(uint32_t p) {
 }
 
 // Image of the weights: per stage (offset, 32-channel block) and block of CC columns the three parts, each the MN-major swizzled
-// operand of 32 lines. One thread per line and eight columns. reverse: offset k of the image is W[K - 1 - k].
+// operand of 32 lines. One thread per line and eight columns. reverse: offset k of the image is W[K - 1 - k]. plain (or NULL): the
+// weights as [K][c_red][c_col] in the image's order of offsets.
 template <int CC>
 __global__ void __launch_bounds__(256) k_f3_image(const float* __restrict__ w, int K, int c_red, int c_col, int n_kb, int blocks,
-                                                  int transpose, int reverse, uint4* __restrict__ image) {
+                                                  int transpose, int reverse, uint4* __restrict__ image,
+                                                  float* __restrict__ plain) {
   after_previous_kernel();
   constexpr uint32_t CPL = CC / 8, CHUNKS = 32 * CPL;
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
@@ -112,7 +118,9 @@ __global__ void __launch_bounds__(256) k_f3_image(const float* __restrict__ w, i
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int co = col0 + (int)f3_n_channel<CC>(c * 8 + q);
-    v[q] = ci >= c_red || co >= c_col ? 0.f : __ldg(wk + (transpose ? (size_t)co * c_red + ci : (size_t)ci * c_col + co));
+    const bool in = ci < c_red && co < c_col;
+    v[q] = in ? __ldg(wk + (transpose ? (size_t)co * c_red + ci : (size_t)ci * c_col + co)) : 0.f;
+    if (plain && in) plain[((size_t)k * c_red + ci) * c_col + co] = v[q];
   }
   uint4* dst = image + (size_t)block * 3 * CHUNKS + p * CPL + swz<CC * 2>(p, c);
 #pragma unroll
@@ -169,23 +177,75 @@ __device__ __forceinline__ float f3_finish(float v, float scale, float shift, in
   return relu ? relu_f32(v) : v;
 }
 
-// One output row (columns col0 .. col0 + width - 1) by fp32 multiply-adds, by a whole warp
-__device__ __noinline__ void exact_row(const F3Args& a, uint32_t row, int col0, int width, const float* s_ep, int lane) {
-  for (int c = lane; c < width && col0 + c < a.c_col; c += 32) {
-    float sum = 0.f;
-    for (int k = 0; k < a.K; ++k) {
-      const int32_t idx = __ldg(a.nbr + (size_t)k * a.n_dst + row);
-      if (idx < 0) continue;
-      const float* x = a.src + (size_t)idx * a.c_red;
-      const float* w = a.w + (size_t)(a.reverse ? a.K - 1 - k : k) * a.c_red * a.c_col;
-      w += a.transpose ? (size_t)(col0 + c) * a.c_red : (size_t)(col0 + c);
-      const int step = a.transpose ? 1 : a.c_col;
-      float part = 0.f;
-      for (int ci = 0; ci < a.c_red; ++ci) part = fmaf(__ldg(x + ci), __ldg(w + (size_t)ci * step), part);
-      sum += part;
+// Rows row0 .. row0 + 3 (columns col0 .. col0 + CC - 1) by fp32 multiply-adds, by a whole warp: a lane per column of every 32
+template <int CC>
+__device__ __forceinline__ void exact_rows(const F3Args& a, uint32_t row0, int col0, const float* s_ep, int lane) {
+  constexpr int NC = CC / 32;
+  if (row0 >= a.n_dst) return;
+  float sum[4][NC];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) sum[r][c] = 0.f;
+  auto entry = [&](int k, int r) { return k < a.K && row0 + r < a.n_dst ? __ldg(a.nbr + (size_t)k * a.n_dst + row0 + r) : -1; };
+  int32_t next[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) next[r] = entry(0, r);
+#pragma unroll 1
+  for (int k = 0; k < a.K; ++k) {
+    int32_t idx[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      idx[r] = next[r];
+      next[r] = entry(k + 1, r);
     }
-    a.out[(size_t)row * a.c_col + col0 + c] = f3_finish(sum, s_ep[c], s_ep[width + c], a.relu);
+    if ((idx[0] & idx[1] & idx[2] & idx[3]) < 0) continue;  // none exists
+    float part[4][NC];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) part[r][c] = 0.f;
+    const float* w = a.w + (size_t)k * a.c_red * a.c_col;
+#pragma unroll 1
+    for (int c0 = 0; c0 < a.c_red; c0 += 32) {
+      float x[4];  // a channel per lane
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        x[r] = idx[r] >= 0 && c0 + lane < a.c_red ? __ldg(a.src + (size_t)idx[r] * a.c_red + c0 + lane) : 0.f;
+#pragma unroll 1
+      for (int ci = 0; ci < 32 && c0 + ci < a.c_red; ci += 4) {
+        float v[4][NC];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const int col = col0 + 32 * c + lane;
+            v[e][c] = __ldg(w + (size_t)(c0 + ci + e) * a.c_col + (col < a.c_col ? col : 0));  // (columns past the last are dropped)
+          }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float xe = __shfl_sync(0xFFFFFFFFu, x[r], ci + e);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) part[r][c] = fmaf(xe, v[e][c], part[r][c]);
+          }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (idx[r] >= 0) sum[r][c] += part[r][c];
   }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int at = 32 * c + lane;
+      if (row0 + r < a.n_dst && col0 + at < a.c_col)
+        a.out[(size_t)(row0 + r) * a.c_col + col0 + at] = f3_finish(sum[r][c], s_ep[at], s_ep[CC + at], a.relu);
+    }
 }
 
 // blockIdx.y: block of CC columns
@@ -194,7 +254,8 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
   using C = F3Cfg<CC, T_>;
   constexpr int T = T_, SLOTS = C::SLOTS, BST = C::B_STAGES, SWB = CC * 2;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint64_t* b_full = reinterpret_cast<uint64_t*>(smem + C::BAR_OFFSET);
+  __shared__ uint32_t s_marks[kF3Marks / 32], s_marked;
+  uint64_t* b_full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* b_empty = b_full + BST;
   uint64_t* a_full = b_empty + BST;              // [stream][slot]
   uint64_t* a_empty = a_full + 2 * SLOTS;        // [stream][slot]
@@ -205,7 +266,9 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
 
   // (uniform for the compiler, see k_conv_ta)
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  if (tid < kF3Marks / 32) s_marks[tid] = 0u;
   if (tid == 0) {
+    s_marked = 0u;
     for (int s = 0; s < BST; ++s) {
       mbar_init(&b_full[s], 1);
       mbar_init(&b_empty[s], T > 1 ? 2 : 1);
@@ -239,7 +302,7 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
   tc_fence_after();
   release_next_kernel();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-  const uint32_t smem_base = smem_u32(smem);
+  const uint32_t smem_base = smem_u32(smem) + C::RING_OFFSET;
   const int n_stages = a.K * a.n_kb;
   // stages of a stream per super-tile
   auto stages_of = [&](int stream) { return T > 1 ? n_stages : (n_stages + 1 - stream) / 2; };
@@ -409,8 +472,8 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
     const int set = (warp - kF3DrainWarp0) >> 2, u = lane & 3;
     const uint32_t quad = warp & 3;
     const int longest = stages_of(0);
-    uint32_t cnt[2] = {0, 0};
-    for (uint32_t st = blockIdx.x; st < a.n_super && !timed_out; st += gridDim.x) {
+    uint32_t cnt[2] = {0, 0}, mark = (T > 1 ? set * 4 : 0) + quad;  // of this warp's block of 32 rows
+    for (uint32_t st = blockIdx.x; st < a.n_super && !timed_out; st += gridDim.x, mark += 4 * T) {
       float sum[HALVES][CC / 8][4];
 #pragma unroll
       for (int h = 0; h < HALVES; ++h)
@@ -450,19 +513,21 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
       for (int h = 0; h < HALVES; ++h) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const uint32_t tile_row0 = st * (kTileM * T) + (T > 1 ? set : 0) * kTileM + quad * 32 + (T > 1 ? h : set) * 16 + i * 8;
-          const uint32_t row = tile_row0 + (lane >> 2);
+          const uint32_t row = st * (kTileM * T) + (T > 1 ? set : 0) * kTileM + quad * 32 + (T > 1 ? h : set) * 16 + i * 8 + (lane >> 2);
           // magnitudes outside [2^-90, the largest number], zero apart
-          bool again = false;
+          bool bad = false;
 #pragma unroll
           for (int v = 0; v < CC / 8; ++v)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const uint32_t bits = __float_as_uint(sum[h][v][2 * i + e]) << 1;
-              again = again || (bits != 0u && bits - (37u << 24) >= (255u - 37u) << 24);
+              bad = bad || (bits != 0u && bits - (37u << 24) >= (255u - 37u) << 24);
             }
-          uint32_t votes = __ballot_sync(0xFFFFFFFFu, again && row < a.n_dst);
-          if (row < a.n_dst && !((votes >> (lane & 28)) & 0xFu)) {
+          if (bad) {  // (rare; sums of rows past the last one are zeros)
+            atomicOr(&s_marks[mark % (kF3Marks / 32)], 1u << ((T > 1 ? h : set) * 16 + i * 8 + (lane >> 2)));
+            s_marked = 1u;
+          }
+          if (row < a.n_dst) {
             float* dst = a.out + (size_t)row * a.c_col;
 #pragma unroll
             for (int v = 0; v < CC / 8; v += 2) {
@@ -477,11 +542,6 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
               }
             }
           }
-          while (votes) {
-            const int r = (__ffs(votes) - 1) >> 2;
-            votes &= ~(0xFu << (4 * r));
-            exact_row(a, tile_row0 + r, col0, CC, s_ep, lane);
-          }
         }
       }
     }
@@ -489,10 +549,19 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
 
   if (timed_out) atomicExch(a.status, (uint32_t)RMN_ERR_TIMEOUT);
   tc_fence_before();
-  __syncthreads();
+  const bool failed = __syncthreads_or(timed_out);
   if (warp == kF3MmaWarp) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+  }
+  // ------------------------------ marked rows ------------------------------------------
+  if (failed || !s_marked || (warp >= kF3MmaWarp && warp < kF3DrainWarp0)) return;
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kF3ExactRegs));
+  const uint32_t worker = warp < kF3MmaWarp ? warp : warp - (kF3DrainWarp0 - kF3MmaWarp);
+  const uint32_t mine = (a.n_super - blockIdx.x + gridDim.x - 1) / gridDim.x * (32 * T);  // groups of four rows
+  for (uint32_t i = worker; i < mine; i += 16) {
+    if (!((s_marks[i / 8 % (kF3Marks / 32)] >> (i % 8 * 4)) & 15u)) continue;
+    exact_rows<CC>(a, (blockIdx.x + i / (32 * T) * gridDim.x) * (kTileM * T) + i % (32 * T) * 4, col0, s_ep, lane);
   }
 }
 
@@ -510,16 +579,17 @@ int launch_f3(F3Args a, uint32_t blocks, uint32_t fit, cudaStream_t stream) {
 }
 
 template <int CC>
-int run_f3(F3Args a, uint8_t* image, cudaStream_t stream) {
+int run_f3(F3Args a, int transpose, int reverse, uint8_t* image, float* plain, cudaStream_t stream) {
   int dev = 0, sms = 148;
   RMN_CUDA_TRY(cudaGetDevice(&dev));
   RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const uint32_t blocks = (uint32_t)(a.c_col + CC - 1) / CC, fit = (uint32_t)sms > blocks ? (uint32_t)sms / blocks : 1u;
   const uint32_t lines = (uint32_t)(a.K * a.n_kb) * blocks * 32 * (CC / 8);
   RMN_CUDA_TRY(launch_overlapped(k_f3_image<CC>, dim3((lines + 255) / 256), dim3(256), 0, stream, a.w, a.K, a.c_red, a.c_col,
-                                 a.n_kb, (int)blocks, a.transpose, a.reverse, reinterpret_cast<uint4*>(image)));
+                                 a.n_kb, (int)blocks, transpose, reverse, reinterpret_cast<uint4*>(image), plain));
   RMN_LAUNCH_CHECK();
   a.image = image;
+  if (plain) a.w = plain;
   // row tiles of the busiest SM: pairs of them share their weights, single ones leave fewer SMs idle at the end
   const uint32_t tiles = (a.n_dst + kTileM - 1) / kTileM, pairs = (tiles + 1) / 2;
   const uint32_t rounds2 = (pairs + fit - 1) / fit * 2, rounds1 = (tiles + fit - 1) / fit;
@@ -531,10 +601,14 @@ int run_f3(F3Args a, uint8_t* image, cudaStream_t stream) {
 
 using namespace rmn;
 
-extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, int c_out) {
-  if (n_dst == 0 || K < 1 || K > 4096 || c_in < 16 || c_in > 1024 || c_in % 8 || c_out < 4 || c_out > 1024 || c_out % 4) return 0;
+// The image of the weights, and behind it the weights themselves in its order
+static size_t f3_image_bytes(int K, int c_in, int c_out) {
   const size_t cc = c_out <= 32 ? 32 : 64, columns = (c_out + cc - 1) / cc * cc;
   return (size_t)K * ((c_in + 31) / 32) * 32 * columns * 3 * 2;
+}
+extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, int c_out) {
+  if (n_dst == 0 || K < 1 || K > 4096 || c_in < 16 || c_in > 1024 || c_in % 8 || c_out < 4 || c_out > 1024 || c_out % 4) return 0;
+  return f3_image_bytes(K, c_in, c_out) + (size_t)K * c_in * c_out * sizeof(float);
 }
 
 // Little work is the multiply-add kernel's: these kernels need the weights prepared by a launch of their own, which a host that
@@ -572,10 +646,11 @@ extern "C" int rmn_conv_forward_f32(const float* d_feats, uint32_t n_src, int c_
   a.c_red = c_in;
   a.c_col = c_out;
   a.n_kb = (c_in + 31) / 32;
-  a.transpose = transpose;
-  a.reverse = reverse;
   a.relu = relu;
   if (!a.status) return RMN_ERR_CUDA;
-  return c_out <= 32 ? tc::run_f3<32>(a, static_cast<uint8_t*>(d_scratch), (cudaStream_t)stream_)
-                     : tc::run_f3<64>(a, static_cast<uint8_t*>(d_scratch), (cudaStream_t)stream_);
+  uint8_t* image = static_cast<uint8_t*>(d_scratch);
+  // (for exact_rows, whose lanes read neighbouring columns)
+  float* plain = transpose || reverse ? reinterpret_cast<float*>(image + f3_image_bytes(K, c_in, c_out)) : nullptr;
+  return c_out <= 32 ? tc::run_f3<32>(a, transpose, reverse, image, plain, (cudaStream_t)stream_)
+                     : tc::run_f3<64>(a, transpose, reverse, image, plain, (cudaStream_t)stream_);
 }

@@ -152,3 +152,57 @@ def test_weights_in_the_middle_of_a_buffer():
         assert inside.is_contiguous() and inside.data_ptr() % 16
         assert torch.equal(ops.conv_forward(feats, inside, nbr), ops.conv_forward(feats, w, nbr))
         assert torch.equal(ops.conv_backward_input(feats, inside, nbr), ops.conv_backward_input(feats, w, nbr))
+
+
+@pytest.mark.parametrize("c_in,c_out,transpose,reverse", [(32, 32, 0, 0), (64, 64, 1, 0), (64, 100, 1, 1), (40, 36, 0, 1)])
+def test_rows_that_are_computed_again(c_in, c_out, transpose, reverse):
+    """Rows of every tile and quarter of a tile, a few of them and all: the multiply-add kernel's values, in about its time
+    (they used to be a serial chain inside the pipeline, an order of magnitude slower than that kernel)."""
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    g = torch.Generator(device="cuda").manual_seed(c_in + c_out)
+    n, K = 40_003, 27
+    nbr = torch.randint(-n, n, (K, n), generator=g, dtype=torch.int32, device="cuda").clamp_(min=-1)
+    nbr[:, 5::7919] = torch.arange(5, n, 7919, dtype=torch.int32, device="cuda")
+    feats = torch.randn((n, c_in), generator=g, device="cuda")
+    w = torch.randn((K, c_in, c_out), generator=g, device="cuda")
+    given = w.flip(0) if reverse else w
+    given = (given.transpose(1, 2) if transpose else given).contiguous()
+    shift = torch.randn(c_out, generator=g, device="cuda")
+    size = lib.rmn_conv_f32_scratch_bytes(n, K, c_in, c_out)
+    scratch, out = torch.empty(size, dtype=torch.uint8, device="cuda"), torch.empty((n, c_out), device="cuda")
+
+    def fast():
+        capi.check(lib.rmn_conv_forward_f32(ops._ptr(feats), n, c_in, ops._ptr(given), K, c_out, transpose, reverse, ops._ptr(nbr),
+                                            n, ops._ptr(out), None, ops._ptr(shift), 0, ops._ptr(scratch), size, ops._stream()),
+                   "rmn_conv_forward_f32")
+        return out
+
+    def plain():
+        again = torch.empty((n, c_out), device="cuda")
+        capi.check(lib.rmn_conv_forward_fused(ops._ptr(feats), n, c_in, ops._ptr(w), K, c_out, ops._ptr(nbr), n, ops._ptr(again),
+                                              capi.F32, None, ops._ptr(shift), 0, ops._stream()), "rmn_conv_forward_fused")
+        return again
+
+    def time(f):
+        best = 1e9
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            f()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    normal = time(plain)
+    feats[5::7919] = float("nan")
+    got, want = fast(), plain()
+    assert torch.equal(got.isnan(), want.isnan()) and bool(got[5::7919].isnan().all()) and bool(got.isfinite().any())
+    ok = want.isfinite()
+    # within twice the bound of a sum of K c_in multiply-adds of this size (see above) of each other
+    assert float((got[ok] - want[ok]).abs().max()) <= 2.0 ** -18 * float(want[ok].abs().max())
+    feats.fill_(float("inf"))
+    assert torch.equal(fast().nan_to_num(7.0), plain().nan_to_num(7.0))
+    assert time(fast) <= 8 * normal
+    capi.check(lib.rmn_device_status(ops._stream()), "rmn_device_status")
