@@ -418,7 +418,8 @@ int rmn_conv_transpose_weights(const void *d_weights, int K, int c_in, int c_out
 
 /*
  * fp32 convolution on the tensor cores: every number as three bf16 parts, products of parts whose error is that of fp32,
- * sums in fp32 (results that are not finite, or below 2^-90, are computed with fp32 multiply-adds). Bytes of scratch (the
+ * sums in fp32. Results that are not finite, or too small to hold what parts of tiny operands lose, are computed with fp32
+ * multiply-adds. Bytes of scratch (the
  * prepared weights) of rmn_conv_forward_f32, 0 where it does not serve (use rmn_conv_forward): c_in a multiple of 8 from 16
  * on, c_out a multiple of 4. rmn_conv_f32_pays: whether it is the faster way for a pass of this size.
  * rmn_conv_forward_f32: rmn_conv_forward_fused for fp32 (d_feats 32-byte aligned, d_out and d_scratch 16-byte aligned:

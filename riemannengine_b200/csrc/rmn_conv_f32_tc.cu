@@ -10,7 +10,11 @@
 // (Read back every other stage, it is 2.7e-7.)
 //
 // Sums that are not finite are computed again with fp32 multiply-adds: infinities and NaN do not survive the split (inf - inf),
-// nor do numbers that round to infinity in bf16. So are sums below 2^-90, where the third parts leave the range of bf16. The
+// nor do numbers that round to infinity in bf16. Numbers below 2^-102 lose their last parts, which fall below the normal numbers of
+// bf16, up to 2^-126 of them in all; products below 2^-102 lose parts in the sums. So the kernel that prepares the weights also
+// finds the largest and the smallest magnitude of the weights and of the features (one pass over these, 13 MB of 102 K rows, which
+// the gathers then find in the L2), and if there is such a number or product, sums below 2^-90 times the largest operand (or 1) are
+// computed again, too, zeros among them: what a sum of up to 2^11 such terms can have lost lies below 2^-25 of any other. The
 // drain only marks their rows, and when the pipeline has ended sixteen of the CTA's warps take the marked ones (exact_rows):
 // nothing in the pipeline waits for them, however many they are. 40 003 rows of infinities, 64 -> 64: 0.88 ms, 5.2 ms
 // where the drain computed each row itself.
@@ -68,10 +72,38 @@ struct F3Args {
   float* out;            // [n_dst, c_col]
   const float* ep_scale;
   const float* ep_shift;
+  const uint4* ranges;  // k_f3_image's
   uint32_t* status;
-  uint32_t n_dst, n_super;
+  uint32_t n_dst, n_super, n_ranges;
   int K, c_red, c_col, n_kb, relu;
 };
+
+// Largest magnitude and smallest but zero of some numbers, as bits without the sign, shifted up by one: .x and .z are the largest
+// (weights, features), .y and .w the smallest minus one, where zero wraps around to the largest integer.
+__device__ __forceinline__ void take_range(float v, uint32_t& most, uint32_t& least) {
+  const uint32_t u = __float_as_uint(v) << 1;
+  most = max(most, u);
+  least = min(least, u - 1u);
+}
+constexpr uint4 kNoRange{0u, ~0u, 0u, ~0u};
+__device__ __forceinline__ void merge_ranges(uint4 r, uint4* shared) {  // by a whole warp
+  r.x = __reduce_max_sync(0xFFFFFFFFu, r.x);
+  r.y = __reduce_min_sync(0xFFFFFFFFu, r.y);
+  r.z = __reduce_max_sync(0xFFFFFFFFu, r.z);
+  r.w = __reduce_min_sync(0xFFFFFFFFu, r.w);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&shared->x, r.x);
+    atomicMin(&shared->y, r.y);
+    atomicMax(&shared->z, r.z);
+    atomicMin(&shared->w, r.w);
+  }
+}
+// Magnitude (bits, shifted up by one) below which a sum is computed again
+__device__ __forceinline__ uint32_t least_sum(uint4 r) {
+  constexpr uint32_t kTiny = 25u << 24;  // 2^-102
+  const bool lossy = r.y < kTiny || r.w < kTiny || (r.y >> 24) + (r.w >> 24) < 2 * 127 - 102;
+  return lossy ? min(max(max(r.x, r.z), 127u << 24), (255u << 24) - 1u) - (90u << 24) : 0u;
+}
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   uint32_t p;
@@ -101,31 +133,53 @@ __device__ __forceinline__ constexpr uint32_t f3_n_channel(uint32_t p) {
 
 // Image of the weights: per stage (offset, 32-channel block) and block of CC columns the three parts, each the MN-major swizzled
 // operand of 32 lines. One thread per line and eight columns. reverse: offset k of the image is W[K - 1 - k]. plain (or NULL): the
-// weights as [K][c_red][c_col] in the image's order of offsets.
+// weights as [K][c_red][c_col] in the image's order of offsets. The blocks from image_blocks on read the n_x numbers of x. ranges:
+// what each block has read.
 template <int CC>
 __global__ void __launch_bounds__(256) k_f3_image(const float* __restrict__ w, int K, int c_red, int c_col, int n_kb, int blocks,
                                                   int transpose, int reverse, uint4* __restrict__ image,
-                                                  float* __restrict__ plain) {
+                                                  float* __restrict__ plain, uint32_t image_blocks, const float4* __restrict__ x,
+                                                  size_t n_x, uint4* __restrict__ ranges) {
   after_previous_kernel();
-  constexpr uint32_t CPL = CC / 8, CHUNKS = 32 * CPL;
-  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
-  if (i >= (uint32_t)(K * n_kb * blocks) * CHUNKS) return;
-  const uint32_t block = i / CHUNKS, p = i % CHUNKS / CPL, c = i % CPL;
-  const int stage = (int)block / blocks, k = stage / n_kb, col0 = ((int)block % blocks) * CC;
-  const int ci = stage % n_kb * 32 + (int)f3_k_channel(p);
-  const float* wk = w + (size_t)(reverse ? K - 1 - k : k) * c_red * c_col;
-  float v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int co = col0 + (int)f3_n_channel<CC>(c * 8 + q);
-    const bool in = ci < c_red && co < c_col;
-    v[q] = in ? __ldg(wk + (transpose ? (size_t)co * c_red + ci : (size_t)ci * c_col + co)) : 0.f;
-    if (plain && in) plain[((size_t)k * c_red + ci) * c_col + co] = v[q];
+  __shared__ uint4 s_range;
+  if (threadIdx.x == 0) s_range = kNoRange;
+  __syncthreads();
+  uint4 range = kNoRange;
+  if (blockIdx.x >= image_blocks) {
+    const size_t step = (size_t)(gridDim.x - image_blocks) * 256;
+#pragma unroll 4
+    for (size_t i = (size_t)(blockIdx.x - image_blocks) * 256 + threadIdx.x; i < n_x / 4; i += step) {
+      const float4 v = __ldg(x + i);
+      take_range(v.x, range.z, range.w);
+      take_range(v.y, range.z, range.w);
+      take_range(v.z, range.z, range.w);
+      take_range(v.w, range.z, range.w);
+    }
   }
-  uint4* dst = image + (size_t)block * 3 * CHUNKS + p * CPL + swz<CC * 2>(p, c);
+  constexpr uint32_t CPL = CC / 8, CHUNKS = 32 * CPL;
+  const uint32_t lines = (uint32_t)(K * n_kb * blocks) * CHUNKS;
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; blockIdx.x < image_blocks && i < lines; i += image_blocks * 256) {
+    const uint32_t block = i / CHUNKS, p = i % CHUNKS / CPL, c = i % CPL;
+    const int stage = (int)block / blocks, k = stage / n_kb, col0 = ((int)block % blocks) * CC;
+    const int ci = stage % n_kb * 32 + (int)f3_k_channel(p);
+    const float* wk = w + (size_t)(reverse ? K - 1 - k : k) * c_red * c_col;
+    float v[8];
 #pragma unroll
-  for (int part = 0; part < 3; ++part)
-    dst[part * CHUNKS] = make_uint4(take_part(v[0], v[1]), take_part(v[2], v[3]), take_part(v[4], v[5]), take_part(v[6], v[7]));
+    for (int q = 0; q < 8; ++q) {
+      const int co = col0 + (int)f3_n_channel<CC>(c * 8 + q);
+      const bool in = ci < c_red && co < c_col;
+      v[q] = in ? __ldg(wk + (transpose ? (size_t)co * c_red + ci : (size_t)ci * c_col + co)) : 0.f;
+      if (plain && in) plain[((size_t)k * c_red + ci) * c_col + co] = v[q];
+      take_range(v[q], range.x, range.y);
+    }
+    uint4* dst = image + (size_t)block * 3 * CHUNKS + p * CPL + swz<CC * 2>(p, c);
+#pragma unroll
+    for (int part = 0; part < 3; ++part)
+      dst[part * CHUNKS] = make_uint4(take_part(v[0], v[1]), take_part(v[2], v[3]), take_part(v[4], v[5]), take_part(v[6], v[7]));
+  }
+  merge_ranges(range, &s_range);
+  __syncthreads();
+  if (threadIdx.x == 0) ranges[blockIdx.x] = s_range;
 }
 
 // 32 channels of a gather warp's 32 rows: lane t holds channels 8 c .. 8 c + 7 and 16 + 8 c .. 16 + 8 c + 7 (c = t / 2 & 1) of row
@@ -255,6 +309,7 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
   constexpr int T = T_, SLOTS = C::SLOTS, BST = C::B_STAGES, SWB = CC * 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint32_t s_marks[kF3Marks / 32], s_marked;
+  __shared__ uint4 s_range;
   uint64_t* b_full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* b_empty = b_full + BST;
   uint64_t* a_full = b_empty + BST;              // [stream][slot]
@@ -269,6 +324,7 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
   if (tid < kF3Marks / 32) s_marks[tid] = 0u;
   if (tid == 0) {
     s_marked = 0u;
+    s_range = kNoRange;
     for (int s = 0; s < BST; ++s) {
       mbar_init(&b_full[s], 1);
       mbar_init(&b_empty[s], T > 1 ? 2 : 1);
@@ -472,6 +528,16 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
     const int set = (warp - kF3DrainWarp0) >> 2, u = lane & 3;
     const uint32_t quad = warp & 3;
     const int longest = stages_of(0);
+    {
+      uint4 range = kNoRange;
+      for (uint32_t i = tid - kF3DrainWarp0 * 32; i < a.n_ranges; i += 256) {
+        const uint4 r = __ldg(a.ranges + i);
+        range = make_uint4(max(range.x, r.x), min(range.y, r.y), max(range.z, r.z), min(range.w, r.w));
+      }
+      merge_ranges(range, &s_range);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    const uint32_t least = least_sum(s_range);
     uint32_t cnt[2] = {0, 0}, mark = (T > 1 ? set * 4 : 0) + quad;  // of this warp's block of 32 rows
     for (uint32_t st = blockIdx.x; st < a.n_super && !timed_out; st += gridDim.x, mark += 4 * T) {
       float sum[HALVES][CC / 8][4];
@@ -514,16 +580,14 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const uint32_t row = st * (kTileM * T) + (T > 1 ? set : 0) * kTileM + quad * 32 + (T > 1 ? h : set) * 16 + i * 8 + (lane >> 2);
-          // magnitudes outside [2^-90, the largest number], zero apart
           bool bad = false;
 #pragma unroll
           for (int v = 0; v < CC / 8; ++v)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const uint32_t bits = __float_as_uint(sum[h][v][2 * i + e]) << 1;
-              bad = bad || (bits != 0u && bits - (37u << 24) >= (255u - 37u) << 24);
+              bad = bad || (__float_as_uint(sum[h][v][2 * i + e]) << 1) - least >= (255u << 24) - least;  // small, or not finite
             }
-          if (bad) {  // (rare; sums of rows past the last one are zeros)
+          if (bad && row < a.n_dst) {  // (rare)
             atomicOr(&s_marks[mark % (kF3Marks / 32)], 1u << ((T > 1 ? h : set) * 16 + i * 8 + (lane >> 2)));
             s_marked = 1u;
           }
@@ -578,16 +642,24 @@ int launch_f3(F3Args a, uint32_t blocks, uint32_t fit, cudaStream_t stream) {
   return RMN_OK;
 }
 
+constexpr uint32_t kF3ImageBlocks = 148 * 2, kF3RangeBlocks = 148 * 4;
+
 template <int CC>
-int run_f3(F3Args a, int transpose, int reverse, uint8_t* image, float* plain, cudaStream_t stream) {
+int run_f3(F3Args a, uint32_t n_src, int transpose, int reverse, uint8_t* image, float* plain, uint4* ranges, cudaStream_t stream) {
   int dev = 0, sms = 148;
   RMN_CUDA_TRY(cudaGetDevice(&dev));
   RMN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const uint32_t blocks = (uint32_t)(a.c_col + CC - 1) / CC, fit = (uint32_t)sms > blocks ? (uint32_t)sms / blocks : 1u;
   const uint32_t lines = (uint32_t)(a.K * a.n_kb) * blocks * 32 * (CC / 8);
-  RMN_CUDA_TRY(launch_overlapped(k_f3_image<CC>, dim3((lines + 255) / 256), dim3(256), 0, stream, a.w, a.K, a.c_red, a.c_col,
-                                 a.n_kb, (int)blocks, transpose, reverse, reinterpret_cast<uint4*>(image), plain));
+  const size_t n_x = (size_t)n_src * a.c_red;
+  const uint32_t image_blocks = (lines + 255) / 256 < kF3ImageBlocks ? (lines + 255) / 256 : kF3ImageBlocks;
+  const uint32_t range_blocks = n_x / 8192 < kF3RangeBlocks ? (uint32_t)(n_x / 8192) + 1 : kF3RangeBlocks;
+  RMN_CUDA_TRY(launch_overlapped(k_f3_image<CC>, dim3(image_blocks + range_blocks), dim3(256), 0, stream, a.w, a.K, a.c_red, a.c_col,
+                                 a.n_kb, (int)blocks, transpose, reverse, reinterpret_cast<uint4*>(image), plain, image_blocks,
+                                 reinterpret_cast<const float4*>(a.src), n_x, ranges));
   RMN_LAUNCH_CHECK();
+  a.ranges = ranges;
+  a.n_ranges = image_blocks + range_blocks;
   a.image = image;
   if (plain) a.w = plain;
   // row tiles of the busiest SM: pairs of them share their weights, single ones leave fewer SMs idle at the end
@@ -601,14 +673,15 @@ int run_f3(F3Args a, int transpose, int reverse, uint8_t* image, float* plain, c
 
 using namespace rmn;
 
-// The image of the weights, and behind it the weights themselves in its order
+// The image of the weights, behind it the weights themselves in its order, then the ranges of k_f3_image's blocks
 static size_t f3_image_bytes(int K, int c_in, int c_out) {
   const size_t cc = c_out <= 32 ? 32 : 64, columns = (c_out + cc - 1) / cc * cc;
   return (size_t)K * ((c_in + 31) / 32) * 32 * columns * 3 * 2;
 }
+static size_t f3_plain_bytes(int K, int c_in, int c_out) { return (size_t)K * c_in * c_out * sizeof(float); }  // (a multiple of 128)
 extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, int c_out) {
   if (n_dst == 0 || K < 1 || K > 4096 || c_in < 16 || c_in > 1024 || c_in % 8 || c_out < 4 || c_out > 1024 || c_out % 4) return 0;
-  return f3_image_bytes(K, c_in, c_out) + (size_t)K * c_in * c_out * sizeof(float);
+  return f3_image_bytes(K, c_in, c_out) + f3_plain_bytes(K, c_in, c_out) + (tc::kF3ImageBlocks + tc::kF3RangeBlocks) * sizeof(uint4);
 }
 
 // Little work is the multiply-add kernel's: these kernels need the weights prepared by a launch of their own, which a host that
@@ -650,7 +723,9 @@ extern "C" int rmn_conv_forward_f32(const float* d_feats, uint32_t n_src, int c_
   if (!a.status) return RMN_ERR_CUDA;
   uint8_t* image = static_cast<uint8_t*>(d_scratch);
   // (for exact_rows, whose lanes read neighbouring columns)
-  float* plain = transpose || reverse ? reinterpret_cast<float*>(image + f3_image_bytes(K, c_in, c_out)) : nullptr;
-  return c_out <= 32 ? tc::run_f3<32>(a, transpose, reverse, image, plain, (cudaStream_t)stream_)
-                     : tc::run_f3<64>(a, transpose, reverse, image, plain, (cudaStream_t)stream_);
+  uint8_t* behind = image + f3_image_bytes(K, c_in, c_out);
+  float* plain = transpose || reverse ? reinterpret_cast<float*>(behind) : nullptr;
+  uint4* ranges = reinterpret_cast<uint4*>(behind + f3_plain_bytes(K, c_in, c_out));
+  return c_out <= 32 ? tc::run_f3<32>(a, n_src, transpose, reverse, image, plain, ranges, (cudaStream_t)stream_)
+                     : tc::run_f3<64>(a, n_src, transpose, reverse, image, plain, ranges, (cudaStream_t)stream_);
 }

@@ -138,6 +138,43 @@ def test_transpose_weights_reverses_the_offsets():
             assert torch.equal(out, (want.flip(0) if reverse else want).contiguous())
 
 
+@pytest.mark.parametrize("x_exponent,w_exponent,both", [
+    (-118, 40, False), (-124, 60, False), (40, -118, False), (60, -124, False),   # one side's last parts below bf16's numbers
+    (-140, 60, False), (60, -140, False),                                        # no parts at all: sums of zero
+    (-70, -70, False), (-60, -45, False),                                        # products below the smallest numbers
+    (-118, 40, True), (30, -120, True), (-140, 60, True),                        # beside operands of ordinary size
+])
+@pytest.mark.parametrize("transpose", [0, 1])
+def test_tiny_operands_of_either_side(x_exponent, w_exponent, both, transpose):
+    """The loss of bits depends on the operands, not on the sum: tiny features beside large weights, and the reverse."""
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    g = torch.Generator(device="cuda").manual_seed(x_exponent + 2 * w_exponent)
+    n, K, c = 1500, 27, 32
+    nbr = torch.randint(-n, n, (K, n), generator=g, dtype=torch.int32, device="cuda").clamp_(min=-1)
+    # (magnitudes of 1 to 2, so that a sum has as many bits as its operands)
+    x = (1 + torch.rand((n, c), generator=g, device="cuda", dtype=torch.float64)) * 2.0 ** x_exponent
+    w = (1 + torch.rand((K, c, c), generator=g, device="cuda", dtype=torch.float64)) * 2.0 ** w_exponent
+    if both:   # rows and columns of ordinary numbers, and rows of zeros
+        x[::3] = torch.randn((n, c), generator=g, device="cuda", dtype=torch.float64)[::3]
+        x[1::5] = 0
+        w[:, :, ::2] = torch.randn((K, c, c), generator=g, device="cuda", dtype=torch.float64)[:, :, ::2]
+    x, w = x.float(), w.float()
+    given = (w.transpose(1, 2) if transpose else w).contiguous()
+    size = lib.rmn_conv_f32_scratch_bytes(n, K, c, c)
+    scratch, out = torch.empty(size, dtype=torch.uint8, device="cuda"), torch.empty((n, c), device="cuda")
+    capi.check(lib.rmn_conv_forward_f32(ops._ptr(x), n, c, ops._ptr(given), K, c, transpose, 0, ops._ptr(nbr), n, ops._ptr(out),
+                                        None, None, 0, ops._ptr(scratch), size, ops._stream()), "rmn_conv_forward_f32")
+    want, most = (torch.zeros((n, c), dtype=torch.float64, device="cuda") for _ in range(2))
+    for k in range(K):
+        hit = nbr[k] >= 0
+        a, b = x[nbr[k][hit].long()].double(), w[k].double()
+        want[hit] += a @ b
+        most[hit] += a.abs() @ b.abs()
+    # 32 multiply-adds of an offset, 27 offsets: 2^-24 of the magnitudes each, 2^-150 where numbers are subnormal
+    assert bool(((out.double() - want).abs() <= 59 * (2.0 ** -24 * most + 2.0 ** -150)).all())
+
+
 def test_weights_in_the_middle_of_a_buffer():
     """Parameters flattened into one buffer start at any element: the same results as aligned ones, in every pass."""
     from riemannengine_b200 import capi, ops
