@@ -4,10 +4,12 @@
 // An fp32 number is the sum of three bf16 numbers x0 + x1 + x2 of eight significant bits each, every one the nearest to what the
 // ones before it leave. Of the nine products of the parts of two numbers the six with i + j <= 2 are multiplied, the smallest
 // first; the others lie below 2^-24 of the product. Tensor memory adds with truncation, so no sum stays there for long: after
-// every stage (32 channels of an offset) it is read back and added, rounded to nearest, to sums in registers. Error against 64
-// bits (2-norm) here / by k_conv_f32, whose sums of an offset are chains of multiply-adds: 101 930 rows of a shell, 32 -> 32
-// 0.99e-7 / 1.19e-7, 64 -> 64 1.25e-7 / 1.56e-7; rooms at 46 %, 32 -> 64 0.90e-7 / 1.19e-7; lidar at 4 % 0.57e-7 / 1.04e-7.
-// (Read back every other stage, it is 2.7e-7.)
+// every stage (32 channels of an offset) it is read back and added, rounded to nearest, to sums in registers. These are added up in
+// groups of stages, whose sums lie in shared memory, so that no long chain rounds at the size of the result (sum_outward: the
+// rounding that takes out the bias of the truncation). Error against 64 bits (2-norm) here / by k_conv_f32, whose sums of an offset
+// are chains of multiply-adds: 30 000 random rows at 66 %, 32 -> 32, numbers of either sign 0.71e-7 / 1.22e-7, positive ones
+// 0.41e-7 / 0.54e-7, 64 -> 64 0.86e-7 / 1.59e-7 and 0.46e-7 / 0.58e-7 (without groups 1.26e-7 and 1.06e-7, and some 4 % faster);
+// 343 offsets 1.16e-7 / 1.46e-7 and 0.58e-7 / 0.55e-7. (Read back every other stage, it is 2.7e-7.)
 //
 // Sums that are not finite are computed again with fp32 multiply-adds: infinities and NaN do not survive the split (inf - inf),
 // nor do numbers that round to infinity in bf16. Numbers below 2^-102 lose their last parts, which fall below the normal numbers of
@@ -34,6 +36,8 @@
 
 #include <cuda_bf16.h>
 
+#include <cmath>
+
 namespace rmn {
 
 const uint32_t* tc_status_device_address();  // rmn_conv_tc.cu
@@ -54,7 +58,9 @@ struct F3Cfg {
   static constexpr int BARRIERS = 2 * B_STAGES + 2 * STREAMS * SLOTS + 2 * STREAMS * ACC_BUFS;
   static constexpr uint32_t EP_OFFSET = 1024;  // behind the barriers: 2 * CC floats of epilogue scale / shift
   static constexpr uint32_t RING_OFFSET = 2048;  // W[k]
-  static constexpr uint32_t SMEM = RING_OFFSET + B_STAGES * B_BYTES;
+  static constexpr uint32_t TOTAL_OFFSET = RING_OFFSET + B_STAGES * B_BYTES;  // sums of the stages before the present group
+  static constexpr int TOTAL_VECS = (T > 1 ? 2 : 1) * CC / 8;                 // float4 of each drain thread
+  static constexpr uint32_t SMEM = TOTAL_OFFSET + TOTAL_VECS * 256 * 16;
   static_assert(FIT >= 2 && BARRIERS * 8 + 4 <= 1024 && (CC == 32 || CC == 64), "tensor / shared memory");
 };
 // Marks of a CTA's rows that are computed again, one bit each; rows beyond this many share them.
@@ -75,7 +81,7 @@ struct F3Args {
   const uint4* ranges;  // k_f3_image's
   uint32_t* status;
   uint32_t n_dst, n_super, n_ranges;
-  int K, c_red, c_col, n_kb, relu;
+  int K, c_red, c_col, n_kb, relu, group;
 };
 
 // Largest magnitude and smallest but zero of some numbers, as bits without the sign, shifted up by one: .x and .z are the largest
@@ -229,6 +235,13 @@ struct F3Rows {
 __device__ __forceinline__ float f3_finish(float v, float scale, float shift, int relu) {
   v = fmaf(v, scale, shift);
   return relu ? relu_f32(v) : v;
+}
+
+// a + b, rounded away from zero. Truncation costs a stage 4 to 5e-8 of its sum on average, so the whole sum as much; the last two
+// sums of groups, rounded like this, give most of it back. Sums that are exact stay so.
+__device__ __forceinline__ float sum_outward(float a, float b) {
+  const float up = __fadd_ru(a, b), down = __fadd_rd(a, b);
+  return up >= 0.f ? up : down;
 }
 
 // Rows row0 .. row0 + 3 (columns col0 .. col0 + CC - 1) by fp32 multiply-adds, by a whole warp: a lane per column of every 32
@@ -537,7 +550,7 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
       merge_ranges(range, &s_range);
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
-    const uint32_t least = least_sum(s_range);
+    float4* total = reinterpret_cast<float4*>(smem + C::TOTAL_OFFSET) + tid - kF3DrainWarp0 * 32;  // vector q: total[256 q]
     uint32_t cnt[2] = {0, 0}, mark = (T > 1 ? set * 4 : 0) + quad;  // of this warp's block of 32 rows
     for (uint32_t st = blockIdx.x; st < a.n_super && !timed_out; st += gridDim.x, mark += 4 * T) {
       float sum[HALVES][CC / 8][4];
@@ -547,34 +560,59 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
         for (int v = 0; v < CC / 8; ++v)
 #pragma unroll
           for (int e = 0; e < 4; ++e) sum[h][v][e] = 0.f;
+      int d = 0;
+      for (bool grouped = false;; grouped = true) {
+        const int end = min(longest, d + a.group);
 #pragma unroll 1
-      for (int d = 0; d < longest && !timed_out; ++d) {
+        for (; d < end && !timed_out; ++d) {
 #pragma unroll
-        for (int x = 0; x < (T > 1 ? 1 : 2); ++x) {
-          const int stream = T > 1 ? set : x;
-          if (d >= stages_of(stream)) continue;
-          const uint32_t acc = stream * 2 + (cnt[x] & 1u), ph = (cnt[x] >> 1) & 1u;
-          ++cnt[x];
-          if (!mbar_wait(&acc_full[acc], ph)) timed_out = true;
-          timed_out = __any_sync(0xFFFFFFFFu, timed_out);
-          if (timed_out) break;
-          tc_fence_after();
+          for (int x = 0; x < (T > 1 ? 1 : 2); ++x) {
+            const int stream = T > 1 ? set : x;
+            if (d >= stages_of(stream)) continue;
+            const uint32_t acc = stream * 2 + (cnt[x] & 1u), ph = (cnt[x] >> 1) & 1u;
+            ++cnt[x];
+            if (!mbar_wait(&acc_full[acc], ph)) timed_out = true;
+            timed_out = __any_sync(0xFFFFFFFFu, timed_out);
+            if (timed_out) break;
+            tc_fence_after();
 #pragma unroll
-          for (int h = 0; h < HALVES; ++h) {
-            const uint32_t taddr = tmem_base + ((quad * 32u + (T > 1 ? h : set) * 16u) << 16) + acc * CC;
-            uint32_t r[CC / 32][16];
+            for (int h = 0; h < HALVES; ++h) {
+              const uint32_t taddr = tmem_base + ((quad * 32u + (T > 1 ? h : set) * 16u) << 16) + acc * CC;
+              uint32_t r[CC / 32][16];
 #pragma unroll
-            for (int q = 0; q < CC / 32; ++q) tc_ld16x256b(taddr + q * 32, r[q]);
-            tc_wait_ld();
+              for (int q = 0; q < CC / 32; ++q) tc_ld16x256b(taddr + q * 32, r[q]);
+              tc_wait_ld();
 #pragma unroll
-            for (int v = 0; v < CC / 2; ++v) sum[h][v / 4][v % 4] += __uint_as_float(r[v / 16][v % 16]);
+              for (int v = 0; v < CC / 2; ++v) sum[h][v / 4][v % 4] += __uint_as_float(r[v / 16][v % 16]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc]);
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_empty[acc]);
+        }
+        auto add_total = [&](auto add) {
+#pragma unroll
+          for (int q = 0; q < C::TOTAL_VECS; ++q) {
+            float(&f)[4] = sum[q / (CC / 8)][q % (CC / 8)];
+            const float4 before = total[256 * q];
+            f[0] = add(before.x, f[0]);
+            f[1] = add(before.y, f[1]);
+            f[2] = add(before.z, f[2]);
+            f[3] = add(before.w, f[3]);
+          }
+        };
+        if (grouped && d + a.group >= longest) add_total([](float x, float y) { return sum_outward(x, y); });  // the last two
+        else if (grouped) add_total([](float x, float y) { return x + y; });
+        if (timed_out || d == longest) break;
+#pragma unroll
+        for (int q = 0; q < C::TOTAL_VECS; ++q) {
+          float(&f)[4] = sum[q / (CC / 8)][q % (CC / 8)];
+          total[256 * q] = make_float4(f[0], f[1], f[2], f[3]);
+          f[0] = f[1] = f[2] = f[3] = 0.f;
         }
       }
       if (timed_out) break;
+      const uint32_t least = least_sum(s_range);
 #pragma unroll
       for (int h = 0; h < HALVES; ++h) {
 #pragma unroll
@@ -635,6 +673,10 @@ int launch_f3(F3Args a, uint32_t blocks, uint32_t fit, cudaStream_t stream) {
   static SmemOptIn opt_in;
   RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_conv_f3<CC, T>), C::SMEM));
   a.n_super = (a.n_dst + kTileM * T - 1) / (kTileM * T);
+  // Stages of a group: n stages in g groups leave a rounding error that goes with sqrt(g + n / g^2), least at g = cbrt(2 n) and
+  // hardly larger at cbrt(n).
+  const int stages = a.K * a.n_kb, groups = (int)(std::cbrt((double)stages) + 1e-6), steps = T > 1 ? stages : (stages + 1) / 2;
+  a.group = (steps + groups - 1) / groups;
   RMN_CUDA_TRY(launch_overlapped(k_conv_f3<CC, T>, dim3(fit < a.n_super ? fit : a.n_super, blocks), dim3(kF3Threads), C::SMEM,
                                  stream, a));
   RMN_LAUNCH_CHECK();

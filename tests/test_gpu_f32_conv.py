@@ -138,6 +138,41 @@ def test_transpose_weights_reverses_the_offsets():
             assert torch.equal(out, (want.flip(0) if reverse else want).contiguous())
 
 
+@pytest.mark.parametrize("n,c_in,c_out,K,fill", [(30_000, 32, 32, 27, 0.66), (9000, 64, 64, 27, 0.5), (20_000, 32, 64, 27, 0.05),
+                                                 (11_000, 32, 64, 8, 0.55), (5000, 256, 64, 27, 0.5), (30_000, 64, 64, 1, 1.0)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "near one", "integers"])
+def test_f32_on_tensor_cores_is_as_close_to_float64_as_multiply_adds(n, c_in, c_out, K, fill, kind):
+    """Sums of either sign and of one sign (where an error that does not average out would show), and exact ones."""
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    g = torch.Generator(device="cuda").manual_seed(n + c_in)
+    nbr = torch.randint(0, n, (K, n), generator=g, dtype=torch.int32, device="cuda")
+    nbr[torch.rand((K, n), generator=g, device="cuda") >= fill] = -1
+    x = torch.randn((n, c_in), generator=g, device="cuda")
+    w = torch.randn((K, c_in, c_out), generator=g, device="cuda")
+    if kind == "positive":
+        x, w = x.abs(), w.abs()
+    elif kind == "near one":
+        x, w = 1 + 0.1 * x.abs(), 1 + 0.1 * w.abs()
+    elif kind == "integers":
+        x, w = (4 * x).round(), (4 * w).round()
+    want = torch.zeros((n, c_out), dtype=torch.float64, device="cuda")
+    for k in range(K):
+        hit = nbr[k] >= 0
+        want[hit] += x[nbr[k][hit].long()].double() @ w[k].double()
+    size = lib.rmn_conv_f32_scratch_bytes(n, K, c_in, c_out)
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    out, plain = torch.empty((n, c_out), device="cuda"), torch.empty((n, c_out), device="cuda")
+    capi.check(lib.rmn_conv_forward_f32(ops._ptr(x), n, c_in, ops._ptr(w), K, c_out, 0, 0, ops._ptr(nbr), n, ops._ptr(out), None,
+                                        None, 0, ops._ptr(scratch), size, ops._stream()), "rmn_conv_forward_f32")
+    capi.check(lib.rmn_conv_forward(ops._ptr(x), n, c_in, ops._ptr(w), K, c_out, ops._ptr(nbr), n, ops._ptr(plain), capi.F32,
+                                    ops._stream()), "rmn_conv_forward")
+    if kind == "integers":
+        assert torch.equal(out.double(), want)
+    else:
+        assert float((out.double() - want).norm()) <= float((plain.double() - want).norm())
+
+
 @pytest.mark.parametrize("x_exponent,w_exponent,both", [
     (-118, 40, False), (-124, 60, False), (40, -118, False), (60, -124, False),   # one side's last parts below bf16's numbers
     (-140, 60, False), (60, -140, False),                                        # no parts at all: sums of zero
