@@ -117,3 +117,71 @@ def test_folded_batch_norm_and_residual_match_float64(n, w_in, w_out, c_in, c_ou
         want = torch.relu(want)
     # fp32 sums rounded to bf16 once: 2^-9 of a value, and the sum's own error
     assert bool(((out[:, :w_out].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4 * want.abs().max()).all())
+
+
+class _Job(ctypes.Structure):   # rmn_weight_job of include/rmn_b200.h
+    _fields_ = [("weights", ctypes.c_void_p), ("image", ctypes.c_void_p)] + [
+        (n, ctypes.c_int) for n in ("K", "w_in", "w_out", "c_in", "c_out")] + [("fold", _Fold)]
+
+
+@pytest.mark.parametrize("n_jobs", [1, 24, 25, 61])   # (24 to a launch)
+def test_weights_of_layers_prepared_together_are_those_prepared_alone(n_jobs):
+    """Layers of mixed shapes, padded ones, batch norms of both parameter types with their own statistics, absent parameters and
+    none at all: the same images, scales and shifts, bit for bit, and nothing beyond them."""
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    g = torch.Generator(device="cuda").manual_seed(n_jobs)
+    shapes = [(27, 4, 32, 32, 32), (8, 64, 128, 64, 128), (27, 32, 64, 32, 64), (1, 32, 20, 32, 32), (27, 256, 256, 256, 256),
+              (9, 100, 250, 128, 256), (81, 64, 33, 64, 64)]
+    together, alone, keep = [], [], []
+    for j in range(n_jobs):
+        K, w_in, w_out, c_in, c_out = shapes[j % len(shapes)]
+        dtype = torch.float32 if j % 2 else torch.bfloat16
+        w = torch.randn((K, w_in, w_out), generator=g, device="cuda").bfloat16()
+        params = [(torch.rand(w_out, generator=g, device="cuda") + 0.5 * i).to(dtype) for i in range(5)]
+        given = [p.data_ptr() if i < 2 or (j >> i) & 1 == 0 else None for i, p in enumerate(params)]
+        size = lib.rmn_conv_weight_image_bytes(K, c_in, c_out, capi.BF16)
+        for jobs in (together, alone):
+            image = torch.full((size + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+            vectors = torch.full((2 * c_out + 8,), 7.0, device="cuda")
+            fold = _Fold(*given, capi.F32 if j % 2 else capi.BF16, 1e-3, vectors.data_ptr(), vectors[c_out:].data_ptr())
+            if j % 5 == 3:
+                fold = _Fold()
+            jobs.append((_Job(w.data_ptr(), image.data_ptr(), K, w_in, w_out, c_in, c_out, fold), image, vectors))
+        keep.append((w, params))
+    capi.check(lib.rmn_conv_weight_images((_Job * n_jobs)(*[job for job, _, _ in together]), n_jobs, ops._stream()), "images")
+    for job, image, _ in alone:
+        fold = ctypes.byref(job.fold) if job.fold.scale else None
+        capi.check(lib.rmn_conv_weight_image(job.weights, job.K, job.w_in, job.w_out, job.c_in, job.c_out, capi.BF16, 0, 0, fold,
+                                             job.image, ops._stream()), "rmn_conv_weight_image")
+    for (_, image, vectors), (_, want_image, want_vectors) in zip(together, alone):
+        assert torch.equal(image, want_image) and torch.equal(vectors, want_vectors)
+
+
+# single tiles whose even and odd stages are summed apart, single tiles of more columns, super-tiles; rows around a tile's edge
+@pytest.mark.parametrize("n,c_in,c_out,K", [(1, 64, 64, 27), (129, 32, 32, 27), (5003, 64, 64, 1), (9000, 128, 256, 27),
+                                            (20_003, 32, 32, 81), (60_001, 64, 128, 27), (100_003, 256, 256, 8)])
+@pytest.mark.parametrize("with_add,with_scale,relu", [(True, True, 1), (True, False, 0), (False, True, 1), (False, False, 0)])
+def test_an_ordered_map_stores_and_adds_every_row_where_it_belongs(n, c_in, c_out, K, with_add, with_scale, relu):
+    """rmn_conv_forward_ordered over a permuted table: bit for bit the rows of rmn_conv_forward_image over the public one."""
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    g = torch.Generator(device="cuda").manual_seed(n + K)
+    nbr = torch.randint(-n, n, (K, n), generator=g, dtype=torch.int32, device="cuda").clamp_(min=-1)
+    order = torch.randperm(n, generator=g, device="cuda").int()
+    ordered = nbr[:, order.long()].contiguous()
+    feats = torch.randn((n, c_in), generator=g, device="cuda").bfloat16()
+    w = (torch.randn((K, c_in, c_out), generator=g, device="cuda") / c_in ** 0.5).bfloat16()
+    add = torch.randn((n, c_out), generator=g, device="cuda").bfloat16() if with_add else None
+    scale, shift = (torch.randn(c_out, generator=g, device="cuda") if with_scale else None for _ in range(2))
+    image = torch.empty(lib.rmn_conv_weight_image_bytes(K, c_in, c_out, capi.BF16), dtype=torch.uint8, device="cuda")
+    capi.check(lib.rmn_conv_weight_image(ops._ptr(w), K, c_in, c_out, c_in, c_out, capi.BF16, 0, 0, None, ops._ptr(image),
+                                         ops._stream()), "rmn_conv_weight_image")
+    got, want = (torch.full((n, c_out), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    capi.check(lib.rmn_conv_forward_ordered(ops._ptr(feats), n, c_in, ops._ptr(image), K, c_out, ops._ptr(ordered), ops._ptr(order),
+                                            n, ops._ptr(got), ops._ptr(scale), ops._ptr(shift), ops._ptr(add), relu,
+                                            ops._stream()), "rmn_conv_forward_ordered")
+    capi.check(lib.rmn_conv_forward_image(ops._ptr(feats), n, c_in, ops._ptr(image), K, c_out, ops._ptr(nbr), None, n,
+                                          ops._ptr(want), ops._ptr(scale), ops._ptr(shift), ops._ptr(add), relu, ops._stream()),
+               "rmn_conv_forward_image")
+    assert torch.equal(got, want)

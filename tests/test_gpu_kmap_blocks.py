@@ -156,3 +156,24 @@ def test_offset_pointers_and_pair_lists_of_small_maps(n, self_map, kernel):
         want = (m.nbr[k] >= 0).nonzero().flatten()
         order = q[lo:hi].argsort()
         assert torch.equal(q[lo:hi][order].long(), want) and torch.equal(a[lo:hi][order], m.nbr[k][want])
+
+
+def test_fused_layers_over_an_ordered_map_give_the_rows_of_the_public_one():
+    """Convolution, batch norm and ReLU as one kernel, over the map that a layer without gradients takes and over the public one,
+    which a request for pair lists leaves in the manager: the same bits."""
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    n = 1_980_000
+    c = _cloud(3, n, 110, 1, "random", 9)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    for c_in, c_out in ((32, 64), (64, 20)):
+        layer = C.RiemannConvolution(c_in, c_out, kernel_size=3, stride=1, bias=True, dimension=3)
+        layer.to("cuda:0")
+        layer.to(torch.bfloat16)
+        feats = torch.randn((n, c_in), generator=g, device="cuda").bfloat16()
+        stats = [torch.rand(c_out, generator=g, device="cuda") + 0.5 for _ in range(4)]
+        ordered, public = C.SparseTensor(feats, c), C.SparseTensor(feats, c)
+        key = public.coordinate_map_key
+        public.coordinate_manager.kernel_map_pairs(key, key, [3] * 3, [1] * 3, [1] * 3)
+        got, want = (C.fused_conv_bn_relu(x, layer, *stats, 1e-5, True).F for x in (ordered, public))
+        assert torch.equal(got, want) and float(got.max()) > 0

@@ -258,3 +258,35 @@ def test_parameters_with_tangents_are_not_dropped():
                 give_tangent(next(p for name, p in net.named_parameters().items() if part in name))
                 with pytest.raises(RuntimeError, match="jvp"):
                     net(C.SparseTensor(feats, small))
+
+
+@pytest.mark.parametrize("norms", ["bf16", "f32"])
+def test_serving_network_with_norms_of_their_own_matches_its_layers(norms):
+    """Weights and batch norms of all layers prepared by one kernel against the layers one after the other (gradients enabled:
+    nothing is prepared), every norm with statistics and parameters of its own: exchanged ones would be far off."""
+    import torch
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    xyz = torch.unique(torch.randint(0, 40, (6000, 3), generator=g, device="cuda"), dim=0)
+    coords = torch.cat([torch.zeros((xyz.size(0), 1), dtype=xyz.dtype, device="cuda"), xyz], 1).int().contiguous()
+    torch.manual_seed(3)
+    net = C.MinkUNet(4, 20, width=32, dimension=3)
+    net.to("cuda:0")
+    net.to(torch.bfloat16 if norms == "bf16" else torch.float32)
+    feats = torch.randn((coords.size(0), 4), generator=g, device="cuda")
+    feats = feats.bfloat16() if norms == "bf16" else feats
+    with torch.no_grad():
+        for name, p in net.named_parameters().items():
+            if "norm" in name:
+                p.copy_(torch.rand(p.shape, generator=g, device="cuda") + (0.5 if "weight" in name else -0.5))
+        for _ in range(4):   # running statistics that are not the identity
+            net(C.SparseTensor(feats, coords))
+    net.train(False)
+    with torch.no_grad():
+        together = net(C.SparseTensor(feats, coords)).F
+    alone = net(C.SparseTensor(feats, coords)).F.detach()
+    size = float(alone.float().pow(2).mean().sqrt())
+    # bf16: thirty layers that round (2^-9) once instead of three times. fp32: the layers run alone on both sides
+    bound = 30 * 2.0 ** -9 if norms == "bf16" else 1e-5
+    assert float((together.float() - alone.float()).pow(2).mean().sqrt()) <= bound * size
