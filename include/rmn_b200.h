@@ -329,6 +329,13 @@ int rmn_kmap_build_host(const void *d_table, const int32_t *d_query, uint32_t n_
 size_t rmn_kmap_ordered_workspace_bytes(uint32_t n_rows, int W, int K);
 int rmn_kmap_build_ordered(const void *d_table, const int32_t *d_coords, uint32_t n_rows, int W, const int32_t *d_offsets,
                            int K, int32_t *d_order, int32_t *d_nbr, void *d_workspace, size_t workspace_bytes, void *stream);
+/*
+ * The map of rmn_kmap_build_self from one of rmn_kmap_build_ordered (same n_rows and K), without another look at the
+ * coordinates; d_workspace (16-byte aligned) of rmn_kmap_workspace_bytes, for the pair lists as after a build. host_ptr (or NULL):
+ * page-locked memory that takes the offset pointers, too.
+ */
+int rmn_kmap_build_from_ordered(const int32_t *d_order, const int32_t *d_ordered_nbr, uint32_t n_rows, int K, int32_t *d_nbr,
+                                int64_t *d_offset_ptr, int64_t *host_ptr, void *d_workspace, size_t workspace_bytes, void *stream);
 
 /*
  * Materialise the pair lists of the last rmn_kmap_build (same d_nbr,

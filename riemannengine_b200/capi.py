@@ -66,6 +66,8 @@ SIGNATURES = {
     "rmn_kmap_ordered_workspace_bytes": (c_size_t, [c_uint32, c_int, c_int]),
     "rmn_kmap_build_ordered": (c_int, [c_void_p, c_void_p, c_uint32, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                        c_size_t, c_void_p]),
+    "rmn_kmap_build_from_ordered": (c_int, [c_void_p, c_void_p, c_uint32, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
+                                            c_void_p]),
     "rmn_conv_forward_ordered": (c_int, [c_void_p, c_uint32, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_uint32,
                                          c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "rmn_conv_f32_scratch_bytes": (c_size_t, [c_uint32, c_int, c_int, c_int]),

@@ -471,6 +471,41 @@ inline cudaError_t clear_entries(int32_t* nbr, size_t n, uint32_t* ticket, cudaS
   return launch_overlapped(k_kmap_clear, dim3((uint32_t)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, nbr, n, ticket);
 }
 
+// The public map from an ordered one: the position of every row, then per offset the entries of its rows, which lie anywhere in
+// the 4 n bytes of that offset. So the offsets come one after the other: what is read again of the 32 bytes around an entry is in
+// the L2 (19 MB an offset for 4.8 M rows), whose 32-byte pieces bound it: 4.8 M shuffled clip rows x 81 offsets 1750 us, 7.1 TB/s of
+// them. Counts are those of k_kmap_probe_self.
+__global__ void __launch_bounds__(256) k_kmap_positions(const int32_t* __restrict__ order, uint32_t n, int32_t* __restrict__ position,
+                                                        uint32_t* __restrict__ scan_ticket) {
+  after_previous_kernel();
+  const uint32_t p = blockIdx.x * 256 + threadIdx.x;
+  if (p == 0) *scan_ticket = 0;
+  if (p < n) position[__ldg(order + p)] = (int32_t)p;
+}
+constexpr int kUnorderBlocks = 4;  // blocks of kKmapBlock rows that a CUDA block takes
+__global__ void __launch_bounds__(kKmapBlock) k_kmap_unorder(const int32_t* __restrict__ ordered, const int32_t* __restrict__ position,
+                                                             uint32_t n, int half, int32_t* __restrict__ nbr,
+                                                             uint32_t* __restrict__ block_counts, uint32_t n_blocks) {
+  after_previous_kernel();
+  const int k = (int)blockIdx.y;
+  const size_t first = (size_t)k * n;
+  const uint32_t block0 = blockIdx.x * kUnorderBlocks;
+  int32_t v[kUnorderBlocks];
+#pragma unroll
+  for (int j = 0; j < kUnorderBlocks; ++j) {
+    const uint32_t row = (block0 + j) * kKmapBlock + threadIdx.x;
+    v[j] = row < n ? __ldg(ordered + first + (uint32_t)__ldg(position + row)) : -1;
+  }
+#pragma unroll
+  for (int j = 0; j < kUnorderBlocks; ++j) {
+    const uint32_t row = (block0 + j) * kKmapBlock + threadIdx.x;
+    if (row < n) __stcs(nbr + first + row, v[j]);
+    if (k > half) continue;
+    const int count = __syncthreads_count(v[j] >= 0);
+    if (threadIdx.x == 0 && block0 + j < n_blocks) block_counts[(size_t)k * n_blocks + block0 + j] = (uint32_t)count;
+  }
+}
+
 __global__ void __launch_bounds__(256) k_kmap_transpose(const int32_t* __restrict__ nbr,
                                                         uint32_t n_query, int K, uint32_t n_a,
                                                         int32_t* __restrict__ nbr_t) {
@@ -697,6 +732,33 @@ extern "C" int rmn_kmap_build_ordered(const void* d_table, const int32_t* d_coor
                                    counts + (size_t)K * nb + K + 2, ix.state, TailScan{}));
     RMN_LAUNCH_CHECK();
   });
+  return RMN_OK;
+}
+
+extern "C" int rmn_kmap_build_from_ordered(const int32_t* d_order, const int32_t* d_ordered_nbr, uint32_t n_rows, int K,
+                                           int32_t* d_nbr, int64_t* d_offset_ptr, int64_t* host_ptr, void* d_workspace,
+                                           size_t workspace_bytes, void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  if (rmn_kmap_ordered_workspace_bytes(n_rows, RMN_MAX_W, K) == 0) return RMN_ERR_UNSUPPORTED;
+  if (!d_order || !d_ordered_nbr || !d_nbr || !d_offset_ptr || !d_workspace || ((uintptr_t)d_workspace & 15)) return RMN_ERR_BAD_ARG;
+  if (workspace_bytes < rmn_kmap_workspace_bytes(n_rows, K)) return RMN_ERR_ALLOC;
+  int64_t* host_alias = nullptr;
+  if (host_ptr) RMN_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&host_alias), host_ptr, 0));
+  const uint32_t nb = kmap_blocks(n_rows);
+  const int half = K / 2;
+  uint32_t* block_counts = static_cast<uint32_t*>(d_workspace);
+  uint32_t* totals = block_counts + (size_t)K * nb;
+  // (where a build has its index)
+  int32_t* position = reinterpret_cast<int32_t*>(static_cast<char*>(d_workspace) + kmap_counts_bytes(n_rows, K));
+  RMN_CUDA_TRY(launch_overlapped(k_kmap_positions, dim3((n_rows + 255) / 256), dim3(256), 0, stream, d_order, n_rows, position,
+                                 totals + K + 2));
+  RMN_LAUNCH_CHECK();
+  RMN_CUDA_TRY(launch_overlapped(k_kmap_unorder, dim3((nb + kUnorderBlocks - 1) / kUnorderBlocks, K), dim3(kKmapBlock), 0, stream,
+                                 d_ordered_nbr, (const int32_t*)position, n_rows, half, d_nbr, block_counts, nb));
+  RMN_LAUNCH_CHECK();
+  RMN_CUDA_TRY(launch_overlapped(k_kmap_scan, dim3(half + 1), dim3(1024), 0, stream, block_counts, nb, K, half, totals, d_offset_ptr,
+                                 host_alias));
+  RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
 

@@ -200,7 +200,8 @@ public:
                                         const stride_type& kernel_dilation, RegionType::Type region_type,
                                         const at::Tensor& offsets, bool is_transpose, bool is_pool);
   // kernel_map for a convolution that only runs forward: a large self map may come in an internal order of its rows
-  // (rmn_kmap_build_ordered; `order` is defined then), unless the public map exists already. Cached apart from the public maps.
+  // (rmn_kmap_build_ordered; `order` is defined then), unless the public map exists already. Cached apart from the public maps, until
+  // the public one is asked for, which is made from it and takes its place.
   std::shared_ptr<KernelMap> layer_map(const CoordinateMapKey& in_key, const CoordinateMapKey& out_key,
                                        const stride_type& kernel_size, const stride_type& kernel_stride,
                                        const stride_type& kernel_dilation, RegionType::Type region_type,

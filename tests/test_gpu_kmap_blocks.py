@@ -177,3 +177,77 @@ def test_fused_layers_over_an_ordered_map_give_the_rows_of_the_public_one():
         public.coordinate_manager.kernel_map_pairs(key, key, [3] * 3, [1] * 3, [1] * 3)
         got, want = (C.fused_conv_bn_relu(x, layer, *stats, 1e-5, True).F for x in (ordered, public))
         assert torch.equal(got, want) and float(got.max()) > 0
+
+
+# rows around a block of 256 and around the four of them that a CUDA block takes; the index used and not used
+@pytest.mark.parametrize("D,n,extent,kernel,order", [(3, 1_970_000, 110, 3, "random"), (3, 1_970_177, 5000, 3, "random"),
+                                                     (3, 1_970_945, 100, 3, "sorted"), (4, 1_980_161, 36, 3, "random")])
+def test_public_map_made_from_an_ordered_one(D, n, extent, kernel, order):
+    """The same table, counts and pair lists as a build of its own, bit for bit."""
+    from riemannengine_b200 import capi, ops
+    c = _cloud(D, n, extent, 1, order, n)
+    table = ops.table_build(c)
+    off = ops.region_offsets(0, [kernel] * D, [1] * D, [1] * D)
+    K = off.shape[0]
+    want = ops.kmap_build(table, table.coords, off, self_map=True)
+    lib = capi.lib()
+    scratch = torch.empty(lib.rmn_kmap_ordered_workspace_bytes(n, D + 1, K), dtype=torch.uint8, device="cuda")
+    rows, ordered = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty((K, n), dtype=torch.int32, device="cuda")
+    offsets = torch.as_tensor(off, dtype=torch.int32, device="cuda").contiguous()
+    capi.check(lib.rmn_kmap_build_ordered(ops._ptr(table.buffer), ops._ptr(table.coords), n, D + 1, ops._ptr(offsets), K,
+                                          ops._ptr(rows), ops._ptr(ordered), ops._ptr(scratch), scratch.numel(), ops._stream()),
+               "rmn_kmap_build_ordered")
+    del scratch
+    size = lib.rmn_kmap_workspace_bytes(n, K)
+    workspace = torch.full((size + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    nbr = torch.full((K, n), -2, dtype=torch.int32, device="cuda")
+    offset_ptr = torch.full((K + 1,), -1, dtype=torch.int64, device="cuda")
+    on_host = torch.full((K + 1,), -1, dtype=torch.int64).pin_memory()
+    args = [ops._ptr(rows), ops._ptr(ordered), n, K, ops._ptr(nbr), ops._ptr(offset_ptr), on_host.data_ptr(), ops._ptr(workspace)]
+    assert lib.rmn_kmap_build_from_ordered(*args, size - 1, ops._stream()) != 0
+    capi.check(lib.rmn_kmap_build_from_ordered(*args, size, ops._stream()), "rmn_kmap_build_from_ordered")
+    torch.cuda.synchronize()
+    assert bool((workspace[size:] == 0xA5).all())
+    for k in range(K):
+        assert torch.equal(nbr[k], want.nbr[k])
+    assert torch.equal(offset_ptr, want.offset_ptr) and torch.equal(on_host, want.offset_ptr.cpu())
+    got = ops.NeighbourTable(nbr, offset_ptr, workspace[:size], n, K, n)
+    for a, b in zip(got.pairs(), want.pairs()):
+        assert torch.equal(torch.as_tensor(a), torch.as_tensor(b))
+
+
+def test_a_layer_without_gradients_leaves_no_second_build_behind():
+    """Pair lists and training passes behind a layer that only ran forward: results, gradients and lists of a manager in which it
+    did not, and no two maps held."""
+    from riemannengine_b200 import cpp
+    C = cpp.load()
+    n = 1_980_000
+    c = _cloud(3, n, 110, 1, "random", 11)
+    g = torch.Generator(device="cuda").manual_seed(11)
+    layer = C.RiemannConvolution(32, 32, kernel_size=3, stride=1, bias=True, dimension=3)
+    layer.to("cuda:0")
+    layer.to(torch.bfloat16)
+    feats, grad = (torch.randn((n, 32), generator=g, device="cuda").bfloat16() for _ in range(2))
+
+    def both_passes(forward_first):
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        f = feats.clone().requires_grad_(True)
+        x = C.SparseTensor(f, c)
+        with torch.no_grad():
+            first = layer(x if forward_first else C.SparseTensor(feats, c)).F
+        layer.zero_grad()
+        out = layer(x).F
+        out.backward(grad)
+        key = x.coordinate_map_key
+        pairs = x.coordinate_manager.kernel_map_pairs(key, key, [3] * 3, [1] * 3, [1] * 3)
+        with torch.no_grad():
+            after = layer(x).F
+        results = [first, out.detach(), f.grad, layer.kernel.grad.clone(), after] + [torch.as_tensor(p) for p in pairs]
+        return results, torch.cuda.memory_allocated() - before
+
+    both_passes(False)   # (what is allocated once)
+    (want, held), (got, held_after) = both_passes(False), both_passes(True)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    assert held_after <= held + 27 * n * 2   # (a second table would be 27 n x 4)
