@@ -159,6 +159,11 @@ namespace {
 // to two 128 x 128 layers' worth. Up to 74 row tiles of 128 the convolution runs single tiles, which take no plan.
 // (ALWAYS: the first wide pass builds the plan.)
 constexpr int64_t kWidePass = 128 * 128, kPlanMinRows = 74 * 128 + 1;
+// whether a pass of this many channels over a table of this size counts towards a plan
+bool counts_for_plan(int64_t weight, int64_t rows, int64_t offsets) {
+  return weight >= kWidePass && rows >= kPlanMinRows && g_plan_policy.load() != PlanPolicy::NEVER &&
+         rmn_conv_plan_bytes(static_cast<uint32_t>(rows), static_cast<int>(offsets)) > 0;
+}
 bool want_plan(int64_t weight_sum, int64_t rows) {
   const int policy = g_plan_policy.load();
   if (policy == PlanPolicy::NEVER || rows < kPlanMinRows) return false;
@@ -1504,7 +1509,10 @@ bool folds_batch_norm(const RiemannConvolutionBaseImpl& conv, const SparseTensor
   return (shape.first != x.size(1) || !x.is_contiguous() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 == 0);
 }
 
-// whether a layer that only runs forward may take an ordered map: its pass goes to the kernels of prepared weights
+// whether a layer that only runs forward may take an ordered map: its pass goes to the kernels of prepared weights, and is not one
+// of those that a plan serves better. us of whole passes over ordered / public maps, layers of 128 -> 128 channels: 2.16 M voxels of
+// lidar sweeps, one layer 1533 / 1535, two 2746 / 2165, four 5179 / 2716; 2.1 M voxels of rooms in spatial order, two layers
+// 3347 / 3154. Narrower layers: shuffled rooms 32 -> 32 665 / 706, 64 -> 64 876 / 894.
 bool takes_ordered_map(const RiemannConvolutionBaseImpl& conv, const SparseTensor& input) {
   auto const& kernel = conv.kernel_;
   auto const& x = input.F();
@@ -1513,6 +1521,7 @@ bool takes_ordered_map(const RiemannConvolutionBaseImpl& conv, const SparseTenso
       x.scalar_type() != at::kBFloat16 || kernel.scalar_type() != at::kBFloat16 || conv.is_transpose_)
     return false;
   const auto shape = run_shape(kernel);
+  if (counts_for_plan(shape.first * shape.second, x.size(0), kernel.size(0))) return false;  // (a self map: as many rows out as in)
   return rmn_conv_weight_image_bytes(static_cast<int>(kernel.size(0)), static_cast<int>(shape.first),
                                      static_cast<int>(shape.second), RMN_BF16) > 0 &&
          (shape.first != x.size(1) || (x.is_contiguous() && reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 == 0));

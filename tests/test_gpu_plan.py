@@ -244,3 +244,38 @@ def test_no_host_builds_a_plan_that_its_kernels_would_drop():
         finally:
             E.KernelMap.plan_policy = 0
         assert built[0] == built[1], (rows, channels)
+
+
+def test_wide_layers_over_large_maps_keep_their_plan():
+    """Layers without gradients take large maps in an internal order, which has no plan: not those wide enough for one."""
+    from riemannengine_b200 import capi, cpp
+    C = cpp.load()
+    n = 1_980_000
+    g = torch.Generator(device="cuda").manual_seed(13)
+    c = torch.unique(torch.randint(0, 130, (3_700_000, 3), generator=g, device="cuda"), dim=0)[:n]
+    c = torch.cat([torch.zeros_like(c[:, :1]), c], 1)
+    c = torch.cat([c, c + torch.tensor([1, 0, 0, 0], device="cuda")])[:n].int().contiguous()
+    layer = C.RiemannConvolution(128, 128, kernel_size=3, stride=1, bias=False, dimension=3)
+    layer.to("cuda:0")
+    layer.to(torch.bfloat16)
+    feats = torch.randn((n, 128), generator=g, device="cuda").bfloat16()
+    lib = capi.lib()
+    launches, results = {}, {}
+    try:
+        for policy in (2, 1):   # never, always
+            C.set_convolution_plan_policy(policy)
+            x = C.SparseTensor(feats, c)
+            counts = []
+            with torch.no_grad():
+                for _ in range(2):   # the second pass finds map and plan
+                    before = lib.rmn_launch_count()
+                    results[policy] = layer(x).F
+                    counts.append(lib.rmn_launch_count() - before)
+            key, third = x.coordinate_map_key, lib.rmn_launch_count()
+            x.coordinate_manager.kernel_map_pairs(key, key, [3] * 3, [1] * 3, [1] * 3)
+            launches[policy] = counts + [lib.rmn_launch_count() - third]
+    finally:
+        C.set_convolution_plan_policy(0)
+    assert torch.equal(results[1], results[2])
+    # the public map is there already: only the lists are written. Over an ordered one it has to be made first.
+    assert launches[1][2] < launches[2][2], launches
