@@ -428,7 +428,8 @@ int rmn_conv_transpose_weights(const void *d_weights, int K, int c_in, int c_out
  * sums in fp32. Results that are not finite, or too small to hold what parts of tiny operands lose, are computed with fp32
  * multiply-adds. Bytes of scratch (the
  * prepared weights) of rmn_conv_forward_f32, 0 where it does not serve (use rmn_conv_forward): c_in a multiple of 8 from 16
- * on, c_out a multiple of 4. rmn_conv_f32_pays: whether it is the faster way for a pass of this size.
+ * on, c_out a multiple of 4. rmn_conv_f32_pays: whether it is the faster way for a pass of this size. (Large passes over tables with
+ * less than a sixteenth of neighbours go to the multiply-add kernel, chosen on the device.)
  * rmn_conv_forward_f32: rmn_conv_forward_fused for fp32 (d_feats 32-byte aligned, d_out and d_scratch 16-byte aligned:
  * RMN_ERR_UNSUPPORTED otherwise; d_weights at any element). transpose: d_weights is [K, c_out, c_in], each offset's matrix used transposed;
  * reverse: offset k uses d_weights[K - 1 - k]. With both, the input gradient of a point-symmetric self map is this call on

@@ -103,8 +103,9 @@ template <int NV>
 __global__ void __launch_bounds__(256)
     k_conv_f32(const float* __restrict__ src, const float* __restrict__ w, const int32_t* __restrict__ nbr, uint32_t n_dst,
                int K, int c_red, int c_col, int splits, float* __restrict__ out, const float* __restrict__ ep_scale,
-               const float* __restrict__ ep_shift, int ep_relu) {
+               const float* __restrict__ ep_shift, int ep_relu, const uint32_t* __restrict__ only_if) {
   after_previous_kernel();
+  if (only_if && !__ldg(only_if)) return;
   using Cfg = F32FwCfg<NV>;
   constexpr int C = Cfg::C, BATCH = Cfg::BATCH, RGS = Cfg::RGS;
   extern __shared__ __align__(16) float smem_f[];
@@ -232,7 +233,8 @@ __global__ void __launch_bounds__(256)
 
 template <int NV>
 static int launch_conv_f32(const float* src, const float* w, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col,
-                           float* out, const float* ep_scale, const float* ep_shift, int ep_relu, cudaStream_t stream) {
+                           float* out, const float* ep_scale, const float* ep_shift, int ep_relu, const uint32_t* only_if,
+                           cudaStream_t stream) {
   using Cfg = F32FwCfg<NV>;
   static SmemOptIn opt_in;
   RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_conv_f32<NV>), 8 * Cfg::WARP_WORDS * 4));
@@ -247,7 +249,7 @@ static int launch_conv_f32(const float* src, const float* w, const int32_t* nbr,
   const uint32_t groups = warps / splits;
   dim3 grid((row_groups + groups - 1) / groups, tiles_n);
   RMN_CUDA_TRY(launch_overlapped(k_conv_f32<NV>, dim3(grid), dim3(warps * 32), (size_t)warps * Cfg::WARP_WORDS * 4, stream,
-                                 src, w, nbr, n_dst, K, c_red, c_col, splits, out, ep_scale, ep_shift, ep_relu));
+                                 src, w, nbr, n_dst, K, c_red, c_col, splits, out, ep_scale, ep_shift, ep_relu, only_if));
   RMN_LAUNCH_CHECK();
   return RMN_OK;
 }
@@ -450,12 +452,18 @@ bool f32_fast_shape(int c_in, int c_out) { return c_in % 4 == 0 && c_out % 4 == 
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// RMN_ERR_UNSUPPORTED where the shape or an alignment is not covered (the generic kernels take it then)
+// RMN_ERR_UNSUPPORTED where the shape or an alignment is not covered (the generic kernels take it then). only_if (or NULL): on the
+// device, nothing is done where it holds 0.
+int f32_conv_if(const float* src, const float* w, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, float* out,
+                const float* ep_scale, const float* ep_shift, int ep_relu, const uint32_t* only_if, cudaStream_t stream) {
+  if (!f32_fast_shape(c_red, c_col) || !aligned16(src) || !aligned16(w) || !aligned16(out)) return RMN_ERR_UNSUPPORTED;
+  return c_col <= 32
+             ? launch_conv_f32<1>(src, w, nbr, n_dst, K, c_red, c_col, out, ep_scale, ep_shift, ep_relu, only_if, stream)
+             : launch_conv_f32<2>(src, w, nbr, n_dst, K, c_red, c_col, out, ep_scale, ep_shift, ep_relu, only_if, stream);
+}
 int f32_conv(const float* src, const float* w, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col,
              float* out, const float* ep_scale, const float* ep_shift, int ep_relu, cudaStream_t stream) {
-  if (!f32_fast_shape(c_red, c_col) || !aligned16(src) || !aligned16(w) || !aligned16(out)) return RMN_ERR_UNSUPPORTED;
-  return c_col <= 32 ? launch_conv_f32<1>(src, w, nbr, n_dst, K, c_red, c_col, out, ep_scale, ep_shift, ep_relu, stream)
-                     : launch_conv_f32<2>(src, w, nbr, n_dst, K, c_red, c_col, out, ep_scale, ep_shift, ep_relu, stream);
+  return f32_conv_if(src, w, nbr, n_dst, K, c_red, c_col, out, ep_scale, ep_shift, ep_relu, nullptr, stream);
 }
 
 size_t f32_wgrad_workspace_bytes(uint32_t n_dst, int K, int c_in, int c_out) {

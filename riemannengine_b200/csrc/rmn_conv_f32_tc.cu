@@ -42,6 +42,8 @@ namespace rmn {
 
 const uint32_t* tc_status_device_address();  // rmn_conv_tc.cu
 void count_tc_launch();
+int f32_conv_if(const float* src, const float* w, const int32_t* nbr, uint32_t n_dst, int K, int c_red, int c_col, float* out,
+                const float* ep_scale, const float* ep_shift, int ep_relu, const uint32_t* only_if, cudaStream_t stream);
 
 namespace tc {
 
@@ -79,6 +81,7 @@ struct F3Args {
   const float* ep_scale;
   const float* ep_shift;
   const uint4* ranges;  // k_f3_image's
+  uint32_t* thin;       // k_f3_image's, or NULL: 1 where k_conv_f32 does this pass
   uint32_t* status;
   uint32_t n_dst, n_super, n_ranges;
   int K, c_red, c_col, n_kb, relu, group;
@@ -140,19 +143,37 @@ __device__ __forceinline__ constexpr uint32_t f3_n_channel(uint32_t p) {
 // Image of the weights: per stage (offset, 32-channel block) and block of CC columns the three parts, each the MN-major swizzled
 // operand of 32 lines. One thread per line and eight columns. reverse: offset k of the image is W[K - 1 - k]. plain (or NULL): the
 // weights as [K][c_red][c_col] in the image's order of offsets. The blocks from image_blocks on read the n_x numbers of x. ranges:
-// what each block has read.
+// what each block has read. thin (or NULL): a last block looks at kF3Samples of the n_entries entries of the table, spread evenly,
+// and says whether fewer than one in sixteen is a neighbour.
+constexpr uint32_t kF3Samples = 4096;
 template <int CC>
 __global__ void __launch_bounds__(256) k_f3_image(const float* __restrict__ w, int K, int c_red, int c_col, int n_kb, int blocks,
                                                   int transpose, int reverse, uint4* __restrict__ image,
                                                   float* __restrict__ plain, uint32_t image_blocks, const float4* __restrict__ x,
-                                                  size_t n_x, uint4* __restrict__ ranges) {
+                                                  size_t n_x, uint4* __restrict__ ranges, const int32_t* __restrict__ nbr,
+                                                  uint64_t n_entries, uint32_t* __restrict__ thin) {
   after_previous_kernel();
+  if (thin && blockIdx.x == gridDim.x - 1) {
+    uint32_t found = 0;
+#pragma unroll 16
+    for (uint32_t i = threadIdx.x; i < kF3Samples; i += 256)  // (multiples of the golden ratio)
+      found += __ldg(nbr + __umul64hi(i * 0x9E3779B97F4A7C15ull, n_entries)) >= 0 ? 1u : 0u;
+    __shared__ uint32_t s_found;
+    if (threadIdx.x == 0) s_found = 0u;
+    __syncthreads();
+    found = __reduce_add_sync(0xFFFFFFFFu, found);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_found, found);
+    __syncthreads();
+    if (threadIdx.x == 0) *thin = s_found < kF3Samples / 16 ? 1u : 0u;
+    return;
+  }
+  const uint32_t range_blocks = gridDim.x - image_blocks - (thin ? 1u : 0u);
   __shared__ uint4 s_range;
   if (threadIdx.x == 0) s_range = kNoRange;
   __syncthreads();
   uint4 range = kNoRange;
   if (blockIdx.x >= image_blocks) {
-    const size_t step = (size_t)(gridDim.x - image_blocks) * 256;
+    const size_t step = (size_t)range_blocks * 256;
 #pragma unroll 4
     for (size_t i = (size_t)(blockIdx.x - image_blocks) * 256 + threadIdx.x; i < n_x / 4; i += step) {
       const float4 v = __ldg(x + i);
@@ -355,6 +376,7 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
   }
   // (tensor memory is taken behind the kernels before this one and ahead of the next: see release_next_kernel)
   wait_previous_kernels();
+  if (a.thin && __ldg(a.thin)) return;
   if (warp == kF3MmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
                  : "memory");
@@ -696,9 +718,10 @@ int run_f3(F3Args a, uint32_t n_src, int transpose, int reverse, uint8_t* image,
   const size_t n_x = (size_t)n_src * a.c_red;
   const uint32_t image_blocks = (lines + 255) / 256 < kF3ImageBlocks ? (lines + 255) / 256 : kF3ImageBlocks;
   const uint32_t range_blocks = n_x / 8192 < kF3RangeBlocks ? (uint32_t)(n_x / 8192) + 1 : kF3RangeBlocks;
-  RMN_CUDA_TRY(launch_overlapped(k_f3_image<CC>, dim3(image_blocks + range_blocks), dim3(256), 0, stream, a.w, a.K, a.c_red, a.c_col,
-                                 a.n_kb, (int)blocks, transpose, reverse, reinterpret_cast<uint4*>(image), plain, image_blocks,
-                                 reinterpret_cast<const float4*>(a.src), n_x, ranges));
+  RMN_CUDA_TRY(launch_overlapped(k_f3_image<CC>, dim3(image_blocks + range_blocks + (a.thin ? 1u : 0u)), dim3(256), 0, stream, a.w,
+                                 a.K, a.c_red, a.c_col, a.n_kb, (int)blocks, transpose, reverse, reinterpret_cast<uint4*>(image),
+                                 plain, image_blocks, reinterpret_cast<const float4*>(a.src), n_x, ranges, a.nbr,
+                                 (uint64_t)a.K * a.n_dst, a.thin));
   RMN_LAUNCH_CHECK();
   a.ranges = ranges;
   a.n_ranges = image_blocks + range_blocks;
@@ -707,7 +730,9 @@ int run_f3(F3Args a, uint32_t n_src, int transpose, int reverse, uint8_t* image,
   // row tiles of the busiest SM: pairs of them share their weights, single ones leave fewer SMs idle at the end
   const uint32_t tiles = (a.n_dst + kTileM - 1) / kTileM, pairs = (tiles + 1) / 2;
   const uint32_t rounds2 = (pairs + fit - 1) / fit * 2, rounds1 = (tiles + fit - 1) / fit;
-  return rounds2 <= rounds1 ? launch_f3<CC, 2>(a, blocks, fit, stream) : launch_f3<CC, 1>(a, blocks, fit, stream);
+  const int st = rounds2 <= rounds1 ? launch_f3<CC, 2>(a, blocks, fit, stream) : launch_f3<CC, 1>(a, blocks, fit, stream);
+  if (st != RMN_OK || !a.thin) return st;
+  return f32_conv_if(a.src, a.w, a.nbr, a.n_dst, a.K, a.c_red, a.c_col, a.out, a.ep_scale, a.ep_shift, a.relu, a.thin, stream);
 }
 
 }  // namespace tc
@@ -723,7 +748,8 @@ static size_t f3_image_bytes(int K, int c_in, int c_out) {
 static size_t f3_plain_bytes(int K, int c_in, int c_out) { return (size_t)K * c_in * c_out * sizeof(float); }  // (a multiple of 128)
 extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, int c_out) {
   if (n_dst == 0 || K < 1 || K > 4096 || c_in < 16 || c_in > 1024 || c_in % 8 || c_out < 4 || c_out > 1024 || c_out % 4) return 0;
-  return f3_image_bytes(K, c_in, c_out) + f3_plain_bytes(K, c_in, c_out) + (tc::kF3ImageBlocks + tc::kF3RangeBlocks) * sizeof(uint4);
+  return f3_image_bytes(K, c_in, c_out) + f3_plain_bytes(K, c_in, c_out) +
+         (tc::kF3ImageBlocks + tc::kF3RangeBlocks + 1) * sizeof(uint4);  // (and k_f3_image's word on the table)
 }
 
 // Little work is the multiply-add kernel's: these kernels need the weights prepared by a launch of their own, which a host that
@@ -733,6 +759,17 @@ extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, in
 // 91 / 72 and 175 / 172; 663 (8000 rows 64 -> 48) 94 / 75 and 181 / 169; 90 (strided, 11 000 rows, 8 offsets) 94 / 99.
 extern "C" int rmn_conv_f32_pays(uint32_t n_dst, int K, int c_in, int c_out) {
   return rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out) > 0 && (double)n_dst * K * c_in * c_out >= 500e6;
+}
+
+// Thin tables are the multiply-add kernel's, which goes with the entries that are neighbours. Whether a table is thin is known on
+// the device alone; both kernels are launched then, and one does nothing, for 5 us. So it is asked where that is little: us of
+// the two kernels here / there, lidar sweeps of 119 755 voxels, 64 -> 64, 27 offsets (4 % neighbours) 139 / 121, 125 offsets (1.2 %)
+// 548 / 270, 343 offsets (0.6 %) 1426 / 578, 32 -> 32 69 / 64, 231 / 172, 611 / 419; a shell at 66 % 142 / 531 and 73 / 176. The
+// lines between lie at 5.0 % (32 -> 64) to 6.6 % (32 -> 32). A self map of 27 offsets has 3.7 % at least.
+// Asked, the passes over 125 and 343 offsets take 183 and 436 (32 -> 32), 280 and 595 (64 -> 64); a shell's over 125 258 -> 263 and
+// 519 -> 527.
+static bool f3_asks_for_thin_tables(uint32_t n_dst, int K, int c_in, int c_out) {
+  return (double)n_dst * K * c_in * c_out >= (K > 27 ? 8e9 : 40e9);
 }
 
 extern "C" int rmn_conv_forward_f32(const float* d_feats, uint32_t n_src, int c_in, const float* d_weights, int K, int c_out,
@@ -764,10 +801,12 @@ extern "C" int rmn_conv_forward_f32(const float* d_feats, uint32_t n_src, int c_
   a.relu = relu;
   if (!a.status) return RMN_ERR_CUDA;
   uint8_t* image = static_cast<uint8_t*>(d_scratch);
-  // (for exact_rows, whose lanes read neighbouring columns)
+  const bool ask = f3_asks_for_thin_tables(n_dst, K, c_in, c_out);
+  // (for exact_rows, whose lanes read neighbouring columns, and k_conv_f32, which reads four elements at a time)
   uint8_t* behind = image + f3_image_bytes(K, c_in, c_out);
-  float* plain = transpose || reverse ? reinterpret_cast<float*>(behind) : nullptr;
+  float* plain = transpose || reverse || (ask && ((uintptr_t)d_weights & 15)) ? reinterpret_cast<float*>(behind) : nullptr;
   uint4* ranges = reinterpret_cast<uint4*>(behind + f3_plain_bytes(K, c_in, c_out));
+  if (ask) a.thin = reinterpret_cast<uint32_t*>(ranges + tc::kF3ImageBlocks + tc::kF3RangeBlocks);
   return c_out <= 32 ? tc::run_f3<32>(a, n_src, transpose, reverse, image, plain, ranges, (cudaStream_t)stream_)
                      : tc::run_f3<64>(a, n_src, transpose, reverse, image, plain, ranges, (cudaStream_t)stream_);
 }

@@ -278,3 +278,38 @@ def test_rows_that_are_computed_again(c_in, c_out, transpose, reverse):
     assert torch.equal(fast().nan_to_num(7.0), plain().nan_to_num(7.0))
     assert time(fast) <= 8 * normal
     capi.check(lib.rmn_device_status(ops._stream()), "rmn_device_status")
+
+
+# the lines of the rule (15 625 rows x 125 offsets, 361 690 rows x 27 offsets of 64 -> 64 channels) from both sides, fills around
+# one in sixteen, an empty and a full table
+@pytest.mark.parametrize("n,c_in,c_out,K,fill,thin", [(15_700, 64, 64, 125, 0.01, True), (15_700, 64, 64, 125, 0.055, True),
+                                                      (15_700, 64, 64, 125, 0.07, False), (15_700, 64, 64, 125, 1.0, False),
+                                                      (15_700, 64, 64, 125, 0.0, True), (15_500, 64, 64, 125, 0.01, False),
+                                                      (62_600, 32, 32, 125, 0.02, True), (21_300, 40, 76, 124, 0.02, True),
+                                                      (362_000, 64, 64, 27, 0.04, True), (361_000, 64, 64, 27, 0.04, False)])
+@pytest.mark.parametrize("transpose,reverse,first", [(0, 0, 0), (1, 0, 0), (0, 1, 1), (1, 1, 3)])
+def test_large_passes_over_thin_tables_are_the_multiply_add_kernels(n, c_in, c_out, K, fill, thin, transpose, reverse, first):
+    """Which kernel did it shows in the last bits: those of rmn_conv_forward_fused where the table is thin."""
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    g = torch.Generator(device="cuda").manual_seed(n + K + int(100 * fill))
+    nbr = torch.randint(0, n, (K, n), generator=g, dtype=torch.int32, device="cuda")
+    nbr[torch.rand((K, n), generator=g, device="cuda") >= fill] = -1
+    x = torch.randn((n, c_in), generator=g, device="cuda")
+    w = torch.randn((K, c_in, c_out), generator=g, device="cuda")
+    given = w.flip(0) if reverse else w
+    given = (given.transpose(1, 2) if transpose else given).contiguous()
+    given = torch.zeros(given.numel() + 4, device="cuda")[first:first + given.numel()].view(given.shape).copy_(given)
+    scale, shift = torch.randn((2, c_out), generator=g, device="cuda")
+    size = lib.rmn_conv_f32_scratch_bytes(n, K, c_in, c_out)
+    scratch = torch.full((size + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    out, plain = (torch.full((n, c_out), 7.0, device="cuda") for _ in range(2))
+    capi.check(lib.rmn_conv_forward_f32(ops._ptr(x), n, c_in, ops._ptr(given), K, c_out, transpose, reverse, ops._ptr(nbr), n,
+                                        ops._ptr(out), ops._ptr(scale), ops._ptr(shift), 1, ops._ptr(scratch), size,
+                                        ops._stream()), "rmn_conv_forward_f32")
+    capi.check(lib.rmn_conv_forward_fused(ops._ptr(x), n, c_in, ops._ptr(w), K, c_out, ops._ptr(nbr), n, ops._ptr(plain), capi.F32,
+                                          ops._ptr(scale), ops._ptr(shift), 1, ops._stream()), "rmn_conv_forward_fused")
+    assert torch.equal(out, plain) == (thin or fill == 0.0)
+    # two sums of up to K c_in products, each within 2^-24 of the magnitudes a term (the grouped sum far less)
+    assert float((out - plain).abs().max()) <= 2.0 ** -18 * max(1.0, float(plain.abs().max()))
+    assert bool((scratch[size:] == 0xA5).all())
