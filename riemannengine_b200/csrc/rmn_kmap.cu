@@ -471,30 +471,48 @@ inline cudaError_t clear_entries(int32_t* nbr, size_t n, uint32_t* ticket, cudaS
   return launch_overlapped(k_kmap_clear, dim3((uint32_t)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, nbr, n, ticket);
 }
 
-// The public map from an ordered one: the position of every row, then per offset the entries of its rows, which lie anywhere in
-// the 4 n bytes of that offset. So the offsets come one after the other: what is read again of the 32 bytes around an entry is in
-// the L2 (19 MB an offset for 4.8 M rows), whose 32-byte pieces bound it: 4.8 M shuffled clip rows x 81 offsets 1750 us, 7.1 TB/s of
-// them. Counts are those of k_kmap_probe_self.
-__global__ void __launch_bounds__(256) k_kmap_positions(const int32_t* __restrict__ order, uint32_t n, int32_t* __restrict__ position,
-                                                        uint32_t* __restrict__ scan_ticket) {
+// The public map from an ordered one. k_kmap_positions: the position of every row, and which of its entries exist, a bit each, in
+// the row's words of `masks` [words][n]. k_kmap_unorder, offset by offset: entries of neighbouring rows lie anywhere in the 4 n bytes
+// of that offset, of which what is read again is in the L2 (19 MB for 4.8 M rows), whose 32-byte pieces bound it; so only the
+// entries that exist are read. The masks lie in the last offsets' places in the public table, which a launch without them fills
+// at the end. Counts are those of k_kmap_probe_self. us, before the masks
+// and with them: 4.8 M shuffled clip rows x 81 offsets at 32 % 1750 and 1363, 2.1 M voxels of rooms x 27 at 46 % 271 and 214, 2.2 M
+// of lidar sweeps x 27 in their own order 117 and 153.
+__global__ void __launch_bounds__(256) k_kmap_positions(const int32_t* __restrict__ order, const int32_t* __restrict__ ordered,
+                                                        uint32_t n, int K, int32_t* __restrict__ position,
+                                                        uint32_t* __restrict__ masks, uint32_t* __restrict__ scan_ticket) {
   after_previous_kernel();
   const uint32_t p = blockIdx.x * 256 + threadIdx.x;
   if (p == 0) *scan_ticket = 0;
-  if (p < n) position[__ldg(order + p)] = (int32_t)p;
+  if (p >= n) return;
+  const uint32_t row = (uint32_t)__ldg(order + p);
+  position[row] = (int32_t)p;
+  for (int k0 = 0; k0 < K; k0 += 32, masks += n) {
+    uint32_t mask = 0;
+#pragma unroll 8
+    for (int k = k0; k < min(k0 + 32, K); ++k) mask |= (__ldcs(ordered + (size_t)k * n + p) >= 0 ? 1u : 0u) << (k - k0);
+    masks[row] = mask;
+  }
 }
 constexpr int kUnorderBlocks = 4;  // blocks of kKmapBlock rows that a CUDA block takes
 __global__ void __launch_bounds__(kKmapBlock) k_kmap_unorder(const int32_t* __restrict__ ordered, const int32_t* __restrict__ position,
-                                                             uint32_t n, int half, int32_t* __restrict__ nbr,
+                                                             const uint32_t* masks, uint32_t n, int k0, int half, int32_t* nbr,
                                                              uint32_t* __restrict__ block_counts, uint32_t n_blocks) {
   after_previous_kernel();
-  const int k = (int)blockIdx.y;
+  const int k = k0 + (int)blockIdx.y;
   const size_t first = (size_t)k * n;
   const uint32_t block0 = blockIdx.x * kUnorderBlocks;
+  uint32_t exists[kUnorderBlocks];
   int32_t v[kUnorderBlocks];
 #pragma unroll
   for (int j = 0; j < kUnorderBlocks; ++j) {
     const uint32_t row = (block0 + j) * kKmapBlock + threadIdx.x;
-    v[j] = row < n ? __ldg(ordered + first + (uint32_t)__ldg(position + row)) : -1;
+    exists[j] = row >= n ? 0u : masks ? (masks[(size_t)(k / 32) * n + row] >> (k & 31)) & 1u : 1u;
+  }
+#pragma unroll
+  for (int j = 0; j < kUnorderBlocks; ++j) {
+    const uint32_t row = (block0 + j) * kKmapBlock + threadIdx.x;
+    v[j] = exists[j] ? __ldg(ordered + first + (uint32_t)__ldg(position + row)) : -1;
   }
 #pragma unroll
   for (int j = 0; j < kUnorderBlocks; ++j) {
@@ -750,12 +768,18 @@ extern "C" int rmn_kmap_build_from_ordered(const int32_t* d_order, const int32_t
   uint32_t* totals = block_counts + (size_t)K * nb;
   // (where a build has its index)
   int32_t* position = reinterpret_cast<int32_t*>(static_cast<char*>(d_workspace) + kmap_counts_bytes(n_rows, K));
-  RMN_CUDA_TRY(launch_overlapped(k_kmap_positions, dim3((n_rows + 255) / 256), dim3(256), 0, stream, d_order, n_rows, position,
-                                 totals + K + 2));
+  const int words = (K + 31) / 32, masked = K - words;
+  uint32_t* masks = reinterpret_cast<uint32_t*>(d_nbr + (size_t)masked * n_rows);
+  RMN_CUDA_TRY(launch_overlapped(k_kmap_positions, dim3((n_rows + 255) / 256), dim3(256), 0, stream, d_order, d_ordered_nbr, n_rows, K,
+                                 position, masks, totals + K + 2));
   RMN_LAUNCH_CHECK();
-  RMN_CUDA_TRY(launch_overlapped(k_kmap_unorder, dim3((nb + kUnorderBlocks - 1) / kUnorderBlocks, K), dim3(kKmapBlock), 0, stream,
-                                 d_ordered_nbr, (const int32_t*)position, n_rows, half, d_nbr, block_counts, nb));
-  RMN_LAUNCH_CHECK();
+  const uint32_t row_blocks = (nb + kUnorderBlocks - 1) / kUnorderBlocks;
+  for (const uint32_t* m = masks;; m = nullptr) {
+    RMN_CUDA_TRY(launch_overlapped(k_kmap_unorder, dim3(row_blocks, m ? masked : words), dim3(kKmapBlock), 0, stream, d_ordered_nbr,
+                                   (const int32_t*)position, m, n_rows, m ? 0 : masked, half, d_nbr, block_counts, nb));
+    RMN_LAUNCH_CHECK();
+    if (!m) break;
+  }
   RMN_CUDA_TRY(launch_overlapped(k_kmap_scan, dim3(half + 1), dim3(1024), 0, stream, block_counts, nb, K, half, totals, d_offset_ptr,
                                  host_alias));
   RMN_LAUNCH_CHECK();

@@ -623,8 +623,8 @@ std::shared_ptr<KernelMap> CoordinateManager::find_or_build(const CoordinateMapK
     auto nbr = static_cast<int32_t*>(ptr(result->nbr_out));
     auto offset_ptr = static_cast<int64_t*>(ptr(result->offset_ptr)), host_ptr = result->host_offset_ptr.data_ptr<int64_t>();
     if (ordered)
-      // A layer has the same map in another order. us so / by a build of its own: 4.8 M clip rows x 81 offsets 1750 / 2330,
-      // 2.1 M voxels of rooms x 27 271 / 332, 2.2 M of lidar sweeps x 27 117 / 336.
+      // A layer has the same map in another order. us so / by a build of its own: 4.8 M clip rows x 81 offsets 1363 / 2348,
+      // 2.1 M voxels of rooms x 27 214 / 334, 2.2 M of lidar sweeps x 27 153 / 334.
       check(rmn_kmap_build_from_ordered(static_cast<const int32_t*>(ptr(ordered->order)),
                                         static_cast<const int32_t*>(ptr(ordered->nbr_out)), out_map.size, K, nbr, offset_ptr,
                                         host_ptr, ptr(result->workspace), ws_bytes, current_stream()),
