@@ -680,7 +680,10 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
   }
   // ------------------------------ marked rows ------------------------------------------
   if (failed || !s_marked || (warp >= kF3MmaWarp && warp < kF3DrainWarp0)) return;
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kF3ExactRegs));
+  __builtin_assume(warp < kF3Warps);
+  if (warp < kF3Warps) {  // (all that are left: whole warpgroups)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kF3ExactRegs));
+  }
   const uint32_t worker = warp < kF3MmaWarp ? warp : warp - (kF3DrainWarp0 - kF3MmaWarp);
   const uint32_t mine = (a.n_super - blockIdx.x + gridDim.x - 1) / gridDim.x * (32 * T);  // groups of four rows
   for (uint32_t i = worker; i < mine; i += 16) {
