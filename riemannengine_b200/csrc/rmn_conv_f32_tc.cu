@@ -27,10 +27,11 @@
 // super-tile (T = 2), or every other stage of a single one (T = 1). Waits are bounded, results bit-reproducible.
 //
 // What bounds it is the gather warps' chain of fetching, splitting (eleven instructions per two numbers) and storing a stage,
-// some 600 cycles, against 12 MMAs of 16 to 32 cycles. us with the weight image / k_conv_f32: 101 930 rows at 66 %, 32 -> 32
-// 59 / 164, 64 -> 64 124 / 519; 48 503 rows at 45 %, 32 -> 64 41 / 117, 64 -> 32 59 / 140; 119 755 lidar voxels, 32 -> 32 53 / 51,
-// 64 -> 64 118 / 110 (k_conv_f32 goes with the rows that exist; blocks of 32 rows none of which exists are not split here: 66
-// and 140 without).
+// some 600 cycles, against 12 MMAs of 16 to 32 cycles: 56 % of the issue slots and 22 % of the tensor pipe are busy at 32 -> 32, 61
+// and 46 % at 64 -> 64. us with the weight image, back to back / k_conv_f32: 101 930 rows at 66 %, 32 -> 32 64 / 166, 64 -> 64
+// 133 / 523; 48 503 rows at 45 %, 32 -> 64 44 / 116, 64 -> 32 62 / 141; 119 755 lidar voxels at 4 %, 32 -> 32 57 / 52, 64 -> 64
+// 127 / 112 (k_conv_f32 goes with the rows that exist: see f3_asks_for_thin_tables. Blocks of 32 rows none of which exists are not
+// split here, which took 13 and 22 us off).
 #include "rmn_common.cuh"
 #include "rmn_tc.cuh"
 
@@ -759,7 +760,8 @@ extern "C" size_t rmn_conv_f32_scratch_bytes(uint32_t n_dst, int K, int c_in, in
 // waits for nothing else pays for, and few rows leave most SMs idle while every row tile walks all offsets in turn. Passes of
 // one layer, us there / here, forward alone and with its gradients, by the rows x offsets x channels in x out of the layer, in
 // millions: 221 (8000 rows 32 -> 32) 69 / 66 and 168 / 173; 442 (32 -> 64) 75 / 67 and 168 / 172; 553 (20 000 rows 32 -> 32)
-// 91 / 72 and 175 / 172; 663 (8000 rows 64 -> 48) 94 / 75 and 181 / 169; 90 (strided, 11 000 rows, 8 offsets) 94 / 99.
+// 91 / 72 and 175 / 172; 663 (8000 rows 64 -> 48) 94 / 75 and 181 / 169; 90 (strided, 11 000 rows, 8 offsets) 94 / 99. (Device
+// time alone, back to back: 221 16.1 / 15.7, 442 23 / 18, 553 39 / 25, 664 41 / 28.)
 extern "C" int rmn_conv_f32_pays(uint32_t n_dst, int K, int c_in, int c_out) {
   return rmn_conv_f32_scratch_bytes(n_dst, K, c_in, c_out) > 0 && (double)n_dst * K * c_in * c_out >= 500e6;
 }

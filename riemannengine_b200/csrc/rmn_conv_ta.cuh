@@ -7,9 +7,9 @@
 // zero row of a missing neighbour (54 % of a room's table) one, and the MMAs read every row back through the same pipe.
 // Here a row goes from global memory to registers (two wavefronts: two lanes fetch 64 bytes at a time with 32-byte
 // loads) and from there to tensor memory (tcgen05.st), where tcgen05.mma takes its A operand: a missing row is read from
-// nowhere. It is not free: its stage is stored and multiplied all the same. 1.2 M x 27 entries, 64 -> 64: 239 us with no entry
-// present, 283 at 46 %, 400 with all; the load/store pipe is 83 % busy at 46 %, half of it with the rows that exist, the tensor
-// pipe 45 %. The order in which the registers of a row reach tensor memory is a permutation
+// nowhere. It is not free: its stage is stored and multiplied all the same. 1.2 M x 27 entries, 64 -> 64: 215 us with no entry
+// present, 270 at 46 %, 371 with all; the load/store pipe is 79 % busy at 46 %, half of it with the rows that exist, the tensor
+// pipe 48 %. The order in which the registers of a row reach tensor memory is a permutation
 // of its channels, which the weight image repeats along K; its columns are permuted so that the epilogue's
 // tcgen05.ld gives every lane 32 contiguous bytes of an output row; and W[k] arrives by one bulk copy per stage.
 //

@@ -956,9 +956,9 @@ extern "C" int rmn_table_build_static(const int32_t* d_coords, uint32_t n_rows, 
   void* scratch = nullptr;
   const int rc = static_scratch_address(&scratch);
   if (rc != RMN_OK) return rc;
-  // Nothing in the scratch has to start at zero: the insert pass writes the slot of every row
-  // and the count pass writes every block counter before anything reads them, so whatever an
-  // earlier call left behind is overwritten.
+  // Nothing in the scratch has to start at zero: the build's first pass clears the bits and counts of
+  // repeated rows and the insert pass writes the slot of every row before anything reads them, so
+  // whatever an earlier call left behind is overwritten.
   return rmn_table_build(d_coords, n_rows, W, d_table, table_bytes, d_mapping, d_inverse,
                          d_unique_coords, scratch, kStaticScratchBytes, stream_);
 }
