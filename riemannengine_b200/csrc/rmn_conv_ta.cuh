@@ -17,7 +17,9 @@
 // serves tile g % T), 2 MMA, 1 weights, 1 idle, 4 epilogue. A (tile, offset) stage costs the warp that issues its MMAs some 150
 // cycles of barrier, fence and commit latency beside 128 of math at 64 columns, and one such warp is what bound tables of few
 // entries. So two issue, each for half of the tiles; where a super-tile is a single tile of up to 64 columns, one takes its even
-// stages and one its odd ones, into accumulators of their own that the epilogue adds (SPLIT). Rows are fetched past the L1: a
+// stages and one its odd ones, into accumulators of their own that the epilogue adds (SPLIT; sums half as
+// long, truncated half as often: of 230 400 results at 900 rows 256 -> 256 222 are not the bf16 number nearest to the 64-bit sum,
+// with one accumulator 404; of 576 000 at 9000 rows 64 -> 64 168 and 261). Rows are fetched past the L1: a
 // hit there passes the load/store pipe in twice the wavefronts of a miss. us before and after both: 1.2 M rows of rooms 64 -> 64
 // 281 and 271, sorted by blocks 300 and 274, 32 -> 32 154 and 149; 240 000 lidar voxels 64 -> 64 57 and 51; 850 rows 256 -> 256
 // 21.5 and 19.6. Waits are bounded (g_tc_status), results are bit-reproducible: every accumulator adds its offsets in ascending
