@@ -5,11 +5,14 @@
 // ones before it leave. Of the nine products of the parts of two numbers the six with i + j <= 2 are multiplied, the smallest
 // first; the others lie below 2^-24 of the product. Tensor memory adds with truncation, so no sum stays there for long: after
 // every stage (32 channels of an offset) it is read back and added, rounded to nearest, to sums in registers. These are added up in
-// groups of stages, whose sums lie in shared memory, so that no long chain rounds at the size of the result (sum_outward: the
-// rounding that takes out the bias of the truncation). Error against 64 bits (2-norm) here / by k_conv_f32, whose sums of an offset
-// are chains of multiply-adds: 30 000 random rows at 66 %, 32 -> 32, numbers of either sign 0.71e-7 / 1.22e-7, positive ones
-// 0.41e-7 / 0.54e-7, 64 -> 64 0.86e-7 / 1.59e-7 and 0.46e-7 / 0.58e-7 (without groups 1.26e-7 and 1.06e-7, and some 4 % faster);
-// 343 offsets 1.16e-7 / 1.46e-7 and 0.58e-7 / 0.55e-7. (Read back every other stage, it is 2.7e-7.)
+// groups of stages, whose sums lie in shared memory, so that no long chain rounds at the size of the result: what the addition of a
+// group leaves out begins the next group's sum (sum_and_rest), and two of the additions are rounded so that they take out the bias of
+// the truncation (sum_outward). Error against 64 bits (2-norm) here / by k_conv_f32, whose sums of an offset are chains of
+// multiply-adds: 30 000 random rows at 66 %, 32 -> 32, numbers of either sign 0.71e-7 / 1.22e-7, positive ones 0.41e-7 / 0.54e-7,
+// 64 -> 64 0.86e-7 / 1.59e-7 and 0.46e-7 / 0.58e-7 (without groups 1.26e-7 and 1.06e-7, and some 4 % faster);
+// 343 offsets, 32 -> 32 1.13e-7 / 1.54e-7 and 0.48e-7 / 0.58e-7, 64 -> 64 1.16e-7 / 1.84e-7 and 0.46e-7 / 0.58e-7 (without what is
+// left out 1.55e-7 and 0.69e-7 there).
+// (Read back every other stage, it is 2.7e-7.)
 //
 // Sums that are not finite are computed again with fp32 multiply-adds: infinities and NaN do not survive the split (inf - inf),
 // nor do numbers that round to infinity in bf16. Numbers below 2^-102 lose their last parts, which fall below the normal numbers of
@@ -259,11 +262,19 @@ __device__ __forceinline__ float f3_finish(float v, float scale, float shift, in
   return relu ? relu_f32(v) : v;
 }
 
-// a + b, rounded away from zero. Truncation costs a stage 4 to 5e-8 of its sum on average, so the whole sum as much; the last two
-// sums of groups, rounded like this, give most of it back. Sums that are exact stay so.
+// a + b, rounded away from zero. Truncation costs a stage some 6e-8 of its sum on average, so the whole sum as much; two of the sums
+// of groups, at about half of the whole and at its end, rounded like this give most of it back (a later one than at half gave back up
+// to 4e-8 too much). Sums that are exact stay so.
 __device__ __forceinline__ float sum_outward(float a, float b) {
   const float up = __fadd_ru(a, b), down = __fadd_rd(a, b);
   return up >= 0.f ? up : down;
+}
+
+// a becomes a + b, and b what its rounding has left out (Knuth's TwoSum), with which the next group begins
+__device__ __forceinline__ void sum_and_rest(float& a, float& b) {
+  const float s = __fadd_rn(a, b), part = __fsub_rn(s, a);
+  b = __fadd_rn(__fsub_rn(a, __fsub_rn(s, part)), __fsub_rn(b, part));
+  a = s;
 }
 
 // Rows row0 .. row0 + 3 (columns col0 .. col0 + CC - 1) by fp32 multiply-adds, by a whole warp: a lane per column of every 32
@@ -613,25 +624,38 @@ __global__ void __launch_bounds__(kF3Threads, 1) k_conv_f3(const __grid_constant
             if (lane == 0) mbar_arrive(&acc_empty[acc]);
           }
         }
-        auto add_total = [&](auto add) {
+        // Outward: the last two sums of two or three groups; of more, the first that holds half of the stages and the last.
+        const bool outward = d == longest || (2 * d >= longest && 2 * (d - a.group) < longest);
+        if (grouped && outward) {
 #pragma unroll
           for (int q = 0; q < C::TOTAL_VECS; ++q) {
             float(&f)[4] = sum[q / (CC / 8)][q % (CC / 8)];
             const float4 before = total[256 * q];
-            f[0] = add(before.x, f[0]);
-            f[1] = add(before.y, f[1]);
-            f[2] = add(before.z, f[2]);
-            f[3] = add(before.w, f[3]);
+            f[0] = sum_outward(before.x, f[0]);
+            f[1] = sum_outward(before.y, f[1]);
+            f[2] = sum_outward(before.z, f[2]);
+            f[3] = sum_outward(before.w, f[3]);
           }
-        };
-        if (grouped && d + a.group >= longest) add_total([](float x, float y) { return sum_outward(x, y); });  // the last two
-        else if (grouped) add_total([](float x, float y) { return x + y; });
+        }
         if (timed_out || d == longest) break;
+        if (grouped && !outward) {
 #pragma unroll
-        for (int q = 0; q < C::TOTAL_VECS; ++q) {
-          float(&f)[4] = sum[q / (CC / 8)][q % (CC / 8)];
-          total[256 * q] = make_float4(f[0], f[1], f[2], f[3]);
-          f[0] = f[1] = f[2] = f[3] = 0.f;
+          for (int q = 0; q < C::TOTAL_VECS; ++q) {
+            float(&f)[4] = sum[q / (CC / 8)][q % (CC / 8)];
+            float4 all = total[256 * q];
+            sum_and_rest(all.x, f[0]);
+            sum_and_rest(all.y, f[1]);
+            sum_and_rest(all.z, f[2]);
+            sum_and_rest(all.w, f[3]);
+            total[256 * q] = all;
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < C::TOTAL_VECS; ++q) {
+            float(&f)[4] = sum[q / (CC / 8)][q % (CC / 8)];
+            total[256 * q] = make_float4(f[0], f[1], f[2], f[3]);
+            f[0] = f[1] = f[2] = f[3] = 0.f;
+          }
         }
       }
       if (timed_out) break;
@@ -699,9 +723,10 @@ int launch_f3(F3Args a, uint32_t blocks, uint32_t fit, cudaStream_t stream) {
   static SmemOptIn opt_in;
   RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_conv_f3<CC, T>), C::SMEM));
   a.n_super = (a.n_dst + kTileM * T - 1) / (kTileM * T);
-  // Stages of a group: n stages in g groups leave a rounding error that goes with sqrt(g + n / g^2), least at g = cbrt(2 n) and
-  // hardly larger at cbrt(n).
-  const int stages = a.K * a.n_kb, groups = (int)(std::cbrt((double)stages) + 1e-6), steps = T > 1 ? stages : (stages + 1) / 2;
+  // Stages of a group: n stages in g groups leave a rounding error within them that goes with sqrt(n) / g, and some of the last sum.
+  // Adding up a group costs the drain what a stage or two do, so few of them where they are short.
+  const int stages = a.K * a.n_kb, steps = T > 1 ? stages : (stages + 1) / 2;
+  const int cube_root = (int)(std::cbrt((double)stages) + 1e-6), groups = cube_root > (stages + 47) / 48 ? cube_root : (stages + 47) / 48;
   a.group = (steps + groups - 1) / groups;
   RMN_CUDA_TRY(launch_overlapped(k_conv_f3<CC, T>, dim3(fit < a.n_super ? fit : a.n_super, blocks), dim3(kF3Threads), C::SMEM,
                                  stream, a));

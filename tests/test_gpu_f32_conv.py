@@ -313,3 +313,40 @@ def test_large_passes_over_thin_tables_are_the_multiply_add_kernels(n, c_in, c_o
     # two sums of up to K c_in products, each within 2^-24 of the magnitudes a term (the grouped sum far less)
     assert float((out - plain).abs().max()) <= 2.0 ** -18 * max(1.0, float(plain.abs().max()))
     assert bool((scratch[size:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("n,c_in,c_out,K,fill", [(20_000, 32, 32, 64, 0.66), (20_000, 32, 32, 125, 0.5), (8000, 64, 64, 125, 0.5),
+                                                 (12_000, 32, 32, 343, 0.66), (4000, 64, 64, 343, 0.66), (6000, 32, 32, 729, 0.66),
+                                                 (4000, 256, 64, 125, 0.5), (20_000, 256, 32, 125, 0.5)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "near one", "integers"])
+def test_f32_sums_of_many_stages_are_as_close_to_float64_as_multiply_adds(n, c_in, c_out, K, fill, kind):
+    """Kernels of five and more along an axis: hundreds of partial sums, whose roundings must not add up. Tables above the line of
+    one neighbour in sixteen: the tensor cores' kernel, with single row tiles and with two."""
+    from riemannengine_b200 import capi, ops
+    lib = capi.lib()
+    g = torch.Generator(device="cuda").manual_seed(n + c_in + K)
+    nbr = torch.randint(0, n, (K, n), generator=g, dtype=torch.int32, device="cuda")
+    nbr[torch.rand((K, n), generator=g, device="cuda") >= fill] = -1
+    x = torch.randn((n, c_in), generator=g, device="cuda")
+    w = torch.randn((K, c_in, c_out), generator=g, device="cuda")
+    if kind == "positive":
+        x, w = x.abs(), w.abs()
+    elif kind == "near one":
+        x, w = 1 + 0.1 * x.abs(), 1 + 0.1 * w.abs()
+    elif kind == "integers":
+        x, w = x.round(), w.round()
+    want = torch.zeros((n, c_out), dtype=torch.float64, device="cuda")
+    for k in range(K):
+        hit = nbr[k] >= 0
+        want[hit] += x[nbr[k][hit].long()].double() @ w[k].double()
+    size = lib.rmn_conv_f32_scratch_bytes(n, K, c_in, c_out)
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    out, plain = torch.empty((n, c_out), device="cuda"), torch.empty((n, c_out), device="cuda")
+    capi.check(lib.rmn_conv_forward_f32(ops._ptr(x), n, c_in, ops._ptr(w), K, c_out, 0, 0, ops._ptr(nbr), n, ops._ptr(out), None,
+                                        None, 0, ops._ptr(scratch), size, ops._stream()), "rmn_conv_forward_f32")
+    capi.check(lib.rmn_conv_forward(ops._ptr(x), n, c_in, ops._ptr(w), K, c_out, ops._ptr(nbr), n, ops._ptr(plain), capi.F32,
+                                    ops._stream()), "rmn_conv_forward")
+    if kind == "integers":
+        assert torch.equal(out.double(), want)
+    else:
+        assert float((out.double() - want).norm()) <= float((plain.double() - want).norm())
