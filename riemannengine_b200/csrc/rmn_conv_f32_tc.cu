@@ -724,9 +724,13 @@ int launch_f3(F3Args a, uint32_t blocks, uint32_t fit, cudaStream_t stream) {
   RMN_CUDA_TRY(opt_in.apply(reinterpret_cast<const void*>(&k_conv_f3<CC, T>), C::SMEM));
   a.n_super = (a.n_dst + kTileM * T - 1) / (kTileM * T);
   // Stages of a group: n stages in g groups leave a rounding error within them that goes with sqrt(n) / g, and some of the last sum.
-  // Adding up a group costs the drain what a stage or two do, so few of them where they are short.
+  // Adding up a group costs the drain what a stage or two do, so few of them where they are short; but two from four stages on, for
+  // the rounding that takes out the bias (7 offsets, 32 -> 64, positive numbers 0.66e-7 with one, 0.48e-7 with two, 0.57e-7
+  // by multiply-adds).
   const int stages = a.K * a.n_kb, steps = T > 1 ? stages : (stages + 1) / 2;
-  const int cube_root = (int)(std::cbrt((double)stages) + 1e-6), groups = cube_root > (stages + 47) / 48 ? cube_root : (stages + 47) / 48;
+  int groups = (int)(std::cbrt((double)stages) + 1e-6);
+  if (groups < 2 && stages >= 4) groups = 2;
+  if (groups < (stages + 47) / 48) groups = (stages + 47) / 48;
   a.group = (steps + groups - 1) / groups;
   RMN_CUDA_TRY(launch_overlapped(k_conv_f3<CC, T>, dim3(fit < a.n_super ? fit : a.n_super, blocks), dim3(kF3Threads), C::SMEM,
                                  stream, a));

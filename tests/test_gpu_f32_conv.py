@@ -350,3 +350,12 @@ def test_f32_sums_of_many_stages_are_as_close_to_float64_as_multiply_adds(n, c_i
         assert torch.equal(out.double(), want)
     else:
         assert float((out.double() - want).norm()) <= float((plain.double() - want).norm())
+
+
+@pytest.mark.parametrize("n,c_in,c_out,K,fill", [(30_000, 32, 64, 4, 0.55), (30_000, 32, 64, 7, 0.55), (30_000, 64, 64, 2, 0.55),
+                                                 (30_000, 64, 64, 3, 0.6), (30_000, 16, 64, 7, 0.55), (30_000, 24, 32, 5, 1.0),
+                                                 (12_000, 32, 64, 7, 0.55), (30_000, 32, 64, 3, 0.6)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "near one", "integers"])
+def test_f32_sums_of_few_stages_are_as_close_to_float64_as_multiply_adds(n, c_in, c_out, K, fill, kind):
+    """Kernels of a few offsets (a cross of seven), whose sums are one group or two; single row tiles and two."""
+    test_f32_sums_of_many_stages_are_as_close_to_float64_as_multiply_adds(n, c_in, c_out, K, fill, kind)
